@@ -259,6 +259,61 @@ LKC_API int lkc_plan_memory(int64_t n, int64_t num_streams, const int64_t* bytes
                             const int64_t* alloc_clock, const int64_t* last_use, int64_t align, int64_t* offsets,
                             int64_t* total);
 
+/* ---- whole-model calls (host code; everything they queue is one of the kernels above) ---------------------------
+ * No counterpart in the reference, whose runtime walks a compiled program; here one call queues what Generator.forward
+ * composes from the entry points above (models/kokoro/model.py:735-781), resp. one AdaINResBlock1 (:235-247). The caller
+ * owns all memory: weights and packs (device pointers) live as long as the handle, the workspace until the work queued by
+ * the call has finished; every intermediate lives in the workspace, overlaid by lkc_plan_memory. */
+typedef struct LkcResblock {
+  int64_t c, k;
+  /* index 2 j + (n - 1): convs{n}.{j} / alpha{n}.{j} / adain{n}.{j}; gb = offset (floats) of that AdaIN's (gamma | beta) in
+   * the style bank; state may be NULL (CUDA-core kernel) */
+  const void *w[6], *b[6], *alpha[6];
+  const LkcConvState* state[6];
+  int64_t gb[6];
+} LkcResblock;
+typedef struct LkcNoiseConv { /* polyphase form of noise_convs.{i}: weights [C, rows, taps], see space_to_depth */
+  const void *w, *b;
+  const LkcConvState* state;
+  int64_t stride, padding, taps, rows;
+} LkcNoiseConv;
+typedef struct LkcGenerator {
+  const void *bank_wt, *bank_b; /* style bank: f32[128, bank_n], f32[bank_n] */
+  int64_t bank_n;
+  LkcNoiseConv noise_conv[2];
+  LkcResblock noise_res[2], res[6];
+  const void* ups_b[2];
+  const LkcConvState* ups_state[2]; /* lkc_convt_state_create */
+  const void *post_w, *post_b, *ident128; /* ident128: identity affine f32[3, 128] */
+  const LkcConvState* post_state;
+} LkcGenerator;
+typedef struct LkcGeneratorIo {
+  const void *x, *har, *s; /* f32[512, t], f32[22, 60 t + 1], f32[128] */
+  void *audio, *post;      /* f32[300 t]; f32[22, 60 t + 1] or NULL */
+  int64_t t, x_pitch, har_pitch, post_pitch;
+  void* workspace;
+  int64_t workspace_bytes;
+  void* side[4];    /* streams for the independent branches (concurrent != 0); joined back before the call's last kernel */
+  int64_t concurrent;
+  int64_t launches; /* out: kernels queued */
+} LkcGeneratorIo;
+typedef struct LkcResblockIo {
+  const void *x, *stats, *bank; /* f32[C, l]; chunk statistics of x or NULL; style bank */
+  void *out, *out_stats;        /* f32[C, l], f32[C, ceil(l / 128), 2] */
+  int64_t l, x_pitch, out_pitch;
+  void* workspace; /* NULL: only workspace_bytes is set, nothing is queued */
+  int64_t workspace_bytes;
+  int64_t launches; /* out */
+} LkcResblockIo;
+typedef struct LkcModel LkcModel;
+/* The handle copies the struct and keeps the events of the stream joins and the memory plans of the last lengths. Calls on
+ * one handle may come from several threads. */
+LKC_API LkcModel* lkc_generator_create(const LkcGenerator* w);
+LKC_API void lkc_model_destroy(LkcModel* m);
+LKC_API int lkc_generator_workspace(LkcModel* m, int64_t t, int concurrent, int64_t* bytes, int64_t* unplanned);
+LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, void* stream);
+LKC_API int lkc_resblock(const LkcResblock* w, LkcResblockIo* io, void* stream);
+
 /* ---- device-side test harness (the data path of the reference's RUN2 message, include/lokinfer/remote/server.h:30-47)
  * lkc_generate_cuda fills a tensor from a seed with the reference's generator (src/remote/server.cpp:739-782;
  * python/lokinfer/remote.py:96-119): splitmix64 of seed + (2 i + 1) golden and seed + (2 i + 2) golden, u = (mix >> 11)

@@ -21,6 +21,41 @@ class LkcArgs(ctypes.Structure):
     ]
 
 
+class LkcResblock(ctypes.Structure):
+    """struct LkcResblock of include/lkc.h."""
+    _fields_ = [("c", ctypes.c_int64), ("k", ctypes.c_int64), ("w", ctypes.c_void_p * 6), ("b", ctypes.c_void_p * 6),
+                ("alpha", ctypes.c_void_p * 6), ("state", ctypes.c_void_p * 6), ("gb", ctypes.c_int64 * 6)]
+
+
+class LkcNoiseConv(ctypes.Structure):
+    _fields_ = [("w", ctypes.c_void_p), ("b", ctypes.c_void_p), ("state", ctypes.c_void_p),
+                ("stride", ctypes.c_int64), ("padding", ctypes.c_int64), ("taps", ctypes.c_int64),
+                ("rows", ctypes.c_int64)]
+
+
+class LkcGenerator(ctypes.Structure):
+    _fields_ = [("bank_wt", ctypes.c_void_p), ("bank_b", ctypes.c_void_p), ("bank_n", ctypes.c_int64),
+                ("noise_conv", LkcNoiseConv * 2), ("noise_res", LkcResblock * 2), ("res", LkcResblock * 6),
+                ("ups_b", ctypes.c_void_p * 2), ("ups_state", ctypes.c_void_p * 2),
+                ("post_w", ctypes.c_void_p), ("post_b", ctypes.c_void_p), ("ident128", ctypes.c_void_p),
+                ("post_state", ctypes.c_void_p)]
+
+
+class LkcGeneratorIo(ctypes.Structure):
+    _fields_ = [("x", ctypes.c_void_p), ("har", ctypes.c_void_p), ("s", ctypes.c_void_p), ("audio", ctypes.c_void_p),
+                ("post", ctypes.c_void_p), ("t", ctypes.c_int64), ("x_pitch", ctypes.c_int64),
+                ("har_pitch", ctypes.c_int64), ("post_pitch", ctypes.c_int64), ("workspace", ctypes.c_void_p),
+                ("workspace_bytes", ctypes.c_int64), ("side", ctypes.c_void_p * 4), ("concurrent", ctypes.c_int64),
+                ("launches", ctypes.c_int64)]
+
+
+class LkcResblockIo(ctypes.Structure):
+    _fields_ = [("x", ctypes.c_void_p), ("stats", ctypes.c_void_p), ("bank", ctypes.c_void_p), ("out", ctypes.c_void_p),
+                ("out_stats", ctypes.c_void_p), ("l", ctypes.c_int64), ("x_pitch", ctypes.c_int64),
+                ("out_pitch", ctypes.c_int64), ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_int64),
+                ("launches", ctypes.c_int64)]
+
+
 RUN_FN = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.POINTER(LkcArgs), ctypes.c_void_p)
 
 _lib = None
@@ -67,6 +102,17 @@ def lib():
         l.lkc_set_conv_io.argtypes = [ctypes.c_int]
         l.lkc_set_conv_path.restype = ctypes.c_int
         l.lkc_set_conv_path.argtypes = [ctypes.c_int]
+        l.lkc_generator_create.restype = ctypes.c_void_p
+        l.lkc_generator_create.argtypes = [ctypes.POINTER(LkcGenerator)]
+        l.lkc_model_destroy.restype = None
+        l.lkc_model_destroy.argtypes = [ctypes.c_void_p]
+        l.lkc_generator_workspace.restype = ctypes.c_int
+        l.lkc_generator_workspace.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_int,
+                                              ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]
+        l.lkc_generator_forward.restype = ctypes.c_int
+        l.lkc_generator_forward.argtypes = [ctypes.c_void_p, ctypes.POINTER(LkcGeneratorIo), ctypes.c_void_p]
+        l.lkc_resblock.restype = ctypes.c_int
+        l.lkc_resblock.argtypes = [ctypes.POINTER(LkcResblock), ctypes.POINTER(LkcResblockIo), ctypes.c_void_p]
         _lib = l
     return _lib
 

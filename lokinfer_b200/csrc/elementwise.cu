@@ -226,6 +226,40 @@ __global__ void gemmBiasKernel(const float* __restrict__ x, const float* __restr
   out[row * n + col] = acc + b[col];
 }
 
+}  // namespace
+
+// ---- launchers shared by the C-ABI entry points below and the whole-model calls (model.cu)
+
+int channelStats(const float* x, float* stats, int64_t c, int64_t l, int64_t pitch, int64_t statsStride, cudaStream_t s) {
+  const int64_t nchunks = statChunks(l);
+  dim3 grid(static_cast<unsigned>(ceilDiv(nchunks, kThreads / 32)), static_cast<unsigned>(c));
+  channelStatsKernel<<<grid, kThreads, 0, s>>>(x, stats, l, nchunks, pitch, statsStride);
+  return launched("channel_stats_f32_cuda");
+}
+
+int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s) {
+  adainAffineKernel<<<static_cast<unsigned>(c), kAffineThreads, 0, s>>>(stats, gb, affine, c, l, statChunks(l), eps);
+  return launched("adain_affine_f32_cuda");
+}
+
+int gemmBias(const float* x, const float* wt, const float* b, float* out, int64_t m, int64_t k, int64_t n, cudaStream_t s) {
+  dim3 grid(static_cast<unsigned>(ceilDiv(n, kThreads)), static_cast<unsigned>(m));
+  gemmBiasKernel<<<grid, kThreads, static_cast<size_t>(k) * 4, s>>>(x, wt, b, out, m, k, n);
+  return launched("gemm_bias_f32_cuda");
+}
+
+int addRows(const float* a, const float* b, float* out, int64_t n, cudaStream_t s) {
+  addKernel<<<gridFor(n), kThreads, 0, s>>>(a, b, out, n);
+  return launched("add_f32_cuda");
+}
+
+int add3Scale(const float* a, const float* b, const float* c, float* out, int64_t n, float scale, cudaStream_t s) {
+  add3ScaleKernel<<<gridFor(n), kThreads, 0, s>>>(a, b, c, out, n, scale);
+  return launched("add3_scale_f32_cuda");
+}
+
+namespace {
+
 int64_t numel(const int64_t* dims, int rank) {
   int64_t n = 1;
   for (int i = 0; i < rank; ++i) n *= dims[i];
@@ -261,17 +295,14 @@ extern "C" LKC_API int lkc_add_f32_cuda(const LkcArgs* a, void* stream) {
   LKC_REQUIRE(a && a->numPtrs == 3, "add_f32_cuda: expected a, b | out");
   const int64_t n = numel(a->ints, rankOf(a, 2));
   if (n == 0) return 0;
-  addKernel<<<gridFor(n), kThreads, 0, S(stream)>>>(F(a, 0), F(a, 1), O(a, 2), n);
-  return launched("add_f32_cuda");
+  return addRows(F(a, 0), F(a, 1), O(a, 2), n, S(stream));
 }
 
 extern "C" LKC_API int lkc_add3_scale_f32_cuda(const LkcArgs* a, void* stream) {
   LKC_REQUIRE(a && a->numPtrs == 4 && a->floats, "add3_scale_f32_cuda: expected a, b, c | out and scale");
   const int64_t n = numel(a->ints, rankOf(a, 3));
   if (n == 0) return 0;
-  add3ScaleKernel<<<gridFor(n), kThreads, 0, S(stream)>>>(F(a, 0), F(a, 1), F(a, 2), O(a, 3), n,
-                                                          static_cast<float>(a->floats[0]));
-  return launched("add3_scale_f32_cuda");
+  return add3Scale(F(a, 0), F(a, 1), F(a, 2), O(a, 3), n, static_cast<float>(a->floats[0]), S(stream));
 }
 
 extern "C" LKC_API int lkc_scale_f32_cuda(const LkcArgs* a, void* stream) {
@@ -309,6 +340,14 @@ __global__ void spaceToDepthKernel(const float* __restrict__ x, float* __restric
   }
 }
 
+namespace lkc {
+int spaceToDepth(const float* x, float* y, int64_t ci, int64_t l, int64_t rows, int64_t ly, int64_t xPitch, int64_t yPitch,
+                 int64_t stride, int64_t pad, cudaStream_t s) {
+  spaceToDepthKernel<<<gridFor(rows * ly, 4), kThreads, 0, s>>>(x, y, ci, l, rows, ly, xPitch, yPitch, int(stride), pad);
+  return launched("space_to_depth_f32_cuda");
+}
+}  // namespace lkc
+
 // ints: x(Ci, L) y(rows, Ly) pad stride [x_pitch y_pitch]
 extern "C" LKC_API int lkc_space_to_depth_f32_cuda(const LkcArgs* a, void* stream) {
   LKC_REQUIRE(a && a->numPtrs == 2 && (a->numInts == 6 || a->numInts == 8), "space_to_depth_f32_cuda: expected x | y, pad, stride");
@@ -317,9 +356,7 @@ extern "C" LKC_API int lkc_space_to_depth_f32_cuda(const LkcArgs* a, void* strea
   LKC_REQUIRE(s >= 1 && s <= 64 && pad >= 0 && ci >= 1 && l >= 1, "space_to_depth_f32_cuda: invalid stride / padding");
   LKC_REQUIRE(rows >= ci * s && ly >= 1 && yPitch >= ly && xPitch >= l,
               "space_to_depth_f32_cuda: y must be f32[rows >= Ci * stride, Ly]");
-  spaceToDepthKernel<<<gridFor(rows * ly, 4), kThreads, 0, S(stream)>>>(F(a, 0), O(a, 1), ci, l, rows, ly, xPitch, yPitch,
-                                                                        int(s), pad);
-  return launched("space_to_depth_f32_cuda");
+  return spaceToDepth(F(a, 0), O(a, 1), ci, l, rows, ly, xPitch, yPitch, s, pad, S(stream));
 }
 
 extern "C" LKC_API int lkc_adain1d_f32_cuda(const LkcArgs* a, void* stream) {
@@ -344,9 +381,7 @@ extern "C" LKC_API int lkc_channel_stats_f32_cuda(const LkcArgs* a, void* stream
               "channel_stats_f32_cuda: stats must be f32[C, ceil(L/128), 2]");
   LKC_REQUIRE(c <= 65535, "channel_stats_f32_cuda: too many channels");
   if (c == 0) return 0;
-  dim3 grid(static_cast<unsigned>(ceilDiv(nchunks, kThreads / 32)), static_cast<unsigned>(c));
-  channelStatsKernel<<<grid, kThreads, 0, S(stream)>>>(F(a, 0), O(a, 1), l, nchunks, pitch, statsStride);
-  return launched("channel_stats_f32_cuda");
+  return channelStats(F(a, 0), O(a, 1), c, l, pitch, statsStride, S(stream));
 }
 
 extern "C" LKC_API int lkc_adain_affine_f32_cuda(const LkcArgs* a, void* stream) {
@@ -359,9 +394,7 @@ extern "C" LKC_API int lkc_adain_affine_f32_cuda(const LkcArgs* a, void* stream)
   if (c == 0) return 0;
   LKC_REQUIRE(c <= 0x7fffffff, "adain_affine_f32_cuda: too many channels");
   LKC_REQUIRE((reinterpret_cast<uintptr_t>(a->ptrs[0]) & 7) == 0, "adain_affine_f32_cuda: stats must be 8-byte aligned");
-  adainAffineKernel<<<static_cast<unsigned>(c), kAffineThreads, 0, S(stream)>>>(F(a, 0), F(a, 1), O(a, 2), c, l, nchunks,
-                                                                               static_cast<float>(a->floats[0]));
-  return launched("adain_affine_f32_cuda");
+  return adainAffine(F(a, 0), F(a, 1), O(a, 2), c, l, static_cast<float>(a->floats[0]), S(stream));
 }
 
 extern "C" LKC_API int lkc_gemm_bias_f32_cuda(const LkcArgs* a, void* stream) {
@@ -371,8 +404,5 @@ extern "C" LKC_API int lkc_gemm_bias_f32_cuda(const LkcArgs* a, void* stream) {
               "gemm_bias_f32_cuda: shapes must be x[M,K] wt[K,N] b[N] out[M,N]");
   LKC_REQUIRE(k * 4 <= 48 * 1024 && m <= 65535, "gemm_bias_f32_cuda: K or M too large for this kernel");
   if (m * n == 0) return 0;
-  dim3 grid(static_cast<unsigned>(ceilDiv(n, kThreads)), static_cast<unsigned>(m));
-  gemmBiasKernel<<<grid, kThreads, static_cast<size_t>(k) * 4, S(stream)>>>(F(a, 0), F(a, 1), F(a, 2), O(a, 3), m, k,
-                                                                           n);
-  return launched("gemm_bias_f32_cuda");
+  return gemmBias(F(a, 0), F(a, 1), F(a, 2), O(a, 3), m, k, n, S(stream));
 }

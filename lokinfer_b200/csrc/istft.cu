@@ -88,7 +88,32 @@ __global__ void __launch_bounds__(NTHREADS) istftKernel(const IstftArgs a) {
   }
 }
 
+// Checks of the caller done: shared-memory limit, launch.
+int istftLaunch(IstftArgs p, cudaStream_t s) {
+  p.bins = p.nfft / 2 + 1;
+  p.nfMax = FB + (p.nfft + p.hop - 1) / p.hop + 2;
+  const size_t smem = sizeof(float) * (size_t(2) * p.bins * p.nfft + p.nfft + size_t(2) * p.bins * p.nfMax +
+                                       size_t(p.nfft) * p.nfMax);
+  LKC_REQUIRE(smem <= 200 * 1024, "istft_logits_f32_cuda: n_fft / hop too large for one block's shared memory");
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    cudaError_t e = cudaFuncSetAttribute(istftKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e != cudaSuccess) return failCuda("istft_logits_f32_cuda: cudaFuncSetAttribute", e);
+    configured[dev] = true;
+  }
+  const int64_t blocks = ceilDiv(p.len, int64_t(FB) * p.hop);
+  LKC_REQUIRE(blocks <= 0x7fffffff, "istft_logits_f32_cuda: grid too large");
+  istftKernel<<<static_cast<unsigned>(blocks), NTHREADS, smem, s>>>(p);
+  return launched("istft_logits_f32_cuda");
+}
+
 }  // namespace
+
+int istftLogits(const float* x, float* out, int64_t l, int64_t pitch, int nfft, int hop, cudaStream_t s) {
+  return istftLaunch({x, out, l, int64_t(hop) * (l - 1), pitch, 0, 0, nfft, hop, 0, 0}, s);
+}
 }  // namespace lkc
 
 using namespace lkc;
@@ -120,21 +145,6 @@ extern "C" LKC_API int lkc_istft_logits_f32_cuda(const LkcArgs* a, void* stream)
   p.pitch = a->numInts >= 6 ? a->ints[5] : lx;  // optional trailing int: row pitch of x
   p.frame0 = frame0, p.i0 = i0;
   LKC_REQUIRE(p.pitch >= lx, "istft_logits_f32_cuda: the row pitch is smaller than the row");
-  p.nfft = int(nfft), p.hop = int(hop), p.bins = int(nfft / 2 + 1);
-  p.nfMax = int(FB + (nfft + hop - 1) / hop + 2);
-  const size_t smem = sizeof(float) * (size_t(2) * p.bins * p.nfft + p.nfft + size_t(2) * p.bins * p.nfMax +
-                                       size_t(p.nfft) * p.nfMax);
-  LKC_REQUIRE(smem <= 200 * 1024, "istft_logits_f32_cuda: n_fft / hop too large for one block's shared memory");
-  static bool configured[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(istftKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return failCuda("istft_logits_f32_cuda: cudaFuncSetAttribute", e);
-    configured[dev] = true;
-  }
-  const int64_t blocks = ceilDiv(len, int64_t(FB) * hop);
-  LKC_REQUIRE(blocks <= 0x7fffffff, "istft_logits_f32_cuda: grid too large");
-  istftKernel<<<static_cast<unsigned>(blocks), NTHREADS, smem, S(stream)>>>(p);
-  return launched("istft_logits_f32_cuda");
+  p.nfft = int(nfft), p.hop = int(hop);
+  return istftLaunch(p, S(stream));
 }

@@ -103,4 +103,15 @@ int convTcStatusAsync(int* hostOut, cudaStream_t s);
 int convTcSetIo(int mode);
 int convTcProfile(int enable, long long* out16);
 
+// Launchers behind the C-ABI entry points of the same names (elementwise.cu, istft.cu, conv_tc.cu); arguments checked by
+// the caller. Row pitches in floats.
+int channelStats(const float* x, float* stats, int64_t c, int64_t l, int64_t pitch, int64_t statsStride, cudaStream_t s);
+int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s);
+int gemmBias(const float* x, const float* wt, const float* b, float* out, int64_t m, int64_t k, int64_t n, cudaStream_t s);
+int addRows(const float* a, const float* b, float* out, int64_t n, cudaStream_t s);
+int add3Scale(const float* a, const float* b, const float* c, float* out, int64_t n, float scale, cudaStream_t s);
+int spaceToDepth(const float* x, float* y, int64_t ci, int64_t l, int64_t rows, int64_t ly, int64_t xPitch, int64_t yPitch,
+                 int64_t stride, int64_t pad, cudaStream_t s);
+int istftLogits(const float* x, float* out, int64_t l, int64_t pitch, int nfft, int hop, cudaStream_t s);
+
 }  // namespace lkc

@@ -1,0 +1,415 @@
+// Whole-model calls: the generator's forward and one AdaINResBlock1 as ONE call each (host code; every kernel it queues
+// is an entry point of this library). What they replace is the op-by-op composition in generator.py, whose 110 calls
+// through Python (argument checks, argument packing, one allocation per result, stream switches) took 5 ms of host time
+// per forward whatever its length, two to ten times what the GPU needs below 10 s of audio.
+//
+// A forward is written once as a sequence of alloc / use / join / launch steps over an Exec and runs in two modes. In
+// plan mode nothing is launched: every tensor's allocation and uses are recorded with the vector clock of the stream
+// they happen on, and lkc_plan_memory turns that into offsets inside one workspace (the branches run on side streams,
+// so a byte range is reused only where a join orders its uses before the new allocation). In run mode the same
+// sequence takes its tensors from the workspace and queues its kernels. The plan depends on the length alone; the last
+// few are kept with the model (a plan costs about 40 us).
+#include <algorithm>
+#include <list>
+#include <memory>
+#include <mutex>
+#include <new>
+#include <vector>
+
+#include "lkc_common.h"
+
+namespace lkc {
+namespace {
+
+constexpr int kStreams = 5;  // the caller's stream and four side streams
+constexpr int kEvents = 12;  // joins of one forward
+constexpr size_t kPlans = 16;
+constexpr float kEps = 1e-5f;  // AdaIN
+
+struct Plan {
+  int64_t key = 0, bytes = 0, unplanned = 0;
+  std::vector<int64_t> offsets;
+};
+
+// A tensor of the workspace, or (id < 0) one of the caller's.
+struct Buf {
+  float* p = nullptr;
+  int64_t pitch = 0;
+  int id = -1;
+};
+
+class Exec {
+ public:
+  // plan mode
+  explicit Exec(bool concurrent) : concurrent_(concurrent) {}
+  // run mode
+  Exec(bool concurrent, const Plan& plan, char* base, cudaStream_t main, const cudaStream_t* side, cudaEvent_t* events)
+      : concurrent_(concurrent), plan_(&plan), base_(base), events_(events) {
+    streams_[0] = main;
+    for (int i = 1; i < kStreams; ++i) streams_[i] = concurrent ? side[i - 1] : main;
+  }
+
+  bool running() const { return plan_ != nullptr; }
+  cudaStream_t stream(int s) const { return streams_[s]; }
+
+  Buf alloc(int s, int64_t floats, int64_t pitch = 0) {
+    Buf b;
+    b.pitch = pitch, b.id = next_++;
+    if (running()) {
+      b.p = reinterpret_cast<float*>(base_ + plan_->offsets[b.id]);
+      return b;
+    }
+    const int l = lane(s);
+    ++clock_[l][l];
+    bytes_.push_back(floats * 4);
+    for (int i = 0; i < kStreams; ++i) allocClock_.push_back(clock_[l][i]), lastUse_.push_back(0);
+    lastUse_[size_t(b.id) * kStreams + l] = clock_[l][l];
+    return b;
+  }
+  // f32[c, l] with rows on 16-byte boundaries
+  Buf rows(int s, int64_t c, int64_t l) { return alloc(s, c * ((l + 3) & ~int64_t(3)), (l + 3) & ~int64_t(3)); }
+
+  // One kernel on stream s that reads or writes `bufs`; fn() queues it and returns 0 or an error code.
+  template <class Fn>
+  void launch(int s, std::initializer_list<Buf> bufs, Fn fn) {
+    if (running()) {
+      if (rc == 0) rc = fn(streams_[s]);
+      ++launches;
+      return;
+    }
+    const int l = lane(s);
+    const int64_t n = ++clock_[l][l];
+    for (const Buf& b : bufs)
+      if (b.id >= 0) lastUse_[size_t(b.id) * kStreams + l] = n;
+  }
+
+  // Nothing queued on `waiter` from here on starts before everything queued on `waited` so far has finished.
+  void join(int waiter, int waited) {
+    if (!concurrent_) return;
+    if (!running()) {
+      for (int i = 0; i < kStreams; ++i) clock_[waiter][i] = std::max(clock_[waiter][i], clock_[waited][i]);
+      return;
+    }
+    if (rc != 0) return;
+    cudaEvent_t e = events_[event_++ % kEvents];
+    cudaError_t err = cudaEventRecord(e, streams_[waited]);
+    if (err == cudaSuccess) err = cudaStreamWaitEvent(streams_[waiter], e, 0);
+    if (err != cudaSuccess) rc = failCuda("model: stream join", err);
+  }
+
+  int finishPlan(Plan* out) {
+    const int64_t n = int64_t(bytes_.size());
+    out->offsets.assign(size_t(n), 0);
+    const std::vector<int32_t> pinned(size_t(n), 0);
+    for (int64_t b : bytes_) out->unplanned += (b + 255) / 256 * 256;
+    return lkc_plan_memory(n, kStreams, bytes_.data(), pinned.data(), allocClock_.data(), lastUse_.data(), 256,
+                           out->offsets.data(), &out->bytes);
+  }
+
+  int rc = 0;
+  int64_t launches = 0;
+
+ private:
+  int lane(int s) const { return concurrent_ ? s : 0; }
+
+  const bool concurrent_;
+  const Plan* plan_ = nullptr;
+  char* base_ = nullptr;
+  cudaStream_t streams_[kStreams] = {};
+  cudaEvent_t* events_ = nullptr;
+  int next_ = 0, event_ = 0;
+  std::vector<int64_t> bytes_, allocClock_, lastUse_;
+  int64_t clock_[kStreams][kStreams] = {};
+};
+
+const float* FP(const void* p) { return static_cast<const float*>(p); }
+
+// One fused conv of the tensor-core family, stride 1: act((x - mean) * scale + beta) -> conv -> + bias [+ residual].
+void conv(Exec& e, int s, Act act, Buf x, int64_t l, int64_t ci, int64_t co, int64_t k, int64_t d, int64_t pad,
+          const void* w, const void* b, Buf affine, const void* alpha, float slope, const LkcConvState* state, Buf residual,
+          Buf out, Buf stats) {
+  e.launch(s, {x, affine, residual, out, stats}, [&](cudaStream_t st) {
+    ConvFusedParams p;
+    p.x = x.p, p.w = FP(w), p.bias = FP(b), p.affine = affine.p, p.alpha = FP(alpha), p.residual = residual.p;
+    p.out = out.p, p.stats = stats.p;
+    p.ci = ci, p.l = l, p.co = co, p.k = k, p.dilation = d, p.padding = pad, p.lo = l + 2 * pad - d * (k - 1);
+    p.xPitch = x.pitch, p.resPitch = residual.pitch, p.outPitch = out.pitch;
+    p.act = act, p.slope = slope, p.state = state;
+    return convFused(p, st);
+  });
+}
+
+// gb = this AdaIN's (gamma | beta) inside the style bank.
+Buf affineOf(Exec& e, int s, Buf stats, Buf bank, int64_t gb, int64_t c, int64_t l) {
+  Buf af = e.alloc(s, 3 * c);
+  e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, bank.p + gb, af.p, c, l, kEps, st); });
+  return af;
+}
+
+Buf statsBuf(Exec& e, int s, int64_t c, int64_t l) { return e.alloc(s, c * statChunks(l) * 2); }
+
+Buf channelStatsOf(Exec& e, int s, Buf x, int64_t c, int64_t l) {
+  Buf st = statsBuf(e, s, c, l);
+  e.launch(s, {x, st}, [&](cudaStream_t cs) { return channelStats(x.p, st.p, c, l, x.pitch, statChunks(l), cs); });
+  return st;
+}
+
+// What the last conv of a block adds: its running x, or what `make` (called with that x before the block's last
+// iteration) returns; `ready` is called just before the last conv is queued.
+struct PlainResidual {
+  Buf make(Buf x) const { return x; }
+  void ready() const {}
+};
+
+// AdaINResBlock1 (models/kokoro/model.py:235-247): three times {affine, Snake conv (dilation 1, 3, 5), affine, Snake conv
+// + residual}. `out` / `outStats` receive the result: the caller's memory where they come with a pointer, else tensors
+// allocated here.
+template <class Residual>
+void resblock(Exec& e, int s, const LkcResblock& w, Buf x, Buf stats, int64_t l, Buf bank, Buf* out, Buf* outStats,
+              Residual residual) {
+  static const int64_t dil[3] = {1, 3, 5};
+  const int64_t c = w.c, k = w.k;
+  const Buf none;
+  for (int j = 0; j < 3; ++j) {
+    const int64_t d = dil[j];
+    const int i1 = 2 * j, i2 = 2 * j + 1;
+    const bool last = j == 2;
+    const Buf res = last ? residual.make(x) : x;
+    Buf af = affineOf(e, s, stats, bank, w.gb[i1], c, l);
+    Buf xt = e.rows(s, c, l), st1 = statsBuf(e, s, c, l);
+    conv(e, s, Act::Snake, x, l, c, c, k, d, d * (k - 1) / 2, w.w[i1], w.b[i1], af, w.alpha[i1], 0.f, w.state[i1], none, xt, st1);
+    af = affineOf(e, s, st1, bank, w.gb[i2], c, l);
+    Buf xn = last && out->p ? *out : e.rows(s, c, l);
+    Buf stn = last && outStats->p ? *outStats : statsBuf(e, s, c, l);
+    if (last) residual.ready();
+    conv(e, s, Act::Snake, xt, l, c, c, k, 1, (k - 1) / 2, w.w[i2], w.b[i2], af, w.alpha[i2], 0.f, w.state[i2], res, xn, stn);
+    x = xn, stats = stn;
+  }
+  *out = x, *outStats = stats;
+}
+
+bool resblockOk(const LkcResblock& w) {
+  if (w.c < 1 || w.k < 1 || w.k % 2 == 0) return false;
+  for (int i = 0; i < 6; ++i)
+    if (!w.w[i] || !w.b[i] || !w.alpha[i] || w.gb[i] < 0) return false;
+  return true;
+}
+
+// The generator (models/kokoro/model.py:735-781), the op sequence of Generator.forward. Streams: 0 the caller's, 1 and 2
+// the noise branches (they need only `har`), 3 and 4 the k = 7 and k = 3 resblocks of a stage.
+void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
+  const int64_t t = io.t, len[2] = {10 * t, 60 * t + 1};
+  const int64_t ch[2] = {256, 128}, cin[2] = {512, 256}, up[2] = {10, 6};
+  const Buf none;
+  Buf x, har;
+  x.p = const_cast<float*>(FP(io.x)), x.pitch = io.x_pitch;
+  har.p = const_cast<float*>(FP(io.har)), har.pitch = io.har_pitch;
+
+  Buf bank = e.alloc(0, m.bank_n);
+  e.launch(0, {bank}, [&](cudaStream_t st) { return gemmBias(FP(io.s), FP(m.bank_wt), FP(m.bank_b), bank.p, 1, 128, m.bank_n, st); });
+  e.join(1, 0), e.join(2, 0);
+
+  auto upsample = [&](int i, Buf in, int64_t lin, Buf res) {
+    Buf u = e.rows(0, ch[i], len[i]);
+    e.launch(0, {in, res, u}, [&](cudaStream_t st) {
+      ConvtParams p;
+      p.x = in.p, p.bias = FP(m.ups_b[i]), p.res = res.p, p.out = u.p;
+      p.ci = cin[i], p.l = lin, p.co = ch[i], p.stride = up[i], p.padLeft = i, p.slope = 0.1f;
+      p.xPitch = in.pitch, p.resPitch = res.pitch, p.outPitch = u.pitch;
+      const ConvState* cs = reinterpret_cast<const ConvState*>(m.ups_state[i]);
+      return convtTc(p, cs->wp, cs->f16, st);
+    });
+    return u;
+  };
+
+  // The first upsampler runs next to the first noise branch, the longer of the two; their sum is formed by that
+  // branch's last conv, whose residual is (its own running x) + (the upsampled input). The sum and its chunk statistics
+  // then leave one epilogue, and neither the upsampler nor a statistics pass stands between the branch and stage 0.
+  const Buf u0 = upsample(0, x, t, none);
+  struct AddUpsampled {
+    Exec& e;
+    Buf u;
+    int64_t c, l;
+    Buf make(Buf x) const {
+      e.join(0, 1);
+      Buf r = e.rows(0, c, l);
+      e.launch(0, {x, u, r}, [&](cudaStream_t st) { return addRows(x.p, u.p, r.p, c * r.pitch, st); });
+      return r;
+    }
+    void ready() const { e.join(1, 0); }
+  };
+  Buf noise[2], noiseStats[2];
+  for (int i = 1; i >= 0; --i) {  // polyphase view of `har`, stride-1 conv, resblock
+    const int s = 1 + i;
+    const LkcNoiseConv& n = m.noise_conv[i];
+    const int64_t ly = len[i] + n.taps - 1;
+    Buf y = e.rows(s, n.rows, ly);
+    e.launch(s, {har, y}, [&](cudaStream_t st) {
+      return spaceToDepth(har.p, y.p, 22, len[1], n.rows, ly, har.pitch, y.pitch, n.stride, n.padding, st);
+    });
+    Buf xs = e.rows(s, ch[i], len[i]), xst = statsBuf(e, s, ch[i], len[i]);
+    conv(e, s, Act::None, y, ly, n.rows, ch[i], n.taps, 1, 0, n.w, n.b, none, nullptr, 0.f, n.state, none, xs, xst);
+    if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], AddUpsampled{e, u0, ch[0], len[0]});
+    else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], PlainResidual{});
+  }
+
+  Buf in = noise[0], inStats = noiseStats[0], mean;
+  for (int i = 0; i < 2; ++i) {
+    const int64_t l = len[i], c = ch[i];
+    e.join(0, 1 + i);
+    if (i == 1) {
+      in = upsample(1, mean, len[0], noise[1]);
+      inStats = channelStatsOf(e, 0, in, c, l);
+    }
+    e.join(3, 0), e.join(4, 0);
+    Buf rb[3], st[3];
+    for (int j = 2; j >= 0; --j)
+      resblock(e, j == 2 ? 0 : (j == 1 ? 3 : 4), m.res[3 * i + j], in, inStats, l, bank, &rb[j], &st[j], PlainResidual{});
+    e.join(0, 3), e.join(0, 4);
+    mean = e.rows(0, c, l);
+    e.launch(0, {rb[0], rb[1], rb[2], mean}, [&](cudaStream_t cs) {
+      return add3Scale(rb[0].p, rb[1].p, rb[2].p, mean.p, c * mean.pitch, 1.f / 3.f, cs);
+    });
+  }
+
+  Buf post, postStats = statsBuf(e, 0, 22, len[1]), ident;
+  if (io.post) post.p = static_cast<float*>(io.post), post.pitch = io.post_pitch;
+  else post = e.rows(0, 22, len[1]);
+  ident.p = const_cast<float*>(FP(m.ident128));
+  conv(e, 0, Act::Leaky, mean, len[1], 128, 22, 7, 1, 3, m.post_w, m.post_b, ident, nullptr, 0.01f, m.post_state, none, post, postStats);
+  e.launch(0, {post}, [&](cudaStream_t st) {
+    return istftLogits(post.p, static_cast<float*>(io.audio), len[1], post.pitch, 20, 5, st);
+  });
+}
+
+}  // namespace
+}  // namespace lkc
+
+using namespace lkc;
+
+struct LkcModel {
+  LkcGenerator w;
+  cudaEvent_t events[kEvents] = {};
+  std::mutex mutex;
+  std::list<std::shared_ptr<const Plan>> plans;  // most recently used first
+
+  int plan(int64_t t, bool concurrent, std::shared_ptr<const Plan>* out) {
+    const int64_t key = 2 * t + (concurrent ? 1 : 0);
+    for (auto it = plans.begin(); it != plans.end(); ++it)
+      if ((*it)->key == key) {
+        plans.splice(plans.begin(), plans, it);
+        *out = plans.front();
+        return 0;
+      }
+    auto p = std::make_shared<Plan>();
+    p->key = key;
+    LkcGeneratorIo io{};
+    io.t = t;
+    Exec e(concurrent);
+    generator(e, w, io);
+    if (int rc = e.finishPlan(p.get())) return rc;
+    plans.push_front(p);
+    if (plans.size() > kPlans) plans.pop_back();
+    *out = p;
+    return 0;
+  }
+};
+
+extern "C" LKC_API LkcModel* lkc_generator_create(const LkcGenerator* w) {
+  const char* bad = nullptr;
+  if (!w) bad = "generator_create: null weights";
+  for (int i = 0; !bad && i < 8; ++i)
+    if (!resblockOk(i < 2 ? w->noise_res[i] : w->res[i - 2])) bad = "generator_create: bad resblock";
+  for (int i = 0; !bad && i < 2; ++i) {
+    const LkcNoiseConv& n = w->noise_conv[i];
+    if (!n.w || !n.b || !n.state || n.stride < 1 || n.taps < 1 || n.rows < 22 * n.stride) bad = "generator_create: bad noise conv";
+    else if (!w->ups_b[i] || !w->ups_state[i]) bad = "generator_create: bad upsampler";
+  }
+  if (!bad && (!w->bank_wt || !w->bank_b || w->bank_n < 1 || !w->post_w || !w->post_b || !w->ident128)) bad = "generator_create: null weight";
+  LkcModel* m = bad ? nullptr : new (std::nothrow) LkcModel;
+  if (!m) {
+    fail(bad ? bad : "generator_create: out of host memory");
+    return nullptr;
+  }
+  m->w = *w;
+  for (cudaEvent_t& ev : m->events) {
+    const cudaError_t err = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (err != cudaSuccess) {
+      failCuda("generator_create: cudaEventCreate", err);
+      lkc_model_destroy(m);
+      return nullptr;
+    }
+  }
+  return m;
+}
+
+extern "C" LKC_API void lkc_model_destroy(LkcModel* m) {
+  if (!m) return;
+  for (cudaEvent_t ev : m->events)
+    if (ev) cudaEventDestroy(ev);
+  delete m;
+}
+
+extern "C" LKC_API int lkc_generator_workspace(LkcModel* m, int64_t t, int concurrent, int64_t* bytes, int64_t* unplanned) {
+  LKC_REQUIRE(m && bytes, "generator_workspace: null argument");
+  LKC_REQUIRE(t >= 1 && t < (int64_t(1) << 24), "generator_workspace: t out of range");
+  std::lock_guard<std::mutex> lock(m->mutex);
+  std::shared_ptr<const Plan> p;
+  if (int rc = m->plan(t, concurrent != 0, &p)) return rc;
+  *bytes = p->bytes;
+  if (unplanned) *unplanned = p->unplanned;
+  return 0;
+}
+
+extern "C" LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, void* stream) {
+  LKC_REQUIRE(m && io && io->x && io->har && io->s && io->audio && io->workspace, "generator_forward: null argument");
+  LKC_REQUIRE(io->t >= 1 && io->t < (int64_t(1) << 24), "generator_forward: t out of range");
+  LKC_REQUIRE(io->x_pitch >= io->t && io->har_pitch >= 60 * io->t + 1 && (!io->post || io->post_pitch >= 60 * io->t + 1),
+              "generator_forward: a row pitch is smaller than the row");
+  LKC_REQUIRE((reinterpret_cast<uintptr_t>(io->workspace) & 255) == 0, "generator_forward: the workspace must be 256-byte aligned");
+  // The events and the order of record and wait on them belong to one forward at a time; queueing is all that happens
+  // under the lock.
+  std::lock_guard<std::mutex> lock(m->mutex);
+  std::shared_ptr<const Plan> p;
+  if (int rc = m->plan(io->t, io->concurrent != 0, &p)) return rc;
+  LKC_REQUIRE(io->workspace_bytes >= p->bytes, "generator_forward: the workspace is too small (lkc_generator_workspace)");
+  Exec e(io->concurrent != 0, *p, static_cast<char*>(io->workspace), S(stream),
+         reinterpret_cast<const cudaStream_t*>(io->side), m->events);
+  generator(e, m->w, *io);
+  io->launches = e.launches;
+  return e.rc;
+}
+
+namespace {
+// The sequence of lkc_resblock in both modes.
+void resblockCall(Exec& e, const LkcResblock& w, const LkcResblockIo& io) {
+  Buf x, st, bank, out, outStats;
+  x.p = const_cast<float*>(FP(io.x)), x.pitch = io.x_pitch;
+  bank.p = const_cast<float*>(FP(io.bank));
+  out.p = static_cast<float*>(io.out), out.pitch = io.out_pitch;
+  outStats.p = static_cast<float*>(io.out_stats);
+  if (io.stats) st.p = const_cast<float*>(FP(io.stats));
+  else st = channelStatsOf(e, 0, x, w.c, io.l);
+  resblock(e, 0, w, x, st, io.l, bank, &out, &outStats, PlainResidual{});
+}
+}  // namespace
+
+extern "C" LKC_API int lkc_resblock(const LkcResblock* w, LkcResblockIo* io, void* stream) {
+  LKC_REQUIRE(w && io && resblockOk(*w) && io->l >= 1, "resblock: bad argument");
+  LKC_REQUIRE(io->x && io->bank && io->out && io->out_stats, "resblock: null operand");
+  LKC_REQUIRE(io->x_pitch >= io->l && io->out_pitch >= io->l, "resblock: a row pitch is smaller than the row");
+  Plan p;
+  Exec plan(false);
+  resblockCall(plan, *w, *io);
+  if (int rc = plan.finishPlan(&p)) return rc;
+  if (!io->workspace) {  // the size only
+    io->workspace_bytes = p.bytes;
+    return 0;
+  }
+  LKC_REQUIRE((reinterpret_cast<uintptr_t>(io->workspace) & 255) == 0 && io->workspace_bytes >= p.bytes,
+              "resblock: the workspace must be 256-byte aligned and hold what the size call says");
+  Exec e(false, p, static_cast<char*>(io->workspace), S(stream), nullptr, nullptr);
+  resblockCall(e, *w, *io);
+  io->launches = e.launches;
+  return e.rc;
+}

@@ -10,10 +10,12 @@ buffers, so a replay costs one launch.
 """
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import torch
 
-from . import ops
+from . import _lib, ops
 from .synth import shapes
 
 DILATIONS = (1, 3, 5)
@@ -26,6 +28,21 @@ class _NullCtx:
 
     def __exit__(self, *exc):
         return False
+
+
+class StyleBank:
+    """fc(style) of every AdaIN as views into one style-bank GEMV (model.py:135-144): bank(name) -> f32[2C]."""
+
+    def __init__(self, bank, off):
+        self.bank, self.off = bank, off
+
+    def __call__(self, name):
+        o, n = self.off[name]
+        return self.bank[o: o + n]
+
+
+def _handle(state):
+    return None if state is None else state.handle
 
 
 class Generator:
@@ -75,6 +92,16 @@ class Generator:
                 self.noise_tc[i] = (wp, state, ident, stride, pad, wn.shape[2] // stride, rows)
         self._graphs = {}
         self._streams = None
+        self._blocks = {}  # prefix -> LkcResblock (pointers into self.w, which keeps them alive)
+        self._model = None  # handle of the whole-forward call
+
+    def __del__(self):
+        try:
+            if self._model:
+                _lib.lib().lkc_model_destroy(self._model)
+                self._model = None
+        except Exception:
+            pass
 
     # ------------------------------------------------------------------ building blocks
 
@@ -94,8 +121,108 @@ class Generator:
 
     def style(self, s):
         """fc(style) of every AdaIN as views into one style-bank GEMV (model.py:135-144): name -> f32[2C]."""
-        bank = ops.gemm_bias_f32_cuda(s.reshape(1, -1), self.bank_wt, self.bank_b).reshape(-1)
-        return lambda name: bank[self.bank_off[name][0]: self.bank_off[name][0] + self.bank_off[name][1]]
+        return StyleBank(ops.gemm_bias_f32_cuda(s.reshape(1, -1), self.bank_wt, self.bank_b).reshape(-1), self.bank_off)
+
+    # One resblock and one forward as single library calls (lkc_resblock, lkc_generator_forward): the same kernels in the
+    # same order as the compositions below, queued without a trip through Python per kernel. The compositions remain for
+    # what looks at single kernels (ops.Profile with timing, ops.tracing), for the CUDA-core path and for shapes that
+    # have no tensor-core state.
+
+    def _block(self, prefix, k):
+        """LkcResblock of the weights under `prefix`, or None when a conv of it has no prepared state."""
+        if prefix not in self._blocks:
+            w, blk = self.w, _lib.LkcResblock()
+            c = int(w[f"{prefix}.convs1.0.weight"].shape[0])
+            blk.c, blk.k = c, k
+            for j in range(3):
+                for n in (1, 2):
+                    i, conv = 2 * j + n - 1, f"{prefix}.convs{n}.{j}"
+                    st = self.conv_state.get(conv)
+                    if st is None or tuple(w[conv + ".weight"].shape) != (c, c, k):
+                        self._blocks[prefix] = None
+                        return None
+                    blk.w[i], blk.b[i] = w[conv + ".weight"].data_ptr(), w[conv + ".bias"].data_ptr()
+                    blk.alpha[i] = w[f"{prefix}.alpha{n}.{j}"].data_ptr()
+                    blk.state[i], blk.gb[i] = st.handle, self.bank_off[f"{prefix}.adain{n}.{j}.fc"][0]
+            self._blocks[prefix] = blk
+        blk = self._blocks[prefix]
+        return blk if blk is not None and blk.k == k else None
+
+    def _whole_model(self):
+        """Handle of lkc_generator_forward, or None when some conv has no tensor-core state."""
+        if self._model is None:
+            m, w = _lib.LkcGenerator(), self.w
+            blocks = [(f"noise_res.{i}", k) for i, k in enumerate((7, 11))] + [
+                (f"resblocks.{3 * i + j}", k) for i in (0, 1) for j, k in enumerate(RES_KERNELS)]
+            blocks = [self._block(p, k) if f"{p}.convs1.0.weight" in w else None for p, k in blocks]
+            if (None in blocks or self.ups_wp is None or None in self.ups_state or len(self.noise_tc) < 2
+                    or "conv_post" not in self.conv_state):
+                self._model = 0
+                return None
+            m.noise_res[:], m.res[:] = blocks[:2], blocks[2:]
+            m.bank_wt, m.bank_b, m.bank_n = self.bank_wt.data_ptr(), self.bank_b.data_ptr(), self.bank_b.shape[0]
+            for i in (0, 1):
+                wp, state, _, stride, pad, taps, rows = self.noise_tc[i]
+                n = m.noise_conv[i]
+                n.w, n.b, n.state = wp.data_ptr(), w[f"noise_convs.{i}.bias"].data_ptr(), state.handle
+                n.stride, n.padding, n.taps, n.rows = stride, pad, taps, rows
+                m.ups_b[i], m.ups_state[i] = w[f"ups.{i}.bias"].data_ptr(), self.ups_state[i].handle
+            m.post_w, m.post_b = w["conv_post.weight"].data_ptr(), w["conv_post.bias"].data_ptr()
+            m.ident128, m.post_state = self.ident128.data_ptr(), self.conv_state["conv_post"].handle
+            with torch.cuda.device(self.device):
+                self._model = _lib.lib().lkc_generator_create(ctypes.byref(m))
+            if not self._model:
+                raise _lib.LkcError(_lib.last_error())
+        return self._model or None
+
+    def _workspace_bytes(self, t, concurrent):
+        """(planned, unplanned) bytes of the intermediates of one forward of length t."""
+        b, u = ctypes.c_int64(0), ctypes.c_int64(0)
+        if _lib.lib().lkc_generator_workspace(self._model, t, int(concurrent), ctypes.byref(b), ctypes.byref(u)) != 0:
+            raise _lib.LkcError(_lib.last_error())
+        return b.value, u.value
+
+    def _forward_whole(self, x, har, s, outputs, concurrent, workspace=None):
+        t, dev = int(x.shape[1]), self.device
+        sh = shapes(t)
+        if workspace is None:
+            workspace = torch.empty(self._workspace_bytes(t, concurrent)[0], dtype=torch.uint8, device=dev)
+        io = _lib.LkcGeneratorIo()
+        res = {"audio": torch.empty(sh["S"], dtype=torch.float32, device=dev)}
+        if "post" in outputs:
+            with ops.padded_rows():
+                res["post"] = ops.empty_rows(22, sh["L1"], dev)
+            io.post, io.post_pitch = res["post"].data_ptr(), res["post"].stride(0)
+        io.x, io.har, io.s, io.audio = x.data_ptr(), har.data_ptr(), s.data_ptr(), res["audio"].data_ptr()
+        io.t, io.x_pitch, io.har_pitch = t, x.stride(0), har.stride(0)
+        io.workspace, io.workspace_bytes = workspace.data_ptr(), workspace.numel()
+        io.concurrent = int(concurrent)
+        if concurrent:
+            io.side[:] = [st.cuda_stream for st in self._side_streams()]
+        if _lib.lib().lkc_generator_forward(self._model, ctypes.byref(io), ops._stream()) != 0:
+            raise _lib.LkcError("generator forward: " + _lib.last_error())
+        ops.count_launches(io.launches)
+        out = tuple(res[o] for o in outputs)
+        return out[0] if len(out) == 1 else out
+
+    def _resblock_whole(self, blk, x, gb, x_stats):
+        c, n = int(x.shape[0]), int(x.shape[1])
+        out = ops.empty_rows(c, n, x.device)
+        stats = ops._alloc((c, ops.ceildiv(n, ops.STAT_CHUNK), 2), x.device)
+        io, fn = _lib.LkcResblockIo(), _lib.lib().lkc_resblock
+        io.x, io.bank, io.out, io.out_stats = x.data_ptr(), gb.bank.data_ptr(), out.data_ptr(), stats.data_ptr()
+        io.stats = None if x_stats is None else x_stats.data_ptr()
+        io.l, io.x_pitch, io.out_pitch = n, x.stride(0), out.stride(0)
+        rc = fn(ctypes.byref(blk), ctypes.byref(io), None)  # sizes the workspace
+        if rc == 0:
+            ws = torch.empty(io.workspace_bytes, dtype=torch.uint8, device=x.device)
+            io.workspace = ws.data_ptr()
+            with torch.cuda.device(x.device):
+                rc = fn(ctypes.byref(blk), ctypes.byref(io), ops._stream())
+        if rc != 0:
+            raise _lib.LkcError("resblock: " + _lib.last_error())
+        ops.count_launches(io.launches)
+        return out, stats
 
     def _snake_conv(self, x, af, alpha_key, conv, k, d, residual=None):
         w = self.w
@@ -105,6 +232,12 @@ class Generator:
 
     def adain_resblock1_fused(self, x, gb, prefix, k, x_stats=None):
         n = x.shape[1]
+        if isinstance(gb, StyleBank) and not ops.op_by_op() and x.is_cuda:
+            blk = self._block(prefix, k)
+            ops._f32(x, *([] if x_stats is None else [x_stats]))
+            if blk is not None and tuple(x.shape) == (blk.c, n) and (
+                    x_stats is None or tuple(x_stats.shape) == (blk.c, ops.ceildiv(n, ops.STAT_CHUNK), 2)):
+                return self._resblock_whole(blk, x, gb, x_stats)
         st = ops.channel_stats_f32_cuda(x) if x_stats is None else x_stats
         for j, d in enumerate(DILATIONS):
             af = ops.adain_affine_f32_cuda(st, gb(f"{prefix}.adain1.{j}.fc"), length=n)
@@ -162,6 +295,12 @@ class Generator:
             # them with the TMA unit (values do not depend on the pitch)
             with ops.padded_rows():
                 return self.forward(x, har, s, fused, outputs, concurrent, pad_rows)
+        if fused and set(outputs) <= {"audio", "post"} and not ops.op_by_op() and ops._pad_rows and self._whole_model():
+            ops._f32(x, har, s)
+            ops.check(all(v.is_cuda and v.device == x.device for v in (x, har, s)) and s.numel() == 128,
+                      "operands must live on one cuda device, s must be f32[128]")
+            with torch.cuda.device(x.device):
+                return self._forward_whole(x, har, s.contiguous(), outputs, concurrent)
         gb = self.style(s)
         cur = torch.cuda.current_stream(self.device)
         par = fused and concurrent
@@ -273,10 +412,10 @@ class Generator:
         """Records forward(fused=True) for input length t into a CUDA graph (once per t). Returns a dict with the
         static buffers `x`, `har`, `s`, `audio` and the `graph`; fill the inputs, then graph.replay().
 
-        planned=True (default): the forward's intermediates live in a planned arena (arena.py): one traced forward
-        gives every tensor's life, the plan overlays tensors that are never alive together (judged by the fork / join
-        structure of the streams, not by program order), and the captured forward takes views of ONE device buffer
-        sized by the plan (`arena_bytes`; `unplanned_bytes` is what keeping every intermediate would take)."""
+        planned=True (default): the forward's intermediates live in a planned arena, ONE device buffer in which tensors
+        that are never alive together (judged by the fork / join structure of the streams, not by program order) overlay
+        each other (`arena_bytes`; `unplanned_bytes` is what keeping every intermediate would take). The plan is the
+        whole-forward call's own; the op-by-op forward of the CUDA-core path is traced and planned by arena.py."""
         if t in self._graphs:
             return self._graphs[t]
         from .arena import PlannedArena, Tracer
@@ -285,13 +424,17 @@ class Generator:
         pitch = -(-t // ops.ROW_ALIGN) * ops.ROW_ALIGN  # rows of x start on 16-byte boundaries for any t
         bufs = {"x": torch.zeros(512, pitch, device=dev)[:, :t], "har": torch.zeros(22, sh["L1"], device=dev),
                 "s": torch.zeros(128, device=dev)}
+        whole = not ops.op_by_op() and self._whole_model() is not None
+        if whole and planned:
+            bufs["arena_bytes"], bufs["unplanned_bytes"] = self._workspace_bytes(t, True)
+            bufs["arena"] = torch.empty(bufs["arena_bytes"], dtype=torch.uint8, device=dev)
         side = self._warm_stream()
         side.wait_stream(torch.cuda.current_stream(dev))
         arena = None
         with torch.cuda.stream(side):
-            for _ in range(2):  # warm-up outside capture: lazy module loading, function attributes
+            for _ in range(1 if whole else 2):  # warm-up outside capture: lazy module loading, function attributes
                 ref = self.forward(bufs["x"], bufs["har"], bufs["s"])
-            if planned:
+            if planned and not whole:
                 with ops.tracing(Tracer()) as tr:
                     tr.pin(self.forward(bufs["x"], bufs["har"], bufs["s"]))
                 arena = PlannedArena(tr, dev)
@@ -305,7 +448,9 @@ class Generator:
         torch.cuda.synchronize(dev)
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
-            if arena is not None:
+            if "arena" in bufs:
+                bufs["audio"] = self._forward_whole(bufs["x"], bufs["har"], bufs["s"], ("audio",), True, bufs["arena"])
+            elif arena is not None:
                 arena.begin()
                 with ops.use_allocator(arena.allocator):
                     bufs["audio"] = self.forward(bufs["x"], bufs["har"], bufs["s"])

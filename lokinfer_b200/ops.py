@@ -104,6 +104,20 @@ class Profile:
 _profile = None
 
 
+def op_by_op() -> bool:
+    """True while every kernel has to go through _run: single kernels are being timed or traced, results come from a
+    custom allocator, or the CUDA-core path is selected. The whole-model calls of generator.py and decoder.py then stand
+    back for their compositions."""
+    return (_tracer is not None or (_profile is not None and _profile.time_kernels) or allocator is not _torch_alloc
+            or _conv_path == "simt")
+
+
+def count_launches(n) -> None:
+    """Adds the kernels that a whole-model call queued to the active Profile."""
+    if _profile is not None:
+        _profile.count += int(n)
+
+
 # Kernels that take row pitches: positions (in operands + outs order) of their [C, L] activation tensors. The
 # pitches are appended to the ints only when one of them differs from the row length.
 _PITCHED = {
