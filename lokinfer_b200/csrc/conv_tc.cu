@@ -46,6 +46,8 @@
 //   warp 13     MMA issuer (one lane): per tap group one wait, the group's MMAs back to back, one release
 //   warp 17     raw-window loader of the aligned route (one lane): two tiled TMA loads per chunk, one chunk ahead
 //   warp 19     idle (completes the fifth warpgroup)
+// Launches with few tiles take a second form of the same kernel (template parameter SPLIT): a cluster of CTAs per
+// 128-column tile, each contracting a part of the input channels, reduced over distributed shared memory.
 // All hand-offs are mbarriers. Every wait is bounded: on a timeout the kernel records a status word, drains its
 // copies in flight and returns (TMEM is freed on every path).
 #include <cuda.h>
@@ -65,6 +67,7 @@ namespace {
 
 constexpr bool kProf = LKC_TC_PROF != 0;
 constexpr int NT = 256;         // time columns per tile (= UMMA N)
+constexpr int NTS = 128;        // time columns per tile of the split form: one statistics chunk
 constexpr int MT = 128;         // output channels per tile (= UMMA M)
 constexpr int KC = 16;          // input channels per staged chunk (one weight stage, two K8 steps)
 constexpr int MAX_NB = 4;       // most activation (hi / lo) buffers
@@ -102,12 +105,16 @@ constexpr int STAGE_PITCH = 33;  // floats per row of an epilogue transpose tile
 constexpr int STAGE_FLOATS = 32 * STAGE_PITCH;
 constexpr int BOX = 32, BOX_BYTES = BOX * BOX * 4;  // residual / output boxes of the aligned route: 32 co x 32 t
 static_assert(BOX_BYTES <= STAGE_FLOATS * 4, "a swizzled box fits in a warp's tile");
+constexpr int PART_PITCH = NTS + 4;  // floats per row of a split tile's partial: rows 16-byte aligned, 4 banks apart
+constexpr int PART_BYTES = MT * PART_PITCH * 4;
+constexpr size_t SPLIT_SMEM = 120 * 1024;  // more than half an SM's: one CTA per SM, for whose TMEM two would compete
+constexpr int MAX_SPLIT = 8;     // CTAs of a split tile (the portable cluster size)
 constexpr int MAX_HALO = 50;     // (K - 1) * dilation of the widest Kokoro conv (K 11, dilation 5)
 constexpr int MAX_W_STAGES = 4, MIN_W_STAGES = 2, PREF_W_STAGES = 2;  // weight ring slots
 constexpr int TAP_GROUP = 6;  // most taps per weight slot: one bulk copy, one wait, MMAs back to back, one release
 constexpr int MAX_CHAIN = 24;  // most chained hi MMAs between two drains of Dhi
 constexpr uint32_t SPIN_LIMIT = 1u << 24;
-constexpr uint32_t SLEEP_EPI_NS = 256, SLEEP_PRO_NS = 128, SLEEP_W_NS = 64, SLEEP_MMA_NS = 32;
+constexpr uint32_t SLEEP_EPI_NS = 256, SLEEP_EPI_SPLIT_NS = 64, SLEEP_PRO_NS = 128, SLEEP_W_NS = 64, SLEEP_MMA_NS = 32;
 constexpr uint64_t WAIT_LIMIT_NS = 200ull * 1000 * 1000;  // 0.2 s: a healthy wait is tens of microseconds
 constexpr int kMaxSmem = 232448;  // 227 KB per CTA on sm_100
 
@@ -116,13 +123,14 @@ constexpr int kMaxSmem = 232448;  // 227 KB per CTA on sm_100
 struct SmemLayout {
   uint32_t act, raw, w, par, bar, total;
 };
-__host__ __device__ inline SmemLayout smemLayout(int ci, int rows, int half, int nb, int wStages, int wG, int actRowBytes,
-                                                 int wStageBytes) {
+__host__ __device__ inline SmemLayout smemLayout(bool split, int ci, int rows, int half, int nb, int wStages, int wG,
+                                                 int actRowBytes, int wStageBytes) {
   SmemLayout s;
-  s.act = EPI_WARPS * STAGE_FLOATS * 4;  // tiles: [0, act)
+  s.act = split ? 0 : EPI_WARPS * STAGE_FLOATS * 4;  // tiles: [0, act)
   s.raw = (s.act + uint32_t(nb) * actRowBytes * rows + 127u) & ~127u;
   s.w = s.raw + uint32_t(NRAW) * 2 * KC * half * 4;  // a multiple of 128
   s.par = s.w + uint32_t(wStages) * wG * wStageBytes;
+  if (split && s.par < uint32_t(PART_BYTES)) s.par = PART_BYTES;  // a split tile's partial lies over the operand buffers
   s.bar = s.par + uint32_t(4) * ci * 4;
   s.total = s.bar + 512;
   return s;
@@ -137,7 +145,7 @@ struct TcArgs {
   int64_t xPitch, resPitch, outPitch;  // row pitches in floats
   int padLeft;       // ConvTranspose: 1 = one-sample left reflect pad
   float slope, outScale;
-  int rows;        // staged time rows per buffer = NT + (k-1)*dilation
+  int rows;        // staged time rows per buffer = tile columns + (k-1)*dilation
   int half;        // raw staging: every channel's window is kept as two runs of `half` floats (two TMA boxes)
   int wStages;     // weight ring depth (slots)
   int nb;          // activation buffers
@@ -147,6 +155,7 @@ struct TcArgs {
   int tmaIn;       // 1: x rows are 16-byte aligned, the raw windows come by tiled TMA loads
   int tmaOut;      // 1: out (and residual) rows are 16-byte aligned, boxes go by TMA
   int numTTiles, numCoBlk;
+  int split;       // 0 = a persistent CTA per SM over 256-column tiles; else the CTAs that share one 128-column tile
   int* status;
   long long* prof;  // null, or 16 cycle counters summed over CTAs (see convTcProfile)
 };
@@ -256,6 +265,35 @@ __device__ __forceinline__ void tmemRelinquish() {
 __device__ __forceinline__ void tmemDealloc(uint32_t addr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
 }
+// Cluster of the split form: this CTA's rank, the barrier of all threads of all its CTAs (release / acquire: shared-memory
+// writes before it are visible to every CTA after it), and loads from the same offset in another CTA's shared memory.
+__device__ __forceinline__ uint32_t clusterRank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void clusterSync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peerAddr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 peerLoad4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ float peerLoad(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
 // D[tmem] (+)= A[smem desc] * B[smem desc], kind::tf32, issued by one thread.
 __device__ __forceinline__ void mmaTf32(uint32_t dTmem, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accum) {
   asm volatile(
@@ -301,11 +339,11 @@ __device__ __forceinline__ uint64_t makeDesc(uint32_t addr, uint32_t lbo, uint32
   return uint64_t((addr >> 4) & 0x3FFFu) | (uint64_t((lbo >> 4) & 0x3FFFu) << 16) |
          (uint64_t((sbo >> 4) & 0x3FFFu) << 32) | (uint64_t(1) << 46);
 }
-// Instruction descriptor: D f32 (bits 4-5 = 1), A and B tf32 (bits 7-9 / 10-12 = 2), both K-major, N >> 3 at bit 17,
-// M >> 4 at bit 24.
-constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t(NT >> 3) << 17) | (uint32_t(MT >> 4) << 24);
-// kind::f16 with f16 operands (format 0) and f32 accumulation.
-constexpr uint32_t kIdescF16 = (1u << 4) | (uint32_t(NT >> 3) << 17) | (uint32_t(MT >> 4) << 24);
+// Instruction descriptor of an M128 x N `n` MMA: D f32 (bits 4-5 = 1), both operands K-major, N >> 3 at bit 17, M >> 4 at
+// bit 24, A and B f16 (format 0) or tf32 (bits 7-9 / 10-12 = 2).
+__host__ __device__ constexpr uint32_t idescOf(bool f16, int n) {
+  return (1u << 4) | (f16 ? 0u : (2u << 7) | (2u << 10)) | (uint32_t(n >> 3) << 17) | (uint32_t(MT >> 4) << 24);
+}
 
 __device__ __forceinline__ float tf32Round(float v) {
   uint32_t r;
@@ -355,18 +393,183 @@ __device__ __forceinline__ void regDec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
+__device__ __forceinline__ float warpSum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// Second half of a split tile, one epilogue warp. `parts` = shared-memory address of the partial tiles, the same in every
+// CTA of the cluster.
+// conv: a unit is one output channel of the tile, four columns per lane; the rank's 128 / split channels go round robin
+// over the epilogue warps, UB at a time so that their loads overlap. What does not depend on the contraction (bias,
+// residual) is loaded by prefetch(), for the first UB units before the accumulation.
+// ConvTranspose: a unit is one output channel x 32 input-rate columns, whose 32 * TS output samples are one run.
+// Bound by the SM-to-SM reads (about 11 bytes per clock and SM measured: 5-7 k clocks for the 56 KB of eight CTAs), which
+// is why the split tile is 128 and not 256 columns wide.
+template <int TS>
+struct SplitTail {
+  static constexpr int UB = 4;
+  float4 res[UB];
+  float bias[UB];
+  int row0, units, tt, cb;
+
+  __device__ __forceinline__ SplitTail(const TcArgs& a, int tile, int rank) {
+    tt = tile / a.numCoBlk, cb = tile - tt * a.numCoBlk;
+    if constexpr (TS == 0) {
+      row0 = MT * rank / a.split, units = MT * (rank + 1) / a.split - row0;
+    } else {
+      constexpr int CH = 4 * (32 / TS);
+      row0 = CH * rank / a.split, units = (NTS / 32) * (CH * (rank + 1) / a.split - row0);  // row0: first channel
+    }
+  }
+
+  __device__ __forceinline__ void prefetch(const TcArgs& a, int u0, int lane) {
+    if constexpr (TS == 0) {
+      const bool vecRes = a.residual && ((reinterpret_cast<uintptr_t>(a.residual) | uintptr_t(a.resPitch * 4)) & 15) == 0;
+      const int64_t col = int64_t(tt) * NTS + lane * 4;
+#pragma unroll
+      for (int e = 0; e < UB; ++e) {
+        const int u = u0 + e * EPI_WARPS, co = cb * MT + row0 + u;
+        res[e] = make_float4(0.f, 0.f, 0.f, 0.f), bias[e] = 0.f;
+        if (u < units && co < a.co) {
+          if (a.bias) bias[e] = a.bias[co];
+          if (a.residual && col < a.lo) {
+            const float* rp = a.residual + int64_t(co) * a.resPitch + col;
+            if (vecRes && col + 4 <= a.lo) {
+              res[e] = *reinterpret_cast<const float4*>(rp);
+            } else {
+              res[e].x = rp[0];
+              if (col + 1 < a.lo) res[e].y = rp[1];
+              if (col + 2 < a.lo) res[e].z = rp[2];
+              if (col + 3 < a.lo) res[e].w = rp[3];
+            }
+          }
+        }
+      }
+    }
+  }
+
+  __device__ __forceinline__ void finish(const TcArgs& a, uint32_t parts, int warp, int lane) {
+    if constexpr (TS == 0) {
+      const bool vecOut = ((reinterpret_cast<uintptr_t>(a.out) | uintptr_t(a.outPitch * 4)) & 15) == 0;
+      const int64_t tChunk = int64_t(tt) * NTS, col = tChunk + lane * 4;
+      // valid columns of the tile, and from this lane's first on
+      const int nValid = a.lo - tChunk < NTS ? int(a.lo - tChunk) : NTS, mine = nValid - lane * 4;
+#pragma unroll 1
+      for (int u0 = warp; u0 < units; u0 += UB * EPI_WARPS) {
+        if (u0 != warp) prefetch(a, u0, lane);
+        float4 acc[UB];
+#pragma unroll
+        for (int e = 0; e < UB; ++e) acc[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const uint32_t at = parts + uint32_t(((row0 + u0) * PART_PITCH + lane * 4) * 4);
+        if (mine > 0) {
+#pragma unroll 4
+          for (int r = 0; r < a.split; ++r) {
+            const uint32_t peer = peerAddr(at, r);
+            float4 v[UB];
+#pragma unroll
+            for (int e = 0; e < UB; ++e)
+              if (u0 + e * EPI_WARPS < units) v[e] = peerLoad4(peer + uint32_t(e * EPI_WARPS * PART_PITCH * 4));
+              else v[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int e = 0; e < UB; ++e) acc[e].x += v[e].x, acc[e].y += v[e].y, acc[e].z += v[e].z, acc[e].w += v[e].w;
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int e = 0; e < UB; ++e) {
+          const int u = u0 + e * EPI_WARPS, co = cb * MT + row0 + u;
+          if (u >= units || co >= a.co) continue;  // warp-uniform
+          float v[4] = {acc[e].x, acc[e].y, acc[e].z, acc[e].w};
+          const float rs[4] = {res[e].x, res[e].y, res[e].z, res[e].w};
+          float sum = 0.f, m2 = 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            v[j] += bias[e];
+            if (a.residual) v[j] = (v[j] + rs[j]) * a.outScale;
+            if (j < mine) sum += v[j];
+          }
+          float* op = a.out + int64_t(co) * a.outPitch + col;
+          if (vecOut && mine >= 4) {
+            *reinterpret_cast<float4*>(op) = make_float4(v[0], v[1], v[2], v[3]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (j < mine) op[j] = v[j];
+          }
+          if (a.stats) {
+            const float mean = warpSum(sum) / float(nValid);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (j < mine) m2 = fmaf(v[j] - mean, v[j] - mean, m2);
+            m2 = warpSum(m2);
+            if (lane == 0) {
+              float* st = a.stats + (int64_t(co) * a.nchunks + tt) * 2;
+              st[0] = mean, st[1] = m2;
+            }
+          }
+        }
+      }
+    } else {
+      constexpr int CQ = 32 / TS, CH = 4 * CQ, SEGS = NTS / 32;
+      const int64_t uEnd = a.lo * TS;
+#pragma unroll 1
+      for (int u = warp; u < units; u += EPI_WARPS) {
+        const int ch = row0 + u / SEGS, seg = u % SEGS, co = cb * CH + ch;
+        const int64_t o0 = (int64_t(tt) * NTS + seg * 32) * TS + lane;
+        if (co >= a.co || o0 - lane >= uEnd) continue;
+        float* const orow = a.out + int64_t(co) * a.outPitch;
+        const float* const rrow = a.residual ? a.residual + int64_t(co) * a.resPitch : nullptr;
+        const float b = a.bias ? a.bias[co] : 0.f;
+        float acc[TS], rs[TS];
+        uint32_t off[TS];
+#pragma unroll
+        for (int f = 0; f < TS; ++f) {
+          const int idx = f * 32 + lane;
+          off[f] = parts + uint32_t((((ch / CQ) * 32 + (ch % CQ) * TS + idx % TS) * PART_PITCH + seg * 32 + idx / TS) * 4);
+          acc[f] = b;
+          rs[f] = rrow && o0 + f * 32 < uEnd ? rrow[a.padLeft + o0 + f * 32] : 0.f;
+        }
+#pragma unroll 2
+        for (int r = 0; r < a.split; ++r)
+#pragma unroll
+          for (int f = 0; f < TS; ++f) acc[f] += peerLoad(peerAddr(off[f], r));
+#pragma unroll
+        for (int f = 0; f < TS; ++f) {
+          const int64_t o = o0 + f * 32;
+          if (o < uEnd) orow[a.padLeft + o] = acc[f] + rs[f];
+          // left reflect pad: out[co, 0] = unpadded[co, 1] + residual[co, 0]
+          if (a.padLeft && o == 1 && o < uEnd) orow[0] = acc[f] + (rrow ? rrow[0] : 0.f);
+        }
+      }
+    }
+  }
+};
+
 // PARTIAL: Co is not a multiple of 128 (the last output-channel block has rows that do not exist).
 // TS: 0 = conv1d; 6 / 10 = polyphase ConvTranspose1d of that stride (see the comment above convtTcPackKernel).
 // TMAO: residual and output boxes travel by TMA (rows 16-byte aligned; conv1d with Co % 128 == 0 only).
-template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO>
+// SPLIT: a cluster of a.split CTAs shares one 128-column tile. Each CTA contracts its own run of input-channel chunks and
+// leaves its partial tile in its shared memory (over the operand buffers, which nothing reads any more); after the
+// cluster barrier it finishes a slice of the output channels: the partials are added in rank order over distributed
+// shared memory, then bias, residual, scale, statistics and coalesced stores. For launches with fewer tiles than SMs,
+// where one tile's serial chain of chunks is the launch's time (see splitFor).
+template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT>
 __global__ void __launch_bounds__(NTHREADS, 1)
     convTcKernel(const TcArgs a, const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapRes,
                  const __grid_constant__ CUtensorMap mapOut) {
   constexpr int W_STAGE_BYTES = Fmt<F16>::W_STAGE_BYTES, W_STAGE_FLOATS = Fmt<F16>::W_STAGE_FLOATS;
+  constexpr int NTK = SPLIT ? NTS : NT;  // time columns of this kernel's tiles
+  constexpr int EC = NTK / 2;            // columns of one epilogue warp
+  // Dhi buffers: a 128-column tile leaves room for two, so that the hi MMAs of a drain group need not wait for the drain
+  // of the one before (the lo MMAs that cover it are shorter here)
+  constexpr int HB = SPLIT ? 2 : 1;
+  constexpr uint32_t kIdesc = idescOf(F16, NTK);
   const int NB = a.nb;
   extern __shared__ __align__(1024) unsigned char smemRaw[];
   const int rows = a.rows, half = a.half;
-  const SmemLayout lay = smemLayout(a.ci, rows, half, NB, a.wStages, a.wG, Fmt<F16>::ACT_BYTES_PER_ROW, W_STAGE_BYTES);
+  const SmemLayout lay = smemLayout(SPLIT, a.ci, rows, half, NB, a.wStages, a.wG, Fmt<F16>::ACT_BYTES_PER_ROW, W_STAGE_BYTES);
   const int actBufFloats = Fmt<F16>::ACT_BYTES_PER_ROW / 4 * rows;  // hi + lo
   const int rawBufFloats = 2 * KC * half;
   float* const sStage = reinterpret_cast<float*>(smemRaw);           // EPI_WARPS tiles
@@ -379,8 +582,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   uint64_t* const wFull = bEmpty + MAX_NB;
   uint64_t* const wEmpty = wFull + MAX_W_STAGES;
   uint64_t* const hiFull = wEmpty + MAX_W_STAGES;
-  uint64_t* const hiEmpty = hiFull + 1;
-  uint64_t* const loFull = hiEmpty + 1;
+  uint64_t* const hiEmpty = hiFull + 2;
+  uint64_t* const loFull = hiEmpty + 2;
   uint64_t* const loEmpty = loFull + 1;
   uint64_t* const rawFull = loEmpty + 1;
   uint64_t* const rawEmpty = rawFull + NRAW;
@@ -400,7 +603,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const bool bal = a.balanced != 0;
   const int W_WARP = bal ? 16 : 9, MMA_WARP = bal ? 17 : 13, RAW_WARP = bal ? 18 : 17;
   const int numTiles = a.numTTiles * a.numCoBlk;
-  const int nChunks16 = a.ci / KC;
+  // tiles of this CTA: tile0, tile0 + tileStep, ...; its chunks of a tile: cBegin .. cBegin + nChunks16
+  const int rank = SPLIT ? int(clusterRank()) : 0;
+  const int tile0 = SPLIT ? int(blockIdx.x) / a.split : int(blockIdx.x), tileStep = SPLIT ? numTiles : int(gridDim.x);
+  const int nChunksAll = a.ci / KC;
+  const int cBegin = SPLIT ? nChunksAll * rank / a.split : 0;
+  const int nChunks16 = SPLIT ? nChunksAll * (rank + 1) / a.split - cBegin : nChunksAll;
   const int nGroups = (nChunks16 + a.drainN - 1) / a.drainN;  // Dhi drains per tile
   // tap groups of a chunk: the first tgExtra groups have tgBase + 1 taps, the others tgBase
   const int nTapGroups = (a.k + a.wG - 1) / a.wG, tgBase = a.k / nTapGroups, tgExtra = a.k % nTapGroups;
@@ -408,7 +616,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (threadIdx.x == 0) {
     for (int i = 0; i < NB; ++i) mbarInit(&bFull[i], PRO_WARPS), mbarInit(&bEmpty[i], 1);
     for (int i = 0; i < MAX_W_STAGES; ++i) mbarInit(&wFull[i], 1), mbarInit(&wEmpty[i], 1);
-    mbarInit(hiFull, 1), mbarInit(hiEmpty, EPI_WARPS), mbarInit(loFull, 1), mbarInit(loEmpty, EPI_WARPS);
+    for (int i = 0; i < HB; ++i) mbarInit(&hiFull[i], 1), mbarInit(&hiEmpty[i], EPI_WARPS);
+    mbarInit(loFull, 1), mbarInit(loEmpty, EPI_WARPS);
     for (int i = 0; i < NRAW; ++i) mbarInit(&rawFull[i], 1), mbarInit(&rawEmpty[i], PRO_WARPS);
     for (int i = 0; i < EPI_WARPS; ++i) mbarInit(&resBar[i], 1);
     *abortFlag = 0;
@@ -464,14 +673,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     static_assert(!TMAO || (TS == 0 && !PARTIAL), "boxes need whole 32-channel row groups of a conv1d");
     constexpr bool tmaOut = TMAO;
     const uint32_t laneBase = uint32_t(q * 32) << 16;
+    constexpr uint32_t kSleepEpi = SPLIT ? SLEEP_EPI_SPLIT_NS : SLEEP_EPI_NS;
     uint32_t groupIt = 0, tileIt = 0, resIt = 0;
     bool dead = false, resInFlight = false;
+    SplitTail<TS> tail(a, tile0, rank);
+    if constexpr (SPLIT) tail.prefetch(a, warp, lane);
     long long wHi = 0, wLo = 0, cPre = 0, cFin = 0;
     const long long tStart = kProf ? clock64() : 0;
-    for (int t = blockIdx.x; t < numTiles && !dead; t += gridDim.x, ++tileIt) {
+    for (int t = tile0; t < numTiles && !dead; t += tileStep, ++tileIt) {
       const int tt = t / a.numCoBlk, cb = t - tt * a.numCoBlk;
       const long long tPre = kProf ? clock64() : 0;
-      const int64_t tChunk = int64_t(tt) * NT + g * 128;  // first output column of this warp's 128-column chunk
+      const int64_t tChunk = int64_t(tt) * NTK + g * EC;  // first output column of this warp's 128-column chunk
       const int64_t nValid64 = a.lo - tChunk;
       const int nValid = nValid64 <= 0 ? 0 : (nValid64 < 128 ? int(nValid64) : 128);
       // conv: the warp's rows are 32 consecutive output channels. ConvTranspose: rows are (channel, phase) pairs,
@@ -485,7 +697,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const int coBase = TS ? (cb * 4 + q) * CQ : cb * MT + q * 32;
       const int co = TS ? coBase + lane / (TS ? TS : 1) : coBase + lane;
       const bool rowOk = TS ? (lane < ROWS && co < a.co) : (!PARTIAL || co < a.co);
-      const float bias = (a.bias && rowOk) ? a.bias[co] : 0.f;
+      const float bias = (!SPLIT && a.bias && rowOk) ? a.bias[co] : 0.f;
       // channels of this warp that exist (may be <= 0 in the last block)
       const int coValid = (TS || PARTIAL) ? (a.co - coBase < CQ ? a.co - coBase : CQ) : 32;
       // Running sums start from the bias. The residual is added one 32-column batch at a time: while the warp waits
@@ -494,8 +706,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // The global latency hides behind a whole group of MMAs and no registers are held while waiting.
       float S[128];
 #pragma unroll
-      for (int j = 0; j < 128; ++j) S[j] = bias;
-      const bool hasRes = a.residual != nullptr;
+      for (int j = 0; j < EC; ++j) S[j] = bias;
+      const bool hasRes = !SPLIT && a.residual != nullptr;
       // ConvTranspose with the left reflect pad: out[co, 0] = unpadded[co, 1] + res[co, 0] (the reference copies
       // the column, then adds the residual). The lane that owns (column 0, phase 1) keeps that element's residual
       // out of its running sum and adds it last, so the reflect column gets the plain conv sum.
@@ -577,15 +789,16 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (kProf) cPre += clock64() - tPre;
       // wait for the group's hi chain, add it to the running sums, hand Dhi back
       auto drainGroup = [&]() -> bool {
-        if (!waitT(hiFull, groupIt & 1, wHi, SLEEP_EPI_NS)) {
+        const uint32_t hb = HB == 2 ? groupIt & 1 : 0;
+        if (!waitT(&hiFull[hb], (HB == 2 ? groupIt >> 1 : groupIt) & 1, wHi, kSleepEpi)) {
           giveUp(1, 1);
           return false;
         }
         tcFenceAfter();
 #pragma unroll
-        for (int b = 0; b < 8; ++b) {
+        for (int b = 0; b < EC / 16; ++b) {
           uint32_t v[16];
-          tmemLoad16Async(tmemHi + laneBase + g * 128 + b * 16, v);
+          tmemLoad16Async(tmemHi + hb * NTK + laneBase + g * EC + b * 16, v);
           tmemWaitLoads();
 #pragma unroll
           for (int j = 0; j < 16; j += 2) {  // packed f32x2 adds: half the instructions of the accumulate loop
@@ -596,7 +809,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
         tcFenceBefore();
         __syncwarp();
-        if (lane == 0) mbarArrive(hiEmpty);
+        if (lane == 0) mbarArrive(&hiEmpty[hb]);
         ++groupIt;
         return true;
       };
@@ -618,17 +831,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (c == nSteps - 1) {
           // Last step of the tile (always a drain): Dlo is complete before the last hi MMAs are, so it is folded in
           // first and handed back, and the next tile's lo MMAs need not wait for the last drain and the final phase.
-          if (!waitT(loFull, tileIt & 1, wLo, SLEEP_EPI_NS)) {
+          if (!waitT(loFull, tileIt & 1, wLo, kSleepEpi)) {
             giveUp(1, 2);
             dead = true;
             break;
           }
           tcFenceAfter();
 #pragma unroll
-          for (int b = 0; b < 4; ++b) {  // two 16-column loads in flight per wait
+          for (int b = 0; b < EC / 32; ++b) {  // two 16-column loads in flight per wait
             uint32_t va[16], vb[16];
-            tmemLoad16Async(tmemLo + laneBase + g * 128 + b * 32, va);
-            tmemLoad16Async(tmemLo + laneBase + g * 128 + b * 32 + 16, vb);
+            tmemLoad16Async(tmemLo + laneBase + g * EC + b * 32, va);
+            tmemLoad16Async(tmemLo + laneBase + g * EC + b * 32 + 16, vb);
             tmemWaitLoads();
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -654,6 +867,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       if (dead) break;
       const long long tFin = kProf ? clock64() : 0;
+      if constexpr (SPLIT) {
+        // the last drain followed every MMA of this CTA, so the operand buffers are free
+        float* const row = reinterpret_cast<float*>(smemRaw) + (q * 32 + lane) * PART_PITCH + g * EC;
+#pragma unroll
+        for (int j = 0; j < EC; j += 4) *reinterpret_cast<float4*>(row + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
+        if (kProf) cFin += clock64() - tFin;
+        continue;
+      }
       if (a.residual && a.outScale != 1.f) {
 #pragma unroll
         for (int j = 0; j < 128; ++j) S[j] *= a.outScale;
@@ -799,6 +1020,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       if (kProf) cFin += clock64() - tFin;
     }
+    if constexpr (SPLIT) {
+      clusterSync();
+      tail.finish(a, smemAddr(smemRaw), warp, lane);
+    }
     // Copies of this warp still in flight must end before the CTA may exit: a residual box after an abort, and the
     // output boxes on every path.
     if (resInFlight) mbarWaitQuiet(myRes, resIt & 1);
@@ -813,11 +1038,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const int cg = pw & 3, hf = pw >> 2;  // channel group of 4 inside the 16-channel chunk; row half
     const int rowsHalf = (rows + 1) >> 1;
     const int r0 = hf * rowsHalf, r1 = (r0 + rowsHalf < rows) ? r0 + rowsHalf : rows;
-    constexpr int SLOTS = (((NT + MAX_HALO + 1) >> 1) + 31) / 32;  // row slots of 32 lanes per warp
+    constexpr int SLOTS = (((NTK + MAX_HALO + 1) >> 1) + 31) / 32;  // row slots of 32 lanes per warp
     const bool tmaIn = a.tmaIn != 0;
     const int runSkip = (KC - 1) * half;  // a raw window index i >= half sits in the second run: + runSkip floats
     // per-channel parameters, once: sPar = [mean | a | b | inv] with a = scale, b = beta (x alpha for Snake), inv = 1/alpha
-    for (int c = pw * 32 + lane; c < a.ci; c += PRO_WARPS * 32) {
+    for (int c = cBegin * KC + pw * 32 + lane; c < (cBegin + nChunks16) * KC; c += PRO_WARPS * 32) {
       const float al = ACT == 1 ? a.alpha[c] : 1.f;
       sPar[c] = a.affine ? a.affine[c] : 0.f;
       sPar[a.ci + c] = (a.affine ? a.affine[a.ci + c] : 1.f) * al;
@@ -830,7 +1055,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // input position posT (= tile column * NT - padding) into staging buffer rb. Pointer increments only: this runs
     // once per chunk on every producer thread.
     auto issueCopies = [&](int64_t posT, int c, int rb) {
-      const float* xc = a.x + int64_t(c * KC + cg * 4) * a.xPitch + posT + r0 + lane;
+      const float* xc = a.x + int64_t((cBegin + c) * KC + cg * 4) * a.xPitch + posT + r0 + lane;
       float* base = sRaw + rb * rawBufFloats + cg * 4 * half;
       int64_t pos = posT + r0 + lane;
       int r = r0 + lane;
@@ -846,11 +1071,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
     };
 
-    int t = blockIdx.x, c = 0;
+    int t = tile0, c = 0;
     uint32_t buf = 0, bufPar = 1, rawBuf = 0, rawPar = 0;  // activation buffer + parity of its last release; raw buffer + parity of its fill
     long long wB = 0, wCp = 0, cTr = 0;
     const long long tStart = kProf ? clock64() : 0;
-    int64_t pos0 = int64_t(t / a.numCoBlk) * NT - a.padding;  // input position of row 0 of the current tile's window
+    int64_t pos0 = int64_t(t / a.numCoBlk) * NTK - a.padding;  // input position of row 0 of the current tile's window
     if (!tmaIn) {
       if (t < numTiles) issueCopies(pos0, c, 0);
       cpAsyncCommit();
@@ -859,8 +1084,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       int tn = t, cn = c + 1;
       int64_t posN = pos0;
       if (cn == nChunks16) {
-        cn = 0, tn = t + gridDim.x;
-        posN = int64_t(tn / a.numCoBlk) * NT - a.padding;
+        cn = 0, tn = t + tileStep;
+        posN = int64_t(tn / a.numCoBlk) * NTK - a.padding;
       }
       // the window's offset inside the staged runs: the aligned route loads from the 16-byte boundary below pos0
       int delta = 0;
@@ -891,7 +1116,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       float2 nm[2], pa[2], pb[2], pi[2];  // channel pairs (0, 1) and (2, 3); nm = -mean
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const float* par = sPar + c * KC + cg * 4 + 2 * h;
+        const float* par = sPar + (cBegin + c) * KC + cg * 4 + 2 * h;
         nm[h] = make_float2(-par[0], -par[1]);
         pa[h] = make_float2(par[a.ci], par[a.ci + 1]);
         pb[h] = make_float2(par[2 * a.ci], par[2 * a.ci + 1]);
@@ -960,11 +1185,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       bool dead = false;
       long long wW = 0;
       const long long tStart = kProf ? clock64() : 0;
-      const int64_t blocksPerCo = int64_t(nChunks16) * a.k;  // one block (hi + lo of one tap) per chunk and tap
+      const int64_t blocksPerCo = int64_t(nChunksAll) * a.k;  // one block (hi + lo of one tap) per chunk and tap
       const int slotFloats = a.wG * W_STAGE_FLOATS;
-      for (int t = blockIdx.x; t < numTiles && !dead; t += gridDim.x) {
+      for (int t = tile0; t < numTiles && !dead; t += tileStep) {
         const int tt = t / a.numCoBlk, cb = t - tt * a.numCoBlk;
-        const float* src = a.wp + int64_t(cb) * blocksPerCo * W_STAGE_FLOATS;
+        const float* src = a.wp + (int64_t(cb) * blocksPerCo + int64_t(cBegin) * a.k) * W_STAGE_FLOATS;
         for (int c = 0; c < nChunks16 && !dead; ++c) {
           for (int gi = 0; gi < nTapGroups; ++gi, ++wIt) {
             const int n = tgBase + (gi < tgExtra ? 1 : 0);
@@ -1001,8 +1226,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         long long wR = 0;
         bool dead = false;
         const uint32_t bytes = uint32_t(rawBufFloats) * 4;
-        for (int t = blockIdx.x; t < numTiles && !dead; t += gridDim.x) {
-          const int64_t pos0 = int64_t(t / a.numCoBlk) * NT - a.padding;
+        for (int t = tile0; t < numTiles && !dead; t += tileStep) {
+          const int64_t pos0 = int64_t(t / a.numCoBlk) * NTK - a.padding;
           const int x0 = int(pos0 - (pos0 & 3));
           for (int c = 0; c < nChunks16; ++c, ++issued) {
             if (!waitT(&rawEmpty[rb], ph, wR, SLEEP_W_NS)) {
@@ -1012,8 +1237,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             }
             float* dst = sRaw + rb * rawBufFloats;
             mbarArriveExpectTx(&rawFull[rb], bytes);
-            tmaLoad2d(dst, &mapX, x0, c * KC, &rawFull[rb]);
-            tmaLoad2d(dst + KC * half, &mapX, x0 + half, c * KC, &rawFull[rb]);
+            tmaLoad2d(dst, &mapX, x0, (cBegin + c) * KC, &rawFull[rb]);
+            tmaLoad2d(dst + KC * half, &mapX, x0 + half, (cBegin + c) * KC, &rawFull[rb]);
             if (++rb == NRAW) rb = 0, ph ^= 1;
           }
         }
@@ -1045,11 +1270,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const uint32_t slotU = uint32_t(a.wG) * kStageU;
       const int dil = a.dilation, wStages = a.wStages, drainN = a.drainN;
       int slot = 0, buf = 0, g = 0;
-      uint32_t slotPh = 0, bufPh = 0, groupPar = 0, tilePar = 0;
+      uint32_t slotPh = 0, bufPh = 0, groupPar = 0, tilePar = 0, hb = 0;
       bool dead = false, ready = false;  // ready: the next round's weight slot is already known to be full
       long long wBf = 0, wHe = 0, wWf = 0, wLe = 0;
       const long long tStart = kProf ? clock64() : 0;
-      for (int tile = blockIdx.x; lane == 0 && tile < numTiles && !dead; tile += gridDim.x) {
+      for (int tile = tile0; lane == 0 && tile < numTiles && !dead; tile += tileStep) {
         for (int c = 0; c < nChunks16 && !dead; ++c) {
           if (!waitT(&bFull[buf], bufPh, wBf, SLEEP_MMA_NS)) {
             giveUp(4, 2);
@@ -1072,18 +1297,19 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             const uint32_t aLo = uint32_t(dA), aHi = uint32_t(dA >> 32), bLo = uint32_t(dB), bHi = uint32_t(dB >> 32);
             // Rolled issue loops: the issuer's code between two MMAs has to be fetched and issued while at most one
             // MMA is in flight, so the loops are kept to a handful of instructions and exist once per order.
+            const uint32_t tmemD = tmemHi + hb * NTK;
             auto issueHi = [&](uint32_t acc) {
               if constexpr (F16) {
                 uint32_t aj = aLo, bj = bLo;
 #pragma unroll 1
                 for (int j = 0; j < gN; ++j, aj += kStageU, bj += uint32_t(dil), acc = 1u)
-                  mmaF16W(tmemHi, aj, aHi, bj, bHi, kIdescF16, acc);
+                  mmaF16W(tmemD, aj, aHi, bj, bHi, kIdesc, acc);
               } else {
                 uint64_t dAh = dA, dBh = dB;
 #pragma unroll 1
                 for (int j = 0; j < gN; ++j, dAh += kStageU, dBh += uint32_t(dil), acc = 1u) {
-                  mmaTf32(tmemHi, dAh, dBh, kIdesc, acc);
-                  mmaTf32(tmemHi, dAh + kKsAU, dBh + ksBU, kIdesc, 1u);
+                  mmaTf32(tmemD, dAh, dBh, kIdesc, acc);
+                  mmaTf32(tmemD, dAh + kKsAU, dBh + ksBU, kIdesc, 1u);
                 }
               }
             };
@@ -1092,8 +1318,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 uint32_t aj = aLo, bj = bLo;
 #pragma unroll 1
                 for (int j = 0; j < gN; ++j, aj += kStageU, bj += uint32_t(dil), acc = 1u) {
-                  mmaF16W(tmemLo, aj + kLoAU, aHi, bj, bHi, kIdescF16, acc);
-                  mmaF16W(tmemLo, aj, aHi, bj + loBU, bHi, kIdescF16, 1u);
+                  mmaF16W(tmemLo, aj + kLoAU, aHi, bj, bHi, kIdesc, acc);
+                  mmaF16W(tmemLo, aj, aHi, bj + loBU, bHi, kIdesc, 1u);
                 }
               } else {
                 uint64_t dAh = dA, dBh = dB;
@@ -1112,7 +1338,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             if (nslot == wStages) nslot = 0, nph ^= 1;
             const bool lastRound = c == nChunks16 - 1 && gi == nTapGroups - 1;  // of the tile
             if (needLo) {  // first round of a tile: hi, then lo (Dhi is handed back before Dlo)
-              if (needHi && !waitT(hiEmpty, groupPar ^ 1, wHe, SLEEP_MMA_NS)) {
+              if (needHi && !waitT(&hiEmpty[hb], groupPar ^ 1, wHe, SLEEP_MMA_NS)) {
                 giveUp(4, 1);
                 dead = true;
                 break;
@@ -1132,7 +1358,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
               // the tile's lo chain is complete: the epilogue folds Dlo under the hi MMAs of this last round
               if (lastRound) mmaCommit(loFull);
               if (needHi) {
-                if (!waitT(hiEmpty, groupPar ^ 1, wHe, SLEEP_MMA_NS)) {
+                if (!waitT(&hiEmpty[hb], groupPar ^ 1, wHe, SLEEP_MMA_NS)) {
                   giveUp(4, 1);
                   dead = true;
                   break;
@@ -1150,10 +1376,14 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           if (dead) break;
           const bool lastChunk = c == nChunks16 - 1;
           // the hi chain of a drain group (drainN chunks, or what is left of the tile) is complete
-          if (g == drainN - 1 || lastChunk) mmaCommit(hiFull);
+          if (g == drainN - 1 || lastChunk) mmaCommit(&hiFull[hb]);
           mmaCommit(&bEmpty[buf]);  // activation buffer free once the MMAs have read it
           if (++buf == NB) buf = 0, bufPh ^= 1;
-          if (++g == drainN || lastChunk) g = 0, groupPar ^= 1;
+          if (++g == drainN || lastChunk) {
+            g = 0;
+            if (HB == 1 || hb == 1) groupPar ^= 1;
+            if (HB == 2) hb ^= 1;
+          }
         }
         tilePar ^= 1;
       }
@@ -1163,6 +1393,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
 
   tcFenceBefore();
+  if constexpr (SPLIT) {
+    if (warp >= EPI_WARPS) clusterSync();  // the epilogue warps' part of the first barrier is in their branch
+    clusterSync();                         // no CTA leaves while another reads its partial tile
+  }
   __syncthreads();
   if (warp == MMA_WARP) {
     tcFenceAfter();
@@ -1256,13 +1490,13 @@ static int rawHalf(int rows) { return (((rows + 3 + 1) / 2) + 3) & ~3; }
 
 // Dynamic shared memory of one CTA and the weight ring it leaves room for: the largest taps-per-slot (<= TAP_GROUP)
 // that still gives PREF_W_STAGES slots, else the deepest ring. Returns 0 when even single-tap slots do not fit.
-static size_t convTcSmemBytes(int64_t ci, int rows, int k, bool f16, int* wStages, int* wG) {
+static size_t convTcSmemBytes(bool split, int64_t ci, int rows, int k, bool f16, int* wStages, int* wG) {
   const int tap = f16 ? Fmt<true>::W_STAGE_BYTES : Fmt<false>::W_STAGE_BYTES;
   const int actRow = f16 ? Fmt<true>::ACT_BYTES_PER_ROW : Fmt<false>::ACT_BYTES_PER_ROW;
   const int nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
   const int half = rawHalf(rows);
   if (half > 256) return 0;
-  const SmemLayout base = smemLayout(int(ci), rows, half, nb, 0, 0, actRow, tap);
+  const SmemLayout base = smemLayout(split, int(ci), rows, half, nb, 0, 0, actRow, tap);
   if (base.total > uint32_t(kMaxSmem)) return 0;
   const size_t avail = size_t(kMaxSmem) - base.total;
   // Large groups matter more than a deep ring (measured: two slots of four taps beat four slots of three, and at
@@ -1281,7 +1515,7 @@ static size_t convTcSmemBytes(int64_t ci, int rows, int k, bool f16, int* wStage
   if (bestG == 0) return 0;
   if (wStages) *wStages = bestWs;
   if (wG) *wG = bestG;
-  return smemLayout(int(ci), rows, half, nb, bestWs, bestG, actRow, tap).total;
+  return smemLayout(split, int(ci), rows, half, nb, bestWs, bestG, actRow, tap).total;
 }
 
 // The hi chain between two drains holds at most MAX_CHAIN MMAs: whole chunks while they fit, and a chunk that alone
@@ -1294,7 +1528,7 @@ bool convTcEligible(const ConvFusedParams& p, bool f16) {
         chainOk(p.k, f16) && (p.k - 1) * p.dilation <= MAX_HALO && p.lo >= 1 && p.padding <= (1 << 20) && p.ci <= 4096 &&
         p.l < (int64_t(1) << 30)))
     return false;
-  return convTcSmemBytes(p.ci, NT + int((p.k - 1) * p.dilation), int(p.k), false, nullptr, nullptr) != 0;  // the larger format
+  return convTcSmemBytes(false, p.ci, NT + int((p.k - 1) * p.dilation), int(p.k), false, nullptr, nullptr) != 0;  // the larger format
 }
 
 int64_t convTcPackFloats(int64_t co, int64_t ci, int64_t k, bool f16) {
@@ -1388,27 +1622,44 @@ struct TcMaps {
   CUtensorMap x, res, out;
 };
 
-template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO>
+template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT>
 static int launchTc4(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cudaStream_t s) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
+  const auto kernel = convTcKernel<ACT, PARTIAL, TS, F16, TMAO, SPLIT>;
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(convTcKernel<ACT, PARTIAL, TS, F16, TMAO>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return failCuda("conv (tensor-core): cudaFuncSetAttribute", e);
     configured[dev] = true;
   }
-  convTcKernel<ACT, PARTIAL, TS, F16, TMAO><<<grid, NTHREADS, smem, s>>>(a, m.x, m.res, m.out);
+  if constexpr (SPLIT) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(a.split), attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(unsigned(grid)), cfg.blockDim = dim3(NTHREADS), cfg.dynamicSmemBytes = smem, cfg.stream = s;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, m.x, m.res, m.out);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return failCuda("conv (tensor-core)", e);
+    }
+  } else {
+    kernel<<<grid, NTHREADS, smem, s>>>(a, m.x, m.res, m.out);
+  }
   return launched("conv (tensor-core)");
 }
 
 template <int ACT, bool PARTIAL, int TS, bool F16>
 static int launchTc3(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cudaStream_t s) {
-  if constexpr (TS == 0 && !PARTIAL) {
-    if (a.tmaOut) return launchTc4<ACT, PARTIAL, TS, F16, true>(a, m, grid, smem, s);
+  if constexpr (F16) {  // the second half of a split tile handles every Co and alignment
+    if (a.split) return launchTc4<ACT, false, TS, F16, false, true>(a, m, grid, smem, s);
   }
-  return launchTc4<ACT, PARTIAL, TS, F16, false>(a, m, grid, smem, s);
+  if constexpr (TS == 0 && !PARTIAL) {
+    if (a.tmaOut) return launchTc4<ACT, PARTIAL, TS, F16, true, false>(a, m, grid, smem, s);
+  }
+  return launchTc4<ACT, PARTIAL, TS, F16, false, false>(a, m, grid, smem, s);
 }
 
 template <int ACT, bool PARTIAL, int TS = 0>
@@ -1442,14 +1693,37 @@ int convTcProfile(int enable, long long* out16) {
   return 0;
 }
 
+// CTAs per tile: 0 = the persistent form. The split form is taken where at least two CTAs per 128-column tile fit on the
+// launch's share of the SMs, all in one wave: there the time is one tile's chain of 16-channel chunks plus about 9 us of
+// fixed cost (launch, first loads, cluster reduction), and the chain shrinks with every CTA. With one CTA per tile
+// it gains little over 256-column tiles (an M128 N128 MMA takes about 0.8 of the time of an N256 one here) and doubles
+// the weight traffic; with a second wave it loses. Measured (us, persistent -> split): [256, 240] K = 11: 52 -> 15;
+// [256, 1210] K = 7: 49 -> 17; [128, 1441] K = 3: 29 -> 12; [1104 -> 1024, 61] K = 3: 130 -> 19; [256, 3200] K = 11, two
+// CTAs per tile: 52 -> 30, and with a second wave (four) 39.
+static int splitFor(const TcArgs& a, bool f16, int sms) {
+  if (!f16) return 0;
+  const int n = a.ci / KC;
+  int sp = int(sms / (ceilDiv(a.lo, NTS) * a.numCoBlk));
+  if (sp > MAX_SPLIT) sp = MAX_SPLIT;
+  if (sp > n) sp = n;
+  if (sp < 2) return 0;
+  const int serial = (n + sp - 1) / sp;
+  return (n + serial - 1) / serial;  // no more CTAs than shorten the longest run
+}
+
 // Launch geometry and tensor maps shared by the conv and ConvTranspose entry points.
-static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int* grid, size_t* smem) {
-  *smem = convTcSmemBytes(a.ci, a.rows, a.k, f16, &a.wStages, &a.wG);
-  LKC_REQUIRE(*smem != 0, "conv (tensor-core): window too large");
-  a.half = rawHalf(a.rows);
-  a.nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
+static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercent, int* grid, size_t* smem) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
+  a.split = splitFor(a, f16, d->smCount * smPercent / 100);
+  const int nt = a.split ? NTS : NT;
+  a.numTTiles = int(ceilDiv(a.lo, nt));
+  a.rows = nt + (a.k - 1) * a.dilation;
+  *smem = convTcSmemBytes(a.split != 0, a.ci, a.rows, a.k, f16, &a.wStages, &a.wG);
+  LKC_REQUIRE(*smem != 0, "conv (tensor-core): window too large");
+  if (a.split && *smem < SPLIT_SMEM) *smem = SPLIT_SMEM;
+  a.half = rawHalf(a.rows);
+  a.nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
   a.status = d->status;
   a.prof = (kProf && gProfileOn) ? d->prof : nullptr;
   // Dhi is drained into the f32 running sums after as many whole chunks as fit in MAX_CHAIN chained MMAs.
@@ -1461,7 +1735,7 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int* grid, s
   // chunk 17 % faster, the launch 4-7 %; at K = 7 the isolated layout is 3 % ahead).
   a.balanced = a.k * (f16 ? 3 : 6) <= 15 ? 1 : 0;
   const int tiles = a.numTTiles * a.numCoBlk;
-  *grid = tiles < d->smCount ? tiles : d->smCount;
+  *grid = a.split ? tiles * a.split : (tiles < d->smCount ? tiles : d->smCount);
   // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
   // argument: it stays zero-filled and is never dereferenced.
   std::memset(&m, 0, sizeof m);
@@ -1485,14 +1759,13 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
   a.xPitch = p.xPitch ? p.xPitch : p.l, a.resPitch = p.resPitch ? p.resPitch : p.lo;
   a.outPitch = p.outPitch ? p.outPitch : p.lo;
   a.slope = p.slope, a.outScale = p.outScale;
-  a.rows = NT + (a.k - 1) * a.dilation;
-  const int64_t tTiles = ceilDiv(p.lo, NT);
+  const int64_t tTiles = ceilDiv(p.lo, NTS);
   const int64_t coBlk = ceilDiv(p.co, MT);  // output channels past Co are zero rows of the pack and never stored
   LKC_REQUIRE(tTiles * coBlk < (1 << 30), "conv (tensor-core): too many tiles");
-  a.numTTiles = int(tTiles), a.numCoBlk = int(coBlk);
+  a.numCoBlk = int(coBlk);
   int grid = 0;
   size_t smem = 0;
-  if (int rc = finishArgs(a, m, f16, true, &grid, &smem)) return rc;
+  if (int rc = finishArgs(a, m, f16, true, p.smPercent, &grid, &smem)) return rc;
   switch (p.act) {
     case Act::None: return launchTc<0>(a, m, f16, grid, smem, s);
     case Act::Snake: return launchTc<1>(a, m, f16, grid, smem, s);
@@ -1505,7 +1778,7 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
 
 bool convtTcEligible(int64_t ci, int64_t co, int64_t k, int64_t stride, int64_t padding) {
   return (stride == 6 || stride == 10) && k == 2 * stride && 2 * padding == stride && ci % KC == 0 && ci >= KC &&
-         ci <= 4096 && co >= 1 && convTcSmemBytes(ci, NT + 2, 3, false, nullptr, nullptr) != 0;
+         ci <= 4096 && co >= 1 && convTcSmemBytes(false, ci, NT + 2, 3, false, nullptr, nullptr) != 0;
 }
 
 int64_t convtTcPackFloats(int64_t ci, int64_t co, int64_t stride, bool f16) {
@@ -1541,13 +1814,12 @@ int convtTc(const ConvtParams& p, const float* wp, bool f16, cudaStream_t s) {
   a.validLo = 0, a.validHi = lx;
   a.xPitch = p.xPitch ? p.xPitch : lx, a.resPitch = p.resPitch ? p.resPitch : lo, a.outPitch = p.outPitch ? p.outPitch : lo;
   a.slope = p.slope, a.outScale = 1.f;
-  a.rows = NT + 2;
-  const int64_t tTiles = ceilDiv(p.l, NT), coBlk = ceilDiv(p.co, 4 * (32 / p.stride));
+  const int64_t tTiles = ceilDiv(p.l, NTS), coBlk = ceilDiv(p.co, 4 * (32 / p.stride));
   LKC_REQUIRE(tTiles * coBlk < (1 << 30) && p.l < (int64_t(1) << 30), "conv_transpose1d_poly (tensor-core): too many tiles");
-  a.numTTiles = int(tTiles), a.numCoBlk = int(coBlk);
+  a.numCoBlk = int(coBlk);
   int grid = 0;
   size_t smem = 0;
-  if (int rc = finishArgs(a, m, f16, false, &grid, &smem)) return rc;
+  if (int rc = finishArgs(a, m, f16, false, p.smPercent, &grid, &smem)) return rc;
   if (p.stride == 6) return launchTc2<2, false, 6>(a, m, f16, grid, smem, s);
   return launchTc2<2, false, 10>(a, m, f16, grid, smem, s);
 }

@@ -62,6 +62,7 @@ struct ConvFusedParams {
   Act act = Act::None;
   float slope = 0.f, outScale = 1.f, inScale = 1.f;
   const void* state = nullptr;
+  int smPercent = 100;  // part of the device's SMs this launch may spread over (others run beside it)
 };
 
 // One fused conv, routed to the tensor-core kernel when the shape qualifies, else to the CUDA-core kernel (api.cu).
@@ -86,6 +87,7 @@ struct ConvtParams {
   // Window extension: x holds haloLeft / haloRight real columns before / after the l columns that produce output
   // (time-sharded tensors; the zero padding of the transposed conv then applies only where a halo is absent).
   int64_t haloLeft = 0, haloRight = 0;
+  int smPercent = 100;  // as in ConvFusedParams
 };
 bool convtTcEligible(int64_t ci, int64_t co, int64_t k, int64_t stride, int64_t padding);
 int64_t convtTcPackFloats(int64_t ci, int64_t co, int64_t stride, bool f16);

@@ -25,6 +25,12 @@ constexpr int kStreams = 5;  // the caller's stream and four side streams
 constexpr int kEvents = 12;  // joins of one forward
 constexpr size_t kPlans = 16;
 constexpr float kEps = 1e-5f;  // AdaIN
+// Percent of the SMs that one launch may spread over, as other branches run beside it (on one stream too, so that both
+// ways add the same partial sums): the k = 3, 7, 11 resblocks of a stage, and the two noise branches. The longer a
+// branch's chain, the more it gets; the first noise branch is waited for one stage earlier than the second. Measured,
+// microseconds per forward of T = 24 / 121 / 240 / 320 frames: no splitting 885 / 933 / 979 / 1057, all of the device for
+// every branch 512 / 854 / 972 / 1056, even parts 443 / 725 / 981 / 1057, these 443 / 701 / 904 / 1044.
+constexpr int kBranchSms[3] = {26, 36, 50}, kNoiseSms[2] = {70, 40};
 
 struct Plan {
   int64_t key = 0, bytes = 0, unplanned = 0;
@@ -127,14 +133,14 @@ const float* FP(const void* p) { return static_cast<const float*>(p); }
 // One fused conv of the tensor-core family, stride 1: act((x - mean) * scale + beta) -> conv -> + bias [+ residual].
 void conv(Exec& e, int s, Act act, Buf x, int64_t l, int64_t ci, int64_t co, int64_t k, int64_t d, int64_t pad,
           const void* w, const void* b, Buf affine, const void* alpha, float slope, const LkcConvState* state, Buf residual,
-          Buf out, Buf stats) {
+          Buf out, Buf stats, int smPercent) {
   e.launch(s, {x, affine, residual, out, stats}, [&](cudaStream_t st) {
     ConvFusedParams p;
     p.x = x.p, p.w = FP(w), p.bias = FP(b), p.affine = affine.p, p.alpha = FP(alpha), p.residual = residual.p;
     p.out = out.p, p.stats = stats.p;
     p.ci = ci, p.l = l, p.co = co, p.k = k, p.dilation = d, p.padding = pad, p.lo = l + 2 * pad - d * (k - 1);
     p.xPitch = x.pitch, p.resPitch = residual.pitch, p.outPitch = out.pitch;
-    p.act = act, p.slope = slope, p.state = state;
+    p.act = act, p.slope = slope, p.state = state, p.smPercent = smPercent;
     return convFused(p, st);
   });
 }
@@ -166,7 +172,7 @@ struct PlainResidual {
 // allocated here.
 template <class Residual>
 void resblock(Exec& e, int s, const LkcResblock& w, Buf x, Buf stats, int64_t l, Buf bank, Buf* out, Buf* outStats,
-              Residual residual) {
+              Residual residual, int smPercent) {
   static const int64_t dil[3] = {1, 3, 5};
   const int64_t c = w.c, k = w.k;
   const Buf none;
@@ -177,12 +183,14 @@ void resblock(Exec& e, int s, const LkcResblock& w, Buf x, Buf stats, int64_t l,
     const Buf res = last ? residual.make(x) : x;
     Buf af = affineOf(e, s, stats, bank, w.gb[i1], c, l);
     Buf xt = e.rows(s, c, l), st1 = statsBuf(e, s, c, l);
-    conv(e, s, Act::Snake, x, l, c, c, k, d, d * (k - 1) / 2, w.w[i1], w.b[i1], af, w.alpha[i1], 0.f, w.state[i1], none, xt, st1);
+    conv(e, s, Act::Snake, x, l, c, c, k, d, d * (k - 1) / 2, w.w[i1], w.b[i1], af, w.alpha[i1], 0.f, w.state[i1], none, xt, st1,
+         smPercent);
     af = affineOf(e, s, st1, bank, w.gb[i2], c, l);
     Buf xn = last && out->p ? *out : e.rows(s, c, l);
     Buf stn = last && outStats->p ? *outStats : statsBuf(e, s, c, l);
     if (last) residual.ready();
-    conv(e, s, Act::Snake, xt, l, c, c, k, 1, (k - 1) / 2, w.w[i2], w.b[i2], af, w.alpha[i2], 0.f, w.state[i2], res, xn, stn);
+    conv(e, s, Act::Snake, xt, l, c, c, k, 1, (k - 1) / 2, w.w[i2], w.b[i2], af, w.alpha[i2], 0.f, w.state[i2], res, xn, stn,
+         smPercent);
     x = xn, stats = stn;
   }
   *out = x, *outStats = stats;
@@ -248,9 +256,10 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
       return spaceToDepth(har.p, y.p, 22, len[1], n.rows, ly, har.pitch, y.pitch, n.stride, n.padding, st);
     });
     Buf xs = e.rows(s, ch[i], len[i]), xst = statsBuf(e, s, ch[i], len[i]);
-    conv(e, s, Act::None, y, ly, n.rows, ch[i], n.taps, 1, 0, n.w, n.b, none, nullptr, 0.f, n.state, none, xs, xst);
-    if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], AddUpsampled{e, u0, ch[0], len[0]});
-    else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], PlainResidual{});
+    conv(e, s, Act::None, y, ly, n.rows, ch[i], n.taps, 1, 0, n.w, n.b, none, nullptr, 0.f, n.state, none, xs, xst,
+         kNoiseSms[i]);
+    if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], AddUpsampled{e, u0, ch[0], len[0]}, kNoiseSms[i]);
+    else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], PlainResidual{}, kNoiseSms[i]);
   }
 
   Buf in = noise[0], inStats = noiseStats[0], mean;
@@ -264,7 +273,8 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
     e.join(3, 0), e.join(4, 0);
     Buf rb[3], st[3];
     for (int j = 2; j >= 0; --j)
-      resblock(e, j == 2 ? 0 : (j == 1 ? 3 : 4), m.res[3 * i + j], in, inStats, l, bank, &rb[j], &st[j], PlainResidual{});
+      resblock(e, j == 2 ? 0 : (j == 1 ? 3 : 4), m.res[3 * i + j], in, inStats, l, bank, &rb[j], &st[j], PlainResidual{},
+               kBranchSms[j]);
     e.join(0, 3), e.join(0, 4);
     mean = e.rows(0, c, l);
     e.launch(0, {rb[0], rb[1], rb[2], mean}, [&](cudaStream_t cs) {
@@ -276,7 +286,8 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
   if (io.post) post.p = static_cast<float*>(io.post), post.pitch = io.post_pitch;
   else post = e.rows(0, 22, len[1]);
   ident.p = const_cast<float*>(FP(m.ident128));
-  conv(e, 0, Act::Leaky, mean, len[1], 128, 22, 7, 1, 3, m.post_w, m.post_b, ident, nullptr, 0.01f, m.post_state, none, post, postStats);
+  conv(e, 0, Act::Leaky, mean, len[1], 128, 22, 7, 1, 3, m.post_w, m.post_b, ident, nullptr, 0.01f, m.post_state, none, post, postStats,
+       100);
   e.launch(0, {post}, [&](cudaStream_t st) {
     return istftLogits(post.p, static_cast<float*>(io.audio), len[1], post.pitch, 20, 5, st);
   });
@@ -390,7 +401,7 @@ void resblockCall(Exec& e, const LkcResblock& w, const LkcResblockIo& io) {
   outStats.p = static_cast<float*>(io.out_stats);
   if (io.stats) st.p = const_cast<float*>(FP(io.stats));
   else st = channelStatsOf(e, 0, x, w.c, io.l);
-  resblock(e, 0, w, x, st, io.l, bank, &out, &outStats, PlainResidual{});
+  resblock(e, 0, w, x, st, io.l, bank, &out, &outStats, PlainResidual{}, 100);
 }
 }  // namespace
 

@@ -114,6 +114,51 @@ def test_conv1d_fused(cuda, ci, co, l, k, d, variant):
         assert rel_l2(out, o2.cpu().numpy()) <= REL_L2
 
 
+# Few tiles: a cluster of CTAs shares a 128-column tile. (Ci, Co, L, K, dilation): three and five channel chunks (CTAs with
+# unequal shares, rows that do not divide evenly), a second output block of one row, one column, one column past a tile,
+# Ci far above Co, and on a 148-SM device the last length with two CTAs per tile and the first without.
+SPLIT_CASES = [(48, 129, 129, 3, 1), (80, 128, 257, 5, 2), (112, 256, 1, 7, 1), (16, 22, 127, 1, 1), (1104, 64, 97, 3, 1),
+               (128, 128, 9472, 3, 1), (128, 128, 9473, 3, 1)]
+
+
+@pytest.mark.parametrize("ci,co,l,k,d", SPLIT_CASES)
+@pytest.mark.parametrize("padded", [False, True])
+def test_conv1d_few_tiles(cuda, ci, co, l, k, d, padded):
+    """Channels of a tile contracted by several CTAs, on both row layouts, with residual and scale: against the float64
+    oracle with the bars of test_conv1d_fused, and twice the same bits (the partial sums are added in a fixed order)."""
+    from lokinfer_b200 import ops
+    x, w, b, affine, _, res = synth.conv_case(ci, co, l, k, ci * 31 + l + k)
+    pad = d * (k - 1) // 2
+    res = np.ascontiguousarray(res[:, :l])
+    dx, dw, db, daf, dres = dev(cuda, x, w, b, affine, res)
+    if padded:
+        dx, dres = _pitched(dx), _pitched(dres)
+    kw = dict(slope=0.2, residual=dres, out_scale=0.7071067811865476, padding=pad, dilation=d,
+              state=ops.conv1d_prepare_f32_cuda(dw))
+    with ops.padded_rows(padded):
+        out, stats = ops.conv1d_leaky_f32_cuda(dx, dw, db, daf, **kw)
+        again, _ = ops.conv1d_leaky_f32_cuda(dx, dw, db, daf, **kw)
+    assert torch.equal(out, again)
+
+    def oracle(dt):
+        a = [O.T(v, dt) for v in (x, w, b, affine, res)]
+        return O.conv1d_fused(a[0], a[1], a[2], a[3], "leaky", slope=0.2, residual=a[4], out_scale=0.7071067811865476,
+                              padding=pad, dilation=d)[0].numpy()
+
+    out, ref64 = out.cpu().numpy(), oracle(torch.float64)
+    assert rel_l2(out, ref64) <= 2 * rel_l2(oracle(torch.float32), ref64) + 2e-7
+    check_stats(stats.cpu().numpy(), out)
+    assert ops.conv_tc_status() == 0
+
+
+def _pitched(t):
+    """The same values as a [:, :L] view of rows padded to a multiple of four floats."""
+    c, l = t.shape
+    buf = torch.full((c, -(-l // 4) * 4), 7.0, device=t.device)
+    buf[:, :l] = t
+    return buf[:, :l]
+
+
 # Shapes for the padded-row (TMA) route: partial last tile, exact tile multiples, windows that start before the row
 # and end after it, odd lengths (pitch = L rounded up to 4), both stage shapes of the 26 s case, several tiles per CTA.
 TMA_CASES = [(128, 128, 1201, 3, 1), (128, 128, 1203, 7, 3), (128, 128, 5000, 11, 5), (256, 256, 641, 11, 5),
