@@ -44,36 +44,43 @@ class Decoder:
                         [w[name + ".pool.weight"], torch.zeros(z, 1, 3, device=self.device)], 0).contiguous()
                     w[name + ".pool.bias"] = torch.cat([w[name + ".pool.bias"], torch.zeros(z, device=self.device)])
             self.gb_pad[name] = cp - cin
-            for conv in (".conv1", ".conv2"):
+            for conv in (".conv1", ".conv2") + ((".conv1x1",) if cin != cout else ()):
                 self.state[name + conv] = ops.conv1d_prepare_f32_cuda(w[name + conv + ".weight"])
+            if cin != cout:
+                w[name + ".conv1x1.bias"] = torch.zeros(cout, device=self.device)
+        self.state["decoder.asr_res.0"] = ops.conv1d_prepare_f32_cuda(w["decoder.asr_res.0.weight"])
         # style bank: every `<name>.fc` of the decoder as one GEMV (models/kokoro/model.py:67-81, names sorted)
         names = sorted(k[: -len(".weight")] for k in w if k.endswith(".fc.weight"))
-        self.bank_wt = torch.cat([w[n + ".weight"].t() for n in names], dim=1).contiguous()
-        self.bank_b = torch.cat([w[n + ".bias"] for n in names]).contiguous()
-        self.bank_off, o = {}, 0
+        # The (gamma | beta) of a norm1 carry their zeros for the appended rows: gamma, zeros, beta, zeros.
+        self.bank_off, o, wt, bias = {}, 0, [], []
         for n in names:
-            self.bank_off[n] = (o, int(w[n + ".bias"].shape[0]))
+            pad = self.gb_pad.get(n[: -len(".norm1.fc")], 0) if n.endswith(".norm1.fc") else 0
+            for t, parts in ((w[n + ".weight"], wt), (w[n + ".bias"], bias)):
+                c = int(t.shape[0]) // 2
+                z = torch.zeros(pad, *t.shape[1:], device=self.device)
+                parts += [t[:c], z, t[c:], z]
+            self.bank_off[n] = (o, int(w[n + ".bias"].shape[0]) + 2 * pad)
             o += self.bank_off[n][1]
-        self._ident = {}
+        self.bank_wt = torch.cat(wt).t().contiguous()
+        self.bank_b = torch.cat(bias).contiguous()
+        self._ident = {c: torch.stack([torch.zeros(c), torch.ones(c), torch.zeros(c)]).to(self.device).contiguous()
+                       for c in {512} | {_pad16(cin) for _, cin, _, _ in DECODER_BLOCKS}}
 
     def _style(self, s):
         bank = ops.gemm_bias_f32_cuda(s.reshape(1, -1), self.bank_wt, self.bank_b).reshape(-1)
 
-        def gb(name, pad=0):
+        def gb(name):
             o, n = self.bank_off[name]
-            v = bank[o: o + n]
-            if pad:  # (gamma | beta) of the appended zero rows: zeros
-                c = n // 2
-                z = torch.zeros(pad, device=self.device)
-                v = torch.cat([v[:c], z, v[c:], z])
-            return v.contiguous()
+            return bank[o: o + n]
 
         return gb
 
-    def _identity(self, c):
-        if c not in self._ident:
-            self._ident[c] = torch.stack([torch.zeros(c), torch.ones(c), torch.zeros(c)]).to(self.device).contiguous()
-        return self._ident[c]
+    def _conv1x1(self, x, name):
+        """Pointwise conv on the tensor cores (K = 1, identity affine): the CUDA-core kernel's one serial chain over up to
+        1104 input channels took 150-340 us whatever the length, this takes 10-35 us."""
+        w = self.w
+        return ops.conv1d_affine_f32_cuda(x, w[name + ".weight"], w[name + ".bias"], self._ident[int(x.shape[0])],
+                                          state=self.state[name])[0]
 
     def _concat(self, parts, cin):
         """concat_rows of the block input, with zero rows up to the next multiple of 16 channels."""
@@ -84,8 +91,8 @@ class Decoder:
 
     def adain_resblk(self, x, gb, name, cin, cout, upsample):
         """AdainResBlk1d through the basic ops (models/kokoro/model.py:158-174). x carries the padded rows."""
-        w, pad = self.w, self.gb_pad[name]
-        r = ops.leaky_relu_f32_cuda(ops.adain1d_f32_cuda(x, gb(name + ".norm1.fc", pad)), slope=0.2)
+        w = self.w
+        r = ops.leaky_relu_f32_cuda(ops.adain1d_f32_cuda(x, gb(name + ".norm1.fc")), slope=0.2)
         if upsample:
             r = ops.conv_transpose1d_dw_f32_cuda(r, w[name + ".pool.weight"], w[name + ".pool.bias"], stride=2,
                                                  padding=1, output_padding=1)
@@ -99,23 +106,23 @@ class Decoder:
 
     def adain_resblk_fused(self, x, gb, name, cin, cout, upsample):
         """The block through the fused conv kernels (models/kokoro/model.py:205-221)."""
-        w, pad = self.w, self.gb_pad[name]
-        gb1 = gb(name + ".norm1.fc", pad)
+        w = self.w
+        gb1 = gb(name + ".norm1.fc")
         af = ops.adain_affine_f32_cuda(ops.channel_stats_f32_cuda(x), gb1, length=int(x.shape[1]))
         if upsample:
             r = ops.leaky_relu_f32_cuda(ops.adain1d_f32_cuda(x, gb1), slope=0.2)
             r = ops.conv_transpose1d_dw_f32_cuda(r, w[name + ".pool.weight"], w[name + ".pool.bias"], stride=2,
                                                  padding=1, output_padding=1)
             h, st = ops.conv1d_affine_f32_cuda(r, w[name + ".conv1.weight"], w[name + ".conv1.bias"],
-                                               self._identity(int(x.shape[0])), padding=1,
+                                               self._ident[int(x.shape[0])], padding=1,
                                                state=self.state[name + ".conv1"])
         else:
             h, st = ops.conv1d_leaky_f32_cuda(x, w[name + ".conv1.weight"], w[name + ".conv1.bias"], af, slope=0.2,
                                               padding=1, state=self.state[name + ".conv1"])
         af = ops.adain_affine_f32_cuda(st, gb(name + ".norm2.fc"), length=int(h.shape[1]))
-        sc = ops.upsample_nearest1d_f32_cuda(x, scale=2) if upsample else x
-        if cin != cout:
-            sc = ops.conv1d_nobias_f32_cuda(sc, w[name + ".conv1x1.weight"])
+        sc = self._conv1x1(x, name + ".conv1x1") if cin != cout else x
+        if upsample:  # nearest neighbour: the same values on either side of a pointwise conv, at half the columns
+            sc = ops.upsample_nearest1d_f32_cuda(sc, scale=2)
         out, _ = ops.conv1d_leaky_f32_cuda(h, w[name + ".conv2.weight"], w[name + ".conv2.bias"], af, slope=0.2,
                                            residual=sc, out_scale=SQRT1_2, padding=1,
                                            state=self.state[name + ".conv2"])
@@ -137,7 +144,10 @@ class Decoder:
         blk = self.adain_resblk_fused if fused else self.adain_resblk
         name, cin, cout, up = DECODER_BLOCKS[0]
         x = blk(self._concat([asr, f0d, nd], cin), gb, name, cin, cout, up)
-        asr_res = ops.conv1d_f32_cuda(asr, w["decoder.asr_res.0.weight"], w["decoder.asr_res.0.bias"])
+        if fused:
+            asr_res = self._conv1x1(asr, "decoder.asr_res.0")
+        else:
+            asr_res = ops.conv1d_f32_cuda(asr, w["decoder.asr_res.0.weight"], w["decoder.asr_res.0.bias"])
         for name, cin, cout, up in DECODER_BLOCKS[1:]:
             x = blk(self._concat([x, asr_res, f0d, nd], cin), gb, name, cin, cout, up)
         return x
