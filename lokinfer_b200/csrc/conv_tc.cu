@@ -138,6 +138,8 @@ __host__ __device__ inline SmemLayout smemLayout(bool split, int ci, int rows, i
 
 struct TcArgs {
   const float *x, *wp, *bias, *affine, *alpha, *residual;
+  const float *statsIn, *gb;  // split form: the AdaIN affine of x is computed here from its chunk statistics (null: `affine`)
+  float eps;
   float *out, *stats;
   int ci, co, k, dilation, padding;
   int64_t l, lo, nchunks;
@@ -1042,7 +1044,43 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const bool tmaIn = a.tmaIn != 0;
     const int runSkip = (KC - 1) * half;  // a raw window index i >= half sits in the second run: + runSkip floats
     // per-channel parameters, once: sPar = [mean | a | b | inv] with a = scale, b = beta (x alpha for Snake), inv = 1/alpha
-    for (int c = cBegin * KC + pw * 32 + lane; c < (cBegin + nChunks16) * KC; c += PRO_WARPS * 32) {
+    // Split form with statsIn: each CTA folds the chunk statistics of its own channels into mean / scale / beta, with the
+    // arithmetic of adainAffineKernel (Chan combine in double), four lanes per channel. A launch of its own costs
+    // 3.5 us plus a gap in front of every conv; here it is one round of loads under the first weight and input copies.
+    const bool fold = SPLIT && a.statsIn != nullptr;
+    if constexpr (SPLIT) {
+      if (fold) {
+        const int64_t nch = (a.l + 127) / 128;
+        const double nT = 128.0, nLast = double(a.l - (nch - 1) * 128);
+        const int cEnd = (cBegin + nChunks16) * KC, sub = lane & 3;
+        for (int c0 = cBegin * KC + pw * 8; c0 < cEnd; c0 += PRO_WARPS * 8) {  // warp-uniform; KC is a multiple of 8
+          const int c = c0 + (lane >> 2);
+          const float2* st = reinterpret_cast<const float2*>(a.statsIn) + int64_t(c) * nch;  // 8-byte aligned, as adain_affine wants
+          double sum = 0.0, m2 = 0.0;
+#pragma unroll 4
+          for (int64_t t = sub; t < nch; t += 4) sum += double(st[t].x) * (t + 1 < nch ? nT : nLast);
+          sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+          sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+          const double mean = sum / double(a.l);
+#pragma unroll 4
+          for (int64_t t = sub; t < nch; t += 4) {
+            const float2 v = st[t];
+            const double dm = double(v.x) - mean;
+            m2 += double(v.y) + (t + 1 < nch ? nT : nLast) * dm * dm;
+          }
+          m2 += __shfl_xor_sync(0xffffffffu, m2, 1);
+          m2 += __shfl_xor_sync(0xffffffffu, m2, 2);
+          if (sub == 0) {
+            const float var = float(m2 / double(a.l)), al = ACT == 1 ? a.alpha[c] : 1.f;
+            sPar[c] = float(mean);
+            sPar[a.ci + c] = (1.f + a.gb[c]) * (1.0f / sqrtf(var + a.eps)) * al;
+            sPar[2 * a.ci + c] = a.gb[a.ci + c] * al;
+            sPar[3 * a.ci + c] = 1.f / al;
+          }
+        }
+      }
+    }
+    for (int c = cBegin * KC + pw * 32 + lane; !fold && c < (cBegin + nChunks16) * KC; c += PRO_WARPS * 32) {
       const float al = ACT == 1 ? a.alpha[c] : 1.f;
       sPar[c] = a.affine ? a.affine[c] : 0.f;
       sPar[a.ci + c] = (a.affine ? a.affine[a.ci + c] : 1.f) * al;
@@ -1700,10 +1738,10 @@ int convTcProfile(int enable, long long* out16) {
 // the weight traffic; with a second wave it loses. Measured (us, persistent -> split): [256, 240] K = 11: 52 -> 15;
 // [256, 1210] K = 7: 49 -> 17; [128, 1441] K = 3: 29 -> 12; [1104 -> 1024, 61] K = 3: 130 -> 19; [256, 3200] K = 11, two
 // CTAs per tile: 52 -> 30, and with a second wave (four) 39.
-static int splitFor(const TcArgs& a, bool f16, int sms) {
+static int splitFor(bool f16, int ci, int64_t lo, int coBlocks, int sms) {
   if (!f16) return 0;
-  const int n = a.ci / KC;
-  int sp = int(sms / (ceilDiv(a.lo, NTS) * a.numCoBlk));
+  const int n = ci / KC;
+  int sp = int(sms / (ceilDiv(lo, NTS) * coBlocks));
   if (sp > MAX_SPLIT) sp = MAX_SPLIT;
   if (sp > n) sp = n;
   if (sp < 2) return 0;
@@ -1715,7 +1753,8 @@ static int splitFor(const TcArgs& a, bool f16, int sms) {
 static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercent, int* grid, size_t* smem) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
-  a.split = splitFor(a, f16, d->smCount * smPercent / 100);
+  a.split = splitFor(f16, a.ci, a.lo, a.numCoBlk, d->smCount * smPercent / 100);
+  LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
   const int nt = a.split ? NTS : NT;
   a.numTTiles = int(ceilDiv(a.lo, nt));
   a.rows = nt + (a.k - 1) * a.dilation;
@@ -1747,6 +1786,12 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercen
   return 0;
 }
 
+bool convTcSplits(const ConvFusedParams& p, bool f16) {
+  const DeviceInfo* d = nullptr;
+  return deviceInfo(&d) == 0 &&
+         splitFor(f16, int(p.ci), p.lo, int(ceilDiv(p.co, MT)), d->smCount * p.smPercent / 100) != 0;
+}
+
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {
   TcArgs a;
   TcMaps m;
@@ -1759,6 +1804,7 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
   a.xPitch = p.xPitch ? p.xPitch : p.l, a.resPitch = p.resPitch ? p.resPitch : p.lo;
   a.outPitch = p.outPitch ? p.outPitch : p.lo;
   a.slope = p.slope, a.outScale = p.outScale;
+  a.statsIn = p.statsIn, a.gb = p.gb, a.eps = p.eps;
   const int64_t tTiles = ceilDiv(p.lo, NTS);
   const int64_t coBlk = ceilDiv(p.co, MT);  // output channels past Co are zero rows of the pack and never stored
   LKC_REQUIRE(tTiles * coBlk < (1 << 30), "conv (tensor-core): too many tiles");
@@ -1814,6 +1860,7 @@ int convtTc(const ConvtParams& p, const float* wp, bool f16, cudaStream_t s) {
   a.validLo = 0, a.validHi = lx;
   a.xPitch = p.xPitch ? p.xPitch : lx, a.resPitch = p.resPitch ? p.resPitch : lo, a.outPitch = p.outPitch ? p.outPitch : lo;
   a.slope = p.slope, a.outScale = 1.f;
+  a.statsIn = nullptr, a.gb = nullptr, a.eps = 0.f;
   const int64_t tTiles = ceilDiv(p.l, NTS), coBlk = ceilDiv(p.co, 4 * (32 / p.stride));
   LKC_REQUIRE(tTiles * coBlk < (1 << 30) && p.l < (int64_t(1) << 30), "conv_transpose1d_poly (tensor-core): too many tiles");
   a.numCoBlk = int(coBlk);

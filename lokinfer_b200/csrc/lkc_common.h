@@ -63,10 +63,16 @@ struct ConvFusedParams {
   float slope = 0.f, outScale = 1.f, inScale = 1.f;
   const void* state = nullptr;
   int smPercent = 100;  // part of the device's SMs this launch may spread over (others run beside it)
+  // Instead of `affine`, where convFoldsAffine: chunk statistics [ci, ceil(l / 128), 2] of x and the (gamma | beta) of its
+  // AdaIN; the conv computes the affine itself.
+  const float *statsIn = nullptr, *gb = nullptr;
+  float eps = 0.f;
 };
 
 // One fused conv, routed to the tensor-core kernel when the shape qualifies, else to the CUDA-core kernel (api.cu).
 int convFused(const ConvFusedParams& p, cudaStream_t s);
+// Whether that route takes p.statsIn / p.gb instead of p.affine (the tensor-core kernel's split form).
+bool convFoldsAffine(const ConvFusedParams& p);
 // CUDA-core implicit-GEMM conv for any shape (conv_simt.cu). stride > 1 only for the plain conv1d.
 int convSimt(const ConvFusedParams& p, int64_t stride, cudaStream_t s);
 
@@ -97,6 +103,7 @@ int convtTc(const ConvtParams& p, const float* wp, bool f16, cudaStream_t s);
 bool convPathForcedSimt();
 bool convPackF16();  // operand format new packs are made in (lkc_set_conv_path)
 bool convTcEligible(const ConvFusedParams& p, bool f16);
+bool convTcSplits(const ConvFusedParams& p, bool f16);  // of an eligible conv
 int64_t convTcPackFloats(int64_t co, int64_t ci, int64_t k, bool f16);
 int convTcPack(const float* w, float* wp, int64_t co, int64_t ci, int64_t k, bool f16, cudaStream_t s);
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s);

@@ -145,11 +145,24 @@ void conv(Exec& e, int s, Act act, Buf x, int64_t l, int64_t ci, int64_t co, int
   });
 }
 
-// gb = this AdaIN's (gamma | beta) inside the style bank.
-Buf affineOf(Exec& e, int s, Buf stats, Buf bank, int64_t gb, int64_t c, int64_t l) {
-  Buf af = e.alloc(s, 3 * c);
-  e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, bank.p + gb, af.p, c, l, kEps, st); });
-  return af;
+// AdaIN -> Snake -> conv [+ residual] of a resblock, c -> c channels of the same length. gb = this AdaIN's (gamma | beta)
+// inside the style bank. The affine is a launch of its own unless the conv's route folds the statistics itself; the
+// plan reserves it either way, as the route may change between two calls (set_conv_path).
+void adainConv(Exec& e, int s, Buf x, Buf stats, int64_t l, int64_t c, int64_t k, int64_t d, const LkcResblock& w, int i,
+               Buf bank, Buf residual, Buf out, Buf outStats, int smPercent) {
+  const Buf af = e.alloc(s, 3 * c);
+  ConvFusedParams p;
+  p.x = x.p, p.w = FP(w.w[i]), p.bias = FP(w.b[i]), p.affine = af.p, p.alpha = FP(w.alpha[i]), p.residual = residual.p;
+  p.out = out.p, p.stats = outStats.p;
+  p.ci = c, p.l = l, p.co = c, p.k = k, p.dilation = d, p.padding = d * (k - 1) / 2, p.lo = l;
+  p.xPitch = x.pitch, p.resPitch = residual.pitch, p.outPitch = out.pitch;
+  p.act = Act::Snake, p.state = w.state[i], p.smPercent = smPercent;
+  const float* gb = bank.p + w.gb[i];
+  if (e.running() && convFoldsAffine(p))
+    p.statsIn = stats.p, p.gb = gb, p.eps = kEps;
+  else
+    e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, c, l, kEps, st); });
+  e.launch(s, {x, stats, bank, af, residual, out, outStats}, [&](cudaStream_t st) { return convFused(p, st); });
 }
 
 Buf statsBuf(Exec& e, int s, int64_t c, int64_t l) { return e.alloc(s, c * statChunks(l) * 2); }
@@ -181,16 +194,12 @@ void resblock(Exec& e, int s, const LkcResblock& w, Buf x, Buf stats, int64_t l,
     const int i1 = 2 * j, i2 = 2 * j + 1;
     const bool last = j == 2;
     const Buf res = last ? residual.make(x) : x;
-    Buf af = affineOf(e, s, stats, bank, w.gb[i1], c, l);
     Buf xt = e.rows(s, c, l), st1 = statsBuf(e, s, c, l);
-    conv(e, s, Act::Snake, x, l, c, c, k, d, d * (k - 1) / 2, w.w[i1], w.b[i1], af, w.alpha[i1], 0.f, w.state[i1], none, xt, st1,
-         smPercent);
-    af = affineOf(e, s, st1, bank, w.gb[i2], c, l);
+    adainConv(e, s, x, stats, l, c, k, d, w, i1, bank, none, xt, st1, smPercent);
     Buf xn = last && out->p ? *out : e.rows(s, c, l);
     Buf stn = last && outStats->p ? *outStats : statsBuf(e, s, c, l);
     if (last) residual.ready();
-    conv(e, s, Act::Snake, xt, l, c, c, k, 1, (k - 1) / 2, w.w[i2], w.b[i2], af, w.alpha[i2], 0.f, w.state[i2], res, xn, stn,
-         smPercent);
+    adainConv(e, s, xt, st1, l, c, k, 1, w, i2, bank, res, xn, stn, smPercent);
     x = xn, stats = stn;
   }
   *out = x, *outStats = stats;
