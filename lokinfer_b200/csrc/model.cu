@@ -26,11 +26,12 @@ constexpr int kEvents = 12;  // joins of one forward
 constexpr size_t kPlans = 16;
 constexpr float kEps = 1e-5f;  // AdaIN
 // Percent of the SMs that one launch may spread over, as other branches run beside it (on one stream too, so that both
-// ways add the same partial sums): the k = 3, 7, 11 resblocks of a stage, and the two noise branches. The longer a
-// branch's chain, the more it gets; the first noise branch is waited for one stage earlier than the second. Measured,
-// microseconds per forward of T = 24 / 121 / 240 / 320 frames: no splitting 885 / 933 / 979 / 1057, all of the device for
-// every branch 512 / 854 / 972 / 1056, even parts 443 / 725 / 981 / 1057, these 443 / 701 / 904 / 1044.
-constexpr int kBranchSms[3] = {26, 36, 50}, kNoiseSms[2] = {70, 40};
+// ways add the same partial sums): [stage] the k = 3, 7, 11 resblocks, and the two noise branches. The longer a branch's
+// chain, the more it gets; the first noise branch is waited for one stage earlier than the second. Measured, microseconds
+// per forward of T = 24 / 121 / 240 / 320 / 400 frames: no splitting 877 / 934 / 980 / 1054 / 1086; noise branches and
+// k = 7, 11 even 400 / 734 / 979 / 1052 / 1088; k = 11 at 50 in both stages 400 / 697 / 915 / 1055 / 1086, at 70 in both
+// 432 / 713 / 853 / 1011 / 1076 (stage 0 of T = 240 and 320 gains, stage 1 of T = 24 loses).
+constexpr int kBranchSms[2][3] = {{26, 36, 70}, {26, 36, 50}}, kNoiseSms[2] = {70, 40};
 
 struct Plan {
   int64_t key = 0, bytes = 0, unplanned = 0;
@@ -283,7 +284,7 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
     Buf rb[3], st[3];
     for (int j = 2; j >= 0; --j)
       resblock(e, j == 2 ? 0 : (j == 1 ? 3 : 4), m.res[3 * i + j], in, inStats, l, bank, &rb[j], &st[j], PlainResidual{},
-               kBranchSms[j]);
+               kBranchSms[i][j]);
     e.join(0, 3), e.join(0, 4);
     mean = e.rows(0, c, l);
     e.launch(0, {rb[0], rb[1], rb[2], mean}, [&](cudaStream_t cs) {
