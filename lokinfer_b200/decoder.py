@@ -77,7 +77,7 @@ class Decoder:
 
     def _conv1x1(self, x, name):
         """Pointwise conv on the tensor cores (K = 1, identity affine): the CUDA-core kernel's one serial chain over up to
-        1104 input channels took 150-340 us whatever the length, this takes 10-35 us."""
+        1104 input channels took 150-340 us whatever the length, this takes 12-40 us (F = 61 / 1040)."""
         w = self.w
         return ops.conv1d_affine_f32_cuda(x, w[name + ".weight"], w[name + ".bias"], self._ident[int(x.shape[0])],
                                           state=self.state[name])[0]
