@@ -24,6 +24,16 @@ def _pad16(c: int) -> int:
     return -(-c // 16) * 16
 
 
+def _prepare_f32_range(w):
+    """A conv state in the tf32 operand format, which has the range of f32: for convs whose input is not normalised."""
+    path = ops._conv_path
+    ops.set_conv_path("tf32")
+    try:
+        return ops.conv1d_prepare_f32_cuda(w)
+    finally:
+        ops.set_conv_path(path)
+
+
 class Decoder:
     def __init__(self, sd: dict, device="cuda"):
         self.device = torch.device(device)
@@ -44,11 +54,12 @@ class Decoder:
                         [w[name + ".pool.weight"], torch.zeros(z, 1, 3, device=self.device)], 0).contiguous()
                     w[name + ".pool.bias"] = torch.cat([w[name + ".pool.bias"], torch.zeros(z, device=self.device)])
             self.gb_pad[name] = cp - cin
-            for conv in (".conv1", ".conv2") + ((".conv1x1",) if cin != cout else ()):
+            for conv in (".conv1", ".conv2"):
                 self.state[name + conv] = ops.conv1d_prepare_f32_cuda(w[name + conv + ".weight"])
             if cin != cout:
+                self.state[name + ".conv1x1"] = _prepare_f32_range(w[name + ".conv1x1.weight"])
                 w[name + ".conv1x1.bias"] = torch.zeros(cout, device=self.device)
-        self.state["decoder.asr_res.0"] = ops.conv1d_prepare_f32_cuda(w["decoder.asr_res.0.weight"])
+        self.state["decoder.asr_res.0"] = _prepare_f32_range(w["decoder.asr_res.0.weight"])
         # style bank: every `<name>.fc` of the decoder as one GEMV (models/kokoro/model.py:67-81, names sorted)
         names = sorted(k[: -len(".weight")] for k in w if k.endswith(".fc.weight"))
         # The (gamma | beta) of a norm1 carry their zeros for the appended rows: gamma, zeros, beta, zeros.
@@ -76,8 +87,9 @@ class Decoder:
         return gb
 
     def _conv1x1(self, x, name):
-        """Pointwise conv on the tensor cores (K = 1, identity affine): the CUDA-core kernel's one serial chain over up to
-        1104 input channels took 150-340 us whatever the length, this takes 12-40 us (F = 61 / 1040)."""
+        """Pointwise conv on the tensor cores (K = 1, identity affine). The CUDA-core kernel's one serial chain over up
+        to 1104 input channels took 150-340 us at any length. The input is raw features, so the operands are tf32
+        halves: the f16 halves of the other convs would limit its range."""
         w = self.w
         return ops.conv1d_affine_f32_cuda(x, w[name + ".weight"], w[name + ".bias"], self._ident[int(x.shape[0])],
                                           state=self.state[name])[0]
