@@ -232,7 +232,8 @@ class Generator:
 
     def adain_resblock1_fused(self, x, gb, prefix, k, x_stats=None):
         n = x.shape[1]
-        if isinstance(gb, StyleBank) and not ops.op_by_op() and x.is_cuda:
+        # the block's offsets are this generator's: a bank of another one (a subset of the same state dict, say) has its own
+        if isinstance(gb, StyleBank) and gb.off is self.bank_off and not ops.op_by_op() and x.is_cuda:
             blk = self._block(prefix, k)
             ops._f32(x, *([] if x_stats is None else [x_stats]))
             if blk is not None and tuple(x.shape) == (blk.c, n) and (

@@ -242,3 +242,19 @@ def test_synthesis_pipeline_matches_synthesize(cuda, gen):
     for o, w in zip(outs, want):
         np.testing.assert_array_equal(o.numpy(), w)
     assert not np.array_equal(want[0], want[1])
+
+
+def test_style_bank_of_another_generator(cuda, gen):
+    """A block of a generator made from a subset of the state dict, with the full model's style bank: the offsets are the
+    bank's own. Same bits as the block run op by op."""
+    from lokinfer_b200 import Generator, ops
+    full = synth.generator_weights(0)
+    part = Generator({n: v for n, v in full.items() if n.startswith("resblocks.4.")}, cuda)
+    s, x = torch.randn(128, device=cuda), torch.randn(128, 1201, device=cuda)
+    bank = gen.style(s)
+    assert part.bank_off["resblocks.4.adain1.0.fc"] != bank.off["resblocks.4.adain1.0.fc"]
+    out, st = part.adain_resblock1_fused(x, bank, "resblocks.4", 7)
+    ref, rst = part.adain_resblock1_fused(x, lambda name: bank(name), "resblocks.4", 7)
+    assert torch.equal(out, ref) and torch.equal(st, rst)
+    own, _ = gen.adain_resblock1_fused(x, bank, "resblocks.4", 7)
+    assert rel_l2(out.cpu().numpy(), own.cpu().numpy()) <= REL_L2
