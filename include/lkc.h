@@ -298,8 +298,8 @@ typedef struct LkcGeneratorIo {
   int64_t launches; /* out: kernels queued */
 } LkcGeneratorIo;
 typedef struct LkcResblockIo {
-  const void *x, *stats, *bank; /* f32[C, l]; chunk statistics of x or NULL; style bank */
-  void *out, *out_stats;        /* f32[C, l], f32[C, ceil(l / 128), 2] */
+  const void *x, *stats, *bank; /* f32[C, l]; chunk statistics of x or NULL (8-byte aligned); style bank: gb[i] + 2 C floats */
+  void *out, *out_stats;        /* f32[C, l], f32[C, ceil(l / 128), 2] (8-byte aligned) */
   int64_t l, x_pitch, out_pitch;
   void* workspace; /* NULL: only workspace_bytes is set, nothing is queued */
   int64_t workspace_bytes;

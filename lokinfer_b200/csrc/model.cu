@@ -419,6 +419,9 @@ extern "C" LKC_API int lkc_resblock(const LkcResblock* w, LkcResblockIo* io, voi
   LKC_REQUIRE(w && io && resblockOk(*w) && io->l >= 1, "resblock: bad argument");
   LKC_REQUIRE(io->x && io->bank && io->out && io->out_stats, "resblock: null operand");
   LKC_REQUIRE(io->x_pitch >= io->l && io->out_pitch >= io->l, "resblock: a row pitch is smaller than the row");
+  LKC_REQUIRE(w->c <= 65535, "resblock: too many channels");  // channel_stats: one grid row per channel
+  LKC_REQUIRE(((reinterpret_cast<uintptr_t>(io->stats) | reinterpret_cast<uintptr_t>(io->out_stats)) & 7) == 0,
+              "resblock: stats and out_stats must be 8-byte aligned");
   Plan p;
   Exec plan(false);
   resblockCall(plan, *w, *io);

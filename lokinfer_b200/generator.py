@@ -224,6 +224,19 @@ class Generator:
         ops.count_launches(io.launches)
         return out, stats
 
+    def _takes_block(self, x, gb, x_stats):
+        """Whether the whole-block call may have these operands, whose addresses go to the kernels unchecked. Everything
+        else is left to the composition, op by op with its checks: a style bank of another generator (the block's offsets
+        are this one's), one that is too short, operands on another device than the weights, an empty x, statistics that
+        are not 8-byte aligned (the kernels read them in pairs)."""
+        if not (isinstance(gb, StyleBank) and gb.off is self.bank_off):
+            return False
+        bank, dev = gb.bank, self.bank_b.device
+        return (x.is_cuda and x.device == dev and x.dim() == 2 and x.shape[1] >= 1
+                and bank.device == dev and bank.dtype == torch.float32 and bank.shape == self.bank_b.shape
+                and bank.is_contiguous()
+                and (x_stats is None or (x_stats.device == dev and x_stats.data_ptr() % 8 == 0)))
+
     def _snake_conv(self, x, af, alpha_key, conv, k, d, residual=None):
         w = self.w
         return ops.conv1d_snake_f32_cuda(x, w[conv + ".weight"], w[conv + ".bias"], af, w[alpha_key],
@@ -232,8 +245,7 @@ class Generator:
 
     def adain_resblock1_fused(self, x, gb, prefix, k, x_stats=None):
         n = x.shape[1]
-        # the block's offsets are this generator's: a bank of another one (a subset of the same state dict, say) has its own
-        if isinstance(gb, StyleBank) and gb.off is self.bank_off and not ops.op_by_op() and x.is_cuda:
+        if not ops.op_by_op() and self._takes_block(x, gb, x_stats):
             blk = self._block(prefix, k)
             ops._f32(x, *([] if x_stats is None else [x_stats]))
             if blk is not None and tuple(x.shape) == (blk.c, n) and (

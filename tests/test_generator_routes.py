@@ -1,10 +1,12 @@
 """Which calls take the whole-resblock / whole-forward library calls and which go through the op-by-op composition, with
 its checks: the host logic in front of the launches, on CPU tensors that claim to live on a GPU."""
+import ctypes
+
 import pytest
 import torch
 
+from lokinfer_b200 import _lib, ops
 from lokinfer_b200 import generator as G
-from lokinfer_b200 import ops
 
 C, N, K = 16, 300, 3
 
@@ -65,3 +67,49 @@ def test_a_bank_of_another_generator_goes_by_its_own_offsets(gen):
     foreign = bank(gen, 24 * C, off={"rb.adain1.0.fc": (5, 2 * C)})
     with pytest.raises(Composition):
         gen.adain_resblock1_fused(x, foreign, "rb", K)
+
+
+@pytest.mark.parametrize("what", ["x on another GPU", "stats on the CPU", "stats on another GPU", "stats not 8-byte aligned",
+                                  "bank on the CPU", "bank on another GPU", "short bank", "strided bank", "f64 bank",
+                                  "empty x"])
+def test_operands_the_whole_call_would_not_check(gen, what):
+    x, b, st = on_gpu(torch.zeros(C, N)), bank(gen), None
+    if what == "x on another GPU":
+        x = on_gpu(torch.zeros(C, N), 1)
+    elif what == "stats on the CPU":
+        st = torch.zeros(C, 3, 2)
+    elif what == "stats on another GPU":
+        st = on_gpu(torch.zeros(C, 3, 2), 1)
+    elif what == "stats not 8-byte aligned":
+        flat = torch.zeros(C * 6 + 1)
+        st = on_gpu(flat[1 if flat.data_ptr() % 8 == 0 else 0:][:C * 6].view(C, 3, 2))
+    elif what == "empty x":
+        x = on_gpu(torch.zeros(C, 0))
+    else:
+        b.bank = {"bank on the CPU": torch.zeros(12 * C), "bank on another GPU": on_gpu(torch.zeros(12 * C), 1),
+                  "short bank": on_gpu(torch.zeros(12 * C - 1)), "strided bank": on_gpu(torch.zeros(24 * C)[::2]),
+                  "f64 bank": on_gpu(torch.zeros(12 * C, dtype=torch.float64))}[what]
+    with pytest.raises(Composition):
+        gen.adain_resblock1_fused(x, b, "rb", K, x_stats=st)
+
+
+def test_resblock_call_rejects_what_its_kernels_cannot_take():
+    """lkc_resblock from C: refused on the host, before anything is queued (no pointer here is a device address)."""
+    blk = _lib.LkcResblock()
+    blk.c, blk.k = C, K
+    blk.w[:], blk.b[:], blk.alpha[:] = [4096] * 6, [4096] * 6, [4096] * 6
+
+    def call(**kw):
+        io = _lib.LkcResblockIo()
+        io.x = io.bank = io.out = io.out_stats = 4096
+        io.l = io.x_pitch = io.out_pitch = N
+        for k, v in kw.items():
+            setattr(io, k, v)
+        return _lib.lib().lkc_resblock(ctypes.byref(blk), ctypes.byref(io), None), io
+
+    rc, io = call()  # without a workspace: its size only
+    assert rc == 0 and io.workspace_bytes > 0
+    for kw in ({"stats": 4100}, {"out_stats": 4100}):
+        assert call(**kw)[0] != 0 and "8-byte aligned" in _lib.last_error()
+    blk.c = 65536
+    assert call()[0] != 0 and "too many channels" in _lib.last_error()

@@ -258,3 +258,32 @@ def test_style_bank_of_another_generator(cuda, gen):
     assert torch.equal(out, ref) and torch.equal(st, rst)
     own, _ = gen.adain_resblock1_fused(x, bank, "resblocks.4", 7)
     assert rel_l2(out.cpu().numpy(), own.cpu().numpy()) <= REL_L2
+
+
+def test_resblock_with_statistics(cuda):
+    """Chunk statistics of x handed in: the same bits as without. Statistics that the kernels could not read are refused
+    before any launch, as are an x or a style bank that does not fit the block."""
+    from lokinfer_b200 import Generator, _lib, ops
+    sd, x, s = synth.resblock_case(48, 1201, 3, 11)  # three channel chunks: CTAs of a split tile with unequal shares
+    g = Generator(sd, cuda)
+    dx, bank = ops.to_cuda(x, cuda), g.style(ops.to_cuda(s, cuda))
+    st = ops.channel_stats_f32_cuda(dx)
+    out, ost = g.adain_resblock1_fused(dx, bank, "rb", 3)
+    again, ast = g.adain_resblock1_fused(dx, bank, "rb", 3, x_stats=st)
+    assert torch.equal(out, again) and torch.equal(ost, ast)
+    sd32 = {n: O.T(v) for n, v in sd.items()}
+    ref, _ = O.adain_resblock1_fused(O.T(x), O.style_bank(sd32, O.T(s)), sd32, "rb", 3)
+    assert rel_l2(out.cpu().numpy(), ref.numpy()) <= 6 * REL_L2
+    odd = torch.empty(st.numel() + 1, device=cuda)[1:].view(st.shape).copy_(st)
+    short = type(bank)(bank.bank[:-1], bank.off)
+    with ops.Profile(time_kernels=False) as prof:
+        for a, kw in (((dx, bank), {"x_stats": st.cpu()}), ((dx, bank), {"x_stats": odd}), ((dx.cpu(), bank), {}),
+                      ((dx[:, :0], bank), {})):
+            with pytest.raises((ops.OpError, _lib.LkcError)):
+                g.adain_resblock1_fused(*a, "rb", 3, **kw)
+        assert prof.count <= 1
+    last = max(bank.off, key=lambda n: bank.off[n][0])
+    assert last in ("rb.adain2.2.fc",)
+    with pytest.raises(ops.OpError):
+        g.adain_resblock1_fused(dx, short, "rb", 3)
+    assert ops.conv_tc_status() == 0
