@@ -310,9 +310,10 @@ class Generator:
                 return self.forward(x, har, s, fused, outputs, concurrent, pad_rows)
         if fused and set(outputs) <= {"audio", "post"} and not ops.op_by_op() and ops._pad_rows and self._whole_model():
             ops._f32(x, har, s)
-            ops.check(all(v.is_cuda and v.device == x.device for v in (x, har, s)) and s.numel() == 128,
-                      "operands must live on one cuda device, s must be f32[128]")
-            with torch.cuda.device(x.device):
+            dev = self.bank_b.device
+            ops.check(all(v.is_cuda and v.device == dev for v in (x, har, s)) and s.numel() == 128,
+                      f"x, har and s must live on the generator's device ({dev}), s must be f32[128]")
+            with torch.cuda.device(dev):
                 return self._forward_whole(x, har, s.contiguous(), outputs, concurrent)
         gb = self.style(s)
         cur = torch.cuda.current_stream(self.device)

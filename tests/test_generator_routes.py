@@ -1,5 +1,6 @@
 """Which calls take the whole-resblock / whole-forward library calls and which go through the op-by-op composition, with
 its checks: the host logic in front of the launches, on CPU tensors that claim to live on a GPU."""
+import contextlib
 import ctypes
 
 import pytest
@@ -113,3 +114,15 @@ def test_resblock_call_rejects_what_its_kernels_cannot_take():
         assert call(**kw)[0] != 0 and "8-byte aligned" in _lib.last_error()
     blk.c = 65536
     assert call()[0] != 0 and "too many channels" in _lib.last_error()
+
+
+@pytest.mark.parametrize("index", [(1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1)])
+def test_forward_refuses_operands_on_another_gpu(gen, monkeypatch, index):
+    monkeypatch.setattr(gen, "_whole_model", lambda: object())
+    monkeypatch.setattr(gen, "_forward_whole", lambda *a, **k: "whole")
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    t = 4
+    args = [torch.zeros(512, t), torch.zeros(22, 60 * t + 1), torch.zeros(128)]
+    assert gen.forward(*[on_gpu(a) for a in args]) == "whole"
+    with pytest.raises(ops.OpError, match="the generator's device"):
+        gen.forward(*[on_gpu(a, i) for a, i in zip(args, index)])
