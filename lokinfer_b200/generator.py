@@ -11,6 +11,7 @@ buffers, so a replay costs one launch.
 from __future__ import annotations
 
 import ctypes
+import operator
 
 import numpy as np
 import torch
@@ -41,8 +42,35 @@ class StyleBank:
         return self.bank[o: o + n]
 
 
-def _handle(state):
-    return None if state is None else state.handle
+class _Held:
+    """The objects whose addresses a library struct holds, and where its tensors were. The references keep the memory; the
+    struct is made anew when one of them was replaced in the generator or moved (`t.data = ...`)."""
+
+    def __init__(self, objs):
+        self.objs = objs
+        self.tensors = [o for o in objs if isinstance(o, torch.Tensor)]
+        self.ptrs = list(map(torch.Tensor.data_ptr, self.tensors))
+
+    def current(self, objs):
+        return all(map(operator.is_, self.objs, objs)) and list(map(torch.Tensor.data_ptr, self.tensors)) == self.ptrs
+
+
+class _Model:
+    """Handle of lkc_generator_create; a call in flight in another thread keeps the one it was given."""
+
+    def __init__(self, struct, held):
+        self.held = held
+        self.handle = _lib.lib().lkc_generator_create(ctypes.byref(struct))
+        if not self.handle:
+            raise _lib.LkcError(_lib.last_error())
+
+    def __del__(self):
+        try:
+            if self.handle:
+                _lib.lib().lkc_model_destroy(self.handle)
+                self.handle = None
+        except Exception:
+            pass
 
 
 class Generator:
@@ -92,16 +120,8 @@ class Generator:
                 self.noise_tc[i] = (wp, state, ident, stride, pad, wn.shape[2] // stride, rows)
         self._graphs = {}
         self._streams = None
-        self._blocks = {}  # prefix -> LkcResblock (pointers into self.w, which keeps them alive)
-        self._model = None  # handle of the whole-forward call
-
-    def __del__(self):
-        try:
-            if self._model:
-                _lib.lib().lkc_model_destroy(self._model)
-                self._model = None
-        except Exception:
-            pass
+        self._blocks = {}  # prefix -> (LkcResblock, the getters of its weights and states, _Held)
+        self._model = None  # (getters of its weights and states, _Model) of the whole-forward call
 
     # ------------------------------------------------------------------ building blocks
 
@@ -128,65 +148,103 @@ class Generator:
     # what looks at single kernels (ops.Profile with timing, ops.tracing), for the CUDA-core path and for shapes that
     # have no tensor-core state.
 
+    def _is(self, t, *shape):
+        """A tensor the kernels can take by its address alone."""
+        return tuple(t.shape) == shape and t.dtype == torch.float32 and t.is_contiguous() and t.device == self.bank_b.device
+
     def _block(self, prefix, k):
         """LkcResblock of the weights under `prefix`, or None when a conv of it has no prepared state."""
-        if prefix not in self._blocks:
-            w, blk = self.w, _lib.LkcResblock()
-            c = int(w[f"{prefix}.convs1.0.weight"].shape[0])
-            blk.c, blk.k = c, k
-            for j in range(3):
-                for n in (1, 2):
-                    i, conv = 2 * j + n - 1, f"{prefix}.convs{n}.{j}"
-                    st = self.conv_state.get(conv)
-                    if st is None or tuple(w[conv + ".weight"].shape) != (c, c, k):
-                        self._blocks[prefix] = None
-                        return None
-                    blk.w[i], blk.b[i] = w[conv + ".weight"].data_ptr(), w[conv + ".bias"].data_ptr()
-                    blk.alpha[i] = w[f"{prefix}.alpha{n}.{j}"].data_ptr()
-                    blk.state[i], blk.gb[i] = st.handle, self.bank_off[f"{prefix}.adain{n}.{j}.fc"][0]
-            self._blocks[prefix] = blk
-        blk = self._blocks[prefix]
-        return blk if blk is not None and blk.k == k else None
+        entry = self._blocks.get(prefix)
+        try:
+            if entry is not None:
+                blk, get_w, get_s, held = entry
+                if held.current(get_w(self.w) + get_s(self.conv_state) + (self.bank_off,)):
+                    return blk if blk.k == k else None
+            convs = [f"{prefix}.convs{n}.{j}" for j in range(3) for n in (1, 2)]
+            get_w = operator.itemgetter(*[c + ".weight" for c in convs], *[c + ".bias" for c in convs],
+                                        *[f"{prefix}.alpha{n}.{j}" for j in range(3) for n in (1, 2)])
+            get_s = operator.itemgetter(*convs)
+            ws, states = get_w(self.w), get_s(self.conv_state)
+            gb = [self.bank_off[f"{prefix}.adain{n}.{j}.fc"] for j in range(3) for n in (1, 2)]
+        except KeyError:
+            return None
+        c = int(ws[0].shape[0])
+        if not (all(st is not None and st.shape == (c, c, k) for st in states) and all(n == 2 * c for _, n in gb)
+                and all(self._is(t, c, c, k) for t in ws[:6]) and all(self._is(t, c) for t in ws[6:])):
+            return None
+        blk, ptrs = _lib.LkcResblock(), [t.data_ptr() for t in ws]
+        blk.c, blk.k = c, k
+        blk.w[:], blk.b[:], blk.alpha[:] = ptrs[:6], ptrs[6:12], ptrs[12:]
+        blk.state[:], blk.gb[:] = [st.handle for st in states], [o for o, _ in gb]
+        self._blocks[prefix] = (blk, get_w, get_s, _Held(ws + states + (self.bank_off,)))
+        return blk
+
+    _BLOCKS = [(f"noise_res.{i}", k) for i, k in enumerate((7, 11))] + [
+        (f"resblocks.{3 * i + j}", k) for i in (0, 1) for j, k in enumerate(RES_KERNELS)]
+    _OTHER_NAMES = ("noise_convs.0.bias", "noise_convs.1.bias", "ups.0.bias", "ups.1.bias", "conv_post.weight",
+                    "conv_post.bias")
+    _OTHERS = operator.itemgetter(*_OTHER_NAMES)
+
+    def _pieces(self, get_w, get_s):
+        """Everything that the whole-forward struct points to."""
+        return (*get_w(self.w), *get_s(self.conv_state), *self.noise_tc.values(), *(n[0] for n in self.noise_tc.values()),
+                *self.ups_state, self.bank_wt, self.bank_b, self.ident128, self.bank_off)
 
     def _whole_model(self):
-        """Handle of lkc_generator_forward, or None when some conv has no tensor-core state."""
-        if self._model is None:
-            m, w = _lib.LkcGenerator(), self.w
-            blocks = [(f"noise_res.{i}", k) for i, k in enumerate((7, 11))] + [
-                (f"resblocks.{3 * i + j}", k) for i in (0, 1) for j, k in enumerate(RES_KERNELS)]
-            blocks = [self._block(p, k) if f"{p}.convs1.0.weight" in w else None for p, k in blocks]
-            if (None in blocks or self.ups_wp is None or None in self.ups_state or len(self.noise_tc) < 2
-                    or "conv_post" not in self.conv_state):
-                self._model = 0
+        """_Model of lkc_generator_forward, or None when some conv has no tensor-core state."""
+        if self.ups_wp is None:
+            return None
+        try:
+            if self._model is not None:
+                get_w, get_s, model = self._model
+                if model.held.current(self._pieces(get_w, get_s)):
+                    return model
+            blocks = [self._block(prefix, k) for prefix, k in self._BLOCKS]
+            if None in blocks:
                 return None
-            m.noise_res[:], m.res[:] = blocks[:2], blocks[2:]
-            m.bank_wt, m.bank_b, m.bank_n = self.bank_wt.data_ptr(), self.bank_b.data_ptr(), self.bank_b.shape[0]
-            for i in (0, 1):
-                wp, state, _, stride, pad, taps, rows = self.noise_tc[i]
-                n = m.noise_conv[i]
-                n.w, n.b, n.state = wp.data_ptr(), w[f"noise_convs.{i}.bias"].data_ptr(), state.handle
-                n.stride, n.padding, n.taps, n.rows = stride, pad, taps, rows
-                m.ups_b[i], m.ups_state[i] = w[f"ups.{i}.bias"].data_ptr(), self.ups_state[i].handle
-            m.post_w, m.post_b = w["conv_post.weight"].data_ptr(), w["conv_post.bias"].data_ptr()
-            m.ident128, m.post_state = self.ident128.data_ptr(), self.conv_state["conv_post"].handle
-            with torch.cuda.device(self.device):
-                self._model = _lib.lib().lkc_generator_create(ctypes.byref(m))
-            if not self._model:
-                raise _lib.LkcError(_lib.last_error())
-        return self._model or None
+            others = self._OTHERS(self.w)
+            noise, ups, post = (self.noise_tc[0], self.noise_tc[1]), tuple(self.ups_state), self.conv_state["conv_post"]
+        except KeyError:
+            return None
+        n = int(self.bank_b.shape[0])
+        tensors = zip((*others, self.bank_wt, self.bank_b, self.ident128),
+                      ((256,), (128,), (256,), (128,), (22, 128, 7), (22,), (128, n), (n,), (3, 128)))
+        states = zip((noise[0][1], noise[1][1], *ups, post),
+                     ((256, noise[0][6], noise[0][5]), (128, noise[1][6], noise[1][5]), (512, 256, 20, 10),
+                      (256, 128, 12, 6), (22, 128, 7)))
+        if not (all(self._is(t, *sh) for t, sh in tensors) and all(st is not None and st.shape == sh for st, sh in states)):
+            return None
+        m = _lib.LkcGenerator()
+        m.noise_res[:], m.res[:] = blocks[:2], blocks[2:]
+        m.bank_wt, m.bank_b, m.bank_n = self.bank_wt.data_ptr(), self.bank_b.data_ptr(), n
+        for i, (wp, state, _, stride, pad, taps, rows) in enumerate(noise):
+            nc = m.noise_conv[i]
+            nc.w, nc.b, nc.state = wp.data_ptr(), others[i].data_ptr(), state.handle
+            nc.stride, nc.padding, nc.taps, nc.rows = stride, pad, taps, rows
+            m.ups_b[i], m.ups_state[i] = others[2 + i].data_ptr(), ups[i].handle
+        m.post_w, m.post_b = others[4].data_ptr(), others[5].data_ptr()
+        m.ident128, m.post_state = self.ident128.data_ptr(), post.handle
+        with torch.cuda.device(self.bank_b.device):
+            names = [n for prefix, _ in self._BLOCKS for n in self.w if n.startswith(prefix + ".") and ".adain" not in n]
+            get_w = operator.itemgetter(*names, *self._OTHER_NAMES)
+            get_s = operator.itemgetter(*(n for n in self.conv_state))
+            model = _Model(m, _Held(self._pieces(get_w, get_s)))
+        self._model = (get_w, get_s, model)
+        return model
 
-    def _workspace_bytes(self, t, concurrent):
+    @staticmethod
+    def _workspace_bytes(model, t, concurrent):
         """(planned, unplanned) bytes of the intermediates of one forward of length t."""
         b, u = ctypes.c_int64(0), ctypes.c_int64(0)
-        if _lib.lib().lkc_generator_workspace(self._model, t, int(concurrent), ctypes.byref(b), ctypes.byref(u)) != 0:
+        if _lib.lib().lkc_generator_workspace(model.handle, t, int(concurrent), ctypes.byref(b), ctypes.byref(u)) != 0:
             raise _lib.LkcError(_lib.last_error())
         return b.value, u.value
 
-    def _forward_whole(self, x, har, s, outputs, concurrent, workspace=None):
+    def _forward_whole(self, model, x, har, s, outputs, concurrent, workspace=None):
         t, dev = int(x.shape[1]), self.device
         sh = shapes(t)
         if workspace is None:
-            workspace = torch.empty(self._workspace_bytes(t, concurrent)[0], dtype=torch.uint8, device=dev)
+            workspace = torch.empty(self._workspace_bytes(model, t, concurrent)[0], dtype=torch.uint8, device=dev)
         io = _lib.LkcGeneratorIo()
         res = {"audio": torch.empty(sh["S"], dtype=torch.float32, device=dev)}
         if "post" in outputs:
@@ -199,7 +257,7 @@ class Generator:
         io.concurrent = int(concurrent)
         if concurrent:
             io.side[:] = [st.cuda_stream for st in self._side_streams()]
-        if _lib.lib().lkc_generator_forward(self._model, ctypes.byref(io), ops._stream()) != 0:
+        if _lib.lib().lkc_generator_forward(model.handle, ctypes.byref(io), ops._stream()) != 0:
             raise _lib.LkcError("generator forward: " + _lib.last_error())
         ops.count_launches(io.launches)
         out = tuple(res[o] for o in outputs)
@@ -308,13 +366,15 @@ class Generator:
             # them with the TMA unit (values do not depend on the pitch)
             with ops.padded_rows():
                 return self.forward(x, har, s, fused, outputs, concurrent, pad_rows)
-        if fused and set(outputs) <= {"audio", "post"} and not ops.op_by_op() and ops._pad_rows and self._whole_model():
+        whole = fused and set(outputs) <= {"audio", "post"} and not ops.op_by_op() and ops._pad_rows
+        model = self._whole_model() if whole else None
+        if model is not None:
             ops._f32(x, har, s)
             dev = self.bank_b.device
             ops.check(all(v.is_cuda and v.device == dev for v in (x, har, s)) and s.numel() == 128,
                       f"x, har and s must live on the generator's device ({dev}), s must be f32[128]")
             with torch.cuda.device(dev):
-                return self._forward_whole(x, har, s.contiguous(), outputs, concurrent)
+                return self._forward_whole(model, x, har, s.contiguous(), outputs, concurrent)
         gb = self.style(s)
         cur = torch.cuda.current_stream(self.device)
         par = fused and concurrent
@@ -438,9 +498,10 @@ class Generator:
         pitch = -(-t // ops.ROW_ALIGN) * ops.ROW_ALIGN  # rows of x start on 16-byte boundaries for any t
         bufs = {"x": torch.zeros(512, pitch, device=dev)[:, :t], "har": torch.zeros(22, sh["L1"], device=dev),
                 "s": torch.zeros(128, device=dev)}
-        whole = not ops.op_by_op() and self._whole_model() is not None
+        model = None if ops.op_by_op() else self._whole_model()
+        whole = model is not None
         if whole and planned:
-            bufs["arena_bytes"], bufs["unplanned_bytes"] = self._workspace_bytes(t, True)
+            bufs["arena_bytes"], bufs["unplanned_bytes"] = self._workspace_bytes(model, t, True)
             bufs["arena"] = torch.empty(bufs["arena_bytes"], dtype=torch.uint8, device=dev)
         side = self._warm_stream()
         side.wait_stream(torch.cuda.current_stream(dev))
@@ -463,7 +524,7 @@ class Generator:
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             if "arena" in bufs:
-                bufs["audio"] = self._forward_whole(bufs["x"], bufs["har"], bufs["s"], ("audio",), True, bufs["arena"])
+                bufs["audio"] = self._forward_whole(model, bufs["x"], bufs["har"], bufs["s"], ("audio",), True, bufs["arena"])
             elif arena is not None:
                 arena.begin()
                 with ops.use_allocator(arena.allocator):

@@ -2,6 +2,7 @@
 its checks: the host logic in front of the launches, on CPU tensors that claim to live on a GPU."""
 import contextlib
 import ctypes
+import types
 
 import pytest
 import torch
@@ -126,3 +127,54 @@ def test_forward_refuses_operands_on_another_gpu(gen, monkeypatch, index):
     assert gen.forward(*[on_gpu(a) for a in args]) == "whole"
     with pytest.raises(ops.OpError, match="the generator's device"):
         gen.forward(*[on_gpu(a, i) for a, i in zip(args, index)])
+
+
+@pytest.fixture
+def block():
+    """A generator of one resblock on CPU tensors, with stand-ins for the prepared states: its pointer struct needs no GPU."""
+    g = G.Generator.__new__(G.Generator)
+    g.device, g.w, g.conv_state, g.bank_off, g._blocks, g._model = torch.device("cpu"), {}, {}, {}, {}, None
+    for j in range(3):
+        for n in (1, 2):
+            conv = f"rb.convs{n}.{j}"
+            g.w[conv + ".weight"], g.w[conv + ".bias"] = torch.zeros(C, C, K), torch.zeros(C)
+            g.w[f"rb.alpha{n}.{j}"] = torch.ones(C)
+            g.conv_state[conv] = types.SimpleNamespace(handle=4096 + 2 * j + n, shape=(C, C, K))
+            g.bank_off[f"rb.adain{n}.{j}.fc"] = (2 * C * (2 * j + n - 1), 2 * C)
+    g.bank_b = torch.zeros(12 * C)
+    return g
+
+
+def test_block_follows_its_weights(block):
+    """A weight that was replaced, or moved in place, is the one that the next call uses."""
+    first = block._block("rb", K)
+    assert first is not None and block._block("rb", K) is first and block._block("rb", K + 2) is None
+    new = torch.ones(C)
+    block.w["rb.convs2.1.bias"] = new
+    assert block._block("rb", K).b[3] == new.data_ptr()
+    moved = torch.ones(C)
+    block.w["rb.alpha1.2"].data = moved
+    assert block._block("rb", K).alpha[4] == moved.data_ptr()
+    block.conv_state["rb.convs1.0"] = types.SimpleNamespace(handle=77, shape=(C, C, K))
+    assert block._block("rb", K).state[0] == 77
+    again = block._block("rb", K)
+    assert block._block("rb", K) is again
+
+
+def test_block_leaves_odd_weights_to_the_composition(block):
+    """Weights that the ops would refuse do not reach the kernels by address, also when they come later."""
+    keep = dict(block.w), dict(block.conv_state)
+    for name, t in (("rb.convs1.1.bias", torch.zeros(C - 1)), ("rb.alpha2.0", torch.zeros(C, dtype=torch.float64)),
+                    ("rb.convs2.2.weight", torch.zeros(C, C, K + 2)), ("rb.convs2.2.bias", torch.zeros(2 * C)[::2]),
+                    ("rb.convs2.2.bias", torch.zeros(C, device="meta"))):
+        assert block._block("rb", K) is not None
+        block.w[name] = t
+        assert block._block("rb", K) is None, name
+        block.w.update(keep[0])
+    del block.w["rb.alpha1.0"]
+    assert block._block("rb", K) is None
+    block.w.update(keep[0])
+    block.conv_state["rb.convs2.0"] = None
+    assert block._block("rb", K) is None
+    block.conv_state.update(keep[1])
+    assert block._block("rb", K) is not None

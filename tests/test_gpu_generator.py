@@ -287,3 +287,21 @@ def test_resblock_with_statistics(cuda):
     with pytest.raises(ops.OpError):
         g.adain_resblock1_fused(dx, short, "rb", 3)
     assert ops.conv_tc_status() == 0
+
+
+def test_replaced_weights_take_effect(cuda):
+    """Biases and alphas written into Generator.w after the first call are the ones that the next call uses, also when the
+    replaced tensors' memory has been given to someone else."""
+    from lokinfer_b200 import Generator
+    g, (_, d) = Generator(synth.generator_weights(0), cuda), _inputs(cuda, 9, seed=4)
+    before = g.forward(*d)
+    for name in ("conv_post.bias", "ups.0.bias", "noise_convs.1.bias", "resblocks.2.convs2.1.bias", "noise_res.0.alpha1.0"):
+        g.w[name] = g.w[name] * 1.25 + 0.01
+        filler = [torch.full_like(g.w[name], float("nan")) for _ in range(4)]
+        after = g.forward(*d)
+        assert torch.isfinite(after).all() and not torch.equal(after, before), name
+        fresh = Generator(synth.generator_weights(0), cuda)
+        fresh.w.update({k: v.clone() for k, v in g.w.items()})
+        assert torch.equal(fresh.forward(*d), after), name
+        before = after
+        del filler
