@@ -134,7 +134,7 @@ LKC_API int lkc_conv1d_leaky_mean3_f32_cuda(const LkcArgs* a, void* stream);
  *   n = lkc_conv1d_tc_pack_floats(Co, Ci, K)       floats of the pack; 0 = shape not eligible (needs Ci % 16 == 0,
  *                                                  K <= 64), the CUDA-core kernel serves it. Co is padded to a
  *                                                  multiple of 128 with zero rows inside the pack
- *   lkc_conv1d_tc_pack_f32_cuda: ptrs w[Co,Ci,K] | wp[n]; ints w(3) wp(1)     hi / lo operand split in the UMMA layout
+ *   lkc_conv1d_tc_pack_f32_cuda: ptrs w[Co,Ci,K] | wp[n]; ints w(3) wp(1) [format]     hi / lo operand split in the UMMA layout
  *   st = lkc_conv1d_state_create(wp, Co, Ci, K)    host-side handle; pass it as LkcArgs.state of the conv1d_* calls
  * A conv call with a state whose shape is eligible ((K - 1) * dilation <= 50, K <= 24 for an f16 pack and <= 12 for
  * a tf32 pack, no mean3 input) runs on the tensor cores; anything else runs on the CUDA-core kernel with identical
@@ -148,8 +148,14 @@ LKC_API int lkc_conv1d_leaky_mean3_f32_cuda(const LkcArgs* a, void* stream);
  * 16-byte aligned (A/B testing). lkc_set_conv_path chooses the path and the operand format of packs made
  * AFTER the call: 0 (default) tensor cores with operands split into f16 hi + f16 lo * 2^-11 (3 kind::f16 MMAs per
  * 16 channels and tap), 2 tensor cores with tf32 hi + tf32 lo (6 kind::tf32 MMAs), 1 the CUDA-core kernel only
- * (A/B testing). lkc_*_pack_floats report sizes for the current format; a state remembers the format of its pack. */
+ * (A/B testing). lkc_*_pack_floats report sizes for the current format; a state remembers the format of its pack.
+ * The `_as` forms take the format as an argument (one of the two below) whatever the current path is, and the two pack
+ * entry points take it as one more trailing int: for one weight in another format, or packs from several threads. */
 typedef struct LkcConvState LkcConvState;
+#define LKC_FORMAT_F16 0
+#define LKC_FORMAT_TF32 2
+LKC_API int64_t lkc_conv1d_tc_pack_floats_as(int64_t co, int64_t ci, int64_t k, int format);
+LKC_API LkcConvState* lkc_conv1d_state_create_as(const void* wp, int64_t co, int64_t ci, int64_t k, int format);
 LKC_API int64_t lkc_conv1d_tc_pack_floats(int64_t co, int64_t ci, int64_t k);
 LKC_API int lkc_conv1d_tc_pack_f32_cuda(const LkcArgs* a, void* stream);
 LKC_API LkcConvState* lkc_conv1d_state_create(const void* wp, int64_t co, int64_t ci, int64_t k);
@@ -186,11 +192,14 @@ LKC_API int lkc_convt_poly_pack_f32_cuda(const LkcArgs* a, void* stream);
 /* Tensor-core path of conv_transpose1d_poly_f32_cuda (no mean3 input; strides 6 and 10 with K = 2 stride,
  * 2 padding = stride, Ci % 16 == 0: the two Kokoro upsamplers), prepared like the conv one:
  *   n = lkc_convt_tc_pack_floats(Ci, Co, K, stride, padding)     0 = not eligible
- *   lkc_convt_tc_pack_f32_cuda: ptrs w[Ci,Co,K] | wp[n]; ints w(3) wp(1) padding stride
+ *   lkc_convt_tc_pack_f32_cuda: ptrs w[Ci,Co,K] | wp[n]; ints w(3) wp(1) padding stride [format]
  *   st = lkc_convt_state_create(wp, Ci, Co, K, stride, padding)   pass as LkcArgs.state of the poly call (the `wp`
  *        operand of that call stays the CUDA-core pack); destroy with lkc_conv1d_state_destroy.
  * The left reflect column is unpadded[co, 1] + res[co, 0] with the plain conv sum, as in the reference
  * (kokoro_conv.cpp:226). */
+LKC_API int64_t lkc_convt_tc_pack_floats_as(int64_t ci, int64_t co, int64_t k, int64_t stride, int64_t padding, int format);
+LKC_API LkcConvState* lkc_convt_state_create_as(const void* wp, int64_t ci, int64_t co, int64_t k, int64_t stride,
+                                                int64_t padding, int format);
 LKC_API int64_t lkc_convt_tc_pack_floats(int64_t ci, int64_t co, int64_t k, int64_t stride, int64_t padding);
 LKC_API int lkc_convt_tc_pack_f32_cuda(const LkcArgs* a, void* stream);
 LKC_API LkcConvState* lkc_convt_state_create(const void* wp, int64_t ci, int64_t co, int64_t k, int64_t stride,

@@ -84,6 +84,14 @@ def lib():
         l.lkc_build_info.restype = ctypes.c_char_p
         l.lkc_conv1d_tc_pack_floats.restype = ctypes.c_int64
         l.lkc_conv1d_tc_pack_floats.argtypes = [ctypes.c_int64] * 3
+        l.lkc_conv1d_tc_pack_floats_as.restype = ctypes.c_int64
+        l.lkc_conv1d_tc_pack_floats_as.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int]
+        l.lkc_conv1d_state_create_as.restype = ctypes.c_void_p
+        l.lkc_conv1d_state_create_as.argtypes = [ctypes.c_void_p] + [ctypes.c_int64] * 3 + [ctypes.c_int]
+        l.lkc_convt_tc_pack_floats_as.restype = ctypes.c_int64
+        l.lkc_convt_tc_pack_floats_as.argtypes = [ctypes.c_int64] * 5 + [ctypes.c_int]
+        l.lkc_convt_state_create_as.restype = ctypes.c_void_p
+        l.lkc_convt_state_create_as.argtypes = [ctypes.c_void_p] + [ctypes.c_int64] * 5 + [ctypes.c_int]
         l.lkc_conv1d_state_create.restype = ctypes.c_void_p
         l.lkc_conv1d_state_create.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64, ctypes.c_int64]
         l.lkc_convt_tc_pack_floats.restype = ctypes.c_int64

@@ -211,58 +211,89 @@ extern "C" LKC_API int lkc_conv1d_leaky_mean3_f32_cuda(const LkcArgs* a, void* s
 extern "C" LKC_API int lkc_conv1d_f32_cuda(const LkcArgs* a, void* s) { return runConv1d(a, s, true); }
 extern "C" LKC_API int lkc_conv1d_nobias_f32_cuda(const LkcArgs* a, void* s) { return runConv1d(a, s, false); }
 
-// ints: w(Co, Ci, K) wp(n)
+namespace {
+// The operand format of a pack: a mode number of lkc_set_conv_path that names one, or the current mode's.
+bool formatOk(int64_t format) { return format == LKC_FORMAT_F16 || format == LKC_FORMAT_TF32; }
+int currentFormat() { return convPackF16() ? LKC_FORMAT_F16 : LKC_FORMAT_TF32; }
+}  // namespace
+
+// ints: w(Co, Ci, K) wp(n) [format]
 extern "C" LKC_API int lkc_conv1d_tc_pack_f32_cuda(const LkcArgs* a, void* stream) {
-  LKC_REQUIRE(a && a->numPtrs == 2 && a->numInts == 4, "conv1d_tc_pack_f32_cuda: expected w | wp");
-  const int64_t co = a->ints[0], ci = a->ints[1], k = a->ints[2];
+  LKC_REQUIRE(a && a->numPtrs == 2 && (a->numInts == 4 || a->numInts == 5), "conv1d_tc_pack_f32_cuda: expected w | wp");
+  const int64_t co = a->ints[0], ci = a->ints[1], k = a->ints[2], format = a->numInts == 5 ? a->ints[4] : currentFormat();
   LKC_REQUIRE(co > 0 && ci > 0 && ci % 16 == 0 && k >= 1 && k <= 64,
               "conv1d_tc_pack_f32_cuda: needs Ci % 16 == 0, 1 <= K <= 64");
-  LKC_REQUIRE(a->ints[3] == convTcPackFloats(co, ci, k, convPackF16()),
+  LKC_REQUIRE(formatOk(format), "conv1d_tc_pack_f32_cuda: no such operand format");
+  const bool f16 = format == LKC_FORMAT_F16;
+  LKC_REQUIRE(a->ints[3] == convTcPackFloats(co, ci, k, f16),
               "conv1d_tc_pack_f32_cuda: wp must hold lkc_conv1d_tc_pack_floats (of the current operand format)");
-  return convTcPack(F(a, 0), O(a, 1), co, ci, k, convPackF16(), S(stream));
+  return convTcPack(F(a, 0), O(a, 1), co, ci, k, f16, S(stream));
+}
+
+extern "C" LKC_API int64_t lkc_conv1d_tc_pack_floats_as(int64_t co, int64_t ci, int64_t k, int format) {
+  if (co <= 0 || ci <= 0 || ci % 16 != 0 || k < 1 || k > 64 || !formatOk(format)) return 0;
+  return convTcPackFloats(co, ci, k, format == LKC_FORMAT_F16);
 }
 
 extern "C" LKC_API int64_t lkc_conv1d_tc_pack_floats(int64_t co, int64_t ci, int64_t k) {
-  if (co <= 0 || ci <= 0 || ci % 16 != 0 || k < 1 || k > 64) return 0;
-  return convTcPackFloats(co, ci, k, convPackF16());
+  return lkc_conv1d_tc_pack_floats_as(co, ci, k, currentFormat());
 }
 
-extern "C" LKC_API LkcConvState* lkc_conv1d_state_create(const void* wp, int64_t co, int64_t ci, int64_t k) {
-  if (!wp || lkc_conv1d_tc_pack_floats(co, ci, k) == 0) {
+extern "C" LKC_API LkcConvState* lkc_conv1d_state_create_as(const void* wp, int64_t co, int64_t ci, int64_t k, int format) {
+  if (!wp || lkc_conv1d_tc_pack_floats_as(co, ci, k, format) == 0) {
     fail("conv1d_state_create: shape not eligible for the tensor-core path or null pack");
     return nullptr;
   }
-  ConvState* st = new (std::nothrow) ConvState{static_cast<const float*>(wp), co, ci, k, 0, convPackF16()};
+  ConvState* st = new (std::nothrow) ConvState{static_cast<const float*>(wp), co, ci, k, 0, format == LKC_FORMAT_F16};
   if (!st) fail("conv1d_state_create: out of host memory");
   return reinterpret_cast<LkcConvState*>(st);
 }
 
+extern "C" LKC_API LkcConvState* lkc_conv1d_state_create(const void* wp, int64_t co, int64_t ci, int64_t k) {
+  return lkc_conv1d_state_create_as(wp, co, ci, k, currentFormat());
+}
+
 extern "C" LKC_API void lkc_conv1d_state_destroy(LkcConvState* st) { delete reinterpret_cast<ConvState*>(st); }
 
-// ints: w(Ci, Co, K) wp(n) padding stride
+// ints: w(Ci, Co, K) wp(n) padding stride [format]
 extern "C" LKC_API int lkc_convt_tc_pack_f32_cuda(const LkcArgs* a, void* stream) {
-  LKC_REQUIRE(a && a->numPtrs == 2 && a->numInts == 6, "convt_tc_pack_f32_cuda: expected w | wp, padding, stride");
+  LKC_REQUIRE(a && a->numPtrs == 2 && (a->numInts == 6 || a->numInts == 7),
+              "convt_tc_pack_f32_cuda: expected w | wp, padding, stride");
   const int64_t ci = a->ints[0], co = a->ints[1], k = a->ints[2], pad = a->ints[4], s = a->ints[5];
+  const int64_t format = a->numInts == 7 ? a->ints[6] : currentFormat();
   LKC_REQUIRE(convtTcEligible(ci, co, k, s, pad),
               "convt_tc_pack_f32_cuda: needs stride 6 or 10, K = 2 stride, 2 padding = stride, Ci % 16 == 0");
-  LKC_REQUIRE(a->ints[3] == convtTcPackFloats(ci, co, s, convPackF16()),
+  LKC_REQUIRE(formatOk(format), "convt_tc_pack_f32_cuda: no such operand format");
+  const bool f16 = format == LKC_FORMAT_F16;
+  LKC_REQUIRE(a->ints[3] == convtTcPackFloats(ci, co, s, f16),
               "convt_tc_pack_f32_cuda: wp must hold lkc_convt_tc_pack_floats (of the current operand format)");
-  return convtTcPack(F(a, 0), O(a, 1), ci, co, k, s, pad, convPackF16(), S(stream));
+  return convtTcPack(F(a, 0), O(a, 1), ci, co, k, s, pad, f16, S(stream));
+}
+
+extern "C" LKC_API int64_t lkc_convt_tc_pack_floats_as(int64_t ci, int64_t co, int64_t k, int64_t stride, int64_t padding,
+                                                       int format) {
+  if (!convtTcEligible(ci, co, k, stride, padding) || !formatOk(format)) return 0;
+  return convtTcPackFloats(ci, co, stride, format == LKC_FORMAT_F16);
 }
 
 extern "C" LKC_API int64_t lkc_convt_tc_pack_floats(int64_t ci, int64_t co, int64_t k, int64_t stride, int64_t padding) {
-  return convtTcEligible(ci, co, k, stride, padding) ? convtTcPackFloats(ci, co, stride, convPackF16()) : 0;
+  return lkc_convt_tc_pack_floats_as(ci, co, k, stride, padding, currentFormat());
+}
+
+extern "C" LKC_API LkcConvState* lkc_convt_state_create_as(const void* wp, int64_t ci, int64_t co, int64_t k,
+                                                           int64_t stride, int64_t padding, int format) {
+  if (!wp || lkc_convt_tc_pack_floats_as(ci, co, k, stride, padding, format) == 0) {
+    fail("convt_state_create: shape not eligible for the tensor-core path or null pack");
+    return nullptr;
+  }
+  ConvState* st = new (std::nothrow) ConvState{static_cast<const float*>(wp), co, ci, k, stride, format == LKC_FORMAT_F16};
+  if (!st) fail("convt_state_create: out of host memory");
+  return reinterpret_cast<LkcConvState*>(st);
 }
 
 extern "C" LKC_API LkcConvState* lkc_convt_state_create(const void* wp, int64_t ci, int64_t co, int64_t k,
                                                         int64_t stride, int64_t padding) {
-  if (!wp || !convtTcEligible(ci, co, k, stride, padding)) {
-    fail("convt_state_create: shape not eligible for the tensor-core path or null pack");
-    return nullptr;
-  }
-  ConvState* st = new (std::nothrow) ConvState{static_cast<const float*>(wp), co, ci, k, stride, convPackF16()};
-  if (!st) fail("convt_state_create: out of host memory");
-  return reinterpret_cast<LkcConvState*>(st);
+  return lkc_convt_state_create_as(wp, ci, co, k, stride, padding, currentFormat());
 }
 
 extern "C" LKC_API int lkc_conv1d_tc_status(int* status, int reset) {

@@ -24,16 +24,6 @@ def _pad16(c: int) -> int:
     return -(-c // 16) * 16
 
 
-def _prepare_f32_range(w):
-    """A conv state in the tf32 operand format, which has the range of f32: for convs whose input is not normalised."""
-    path = ops._conv_path
-    ops.set_conv_path("tf32")
-    try:
-        return ops.conv1d_prepare_f32_cuda(w)
-    finally:
-        ops.set_conv_path(path)
-
-
 class Decoder:
     def __init__(self, sd: dict, device="cuda"):
         self.device = torch.device(device)
@@ -57,9 +47,9 @@ class Decoder:
             for conv in (".conv1", ".conv2"):
                 self.state[name + conv] = ops.conv1d_prepare_f32_cuda(w[name + conv + ".weight"])
             if cin != cout:
-                self.state[name + ".conv1x1"] = _prepare_f32_range(w[name + ".conv1x1.weight"])
+                self.state[name + ".conv1x1"] = ops.conv1d_prepare_f32_cuda(w[name + ".conv1x1.weight"], "tf32")
                 w[name + ".conv1x1.bias"] = torch.zeros(cout, device=self.device)
-        self.state["decoder.asr_res.0"] = _prepare_f32_range(w["decoder.asr_res.0.weight"])
+        self.state["decoder.asr_res.0"] = ops.conv1d_prepare_f32_cuda(w["decoder.asr_res.0.weight"], "tf32")
         # style bank: every `<name>.fc` of the decoder as one GEMV (models/kokoro/model.py:67-81, names sorted)
         names = sorted(k[: -len(".weight")] for k in w if k.endswith(".fc.weight"))
         # The (gamma | beta) of a norm1 carry their zeros for the appended rows: gamma, zeros, beta, zeros.

@@ -639,9 +639,9 @@ class ConvState:
     """Prepared state of one constant conv weight for the tensor-core kernel: the hi / lo operand pack in the UMMA
     layout plus the host handle passed as `state` (the reference's prepare hook result, kernel.h:56-58)."""
 
-    def __init__(self, handle, wp, shape):
+    def __init__(self, handle, wp, shape, fmt):
         self.handle, self.wp, self.shape = handle, wp, shape
-        self.fmt = "tf32" if _conv_path == "tf32" else "f16"  # operand format of the pack
+        self.fmt = fmt  # operand format of the pack
 
     def __del__(self):
         try:
@@ -652,26 +652,27 @@ class ConvState:
             pass
 
 
-def conv1d_prepare_f32_cuda(w):
+def conv1d_prepare_f32_cuda(w, fmt=None):
     """Packs a constant conv weight f32[Co, Ci, K] once for the tensor-core path (run at init, like the reference's
     hoisted weight preparation, docs/passes/hoist-init.md). Returns None when the shape is served by the CUDA-core
-    kernel instead (Ci % 16 != 0 or K > 64)."""
+    kernel instead (Ci % 16 != 0 or K > 64). fmt = operand format, "f16" or "tf32" (the range of f32); None: what
+    set_conv_path says, with tf32 for a weight beyond the f16 range."""
     _f32(w, rank=3)
     check(w.is_contiguous(), "w must be contiguous")
     co, ci, k = (int(d) for d in w.shape)
 
-    def pack():
-        n = int(_lib.lib().lkc_conv1d_tc_pack_floats(co, ci, k))
+    def pack(fmt):
+        n = int(_lib.lib().lkc_conv1d_tc_pack_floats_as(co, ci, k, _FORMATS[fmt]))
         if n == 0:
             return None
         wp = torch.empty((n,), dtype=torch.float32, device=w.device)
-        _run("conv1d_tc_pack_f32_cuda", [w], [wp])
-        handle = _lib.lib().lkc_conv1d_state_create(wp.data_ptr(), co, ci, k)
+        _run("conv1d_tc_pack_f32_cuda", [w], [wp], attrs_int=[_FORMATS[fmt]])
+        handle = _lib.lib().lkc_conv1d_state_create_as(wp.data_ptr(), co, ci, k, _FORMATS[fmt])
         if not handle:
             raise _lib.LkcError(_lib.last_error())
-        return ConvState(handle, wp, (co, ci, k))
+        return ConvState(handle, wp, (co, ci, k), fmt)
 
-    return _pack_checked(pack)
+    return _pack_checked(pack, fmt)
 
 
 def conv_transpose1d_prepare_f32_cuda(w, stride, padding):
@@ -683,16 +684,16 @@ def conv_transpose1d_prepare_f32_cuda(w, stride, padding):
     check(w.is_contiguous(), "w must be contiguous")
     ci, co, k = (int(d) for d in w.shape)
 
-    def pack():
-        n = int(_lib.lib().lkc_convt_tc_pack_floats(ci, co, k, s, p))
+    def pack(fmt):
+        n = int(_lib.lib().lkc_convt_tc_pack_floats_as(ci, co, k, s, p, _FORMATS[fmt]))
         if n == 0:
             return None
         wp = torch.empty((n,), dtype=torch.float32, device=w.device)
-        _run("convt_tc_pack_f32_cuda", [w], [wp], attrs_int=[p, s])
-        handle = _lib.lib().lkc_convt_state_create(wp.data_ptr(), ci, co, k, s, p)
+        _run("convt_tc_pack_f32_cuda", [w], [wp], attrs_int=[p, s, _FORMATS[fmt]])
+        handle = _lib.lib().lkc_convt_state_create_as(wp.data_ptr(), ci, co, k, s, p, _FORMATS[fmt])
         if not handle:
             raise _lib.LkcError(_lib.last_error())
-        return ConvState(handle, wp, (ci, co, k, s))
+        return ConvState(handle, wp, (ci, co, k, s), fmt)
 
     return _pack_checked(pack)
 
@@ -701,24 +702,24 @@ STATUS_F16_ACT, STATUS_F16_WEIGHTS = 0x10000, 0x20000
 _conv_path = "auto"
 
 
-def _pack_checked(pack):
-    """Runs a weight pack and, if the f16 split reported a weight beyond the f16 range (status bit 0x20000: the value
-    was clamped), packs the weight again in the tf32 format, which has the range of f32. Reads the status word, so it
-    synchronises the device: packing is init-time work."""
+_FORMATS = {"f16": 0, "tf32": 2}  # LKC_FORMAT_* of include/lkc.h
+
+
+def _pack_checked(pack, fmt=None):
+    """Runs a weight pack in format `fmt`, or (None) in the format of the current conv path; there, if the f16 split
+    reported a weight beyond the f16 range (status bit 0x20000: the value was clamped), packs the weight again in the tf32
+    format, which has the range of f32. Reads the status word, so it synchronises the device: packing is init-time work.
+    The format goes down to the pack as an argument: other threads may be packing or launching meanwhile."""
+    check(fmt is None or fmt in _FORMATS, "fmt must be 'f16' or 'tf32'")
     with torch.cuda.device(torch.cuda.current_device()):
-        st = pack()
-        if st is None or _conv_path != "auto":
+        path = _conv_path
+        st = pack(fmt or ("tf32" if path == "tf32" else "f16"))
+        if st is None or fmt is not None or path != "auto":
             return st
         status = conv_tc_status()
         if status & ~STATUS_F16_WEIGHTS:
             raise RuntimeError(f"tensor-core conv kernels reported status {status:#x} before this weight was packed")
-        if status & STATUS_F16_WEIGHTS:
-            set_conv_path("tf32")
-            try:
-                st = pack()
-            finally:
-                set_conv_path("auto")
-        return st
+        return pack("tf32") if status & STATUS_F16_WEIGHTS else st
 
 
 def conv_tc_status(reset=True) -> int:
