@@ -347,9 +347,12 @@ __host__ __device__ constexpr uint32_t idescOf(bool f16, int n) {
   return (1u << 4) | (f16 ? 0u : (2u << 7) | (2u << 10)) | (uint32_t(n >> 3) << 17) | (uint32_t(MT >> 4) << 24);
 }
 
+// hi half of the tf32 split. Saturating: a value next to the largest float, or infinite, gets the largest finite hi, so that
+// lo = v - hi stays finite resp. infinite and the products keep the sum's value; rounded up to infinity, hi would make
+// lo = -inf and the sum NaN.
 __device__ __forceinline__ float tf32Round(float v) {
   uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
+  asm("cvt.rna.satfinite.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
   return __uint_as_float(r);
 }
 

@@ -159,6 +159,35 @@ def _pitched(t):
     return buf[:, :l]
 
 
+@pytest.mark.parametrize("l", [1, 61, 300])
+def test_tf32_split_keeps_the_ends_of_the_range(cuda, l):
+    """A pointwise conv with tf32 halves, per column as the CUDA-core kernel: the largest finite values stay finite,
+    infinities keep their sign, NaN stays NaN, in the operand and in the weights, and no column touches another."""
+    from lokinfer_b200 import ops
+    r = np.random.default_rng(l)
+    top = np.finfo(np.float32).max
+    w = (r.uniform(0.01, 0.03, (40, 32, 1)) * r.choice([-1, 1], (40, 32, 1))).astype(np.float32)
+    b, ident = np.zeros(40, np.float32), np.stack([np.zeros(32), np.ones(32), np.zeros(32)]).astype(np.float32)
+    x = r.standard_normal((32, l + 6)).astype(np.float32)
+    for i, v in enumerate((top, -top, np.inf, -np.inf, np.nan)):
+        x[3 * i, i] = v
+    wtop = w.copy()
+    wtop[7, 5, 0] = top
+    for wt, xs in ((w, x), (wtop, (x[:, 5:] * 1e-3).astype(np.float32))):
+        dx, dw, db, did = dev(cuda, xs, wt, b, ident)
+        got, _ = ops.conv1d_affine_f32_cuda(dx, dw, db, did, state=ops.conv1d_prepare_f32_cuda(dw, "tf32"))
+        with np.errstate(invalid="ignore", over="ignore"):
+            want = (wt[:, :, 0].astype(np.float64) @ xs.astype(np.float64)).astype(np.float32)
+        got = got.cpu().numpy()
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+        np.testing.assert_array_equal(np.where(np.isinf(got), got, 0), np.where(np.isinf(want), want, 0))
+        ok = np.isfinite(want)
+        # 22 bits of each operand and a chain of 32 products, per column (columns differ by 38 orders of magnitude)
+        for t in range(xs.shape[1]):
+            assert rel_l2(got[ok[:, t], t], want[ok[:, t], t]) <= 1e-6 if ok[:, t].any() else True
+        assert ops.conv_tc_status() == 0
+
+
 # Shapes for the padded-row (TMA) route: partial last tile, exact tile multiples, windows that start before the row
 # and end after it, odd lengths (pitch = L rounded up to 4), both stage shapes of the 26 s case, several tiles per CTA.
 TMA_CASES = [(128, 128, 1201, 3, 1), (128, 128, 1203, 7, 3), (128, 128, 5000, 11, 5), (256, 256, 641, 11, 5),
