@@ -113,6 +113,12 @@ constexpr int MAX_HALO = 50;     // (K - 1) * dilation of the widest Kokoro conv
 constexpr int MAX_W_STAGES = 4, MIN_W_STAGES = 2, PREF_W_STAGES = 2;  // weight ring slots
 constexpr int TAP_GROUP = 6;  // most taps per weight slot: one bulk copy, one wait, MMAs back to back, one release
 constexpr int MAX_CHAIN = 24;  // most chained hi MMAs between two drains of Dhi
+// The same of a pointwise conv with tf32 halves, whose alternative is one f32 sum over the channels on the CUDA cores.
+// The drift of a chain of 24 made it the less exact of the two below about 700 channels. Error against float64 (1e-7 of
+// the result) of the decoder's 528- and 512-channel convs over 8..1040 columns: CUDA cores 1.2-2.8 and 3.8-4.2, chains of
+// 24: 1.5-3.2 and 4.5-4.7, of 12: 1.1-2.0 and 2.6-2.7, of 8: 0.9-1.6 and 1.9-2.2; of its 1104-channel convs: CUDA cores
+// 4.3-5.4, chains of 24: 3.5-4.4, of 8: 1.6-1.9. 528 -> 1024 channels at 320 columns: 42.9 us at 24, 43.5 at 8.
+constexpr int MAX_CHAIN_POINT32 = 8;
 constexpr uint32_t SPIN_LIMIT = 1u << 24;
 constexpr uint32_t SLEEP_EPI_NS = 256, SLEEP_EPI_SPLIT_NS = 64, SLEEP_PRO_NS = 128, SLEEP_W_NS = 64, SLEEP_MMA_NS = 32;
 constexpr uint64_t WAIT_LIMIT_NS = 200ull * 1000 * 1000;  // 0.2 s: a healthy wait is tens of microseconds
@@ -1768,9 +1774,9 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercen
   a.nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
   a.status = d->status;
   a.prof = (kProf && gProfileOn) ? d->prof : nullptr;
-  // Dhi is drained into the f32 running sums after as many whole chunks as fit in MAX_CHAIN chained MMAs.
+  // Dhi is drained into the f32 running sums after as many whole chunks as fit in the longest chain of MMAs.
   const int perChunk = a.k * (f16 ? 1 : 2);
-  const int n = MAX_CHAIN / perChunk;
+  const int n = (!f16 && a.k == 1 ? MAX_CHAIN_POINT32 : MAX_CHAIN) / perChunk;
   a.drainN = n < 1 ? 1 : n;
   // Launches with at most 15 MMAs per chunk (K <= 5 with f16 halves; the ConvTranspose launches: three taps) are
   // bound by the activation producers: they take the balanced warp layout (measured at K = 3: the transform of a

@@ -77,9 +77,9 @@ class Decoder:
         return gb
 
     def _conv1x1(self, x, name):
-        """Pointwise conv on the tensor cores (K = 1, identity affine). The CUDA-core kernel's one serial chain over up
-        to 1104 input channels took 150-340 us at any length. The input is raw features, so the operands are tf32
-        halves: the f16 halves of the other convs would limit its range."""
+        """Pointwise conv on the tensor cores (K = 1, identity affine), 42-99 us at 61 to 1040 columns. The input is raw
+        features, so the operands are tf32 halves: the f16 halves of the other convs would limit its range. Error against
+        float64 0.38-0.75 of that of the CUDA cores' f32 sums over 512 to 1104 channels."""
         w = self.w
         return ops.conv1d_affine_f32_cuda(x, w[name + ".weight"], w[name + ".bias"], self._ident[int(x.shape[0])],
                                           state=self.state[name])[0]
