@@ -80,8 +80,7 @@ class Exec {
   template <class Fn>
   void launch(int s, std::initializer_list<Buf> bufs, Fn fn) {
     if (running()) {
-      if (rc == 0) rc = fn(streams_[s]);
-      ++launches;
+      if (rc == 0 && (rc = fn(streams_[s])) == 0) ++launches;
       return;
     }
     const int l = lane(s);
@@ -98,10 +97,16 @@ class Exec {
       return;
     }
     if (rc != 0) return;
-    cudaEvent_t e = events_[event_++ % kEvents];
-    cudaError_t err = cudaEventRecord(e, streams_[waited]);
-    if (err == cudaSuccess) err = cudaStreamWaitEvent(streams_[waiter], e, 0);
+    const cudaError_t err = order(waiter, waited);
     if (err != cudaSuccess) rc = failCuda("model: stream join", err);
+    else if (waited == 0) forked_[waiter] = true;
+  }
+
+  // After an error: what the side streams were given still uses the workspace, so the caller's stream waits for it like
+  // after a whole forward (and a capture can end). The first error is the one that is reported.
+  void joinForked() {
+    for (int s = 1; s < kStreams; ++s)
+      if (forked_[s]) order(0, s);
   }
 
   int finishPlan(Plan* out) {
@@ -117,6 +122,13 @@ class Exec {
   int64_t launches = 0;
 
  private:
+  cudaError_t order(int waiter, int waited) {
+    cudaEvent_t e = events_[event_++ % kEvents];
+    cudaError_t err = cudaEventRecord(e, streams_[waited]);
+    if (err == cudaSuccess) err = cudaStreamWaitEvent(streams_[waiter], e, 0);
+    if (err != cudaSuccess) cudaGetLastError();  // reported by the caller; the next launch's check must not see it
+    return err;
+  }
   int lane(int s) const { return concurrent_ ? s : 0; }
 
   const bool concurrent_;
@@ -124,6 +136,7 @@ class Exec {
   char* base_ = nullptr;
   cudaStream_t streams_[kStreams] = {};
   cudaEvent_t* events_ = nullptr;
+  bool forked_[kStreams] = {};
   int next_ = 0, event_ = 0;
   std::vector<int64_t> bytes_, allocClock_, lastUse_;
   int64_t clock_[kStreams][kStreams] = {};
@@ -397,6 +410,7 @@ extern "C" LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, vo
   Exec e(io->concurrent != 0, *p, static_cast<char*>(io->workspace), S(stream),
          reinterpret_cast<const cudaStream_t*>(io->side), m->events);
   generator(e, m->w, *io);
+  if (e.rc != 0) e.joinForked();
   io->launches = e.launches;
   return e.rc;
 }

@@ -305,3 +305,28 @@ def test_replaced_weights_take_effect(cuda):
         assert torch.equal(fresh.forward(*d), after), name
         before = after
         del filler
+
+
+def test_error_inside_a_forward_joins_its_streams(cuda):
+    """A conv in the middle of the forward is refused on the host (its prepared state says another channel count) after
+    work has been queued on the side streams. The caller's stream is ordered behind that work: a capture can end (with a
+    stream left unjoined it cannot), and the generator works on afterwards."""
+    import ctypes
+    from lokinfer_b200 import Generator, _lib, ops
+    g, (_, d) = Generator(synth.generator_weights(0), cuda), _inputs(cuda, 9, seed=6)
+    want = g.forward(*d)
+    ci = ctypes.c_int64.from_address(g.conv_state["resblocks.3.convs2.1"].handle + 16)  # wp, co, ci, k, ...
+    assert ci.value == 128
+    ci.value = 64
+    graph = torch.cuda.CUDAGraph()
+    try:
+        with ops.Profile(time_kernels=False), pytest.raises(_lib.LkcError, match="does not match the weight shape"):
+            g.forward(*d)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph):
+            with pytest.raises(_lib.LkcError, match="does not match the weight shape"):
+                g.forward(*d)
+    finally:
+        ci.value = 128
+    torch.cuda.synchronize()
+    assert torch.equal(g.forward(*d), want) and ops.conv_tc_status() == 0
