@@ -33,6 +33,9 @@ constexpr float kEps = 1e-5f;  // AdaIN
 // 432 / 713 / 853 / 1011 / 1076 (stage 0 of T = 240 and 320 gains, stage 1 of T = 24 loses).
 constexpr int kBranchSms[2][3] = {{26, 36, 70}, {26, 36, 50}}, kNoiseSms[2] = {70, 40};
 
+// Channels of the two stages, of what goes into their upsamplers, and the upsampling factors.
+constexpr int64_t kCh[2] = {256, 128}, kChIn[2] = {512, 256}, kUp[2] = {10, 6};
+
 struct Plan {
   int64_t key = 0, bytes = 0, unplanned = 0;
   std::vector<int64_t> offsets;
@@ -230,7 +233,6 @@ bool resblockOk(const LkcResblock& w) {
 // the noise branches (they need only `har`), 3 and 4 the k = 7 and k = 3 resblocks of a stage.
 void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
   const int64_t t = io.t, len[2] = {10 * t, 60 * t + 1};
-  const int64_t ch[2] = {256, 128}, cin[2] = {512, 256}, up[2] = {10, 6};
   const Buf none;
   Buf x, har;
   x.p = const_cast<float*>(FP(io.x)), x.pitch = io.x_pitch;
@@ -241,11 +243,11 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
   e.join(1, 0), e.join(2, 0);
 
   auto upsample = [&](int i, Buf in, int64_t lin, Buf res) {
-    Buf u = e.rows(0, ch[i], len[i]);
+    Buf u = e.rows(0, kCh[i], len[i]);
     e.launch(0, {in, res, u}, [&](cudaStream_t st) {
       ConvtParams p;
       p.x = in.p, p.bias = FP(m.ups_b[i]), p.res = res.p, p.out = u.p;
-      p.ci = cin[i], p.l = lin, p.co = ch[i], p.stride = up[i], p.padLeft = i, p.slope = 0.1f;
+      p.ci = kChIn[i], p.l = lin, p.co = kCh[i], p.stride = kUp[i], p.padLeft = i, p.slope = 0.1f;
       p.xPitch = in.pitch, p.resPitch = res.pitch, p.outPitch = u.pitch;
       const ConvState* cs = reinterpret_cast<const ConvState*>(m.ups_state[i]);
       return convtTc(p, cs->wp, cs->f16, st);
@@ -278,16 +280,16 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
     e.launch(s, {har, y}, [&](cudaStream_t st) {
       return spaceToDepth(har.p, y.p, 22, len[1], n.rows, ly, har.pitch, y.pitch, n.stride, n.padding, st);
     });
-    Buf xs = e.rows(s, ch[i], len[i]), xst = statsBuf(e, s, ch[i], len[i]);
-    conv(e, s, Act::None, y, ly, n.rows, ch[i], n.taps, 1, 0, n.w, n.b, none, nullptr, 0.f, n.state, none, xs, xst,
+    Buf xs = e.rows(s, kCh[i], len[i]), xst = statsBuf(e, s, kCh[i], len[i]);
+    conv(e, s, Act::None, y, ly, n.rows, kCh[i], n.taps, 1, 0, n.w, n.b, none, nullptr, 0.f, n.state, none, xs, xst,
          kNoiseSms[i]);
-    if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], AddUpsampled{e, u0, ch[0], len[0]}, kNoiseSms[i]);
+    if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], AddUpsampled{e, u0, kCh[0], len[0]}, kNoiseSms[i]);
     else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], PlainResidual{}, kNoiseSms[i]);
   }
 
   Buf in = noise[0], inStats = noiseStats[0], mean;
   for (int i = 0; i < 2; ++i) {
-    const int64_t l = len[i], c = ch[i];
+    const int64_t l = len[i], c = kCh[i];
     e.join(0, 1 + i);
     if (i == 1) {
       in = upsample(1, mean, len[0], noise[1]);
@@ -349,17 +351,39 @@ struct LkcModel {
   }
 };
 
+namespace {
+// Whether a prepared state was made for this shape (conv: stride 0), as the sequence below assumes without looking again.
+bool stateFits(const LkcConvState* state, int64_t co, int64_t ci, int64_t k, int64_t stride) {
+  const ConvState* st = reinterpret_cast<const ConvState*>(state);
+  return st && st->wp && st->co == co && st->ci == ci && st->k == k && st->stride == stride;
+}
+// A resblock of c channels whose AdaIN parameters lie inside a bank of bankN floats.
+bool resblockFits(const LkcResblock& w, int64_t c, int64_t bankN) {
+  if (!resblockOk(w) || w.c != c) return false;
+  for (int i = 0; i < 6; ++i)
+    if (w.gb[i] > bankN - 2 * c || (w.state[i] && !stateFits(w.state[i], c, c, w.k, 0))) return false;
+  return true;
+}
+}  // namespace
+
 extern "C" LKC_API LkcModel* lkc_generator_create(const LkcGenerator* w) {
   const char* bad = nullptr;
   if (!w) bad = "generator_create: null weights";
-  for (int i = 0; !bad && i < 8; ++i)
-    if (!resblockOk(i < 2 ? w->noise_res[i] : w->res[i - 2])) bad = "generator_create: bad resblock";
+  if (!bad && (!w->bank_wt || !w->bank_b || w->bank_n < 1 || w->bank_n > 0x7fffffff || !w->post_w || !w->post_b || !w->ident128))
+    bad = "generator_create: null weight";
+  for (int i = 0; !bad && i < 8; ++i) {
+    const LkcResblock& rb = i < 2 ? w->noise_res[i] : w->res[i - 2];
+    if (!resblockFits(rb, kCh[i < 2 ? i : (i - 2) / 3], w->bank_n)) bad = "generator_create: bad resblock";
+  }
   for (int i = 0; !bad && i < 2; ++i) {
     const LkcNoiseConv& n = w->noise_conv[i];
-    if (!n.w || !n.b || !n.state || n.stride < 1 || n.taps < 1 || n.rows < 22 * n.stride) bad = "generator_create: bad noise conv";
-    else if (!w->ups_b[i] || !w->ups_state[i]) bad = "generator_create: bad upsampler";
+    if (!n.w || !n.b || n.stride < 1 || n.stride > 64 || n.padding < 0 || n.taps < 1 || n.rows < 22 * n.stride ||
+        !stateFits(n.state, kCh[i], n.rows, n.taps, 0))
+      bad = "generator_create: bad noise conv";
+    else if (!w->ups_b[i] || !stateFits(w->ups_state[i], kCh[i], kChIn[i], 2 * kUp[i], kUp[i]))
+      bad = "generator_create: bad upsampler";
   }
-  if (!bad && (!w->bank_wt || !w->bank_b || w->bank_n < 1 || !w->post_w || !w->post_b || !w->ident128)) bad = "generator_create: null weight";
+  if (!bad && w->post_state && !stateFits(w->post_state, 22, kCh[1], 7, 0)) bad = "generator_create: bad conv_post";
   LkcModel* m = bad ? nullptr : new (std::nothrow) LkcModel;
   if (!m) {
     fail(bad ? bad : "generator_create: out of host memory");
