@@ -5,6 +5,8 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <exception>
+#include <new>
 
 #include "lkc.h"
 
@@ -26,6 +28,18 @@ inline int launched(const char* what) {
     return failCuda(what, e);
   }
   return 0;
+}
+
+// Runs the body of a C entry point that allocates host memory: an exception becomes an error code.
+template <class Fn>
+int noThrow(Fn body) {
+  try {
+    return body();
+  } catch (const std::bad_alloc&) {
+    return fail("out of host memory");
+  } catch (const std::exception&) {
+    return fail("unexpected exception");
+  }
 }
 
 #define LKC_REQUIRE(cond, msg) \

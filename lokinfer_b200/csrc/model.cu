@@ -411,12 +411,14 @@ extern "C" LKC_API void lkc_model_destroy(LkcModel* m) {
 extern "C" LKC_API int lkc_generator_workspace(LkcModel* m, int64_t t, int concurrent, int64_t* bytes, int64_t* unplanned) {
   LKC_REQUIRE(m && bytes, "generator_workspace: null argument");
   LKC_REQUIRE(t >= 1 && t < (int64_t(1) << 24), "generator_workspace: t out of range");
-  std::lock_guard<std::mutex> lock(m->mutex);
-  std::shared_ptr<const Plan> p;
-  if (int rc = m->plan(t, concurrent != 0, &p)) return rc;
-  *bytes = p->bytes;
-  if (unplanned) *unplanned = p->unplanned;
-  return 0;
+  return noThrow([&] {
+    std::lock_guard<std::mutex> lock(m->mutex);
+    std::shared_ptr<const Plan> p;
+    if (int rc = m->plan(t, concurrent != 0, &p)) return rc;
+    *bytes = p->bytes;
+    if (unplanned) *unplanned = p->unplanned;
+    return 0;
+  });
 }
 
 extern "C" LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, void* stream) {
@@ -427,16 +429,18 @@ extern "C" LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, vo
   LKC_REQUIRE((reinterpret_cast<uintptr_t>(io->workspace) & 255) == 0, "generator_forward: the workspace must be 256-byte aligned");
   // The events and the order of record and wait on them belong to one forward at a time; queueing is all that happens
   // under the lock.
-  std::lock_guard<std::mutex> lock(m->mutex);
-  std::shared_ptr<const Plan> p;
-  if (int rc = m->plan(io->t, io->concurrent != 0, &p)) return rc;
-  LKC_REQUIRE(io->workspace_bytes >= p->bytes, "generator_forward: the workspace is too small (lkc_generator_workspace)");
-  Exec e(io->concurrent != 0, *p, static_cast<char*>(io->workspace), S(stream),
-         reinterpret_cast<const cudaStream_t*>(io->side), m->events);
-  generator(e, m->w, *io);
-  if (e.rc != 0) e.joinForked();
-  io->launches = e.launches;
-  return e.rc;
+  return noThrow([&] {
+    std::lock_guard<std::mutex> lock(m->mutex);
+    std::shared_ptr<const Plan> p;
+    if (int rc = m->plan(io->t, io->concurrent != 0, &p)) return rc;
+    LKC_REQUIRE(io->workspace_bytes >= p->bytes, "generator_forward: the workspace is too small (lkc_generator_workspace)");
+    Exec e(io->concurrent != 0, *p, static_cast<char*>(io->workspace), S(stream),
+           reinterpret_cast<const cudaStream_t*>(io->side), m->events);
+    generator(e, m->w, *io);
+    if (e.rc != 0) e.joinForked();
+    io->launches = e.launches;
+    return e.rc;
+  });
 }
 
 namespace {
@@ -460,18 +464,20 @@ extern "C" LKC_API int lkc_resblock(const LkcResblock* w, LkcResblockIo* io, voi
   LKC_REQUIRE(w->c <= 65535, "resblock: too many channels");  // channel_stats: one grid row per channel
   LKC_REQUIRE(((reinterpret_cast<uintptr_t>(io->stats) | reinterpret_cast<uintptr_t>(io->out_stats)) & 7) == 0,
               "resblock: stats and out_stats must be 8-byte aligned");
-  Plan p;
-  Exec plan(false);
-  resblockCall(plan, *w, *io);
-  if (int rc = plan.finishPlan(&p)) return rc;
-  if (!io->workspace) {  // the size only
-    io->workspace_bytes = p.bytes;
-    return 0;
-  }
-  LKC_REQUIRE((reinterpret_cast<uintptr_t>(io->workspace) & 255) == 0 && io->workspace_bytes >= p.bytes,
-              "resblock: the workspace must be 256-byte aligned and hold what the size call says");
-  Exec e(false, p, static_cast<char*>(io->workspace), S(stream), nullptr, nullptr);
-  resblockCall(e, *w, *io);
-  io->launches = e.launches;
-  return e.rc;
+  return noThrow([&] {
+    Plan p;
+    Exec plan(false);
+    resblockCall(plan, *w, *io);
+    if (int rc = plan.finishPlan(&p)) return rc;
+    if (!io->workspace) {  // the size only
+      io->workspace_bytes = p.bytes;
+      return 0;
+    }
+    LKC_REQUIRE((reinterpret_cast<uintptr_t>(io->workspace) & 255) == 0 && io->workspace_bytes >= p.bytes,
+                "resblock: the workspace must be 256-byte aligned and hold what the size call says");
+    Exec e(false, p, static_cast<char*>(io->workspace), S(stream), nullptr, nullptr);
+    resblockCall(e, *w, *io);
+    io->launches = e.launches;
+    return e.rc;
+  });
 }

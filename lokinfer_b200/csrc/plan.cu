@@ -15,9 +15,8 @@
 // clock of the allocating stream when tensor i was allocated; last_use[i * S + s]: the largest count of stream s at
 // which tensor i was used (its allocation included; 0 = never on that stream). align: power of two. Writes
 // offsets[i] and *total (arena bytes). Returns 0, or non-zero with lkc_last_error() on bad arguments.
-extern "C" LKC_API int lkc_plan_memory(int64_t n, int64_t num_streams, const int64_t* bytes, const int32_t* pinned,
-                                       const int64_t* alloc_clock, const int64_t* last_use, int64_t align,
-                                       int64_t* offsets, int64_t* total) {
+static int plan(int64_t n, int64_t num_streams, const int64_t* bytes, const int32_t* pinned, const int64_t* alloc_clock,
+                const int64_t* last_use, int64_t align, int64_t* offsets, int64_t* total) {
   LKC_REQUIRE(n >= 0 && num_streams >= 1 && align >= 1 && (align & (align - 1)) == 0, "plan_memory: bad sizes");
   LKC_REQUIRE(n == 0 || (bytes && pinned && alloc_clock && last_use && offsets), "plan_memory: null array");
   LKC_REQUIRE(total, "plan_memory: null total");
@@ -45,4 +44,10 @@ extern "C" LKC_API int lkc_plan_memory(int64_t n, int64_t num_streams, const int
   }
   *total = top;
   return 0;
+}
+
+extern "C" LKC_API int lkc_plan_memory(int64_t n, int64_t num_streams, const int64_t* bytes, const int32_t* pinned,
+                                       const int64_t* alloc_clock, const int64_t* last_use, int64_t align,
+                                       int64_t* offsets, int64_t* total) {
+  return lkc::noThrow([&] { return plan(n, num_streams, bytes, pinned, alloc_clock, last_use, align, offsets, total); });
 }
