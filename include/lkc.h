@@ -272,7 +272,8 @@ LKC_API int lkc_plan_memory(int64_t n, int64_t num_streams, const int64_t* bytes
  * No counterpart in the reference, whose runtime walks a compiled program; here one call queues what Generator.forward
  * composes from the entry points above (models/kokoro/model.py:735-781), resp. one AdaINResBlock1 (:235-247). The caller
  * owns all memory: weights and packs (device pointers) live as long as the handle, the workspace until the work queued by
- * the call has finished; every intermediate lives in the workspace, overlaid by lkc_plan_memory. */
+ * the call has finished; every intermediate lives in the workspace, overlaid by lkc_plan_memory.
+ * lkc_generator_workspace takes the `concurrent` of the forward it is asked for. */
 typedef struct LkcResblock {
   int64_t c, k;
   /* index 2 j + (n - 1): convs{n}.{j} / alpha{n}.{j} / adain{n}.{j}; gb = offset (floats) of that AdaIN's (gamma | beta) in
@@ -296,14 +297,16 @@ typedef struct LkcGenerator {
   const void *post_w, *post_b, *ident128; /* ident128: identity affine f32[3, 128] */
   const LkcConvState* post_state;
 } LkcGenerator;
+#define LKC_UNPLANNED 2
 typedef struct LkcGeneratorIo {
   const void *x, *har, *s; /* f32[512, t], f32[22, 60 t + 1], f32[128] */
   void *audio, *post;      /* f32[300 t]; f32[22, 60 t + 1] or NULL */
   int64_t t, x_pitch, har_pitch, post_pitch;
   void* workspace;
   int64_t workspace_bytes;
-  void* side[4];    /* streams for the independent branches (concurrent != 0); joined back before the call's last kernel */
-  int64_t concurrent;
+  void* side[4];    /* streams for the independent branches (if concurrent); joined back before the call's last kernel */
+  int64_t concurrent; /* 0: one stream; otherwise the branches run side by side. LKC_UNPLANNED and LKC_UNPLANNED | 1: 0 and
+                         1 with bytes of its own for every intermediate, nothing overlaid */
   int64_t launches; /* out: kernels queued */
 } LkcGeneratorIo;
 typedef struct LkcResblockIo {

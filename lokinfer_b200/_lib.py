@@ -41,6 +41,9 @@ class LkcGenerator(ctypes.Structure):
                 ("post_state", ctypes.c_void_p)]
 
 
+LKC_UNPLANNED = 2
+
+
 class LkcGeneratorIo(ctypes.Structure):
     _fields_ = [("x", ctypes.c_void_p), ("har", ctypes.c_void_p), ("s", ctypes.c_void_p), ("audio", ctypes.c_void_p),
                 ("post", ctypes.c_void_p), ("t", ctypes.c_int64), ("x_pitch", ctypes.c_int64),

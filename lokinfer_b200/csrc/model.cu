@@ -112,10 +112,11 @@ class Exec {
       if (forked_[s]) order(0, s);
   }
 
-  int finishPlan(Plan* out) {
+  // overlay = false: every tensor gets bytes of its own.
+  int finishPlan(Plan* out, bool overlay = true) {
     const int64_t n = int64_t(bytes_.size());
     out->offsets.assign(size_t(n), 0);
-    const std::vector<int32_t> pinned(size_t(n), 0);
+    const std::vector<int32_t> pinned(size_t(n), overlay ? 0 : 1);
     for (int64_t b : bytes_) out->unplanned += (b + 255) / 256 * 256;
     return lkc_plan_memory(n, kStreams, bytes_.data(), pinned.data(), allocClock_.data(), lastUse_.data(), 256,
                            out->offsets.data(), &out->bytes);
@@ -323,14 +324,20 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
 
 using namespace lkc;
 
+namespace {
+bool isConcurrent(int64_t mode) { return mode != 0 && mode != LKC_UNPLANNED; }
+}  // namespace
+
 struct LkcModel {
   LkcGenerator w;
   cudaEvent_t events[kEvents] = {};
   std::mutex mutex;
   std::list<std::shared_ptr<const Plan>> plans;  // most recently used first
 
-  int plan(int64_t t, bool concurrent, std::shared_ptr<const Plan>* out) {
-    const int64_t key = 2 * t + (concurrent ? 1 : 0);
+  // mode = LkcGeneratorIo.concurrent
+  int plan(int64_t t, int64_t mode, std::shared_ptr<const Plan>* out) {
+    const bool overlay = mode != LKC_UNPLANNED && mode != (LKC_UNPLANNED | 1), concurrent = isConcurrent(mode);
+    const int64_t key = 4 * t + (overlay ? 2 : 0) + (concurrent ? 1 : 0);
     for (auto it = plans.begin(); it != plans.end(); ++it)
       if ((*it)->key == key) {
         plans.splice(plans.begin(), plans, it);
@@ -343,7 +350,7 @@ struct LkcModel {
     io.t = t;
     Exec e(concurrent);
     generator(e, w, io);
-    if (int rc = e.finishPlan(p.get())) return rc;
+    if (int rc = e.finishPlan(p.get(), overlay)) return rc;
     plans.push_front(p);
     if (plans.size() > kPlans) plans.pop_back();
     *out = p;
@@ -414,7 +421,7 @@ extern "C" LKC_API int lkc_generator_workspace(LkcModel* m, int64_t t, int concu
   return noThrow([&] {
     std::lock_guard<std::mutex> lock(m->mutex);
     std::shared_ptr<const Plan> p;
-    if (int rc = m->plan(t, concurrent != 0, &p)) return rc;
+    if (int rc = m->plan(t, concurrent, &p)) return rc;
     *bytes = p->bytes;
     if (unplanned) *unplanned = p->unplanned;
     return 0;
@@ -432,9 +439,9 @@ extern "C" LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, vo
   return noThrow([&] {
     std::lock_guard<std::mutex> lock(m->mutex);
     std::shared_ptr<const Plan> p;
-    if (int rc = m->plan(io->t, io->concurrent != 0, &p)) return rc;
+    if (int rc = m->plan(io->t, io->concurrent, &p)) return rc;
     LKC_REQUIRE(io->workspace_bytes >= p->bytes, "generator_forward: the workspace is too small (lkc_generator_workspace)");
-    Exec e(io->concurrent != 0, *p, static_cast<char*>(io->workspace), S(stream),
+    Exec e(isConcurrent(io->concurrent), *p, static_cast<char*>(io->workspace), S(stream),
            reinterpret_cast<const cudaStream_t*>(io->side), m->events);
     generator(e, m->w, *io);
     if (e.rc != 0) e.joinForked();

@@ -233,18 +233,20 @@ class Generator:
         return model
 
     @staticmethod
-    def _workspace_bytes(model, t, concurrent):
-        """(planned, unplanned) bytes of the intermediates of one forward of length t."""
+    def _workspace_bytes(model, t, concurrent, planned=True):
+        """(bytes of the workspace, bytes without a plan) of the intermediates of one forward of length t."""
         b, u = ctypes.c_int64(0), ctypes.c_int64(0)
-        if _lib.lib().lkc_generator_workspace(model.handle, t, int(concurrent), ctypes.byref(b), ctypes.byref(u)) != 0:
+        mode = int(concurrent) if planned else int(concurrent) | _lib.LKC_UNPLANNED
+        if _lib.lib().lkc_generator_workspace(model.handle, t, mode, ctypes.byref(b), ctypes.byref(u)) != 0:
             raise _lib.LkcError(_lib.last_error())
         return b.value, u.value
 
-    def _forward_whole(self, model, x, har, s, outputs, concurrent, workspace=None):
+    def _forward_whole(self, model, x, har, s, outputs, concurrent, workspace=None, planned=True):
+        """planned=False: every intermediate has bytes of its own in the workspace."""
         t, dev = int(x.shape[1]), self.device
         sh = shapes(t)
         if workspace is None:
-            workspace = torch.empty(self._workspace_bytes(model, t, concurrent)[0], dtype=torch.uint8, device=dev)
+            workspace = torch.empty(self._workspace_bytes(model, t, concurrent, planned)[0], dtype=torch.uint8, device=dev)
         io = _lib.LkcGeneratorIo()
         res = {"audio": torch.empty(sh["S"], dtype=torch.float32, device=dev)}
         if "post" in outputs:
@@ -254,7 +256,7 @@ class Generator:
         io.x, io.har, io.s, io.audio = x.data_ptr(), har.data_ptr(), s.data_ptr(), res["audio"].data_ptr()
         io.t, io.x_pitch, io.har_pitch = t, x.stride(0), har.stride(0)
         io.workspace, io.workspace_bytes = workspace.data_ptr(), workspace.numel()
-        io.concurrent = int(concurrent)
+        io.concurrent = int(concurrent) if planned else int(concurrent) | _lib.LKC_UNPLANNED
         if concurrent:
             io.side[:] = [st.cuda_stream for st in self._side_streams()]
         if _lib.lib().lkc_generator_forward(model.handle, ctypes.byref(io), ops._stream()) != 0:
@@ -489,7 +491,8 @@ class Generator:
         planned=True (default): the forward's intermediates live in a planned arena, ONE device buffer in which tensors
         that are never alive together (judged by the fork / join structure of the streams, not by program order) overlay
         each other (`arena_bytes`; `unplanned_bytes` is what keeping every intermediate would take). The plan is the
-        whole-forward call's own; the op-by-op forward of the CUDA-core path is traced and planned by arena.py."""
+        whole-forward call's own; the op-by-op forward of the CUDA-core path is traced and planned by arena.py.
+        planned=False: every intermediate has memory of its own, in the graph's pool."""
         if t in self._graphs:
             return self._graphs[t]
         from .arena import PlannedArena, Tracer
@@ -523,8 +526,9 @@ class Generator:
         torch.cuda.synchronize(dev)
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
-            if "arena" in bufs:
-                bufs["audio"] = self._forward_whole(model, bufs["x"], bufs["har"], bufs["s"], ("audio",), True, bufs["arena"])
+            if whole:
+                bufs["audio"] = self._forward_whole(model, bufs["x"], bufs["har"], bufs["s"], ("audio",), True,
+                                                    bufs.get("arena"), planned)
             elif arena is not None:
                 arena.begin()
                 with ops.use_allocator(arena.allocator):

@@ -138,6 +138,10 @@ def test_generator_config2_stages_vs_oracle(cuda, gen):
             assert rel_l2(got_rb[j].cpu().numpy(), ref[name][j].numpy()) <= 24 * REL_L2, (name, j)
     assert rel_l2(post.cpu().numpy(), ref["post"].numpy()) <= 48 * REL_L2
     assert np.abs(audio.cpu().numpy() - ref["audio"].numpy()).max() <= WAVE_MAXABS
+    # stage0 / stage1 make the forward run op by op; without them it is one library call
+    post, audio = gen.forward(*d, outputs=("post", "audio"))
+    assert rel_l2(post.cpu().numpy(), ref["post"].numpy()) <= 48 * REL_L2
+    assert np.abs(audio.cpu().numpy() - ref["audio"].numpy()).max() <= WAVE_MAXABS
     from lokinfer_b200 import ops
     assert ops.conv_tc_status() == 0
 
@@ -153,8 +157,8 @@ def test_graph_replay_matches_eager(cuda, gen):
 
 
 def test_planned_arena(cuda):
-    """The captured forward lives in a planned arena: identical samples to the eager forward (every intermediate its
-    own allocation) and to a capture without the plan, in well under the memory of keeping every intermediate."""
+    """The captured forward lives in a planned arena: identical samples to a capture without the plan (every intermediate
+    has memory of its own) and to the eager forward, in well under the memory of keeping every intermediate."""
     from lokinfer_b200 import Generator, ops
     t = 416
     inp = synth.generator_inputs(t, 9)
@@ -330,3 +334,63 @@ def test_error_inside_a_forward_joins_its_streams(cuda):
         ci.value = 128
     torch.cuda.synchronize()
     assert torch.equal(g.forward(*d), want) and ops.conv_tc_status() == 0
+
+
+@pytest.mark.parametrize("t", [1, 7, 24, 121, 320, 747, 801])
+@pytest.mark.parametrize("concurrent", [True, False])
+def test_memory_plan_changes_nothing(cuda, gen, t, concurrent):
+    """The whole-forward call in its planned workspace against the same call with memory of its own for every intermediate:
+    the same bits, from workspaces full of NaN, one and several forwards of different lengths in flight."""
+    from lokinfer_b200 import ops
+    inp, d = _inputs(cuda, t, seed=60 + t)
+    model = gen._whole_model()
+    got = []
+    for planned in (False, True, True):
+        n, unplanned = gen._workspace_bytes(model, t, concurrent, planned)
+        assert n <= unplanned if planned else n == unplanned
+        ws = torch.full((n,), 255, dtype=torch.uint8, device=cuda)  # every float a NaN
+        got.append(gen._forward_whole(model, *d, ("post", "audio"), concurrent, ws, planned))
+    torch.cuda.synchronize()
+    for post, audio in got[1:]:
+        assert torch.equal(post, got[0][0]) and torch.equal(audio, got[0][1])
+    assert torch.isfinite(got[0][1]).all() and ops.conv_tc_status() == 0
+
+
+@pytest.mark.parametrize("t", [5, 24, 121, 320])
+def test_whole_forward_agrees_with_the_composition(cuda, gen, t):
+    """The whole-forward call and the op-by-op form differ in where the upsampled input is added, in who folds the
+    statistics and in how partial sums are split, not beyond rounding."""
+    from lokinfer_b200 import ops
+    _, d = _inputs(cuda, t, seed=80 + t)
+    post, audio = gen.forward(*d, outputs=("post", "audio"))
+    post2, audio2, _ = gen.forward(*d, outputs=("post", "audio", "stage0"))
+    assert rel_l2(post.cpu().numpy(), post2.cpu().numpy()) <= 48 * REL_L2
+    assert (audio - audio2).abs().max().item() <= WAVE_MAXABS
+
+
+def test_one_generator_in_several_threads(cuda, gen):
+    """Forwards of different lengths from four threads, each on its own stream: every result as from one thread."""
+    import threading
+    jobs = [(t, _inputs(cuda, t, seed=90 + t)[1]) for t in (9, 24, 61, 130)]
+    want = [gen.forward(*d).clone() for _, d in jobs]
+    torch.cuda.synchronize()
+    wrong, errors = [], []
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream(device=cuda)):
+                for _ in range(10):
+                    model = gen._whole_model()
+                    out = gen._forward_whole(model, *jobs[i][1], ("audio",), True)
+                    if not torch.equal(out, want[i]):
+                        wrong.append(jobs[i][0])
+        except Exception as e:  # a thread's exception would be lost
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    torch.cuda.synchronize()
+    assert not errors and not wrong
