@@ -160,6 +160,10 @@ LKC_API int64_t lkc_conv1d_tc_pack_floats(int64_t co, int64_t ci, int64_t k);
 LKC_API int lkc_conv1d_tc_pack_f32_cuda(const LkcArgs* a, void* stream);
 LKC_API LkcConvState* lkc_conv1d_state_create(const void* wp, int64_t co, int64_t ci, int64_t k);
 LKC_API void lkc_conv1d_state_destroy(LkcConvState* st);
+/* The rule by which a conv with f16 halves is split (host code, nothing is launched): CTAs that contract one 128-column x
+ * 128-channel tile together, 0 = a CTA per tile. sms = SMs the launch may use; clusters[n], n = 2..8 = clusters of n CTAs
+ * resident at a time on the device (9 entries; cudaOccupancyMaxActiveClusters). */
+LKC_API int lkc_conv1d_tc_split(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* clusters);
 LKC_API int lkc_conv1d_tc_status(int* status, int reset);
 /* Stream-ordered form for callers that keep several utterances in flight: queues a 4-byte copy of the status word
  * into status_host (pinned host memory) behind the work already on `stream`; synchronises nothing, clears nothing. */

@@ -253,6 +253,11 @@ extern "C" LKC_API LkcConvState* lkc_conv1d_state_create(const void* wp, int64_t
   return lkc_conv1d_state_create_as(wp, co, ci, k, currentFormat());
 }
 
+extern "C" LKC_API int lkc_conv1d_tc_split(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* clusters) {
+  if (ci < 16 || ci % 16 != 0 || ci > 4096 || co < 1 || co > (1 << 30) || lo < 1 || lo > (1 << 30) || sms < 1 || !clusters) return 0;
+  return convTcSplitRule(ci, co, lo, sms, clusters);
+}
+
 extern "C" LKC_API void lkc_conv1d_state_destroy(LkcConvState* st) { delete reinterpret_cast<ConvState*>(st); }
 
 // ints: w(Ci, Co, K) wp(n) padding stride [format]

@@ -51,6 +51,8 @@
 // All hand-offs are mbarriers. Every wait is bounded: on a timeout the kernel records a status word, drains its
 // copies in flight and returns (TMEM is freed on every path).
 #include <cuda.h>
+
+#include <algorithm>
 #include <cuda_fp16.h>
 
 #include <cstdlib>
@@ -1587,7 +1589,31 @@ struct DeviceInfo {
   int* status = nullptr;
   long long* prof = nullptr;
   int smCount = 0;
+  int32_t clusters[MAX_SPLIT + 1] = {};  // [n]: clusters of n CTAs of the split form that the device holds at a time
 };
+// A cluster lives inside one GPC, of whose SMs a remainder is left over: 148 SMs hold 74 clusters of two, but 45 of three,
+// 33 of four, 26 of five, 22 of six, 15 of seven or eight (one B200; which SMs are fused off differs).
+static void countClusters(DeviceInfo& d) {
+  const auto kernel = convTcKernel<1, false, 0, true, false, true>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) {
+    cudaGetLastError();
+    return;  // no split launches
+  }
+  for (int n = 2; n <= MAX_SPLIT; ++n) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(n), attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(unsigned(n) * unsigned(d.smCount)), cfg.blockDim = dim3(NTHREADS), cfg.dynamicSmemBytes = SPLIT_SMEM;
+    cfg.attrs = attr, cfg.numAttrs = 1;
+    int count = 0;
+    if (cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      count = 0;
+    }
+    d.clusters[n] = count;
+  }
+}
 static int deviceInfo(const DeviceInfo** out) {
   static DeviceInfo info[64];
   int dev = 0;
@@ -1604,6 +1630,7 @@ static int deviceInfo(const DeviceInfo** out) {
     e = cudaGetSymbolAddress(reinterpret_cast<void**>(&pp), gTcProf);
     if (e != cudaSuccess) return failCuda("conv (tensor-core): cudaGetSymbolAddress", e);
     d.prof = pp;
+    countClusters(d);
     d.status = ptr;
   }
   *out = &d;
@@ -1741,28 +1768,33 @@ int convTcProfile(int enable, long long* out16) {
 }
 
 // CTAs per tile: 0 = the persistent form. The split form is taken where at least two CTAs per 128-column tile fit on the
-// launch's share of the SMs, all in one wave: there the time is one tile's chain of 16-channel chunks plus about 9 us of
-// fixed cost (launch, first loads, cluster reduction), and the chain shrinks with every CTA. With one CTA per tile
-// it gains little over 256-column tiles (an M128 N128 MMA takes about 0.8 of the time of an N256 one here) and doubles
-// the weight traffic; with a second wave it loses. Measured (us, persistent -> split): [256, 240] K = 11: 52 -> 15;
-// [256, 1210] K = 7: 49 -> 17; [128, 1441] K = 3: 29 -> 12; [1104 -> 1024, 61] K = 3: 130 -> 19; [256, 3200] K = 11, two
-// CTAs per tile: 52 -> 30, and with a second wave (four) 39.
-static int splitFor(bool f16, int ci, int64_t lo, int coBlocks, int sms) {
+// launch's share of the SMs and all its clusters are resident at a time (clusters[n], see countClusters): there the time is
+// one tile's chain of 16-channel chunks plus about 9 us of fixed cost (launch, first loads, cluster reduction), and the
+// chain shrinks with every CTA. With one CTA per tile it gains little over 256-column tiles (an M128 N128 MMA takes about
+// 0.8 of the time of an N256 one here) and doubles the weight traffic; with a second wave it loses: [128, 6144] K = 11,
+// 48 clusters of three where 45 fit, 36 us against 30 us unsplit and 21 us with two CTAs per tile.
+// Measured (us, persistent -> split): [256, 240] K = 11: 52 -> 15; [256, 1210] K = 7: 49 -> 17; [128, 1441] K = 3: 29 -> 12;
+// [1104 -> 1024, 61] K = 3: 130 -> 19; [256, 3200] K = 11, two CTAs per tile: 52 -> 30.
+static int splitFor(bool f16, int ci, int64_t lo, int64_t coBlocks, int sms, const int32_t* clusters) {
   if (!f16) return 0;
   const int n = ci / KC;
-  int sp = int(sms / (ceilDiv(lo, NTS) * coBlocks));
-  if (sp > MAX_SPLIT) sp = MAX_SPLIT;
-  if (sp > n) sp = n;
-  if (sp < 2) return 0;
-  const int serial = (n + sp - 1) / sp;
-  return (n + serial - 1) / serial;  // no more CTAs than shorten the longest run
+  const int64_t tiles = ceilDiv(lo, NTS) * coBlocks;
+  for (int sp = int(std::min<int64_t>(std::min(MAX_SPLIT, n), sms / tiles)); sp >= 2; --sp) {
+    const int serial = (n + sp - 1) / sp, ctas = (n + serial - 1) / serial;  // no more CTAs than shorten the longest run
+    if (tiles <= clusters[ctas]) return ctas;
+  }
+  return 0;
+}
+
+int convTcSplitRule(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* clusters) {
+  return splitFor(true, int(ci), lo, ceilDiv(co, MT), sms, clusters);
 }
 
 // Launch geometry and tensor maps shared by the conv and ConvTranspose entry points.
 static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercent, int* grid, size_t* smem) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
-  a.split = splitFor(f16, a.ci, a.lo, a.numCoBlk, d->smCount * smPercent / 100);
+  a.split = splitFor(f16, a.ci, a.lo, a.numCoBlk, d->smCount * smPercent / 100, d->clusters);
   LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
   const int nt = a.split ? NTS : NT;
   a.numTTiles = int(ceilDiv(a.lo, nt));
@@ -1798,7 +1830,7 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercen
 bool convTcSplits(const ConvFusedParams& p, bool f16) {
   const DeviceInfo* d = nullptr;
   return deviceInfo(&d) == 0 &&
-         splitFor(f16, int(p.ci), p.lo, int(ceilDiv(p.co, MT)), d->smCount * p.smPercent / 100) != 0;
+         splitFor(f16, int(p.ci), p.lo, ceilDiv(p.co, MT), d->smCount * p.smPercent / 100, d->clusters) != 0;
 }
 
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {

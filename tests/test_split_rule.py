@@ -1,0 +1,39 @@
+"""The rule that splits a conv's tiles over clusters of CTAs (host code): every cluster of a launch is resident at once."""
+import ctypes
+
+import pytest
+
+from lokinfer_b200 import _lib
+
+SMS = 148
+CLUSTERS = (0, 0, 74, 45, 33, 26, 22, 15, 15)  # what cudaOccupancyMaxActiveClusters answers on a B200
+
+
+def split(ci, co, lo, sms=SMS, clusters=CLUSTERS):
+    table = (ctypes.c_int32 * 9)(*clusters)
+    return _lib.lib().lkc_conv1d_tc_split(ci, co, lo, sms, table)
+
+
+@pytest.mark.parametrize("c", [16, 32, 48, 112, 128, 256, 512, 1104, 4096])
+@pytest.mark.parametrize("sms", [SMS, SMS * 26 // 100, SMS * 70 // 100, 1, 7])
+def test_every_split_launch_is_resident_at_once(c, sms):
+    blocks, chunks = -(-c // 128), c // 16
+    for lo in [*range(1, 1400, 41), *range(1023, 9700, 129), 9472, 9473, 20000]:
+        for clusters in (CLUSTERS, (0,) * 9, (0, 0, 60, 40, 30, 20, 20, 8, 1)):
+            n, tiles = split(c, c, lo, sms, clusters), -(-lo // 128) * blocks
+            assert n == 0 or 2 <= n <= min(8, chunks)
+            if n:
+                assert tiles <= clusters[n] and tiles * n <= sms
+                assert -(-chunks // n) < -(-chunks // (n - 1))  # no CTA that shortens no run
+            else:  # nothing would fit
+                for m in range(2, min(8, chunks, sms // tiles) + 1):
+                    ctas = -(-chunks // -(-chunks // m))
+                    assert tiles > clusters[ctas]
+
+
+def test_lengths_around_the_limits():
+    assert split(128, 128, 15 * 128) == 8 and split(128, 128, 15 * 128 + 1) == 4  # 16 tiles: 15 clusters of eight fit
+    assert split(128, 128, 48 * 128) == 2  # 45 clusters of three fit
+    assert split(256, 256, 896) == 8 and split(256, 256, 897) == 6
+    assert split(128, 128, 9472) == 2 and split(128, 128, 9473) == 0
+    assert split(16, 16, 1) == 0 and split(100, 16, 1) == 0 and split(128, 128, 0) == 0
