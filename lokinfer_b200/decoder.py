@@ -49,7 +49,8 @@ class Decoder:
             if cin != cout:
                 self.state[name + ".conv1x1"] = ops.conv1d_prepare_f32_cuda(w[name + ".conv1x1.weight"], "tf32")
                 w[name + ".conv1x1.bias"] = torch.zeros(cout, device=self.device)
-        self.state["decoder.asr_res.0"] = ops.conv1d_prepare_f32_cuda(w["decoder.asr_res.0.weight"], "tf32")
+        if "decoder.asr_res.0.weight" in w:  # only forward() needs it: a state dict of the blocks is enough for adain_resblk*
+            self.state["decoder.asr_res.0"] = ops.conv1d_prepare_f32_cuda(w["decoder.asr_res.0.weight"], "tf32")
         # style bank: every `<name>.fc` of the decoder as one GEMV (models/kokoro/model.py:67-81, names sorted)
         names = sorted(k[: -len(".weight")] for k in w if k.endswith(".fc.weight"))
         # The (gamma | beta) of a norm1 carry their zeros for the appended rows: gamma, zeros, beta, zeros.

@@ -35,6 +35,13 @@ def test_decoder_leaves_the_conv_path_alone(no_gpu, monkeypatch):
     assert all(f in ("f16", "tf32") for f in fmt.values())
 
 
+def test_decoder_of_the_blocks_alone(no_gpu):
+    """adain_resblk* need the blocks' weights only; asr_res, F0_conv and N_conv are forward()'s."""
+    sd = synth.decoder_weights(0)
+    dec = decoder.Decoder({n: v for n, v in sd.items() if n.startswith(("decoder.encode.", "decoder.decode."))}, "cpu")
+    assert set(dec.state) == set(decoder.Decoder(sd, "cpu").state) - {"decoder.asr_res.0"}
+
+
 def test_weight_beyond_f16_is_packed_again_without_a_switch(no_gpu, monkeypatch):
     switched = []
     monkeypatch.setattr(ops, "set_conv_path", lambda mode: switched.append(mode))
