@@ -535,7 +535,7 @@ class Generator:
                     bufs["audio"] = self.forward(bufs["x"], bufs["har"], bufs["s"])
             else:
                 bufs["audio"] = self.forward(bufs["x"], bufs["har"], bufs["s"])
-        bufs["graph"] = g
+        bufs["graph"], bufs["model"] = g, model  # the model keeps the weights that the graph reads, whatever replaces them
         if arena is not None:
             bufs["arena"], bufs["arena_bytes"], bufs["unplanned_bytes"] = arena, arena.nbytes, arena.unplanned_bytes
         self._graphs[t] = bufs

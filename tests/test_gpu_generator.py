@@ -394,3 +394,21 @@ def test_one_generator_in_several_threads(cuda, gen):
         th.join()
     torch.cuda.synchronize()
     assert not errors and not wrong
+
+
+def test_captured_forward_keeps_its_weights(cuda):
+    """A weight replaced after a capture: the graph goes on with the weights it was made from, also once the next forward
+    has taken the new one and the old tensor is gone from the generator."""
+    from lokinfer_b200 import Generator
+    g, (_, d) = Generator(synth.generator_weights(0), cuda), _inputs(cuda, 9, seed=8)
+    want, b = g.forward(*d), g.capture(9)
+    for k, v in zip(("x", "har", "s"), d):
+        b[k].copy_(v)
+    for name in ("conv_post.bias", "resblocks.0.convs1.0.bias", "noise_res.1.alpha2.2"):
+        g.w[name] = g.w[name] + 0.5
+    assert not torch.equal(g.forward(*d), want)
+    filler = [torch.full((n,), float("nan"), device=cuda) for n in (22, 128, 256) for _ in range(20)]
+    b["graph"].replay()
+    torch.cuda.synchronize()
+    assert torch.equal(b["audio"], want)
+    del filler
