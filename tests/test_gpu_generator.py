@@ -23,7 +23,7 @@ def _inputs(cuda, t, seed=1):
     return inp, [ops.to_cuda(inp[k], cuda) for k in ("x", "har", "s")]
 
 
-@pytest.mark.parametrize("c,l,k", [(16, 300, 7), (128, 1201, 3), (128, 2000, 11), (256, 640, 7)])
+@pytest.mark.parametrize("c,l,k", [(16, 300, 7), (128, 1201, 3), (128, 2000, 11), (256, 640, 7), (80, 5700, 3)])
 def test_resblock(cuda, c, l, k):
     """Config 0 at reduced length: one AdaINResBlock1 (kernel k, dilations 1/3/5) through the fused ops."""
     from lokinfer_b200 import Generator, ops

@@ -151,6 +151,66 @@ def test_conv1d_few_tiles(cuda, ci, co, l, k, d, padded):
     assert ops.conv_tc_status() == 0
 
 
+# The other activations, with unequal shares: five chunks over three CTAs (34 to 45 tiles on a 148-SM device), three over
+# two; [80, 257] has one chunk per CTA. Above 45 tiles clusters of three no longer fit, below 15 clusters of eight do.
+@pytest.mark.parametrize("ci,co,l,k,d", [(80, 128, 5700, 5, 2), (48, 129, 3800, 7, 1), (80, 80, 257, 3, 1),
+                                         (128, 128, 1920, 3, 1), (128, 128, 1921, 3, 5), (128, 128, 5761, 11, 1)])
+@pytest.mark.parametrize("variant", ["snake", "snake_res", "affine"])
+def test_conv1d_few_tiles_other_activations(cuda, ci, co, l, k, d, variant):
+    from lokinfer_b200 import ops
+    x, w, b, affine, alpha, res = synth.conv_case(ci, co, l, k, ci * 37 + l + k)
+    dx, dw, db, daf, dal, dres = dev(cuda, x, w, b, affine, alpha, res)
+    kw = dict(padding=d * (k - 1) // 2, dilation=d)
+    state = ops.conv1d_prepare_f32_cuda(dw)
+
+    def call():
+        if variant == "affine":
+            return ops.conv1d_affine_f32_cuda(dx, dw, db, daf, state=state, **kw)
+        return ops.conv1d_snake_f32_cuda(dx, dw, db, daf, dal, residual=dres if variant == "snake_res" else None,
+                                         state=state, **kw)
+
+    def oracle(dt):
+        a = [O.T(v, dt) for v in (x, w, b, affine, alpha, res)]
+        if variant == "affine":
+            return O.conv1d_fused(a[0], a[1], a[2], a[3], "none", **kw)[0].numpy()
+        return O.conv1d_fused(a[0], a[1], a[2], a[3], "snake", alpha=a[4],
+                              residual=a[5] if variant == "snake_res" else None, **kw)[0].numpy()
+
+    (out, stats), (again, _) = call(), call()
+    assert torch.equal(out, again)
+    out, ref64 = out.cpu().numpy(), oracle(torch.float64)
+    assert rel_l2(out, ref64) <= 2 * rel_l2(oracle(torch.float32), ref64) + 2e-7
+    check_stats(stats.cpu().numpy(), out)
+    assert ops.conv_tc_status() == 0
+
+
+@pytest.mark.parametrize("ci,l,cut,k,d", [(128, 1201, 640, 3, 1), (256, 1000, 384, 11, 5), (48, 700, 128, 7, 3)])
+def test_conv1d_few_tiles_window(cuda, ci, l, cut, k, d):
+    """A row in two parts as the time-sharded path holds it: each part a window with real columns of its neighbour beside
+    it, what lies beyond the utterance not zero, its statistics a slice of the whole row's."""
+    from lokinfer_b200 import ops
+    x, w, b, affine, alpha, res = synth.conv_case(ci, ci, l, k, ci + l + k)
+    pad, m, n = d * (k - 1) // 2, 64, -(-l // 128)
+    dx, dw, db, daf, dal, dres = dev(cuda, x, w, b, affine, alpha, res)
+    state = ops.conv1d_prepare_f32_cuda(dw)
+    want, wstats = ops.conv1d_snake_f32_cuda(dx, dw, db, daf, dal, residual=dres, padding=pad, dilation=d, state=state)
+    out, stats = torch.full((ci, l), 9.0, device=cuda), torch.full((ci, n, 2), 9.0, device=cuda)
+    filler = torch.full((ci, m), 3.0, device=cuda)
+    for lo, hi in ((0, cut), (cut, l)):
+        left, right = (filler if lo == 0 else dx[:, lo - m:lo]), (filler if hi == l else dx[:, hi:hi + m])
+        buf = torch.cat([left, dx[:, lo:hi], right], 1).contiguous()
+        mine = stats[:, lo // 128:-(-hi // 128)]
+        width = int(buf.shape[1])
+        ops._run("conv1d_snake_res_f32_cuda", [buf, dw, db, daf, dal, dres[:, lo:hi]], [out[:, lo:hi], mine],
+                 attrs_int=[d, pad, ops.conv_tile(ci, k)], state=state.handle,
+                 window=[n, m, m if lo == 0 else 0, m + hi - lo if hi == l else width])
+    # the parts may be split over other numbers of CTAs than the whole: the same sums in another order
+    assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 2e-6
+    check_stats(stats.cpu().numpy(), out.cpu().numpy())
+    np.testing.assert_allclose(stats.cpu().numpy(), wstats.cpu().numpy(), atol=2e-4, rtol=1e-4)
+    assert ops.conv_tc_status() == 0
+
+
 def _pitched(t):
     """The same values as a [:, :L] view of rows padded to a multiple of four floats."""
     c, l = t.shape
