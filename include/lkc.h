@@ -143,7 +143,7 @@ LKC_API int lkc_conv1d_leaky_mean3_f32_cuda(const LkcArgs* a, void* stream);
  * code of the first bounded wait that gave up (0 = none); bit 0x10000 = an activation exceeded the f16 range (65504)
  * under the f16 operand split (it became an infinite operand: the output of that launch is not finite); bit 0x20000
  * = a weight exceeded that range when an f16 pack was made
- * (pack it again after lkc_set_conv_path(2): the tf32 format has the range of f32). lkc_set_conv_io(1) makes later
+ * (pack it again in LKC_FORMAT_TF32, which has the range of f32). lkc_set_conv_io(1) makes later
  * launches use 4-byte accesses even for aligned rows, lkc_set_conv_io(0) (default) the TMA unit where rows are
  * 16-byte aligned (A/B testing). lkc_set_conv_path chooses the path and the operand format of packs made
  * AFTER the call: 0 (default) tensor cores with operands split into f16 hi + f16 lo * 2^-11 (3 kind::f16 MMAs per

@@ -22,15 +22,19 @@ namespace lkc {
 namespace {
 
 constexpr int kStreams = 5;  // the caller's stream and four side streams
-constexpr int kEvents = 12;  // joins of one forward
+// Events of the joins, used in turn. A forward makes 14 joins: an event may be recorded again as soon as the wait on it has
+// been queued, which is the case when join() returns.
+constexpr int kEvents = 12;
 constexpr size_t kPlans = 16;
 constexpr float kEps = 1e-5f;  // AdaIN
 // Percent of the SMs that one launch may spread over, as other branches run beside it (on one stream too, so that both
-// ways add the same partial sums): [stage] the k = 3, 7, 11 resblocks, and the two noise branches. The longer a branch's
-// chain, the more it gets; the first noise branch is waited for one stage earlier than the second. Measured, microseconds
+// ways add the same partial sums): [stage] the k = 3, 7, 11 resblocks, and the two noise branches. What runs beside each
+// other may add up to more than 100: launches of branches rarely coincide for long, and clusters that find no room start
+// when others end. The longer a branch's chain, the more it gets; the first noise branch is waited for one stage earlier than the second. Measured, microseconds
 // per forward of T = 24 / 121 / 240 / 320 / 400 frames: no splitting 877 / 934 / 980 / 1054 / 1086; noise branches and
 // k = 7, 11 even 400 / 734 / 979 / 1052 / 1088; k = 11 at 50 in both stages 400 / 697 / 915 / 1055 / 1086, at 70 in both
-// 432 / 713 / 853 / 1011 / 1076 (stage 0 of T = 240 and 320 gains, stage 1 of T = 24 loses).
+// 432 / 713 / 853 / 1011 / 1076 (stage 0 of T = 240 and 320 gains, stage 1 of T = 24 loses); as below, and with only as
+// many CTAs per tile as the device holds clusters for: 400 / 711 / 853 / 1013 / 1091.
 constexpr int kBranchSms[2][3] = {{26, 36, 70}, {26, 36, 50}}, kNoiseSms[2] = {70, 40};
 
 // Channels of the two stages, of what goes into their upsamplers, and the upsampling factors.

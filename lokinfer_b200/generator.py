@@ -52,7 +52,8 @@ class _Held:
         self.ptrs = list(map(torch.Tensor.data_ptr, self.tensors))
 
     def current(self, objs):
-        return all(map(operator.is_, self.objs, objs)) and list(map(torch.Tensor.data_ptr, self.tensors)) == self.ptrs
+        return (len(objs) == len(self.objs) and all(map(operator.is_, self.objs, objs))
+                and list(map(torch.Tensor.data_ptr, self.tensors)) == self.ptrs)
 
 
 class _Model:
@@ -143,10 +144,13 @@ class Generator:
         """fc(style) of every AdaIN as views into one style-bank GEMV (model.py:135-144): name -> f32[2C]."""
         return StyleBank(ops.gemm_bias_f32_cuda(s.reshape(1, -1), self.bank_wt, self.bank_b).reshape(-1), self.bank_off)
 
-    # One resblock and one forward as single library calls (lkc_resblock, lkc_generator_forward): the same kernels in the
-    # same order as the compositions below, queued without a trip through Python per kernel. The compositions remain for
-    # what looks at single kernels (ops.Profile with timing, ops.tracing), for the CUDA-core path and for shapes that
-    # have no tensor-core state.
+    # One resblock and one forward as single library calls (lkc_resblock, lkc_generator_forward), queued without a trip
+    # through Python per kernel. The compositions below compute the same in single ops, not launch for launch: the whole
+    # forward adds the first upsampled input in the noise block's last conv, takes stage 0's statistics from that conv's
+    # epilogue and gives each branch a share of the SMs, and in both calls split convs fold the statistics themselves. So the
+    # last bits differ, and timings of single kernels (ops.Profile) are those of the composition. It remains for what
+    # looks at single kernels (ops.Profile with timing, ops.tracing, the stage outputs), for the CUDA-core path, for shapes
+    # that have no tensor-core state and for operands that a whole call would not check.
 
     def _is(self, t, *shape):
         """A tensor the kernels can take by its address alone."""

@@ -106,8 +106,8 @@ _profile = None
 
 def op_by_op() -> bool:
     """True while every kernel has to go through _run: single kernels are being timed or traced, results come from a
-    custom allocator, or the CUDA-core path is selected. The whole-model calls of generator.py and decoder.py then stand
-    back for their compositions."""
+    custom allocator, or the CUDA-core path is selected. The whole-block and whole-forward calls of generator.py then
+    stand back for their compositions."""
     return (_tracer is not None or (_profile is not None and _profile.time_kernels) or allocator is not _torch_alloc
             or _conv_path == "simt")
 
