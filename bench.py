@@ -589,7 +589,8 @@ def run_ours(args, rank: int, local_rank: int, world: int):
                     "product)",
                     "conv_ms_per_step": conv_ms, "conv_flops_per_step": conv_flops,
                     "note": "launches of the op-by-op form of the forward; the timed step queues the same convs in one "
-                            "library call (stage 0's statistics come from an epilogue there); conv_ms_per_step sums the launches timed one at a time on one stream (each alone on the "
+                            "library call (stage 0's statistics come from an epilogue there); conv_ms_per_step sums the "
+                            "launches timed one at a time on one stream (each alone on the "
                             "GPU, 4 graph-captured repeats per launch inside its event pair); ms_per_step is the "
                             "captured forward, where independent branches run on side streams and the tail of one "
                             "persistent conv overlaps the start of another, so it can be smaller than conv_ms_per_step",

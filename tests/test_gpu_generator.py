@@ -190,6 +190,8 @@ def test_many_captures_keep_their_plans_valid(cuda):
         inp = synth.generator_inputs(t, 500 + i)
         d = [ops.to_cuda(inp[k], cuda) for k in ("x", "har", "s")]
         eager = g.forward(*d)
+        unplanned = g._forward_whole(g._whole_model(), *d, ("audio",), True, planned=False)
+        assert torch.equal(unplanned, eager), (i, t)
         b = g.capture(t)
         for k, v in zip(("x", "har", "s"), d):
             b[k].copy_(v)
