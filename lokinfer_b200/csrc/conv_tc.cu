@@ -24,27 +24,20 @@
 // take 4-byte cp.async loads and transposed 4-byte stores instead; the arithmetic is the same on both routes.
 // No copy uses cluster multicast, and every tensor map covers memory of this GPU only.
 //
-// One persistent CTA per SM, 20 warps in 5 warpgroups, warp-specialised (registers rebalanced with setmaxnreg). A warp
-// is issued by scheduler (warp id % 4) of the SM. The MMA issuer's instructions between two MMAs are what keeps the
-// tensor pipe fed, so its scheduler (1) hosts no activation producer, only the other two light control warps and the
-// two epilogue warps that TMEM's lane rule puts there (measured: the issuer's own time outside waits fell by 15-19 %
-// against a layout with two producers on its scheduler):
+// One persistent CTA per SM, 20 warps in 5 warpgroups, warp-specialised (registers rebalanced with setmaxnreg):
 //   warps 0-7   accumulate + epilogue: 128 running sums per thread, started from the bias; the residual is added one
 //               32-column batch at a time (fetched into the warp's tile behind a Dhi drain); per drain group += Dhi
 //               (tcgen05.ld); per tile += Dlo (folded in before the tile's last drain: Dlo is complete one run of hi
 //               MMAs before Dhi is), oscale, chunk statistics and the store
-//   (launches that are bound by the producers, few MMAs per chunk, use the plain layout instead: producers 8-15,
-//   two per scheduler, control warps 16-18)
-//   warps 8, 10, 11, 12, 14, 15, 16, 18
-//               activation producers: affine -> Snake / leaky -> hi / lo split of the current chunk's raw window into
+//   warps 8-15  activation producers, two per warp scheduler: affine -> Snake / leaky -> hi / lo split of the current chunk's raw window into
 //               shared memory in the K-major no-swizzle UMMA layout [16-byte K chunk][time row][4 f32 or 8 f16
 //               channels]: a tap shift of kk*d time steps is a +16*kk*d byte offset of the descriptor start address,
 //               so one staged window serves all taps (on the unaligned route they also issue the cp.async of the next
 //               chunk's raw window)
-//   warp 9      weight producer: one cp.async.bulk per tap group (up to 6 taps; hi | lo of [128 co x 16 ci] per tap,
+//   warp 16     weight producer: one cp.async.bulk per tap group (up to 6 taps; hi | lo of [128 co x 16 ci] per tap,
 //               pre-packed in the UMMA layout, L2-resident) into a ring of shared-memory slots
-//   warp 13     MMA issuer (one lane): per tap group one wait, the group's MMAs back to back, one release
-//   warp 17     raw-window loader of the aligned route (one lane): two tiled TMA loads per chunk, one chunk ahead
+//   warp 17     MMA issuer (one elected lane): per tap group one wait, the group's MMAs back to back, one release
+//   warp 18     raw-window loader of the aligned route (one lane): two tiled TMA loads per chunk, one chunk ahead
 //   warp 19     idle (completes the fifth warpgroup)
 // Launches with few tiles take a second form of the same kernel (template parameter SPLIT): a cluster of CTAs per
 // 128-column tile, each contracting a part of the input channels, reduced over distributed shared memory.
@@ -75,15 +68,16 @@ constexpr int KC = 16;          // input channels per staged chunk (one weight s
 constexpr int MAX_NB = 4;       // most activation (hi / lo) buffers
 constexpr int NRAW = 2;         // raw-input staging buffers, filled one chunk ahead
 constexpr int EPI_WARPS = 8, PRO_WARPS = 8;
-constexpr int IDLE_WARP = 19;
+constexpr int W_WARP = EPI_WARPS + PRO_WARPS, MMA_WARP = W_WARP + 1, RAW_WARP = W_WARP + 2;
 constexpr int NWARPS = EPI_WARPS + PRO_WARPS + 4;
 constexpr int NTHREADS = NWARPS * 32;  // 640
-// warpgroups 2-4 mix producers and control warps, and setmaxnreg takes one value per warpgroup
-constexpr int LAUNCH_REGS = 96, EPI_REGS = 152, PRO_REGS = 56, CTL_REGS = PRO_REGS;
+// setmaxnreg takes one value per warpgroup: 0-1 epilogue, 2-3 producers, 4 control
+constexpr int LAUNCH_REGS = 96, EPI_REGS = 160, PRO_REGS = 56, CTL_REGS = 48;
 static_assert(NTHREADS * LAUNCH_REGS <= 65536, "launch register budget");
 // setmaxnreg moves registers inside the CTA's own launch allocation (NTHREADS * LAUNCH_REGS); an increase beyond what
 // the decreases release would block forever.
-static_assert(EPI_WARPS * 32 * EPI_REGS + (NWARPS - EPI_WARPS) * 32 * PRO_REGS <= NTHREADS * LAUNCH_REGS,
+static_assert(EPI_WARPS * 32 * EPI_REGS + PRO_WARPS * 32 * PRO_REGS + (NWARPS - EPI_WARPS - PRO_WARPS) * 32 * CTL_REGS <=
+                  NTHREADS * LAUNCH_REGS,
               "register pool");
 // Operand formats (template parameter F16 of the kernel):
 //   tf32 split (F16 = false): hi = tf32(v), lo = v - hi, both stored as f32; per tap and 16 channels 6 MMAs of
@@ -161,7 +155,6 @@ struct TcArgs {
   int nb;          // activation buffers
   int wG;          // taps per weight slot: the k taps of a chunk go in ceil(k / wG) groups of near-equal size
   int drainN;      // 16-channel chunks accumulated in Dhi between two drains into the running sums
-  int balanced;    // warp-role layout (see the kernel)
   int tmaIn;       // 1: x rows are 16-byte aligned, the raw windows come by tiled TMA loads
   int tmaOut;      // 1: out (and residual) rows are 16-byte aligned, boxes go by TMA
   int numTTiles, numCoBlk;
@@ -203,6 +196,18 @@ __device__ __forceinline__ uint64_t globalTimerNs() {
   uint64_t t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
+}
+// One poll that never parks the thread.
+__device__ __forceinline__ bool mbarTestWait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smemAddr(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
 }
 // Bounded wait: gives up (false) after SPIN_LIMIT polls or WAIT_LIMIT_NS of wall time, whichever comes first, or as
 // soon as another role has aborted. Between polls the warp sleeps `sleepNs`: the warp scheduler issues greedily from
@@ -325,6 +330,14 @@ __device__ __forceinline__ void mmaF16W(uint32_t dTmem, uint32_t aLo, uint32_t a
       "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(dTmem),
       "r"(aLo), "r"(aHi), "r"(bLo), "r"(bHi), "r"(idesc), "r"(accum)
       : "memory");
+}
+// One lane of a converged warp. The MMA and commit instructions take their operands from uniform registers; under a test on
+// the lane number the compiler has to wrap each of them in a loop over the lanes that might be active, under elect.sync it
+// knows there is one (measured: 1.3 k clocks per 16-channel chunk less in the issuing thread, half the machine code).
+__device__ __forceinline__ bool electOne() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
 }
 __device__ __forceinline__ void mmaCommit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smemAddr(bar))
@@ -610,11 +623,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     if (threadIdx.x == 0) atomicOr(a.status, (6 << 8) | 1);
     return;
   }
-  // Two warp-role layouts. Isolated (a.balanced == 0): the three control warps on scheduler 1 (warp id % 4 == 1), no
-  // producer next to the MMA issuer. Balanced: producers 8-15 (two per scheduler), control warps 16-18; for launches
-  // that are bound by the activation producers, where the issuer's pace does not matter.
-  const bool bal = a.balanced != 0;
-  const int W_WARP = bal ? 16 : 9, MMA_WARP = bal ? 17 : 13, RAW_WARP = bal ? 18 : 17;
   const int numTiles = a.numTTiles * a.numCoBlk;
   // tiles of this CTA: tile0, tile0 + tileStep, ...; its chunks of a tile: cBegin .. cBegin + nChunks16
   const int rank = SPLIT ? int(clusterRank()) : 0;
@@ -661,9 +669,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     if (kProf && a.prof && lane == 0)
       atomicAdd(reinterpret_cast<unsigned long long*>(a.prof + slot), (unsigned long long)v);
   };
-  // First timeout wins the low 16 bits; the flag bits above them are kept.
+  // First timeout wins the low 16 bits; the flag bits above them are kept. One lane of a role reports; in the MMA issuer the
+  // only lane that runs, whichever it is.
   auto giveUp = [&](int role, int code) {
-    if (lane == 0) {
+    if (lane == 0 || warp == MMA_WARP) {
       int old = *a.status;
       while ((old & kStatusWaitMask) == 0) {
         const int seen = atomicCAS(a.status, old, old | (role << 8) | code);
@@ -1043,11 +1052,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     if (tmaOut && lane == 0) bulkWaitAll();
     if (kProf && warp == 0)
       profAdd(5, wHi), profAdd(6, wLo), profAdd(7, cPre), profAdd(8, cFin), profAdd(9, clock64() - tStart);
-  } else if (bal ? warp < EPI_WARPS + PRO_WARPS : ((warp & 3) != 1 && warp != IDLE_WARP)) {
+  } else if (warp < EPI_WARPS + PRO_WARPS) {
     // ------------------------------------------------------------------ activation producers
     regDec<PRO_REGS>();
-    const int pw = bal ? warp - EPI_WARPS
-                       : (warp - EPI_WARPS) - ((warp - EPI_WARPS + 2) >> 2);  // 8, 10, 11, 12, 14, 15, 16, 18 -> 0..7
+    const int pw = warp - EPI_WARPS;
     const int cg = pw & 3, hf = pw >> 2;  // channel group of 4 inside the 16-channel chunk; row half
     const int rowsHalf = (rows + 1) >> 1;
     const int r0 = hf * rowsHalf, r1 = (r0 + rowsHalf < rows) ? r0 + rowsHalf : rows;
@@ -1305,11 +1313,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // executes between two MMAs is covered by no more than the one MMA in flight. So the bookkeeping for the next
       // round (ring counters, a first poll of the next slot's barrier) sits where it is free, and only the release
       // and, rarely, a real wait separate two rounds.
-      // Order inside a round: the lo MMAs first, then the hi MMAs, so that the wait for the Dhi drain at the start
-      // of a drain group is covered by the round's own lo MMAs. The first round of a tile goes the other way round,
-      // because there Dhi is handed back before Dlo. (Issuing hi first in the last round of a drain group as well,
-      // which lengthens the cover of the drain to this round's and the next round's lo MMAs, shortened the waits
-      // but not the tile: the extra code in this loop cost what the waits gave back.)
+      // Order inside a round: the lo MMAs first, then the hi MMAs, so that the wait for the Dhi drain at the start of a
+      // drain group is covered by the round's own lo MMAs. At the start of a tile too: the epilogue folds Dlo before the
+      // tile's last drain, so Dlo is handed back first. (Issuing hi first in the last round of a drain group, which
+      // lengthens the cover of the drain to this round's and the next round's lo MMAs, shortened the waits but not the
+      // tile: the extra code in this loop cost what the waits gave back.)
       const uint64_t dA0 = makeDesc(smemAddr(sW), MT * 16, 128);
       const uint64_t dB0 = makeDesc(smemAddr(sAct), rows * 16, 128);
       constexpr uint32_t kStageU = W_STAGE_BYTES >> 4, kLoAU = (W_STAGE_BYTES / 2) >> 4, kKsAU = (2 * MT * 16) >> 4;
@@ -1323,7 +1331,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       bool dead = false, ready = false;  // ready: the next round's weight slot is already known to be full
       long long wBf = 0, wHe = 0, wWf = 0, wLe = 0;
       const long long tStart = kProf ? clock64() : 0;
-      for (int tile = tile0; lane == 0 && tile < numTiles && !dead; tile += tileStep) {
+      const bool leader = electOne();
+      for (int tile = tile0; leader && tile < numTiles && !dead; tile += tileStep) {
         for (int c = 0; c < nChunks16 && !dead; ++c) {
           if (!waitT(&bFull[buf], bufPh, wBf, SLEEP_MMA_NS)) {
             giveUp(4, 2);
@@ -1386,38 +1395,28 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             uint32_t nph = slotPh;
             if (nslot == wStages) nslot = 0, nph ^= 1;
             const bool lastRound = c == nChunks16 - 1 && gi == nTapGroups - 1;  // of the tile
-            if (needLo) {  // first round of a tile: hi, then lo (Dhi is handed back before Dlo)
-              if (needHi && !waitT(&hiEmpty[hb], groupPar ^ 1, wHe, SLEEP_MMA_NS)) {
-                giveUp(4, 1);
-                dead = true;
-                break;
-              }
-              tcFenceAfter();
-              issueHi(accHi);
+            if (needLo) {
               if (!waitT(loEmpty, tilePar ^ 1, wLe, SLEEP_MMA_NS)) {
                 giveUp(4, 4);
                 dead = true;
                 break;
               }
               tcFenceAfter();
-              issueLo(accLo);
-              if (lastRound) mmaCommit(loFull);
-            } else {
-              issueLo(accLo);
-              // the tile's lo chain is complete: the epilogue folds Dlo under the hi MMAs of this last round
-              if (lastRound) mmaCommit(loFull);
-              if (needHi) {
-                if (!waitT(&hiEmpty[hb], groupPar ^ 1, wHe, SLEEP_MMA_NS)) {
-                  giveUp(4, 1);
-                  dead = true;
-                  break;
-                }
-                tcFenceAfter();
-              }
-              issueHi(accHi);
             }
+            issueLo(accLo);
+            // the tile's lo chain is complete: the epilogue folds Dlo under the hi MMAs of this last round
+            if (lastRound) mmaCommit(loFull);
+            if (needHi) {
+              if (!waitT(&hiEmpty[hb], groupPar ^ 1, wHe, SLEEP_MMA_NS)) {
+                giveUp(4, 1);
+                dead = true;
+                break;
+              }
+              tcFenceAfter();
+            }
+            issueHi(accHi);
             // first poll of the next slot's barrier, with the whole round queued behind it
-            ready = mbarTryWait(&wFull[nslot], nph);
+            ready = mbarTestWait(&wFull[nslot], nph);
             mmaCommit(&wEmpty[slot]);  // weight slot free once the MMAs have read it
             kk += gN;
             slot = nslot, slotPh = nph;
@@ -1810,10 +1809,6 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercen
   const int perChunk = a.k * (f16 ? 1 : 2);
   const int n = (!f16 && a.k == 1 ? MAX_CHAIN_POINT32 : MAX_CHAIN) / perChunk;
   a.drainN = n < 1 ? 1 : n;
-  // Launches with at most 15 MMAs per chunk (K <= 5 with f16 halves; the ConvTranspose launches: three taps) are
-  // bound by the activation producers: they take the balanced warp layout (measured at K = 3: the transform of a
-  // chunk 17 % faster, the launch 4-7 %; at K = 7 the isolated layout is 3 % ahead).
-  a.balanced = a.k * (f16 ? 3 : 6) <= 15 ? 1 : 0;
   const int tiles = a.numTTiles * a.numCoBlk;
   *grid = a.split ? tiles * a.split : (tiles < d->smCount ? tiles : d->smCount);
   // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
