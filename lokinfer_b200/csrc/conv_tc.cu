@@ -50,6 +50,7 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "lkc_common.h"
 
@@ -125,12 +126,12 @@ constexpr int kMaxSmem = 232448;  // 227 KB per CTA on sm_100
 struct SmemLayout {
   uint32_t act, raw, w, par, bar, total;
 };
-__host__ __device__ inline SmemLayout smemLayout(bool split, int ci, int rows, int half, int nb, int wStages, int wG,
+__host__ __device__ inline SmemLayout smemLayout(bool split, int ci, int rows, int ext, int nb, int wStages, int wG,
                                                  int actRowBytes, int wStageBytes) {
   SmemLayout s;
   s.act = split ? 0 : EPI_WARPS * STAGE_FLOATS * 4;  // tiles: [0, act)
   s.raw = (s.act + uint32_t(nb) * actRowBytes * rows + 127u) & ~127u;
-  s.w = s.raw + uint32_t(NRAW) * 2 * KC * half * 4;  // a multiple of 128
+  s.w = s.raw + uint32_t(NRAW) * KC * ((split ? NTS : NT) + ext) * 4;  // a multiple of 128
   s.par = s.w + uint32_t(wStages) * wG * wStageBytes;
   if (split && s.par < uint32_t(PART_BYTES)) s.par = PART_BYTES;  // a split tile's partial lies over the operand buffers
   s.bar = s.par + uint32_t(4) * ci * 4;
@@ -149,8 +150,9 @@ struct TcArgs {
   int64_t xPitch, resPitch, outPitch;  // row pitches in floats
   int padLeft;       // ConvTranspose: 1 = one-sample left reflect pad
   float slope, outScale;
-  int rows;        // staged time rows per buffer = tile columns + (k-1)*dilation
-  int half;        // raw staging: every channel's window is kept as two runs of `half` floats (two TMA boxes)
+  int delta;       // columns between the 16-byte boundary a tile's window is loaded from and its first column (0: 4-byte route)
+  int rows;        // staged time rows per buffer = tile columns + (k-1)*dilation + delta
+  int ext;         // raw staging: [16][tile columns], then [16][ext] with the rows - tile columns beyond them (two TMA boxes)
   int wStages;     // weight ring depth (slots)
   int nb;          // activation buffers
   int wG;          // taps per weight slot: the k taps of a chunk go in ceil(k / wG) groups of near-equal size
@@ -398,7 +400,7 @@ __device__ __forceinline__ float2 sinSq2(float2 u) {
   return make_float2((__float_as_int(t.x) & 1) ? 1.f - q.x : q.x, (__float_as_int(t.y) & 1) ? 1.f - q.y : q.y);
 }
 
-// Prologue with per-channel constants folded once per launch (sPar rows mean, a, b, inv):
+// Prologue with per-channel constants folded once per launch (sPar rows -mean, a, b, inv):
 //   Snake: u = (x - mean) * (alpha scale) + alpha beta; result = (u + sin^2(u)) / alpha  (= v + sin^2(alpha v) / alpha)
 //   leaky / none: v = (x - mean) * scale + beta
 // Centering first keeps the precision when the variance is tiny next to the mean, as in the reference.
@@ -408,6 +410,12 @@ __device__ __forceinline__ float2 activate2(float2 x, float2 negm, float2 a, flo
   if (ACT == 1) return __fmul2_rn(__fadd2_rn(v, sinSq2(v)), inv);
   if (ACT == 2) return make_float2(v.x >= 0.f ? v.x : v.x * slope, v.y >= 0.f ? v.y : v.y * slope);
   return v;
+}
+
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
 template <int N>
@@ -583,8 +591,8 @@ struct SplitTail {
 // where one tile's serial chain of chunks is the launch's time (see splitFor).
 template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT>
 __global__ void __launch_bounds__(NTHREADS, 1)
-    convTcKernel(const TcArgs a, const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapRes,
-                 const __grid_constant__ CUtensorMap mapOut) {
+    convTcKernel(const TcArgs a, const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapExt,
+                 const __grid_constant__ CUtensorMap mapRes, const __grid_constant__ CUtensorMap mapOut) {
   constexpr int W_STAGE_BYTES = Fmt<F16>::W_STAGE_BYTES, W_STAGE_FLOATS = Fmt<F16>::W_STAGE_FLOATS;
   constexpr int NTK = SPLIT ? NTS : NT;  // time columns of this kernel's tiles
   constexpr int EC = NTK / 2;            // columns of one epilogue warp
@@ -594,13 +602,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   constexpr uint32_t kIdesc = idescOf(F16, NTK);
   const int NB = a.nb;
   extern __shared__ __align__(1024) unsigned char smemRaw[];
-  const int rows = a.rows, half = a.half;
-  const SmemLayout lay = smemLayout(SPLIT, a.ci, rows, half, NB, a.wStages, a.wG, Fmt<F16>::ACT_BYTES_PER_ROW, W_STAGE_BYTES);
+  const int rows = a.rows, ext = a.ext;
+  const SmemLayout lay = smemLayout(SPLIT, a.ci, rows, ext, NB, a.wStages, a.wG, Fmt<F16>::ACT_BYTES_PER_ROW, W_STAGE_BYTES);
   const int actBufFloats = Fmt<F16>::ACT_BYTES_PER_ROW / 4 * rows;  // hi + lo
-  const int rawBufFloats = 2 * KC * half;
+  const int rawBufFloats = KC * (NTK + ext);
   float* const sStage = reinterpret_cast<float*>(smemRaw);           // EPI_WARPS tiles
   float* const sAct = reinterpret_cast<float*>(smemRaw + lay.act);   // NB buffers of [2 (hi, lo)][16-byte K chunks][rows]
-  float* const sRaw = reinterpret_cast<float*>(smemRaw + lay.raw);   // NRAW buffers of [2 runs][KC][half] raw input
+  float* const sRaw = reinterpret_cast<float*>(smemRaw + lay.raw);   // NRAW buffers of [KC][NTK], [KC][ext] raw input
   float* const sW = reinterpret_cast<float*>(smemRaw + lay.w);       // wStages slots of wG taps of [2 (hi, lo)][16-byte K chunks][MT]
   float* const sPar = reinterpret_cast<float*>(smemRaw + lay.par);   // [4][ci]: folded prologue constants
   uint64_t* const bFull = reinterpret_cast<uint64_t*>(smemRaw + lay.bar);
@@ -1056,13 +1064,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // ------------------------------------------------------------------ activation producers
     regDec<PRO_REGS>();
     const int pw = warp - EPI_WARPS;
-    const int cg = pw & 3, hf = pw >> 2;  // channel group of 4 inside the 16-channel chunk; row half
-    const int rowsHalf = (rows + 1) >> 1;
-    const int r0 = hf * rowsHalf, r1 = (r0 + rowsHalf < rows) ? r0 + rowsHalf : rows;
-    constexpr int SLOTS = (((NTK + MAX_HALO + 1) >> 1) + 31) / 32;  // row slots of 32 lanes per warp
+    const int cg = pw & 3, hf = pw >> 2;  // channel group of 4 inside the 16-channel chunk; half of the tile's columns
+    // A warp stages the rows of its half, SLOTS per lane, with addresses that are immediates. The rows beyond the tile's
+    // columns (at most 53) take one more slot for up to 32 of them: the first 32 go to the warps of half `raw buffer`, so
+    // that the halves take turns, the rest to the other half.
+    constexpr int SLOTS = NTK / 64;
     const bool tmaIn = a.tmaIn != 0;
-    const int runSkip = (KC - 1) * half;  // a raw window index i >= half sits in the second run: + runSkip floats
-    // per-channel parameters, once: sPar = [mean | a | b | inv] with a = scale, b = beta (x alpha for Snake), inv = 1/alpha
+    // per-channel parameters, once: sPar = [-mean | a | b | inv] with a = scale, b = beta (x alpha for Snake), inv = 1/alpha
     // Split form with statsIn: each CTA folds the chunk statistics of its own channels into mean / scale / beta, with the
     // arithmetic of adainAffineKernel (Chan combine in double), four lanes per channel. A launch of its own costs
     // 3.5 us plus a gap in front of every conv; here it is one round of loads under the first weight and input copies.
@@ -1091,7 +1099,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           m2 += __shfl_xor_sync(0xffffffffu, m2, 2);
           if (sub == 0) {
             const float var = float(m2 / double(a.l)), al = ACT == 1 ? a.alpha[c] : 1.f;
-            sPar[c] = float(mean);
+            sPar[c] = -float(mean);
             sPar[a.ci + c] = (1.f + a.gb[c]) * (1.0f / sqrtf(var + a.eps)) * al;
             sPar[2 * a.ci + c] = a.gb[a.ci + c] * al;
             sPar[3 * a.ci + c] = 1.f / al;
@@ -1101,31 +1109,35 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
     for (int c = cBegin * KC + pw * 32 + lane; !fold && c < (cBegin + nChunks16) * KC; c += PRO_WARPS * 32) {
       const float al = ACT == 1 ? a.alpha[c] : 1.f;
-      sPar[c] = a.affine ? a.affine[c] : 0.f;
+      sPar[c] = a.affine ? -a.affine[c] : 0.f;
       sPar[a.ci + c] = (a.affine ? a.affine[a.ci + c] : 1.f) * al;
       sPar[2 * a.ci + c] = (a.affine ? a.affine[2 * a.ci + c] : 0.f) * al;
       sPar[3 * a.ci + c] = 1.f / al;
     }
     asm volatile("bar.sync 1, %0;" ::"n"(PRO_WARPS * 32) : "memory");  // producer warps only
 
+    // First row beyond the tile's columns that this lane stages from raw buffer rb.
+    auto extRow = [&](uint32_t rb) { return NTK + (uint32_t(hf) == rb ? 0 : 32) + lane; };
+
     // Unaligned route: cp.async of this thread's part of the raw window of chunk c of the tile whose window starts at
     // input position posT (= tile column * NT - padding) into staging buffer rb. Pointer increments only: this runs
-    // once per chunk on every producer thread.
+    // once per chunk on every producer thread. A thread copies what it will itself read back.
     auto issueCopies = [&](int64_t posT, int c, int rb) {
-      const float* xc = a.x + int64_t((cBegin + c) * KC + cg * 4) * a.xPitch + posT + r0 + lane;
-      float* base = sRaw + rb * rawBufFloats + cg * 4 * half;
-      int64_t pos = posT + r0 + lane;
-      int r = r0 + lane;
+      const float* xc = a.x + int64_t((cBegin + c) * KC + cg * 4) * a.xPitch + posT;
+      float* const base = sRaw + rb * rawBufFloats;
+      auto copy = [&](int r, float* dst, int pitch) {
+        const int64_t pos = posT + r;
+        if (pos >= 0 && pos < a.l) {
+          const float* src = xc + r;
 #pragma unroll
-      for (int sl = 0; sl < SLOTS; ++sl, r += 32, pos += 32, xc += 32) {
-        if (r < r1 && pos >= 0 && pos < a.l) {
-          float* dst = base + r + (r >= half ? runSkip : 0);
-          cpAsync4(dst, xc);
-          cpAsync4(dst + half, xc + a.xPitch);
-          cpAsync4(dst + 2 * half, xc + 2 * a.xPitch);
-          cpAsync4(dst + 3 * half, xc + 3 * a.xPitch);
+          for (int j = 0; j < 4; ++j) cpAsync4(dst + j * pitch, src + j * a.xPitch);
         }
-      }
+      };
+      const int r0 = hf * (NTK / 2) + lane;
+#pragma unroll
+      for (int sl = 0; sl < SLOTS; ++sl) copy(r0 + sl * 32, base + cg * 4 * NTK + r0 + sl * 32, NTK);
+      const int r = extRow(rb);
+      if (r < rows) copy(r, base + KC * NTK + cg * 4 * ext + r - NTK, ext);
     };
 
     int t = tile0, c = 0;
@@ -1144,10 +1156,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         cn = 0, tn = t + tileStep;
         posN = int64_t(tn / a.numCoBlk) * NTK - a.padding;
       }
-      // the window's offset inside the staged runs: the aligned route loads from the 16-byte boundary below pos0
-      int delta = 0;
       if (tmaIn) {
-        delta = int(pos0 & 3);
         if (!waitT(&rawFull[rawBuf], rawPar, wCp, SLEEP_PRO_NS)) {
           giveUp(2, 2);
           break;
@@ -1165,47 +1174,41 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       const long long tTr = kProf ? clock64() : 0;
       // tf32 split: [cg][rows][4 f32]; f16 split: [cg / 2][rows][8 f16], this thread's 4 channels = half of a chunk
-      float* hi = F16 ? sAct + buf * actBufFloats + (cg >> 1) * rows * 4 + (cg & 1) * 2
-                      : sAct + buf * actBufFloats + cg * rows * 4;
-      float* lo = hi + actBufFloats / 2;
-      const float* src = sRaw + rawBuf * rawBufFloats + cg * 4 * half + delta;
+      float* const hi = F16 ? sAct + buf * actBufFloats + (cg >> 1) * rows * 4 + (cg & 1) * 2
+                            : sAct + buf * actBufFloats + cg * rows * 4;
+      float* const lo = hi + actBufFloats / 2;
+      const float* const raw = sRaw + rawBuf * rawBufFloats;
       // this thread's four channels: constants in registers for the whole chunk
-      float2 nm[2], pa[2], pb[2], pi[2];  // channel pairs (0, 1) and (2, 3); nm = -mean
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float* par = sPar + (cBegin + c) * KC + cg * 4 + 2 * h;
-        nm[h] = make_float2(-par[0], -par[1]);
-        pa[h] = make_float2(par[a.ci], par[a.ci + 1]);
-        pb[h] = make_float2(par[2 * a.ci], par[2 * a.ci + 1]);
-        pi[h] = make_float2(par[3 * a.ci], par[3 * a.ci + 1]);
-      }
+      const float* par = sPar + (cBegin + c) * KC + cg * 4;
+      const float4 nm = *reinterpret_cast<const float4*>(par), pa = *reinterpret_cast<const float4*>(par + a.ci),
+                   pb = *reinterpret_cast<const float4*>(par + 2 * a.ci), pi = *reinterpret_cast<const float4*>(par + 3 * a.ci);
       float big = 0.f;  // largest |value| this thread staged in the chunk (f16 range check, once per chunk)
-#pragma unroll
-      for (int sl = 0; sl < SLOTS; ++sl) {
-        // Branch-free body, so that the iterations' dependency chains interleave: rows beyond the thread's range
-        // recompute its last row and skip the stores; positions outside the valid range select zero.
-        const int rq = r0 + sl * 32 + lane;
-        const bool inr = rq < r1;
-        const int r = inr ? rq : r1 - 1;
-        const int64_t pos = pos0 + r;
-        const bool ok = pos >= a.validLo && pos < a.validHi;
-        const float* sp = src + r + (r + delta >= half ? runSkip : 0);
-        float2 v01 = activate2<ACT>(make_float2(sp[0], sp[half]), nm[0], pa[0], pb[0], pi[0], a.slope);
-        float2 v23 = activate2<ACT>(make_float2(sp[2 * half], sp[3 * half]), nm[1], pa[1], pb[1], pi[1], a.slope);
-        v01.x = ok ? v01.x : 0.f, v01.y = ok ? v01.y : 0.f, v23.x = ok ? v23.x : 0.f, v23.y = ok ? v23.y : 0.f;
+      // rows [okLo, okHi) are inside the valid range, the others are zero padding (after the activation)
+      const int64_t x0 = pos0 - a.delta;
+      const int okLo = x0 >= a.validLo ? 0 : int(a.validLo - x0 < rows ? a.validLo - x0 : rows);
+      const int okHi = a.validHi - x0 >= rows ? rows : int(a.validHi - x0);
+      // One row of four channels; sp: this thread's first channel of the row, the others `pitch` floats on. Branch-free, so
+      // that the slots' dependency chains interleave.
+      auto stage = [&](auto edge, int r, const float* sp, int pitch) {
+        float2 v01 = activate2<ACT>(make_float2(sp[0], sp[pitch]), make_float2(nm.x, nm.y), make_float2(pa.x, pa.y),
+                                    make_float2(pb.x, pb.y), make_float2(pi.x, pi.y), a.slope);
+        float2 v23 = activate2<ACT>(make_float2(sp[2 * pitch], sp[3 * pitch]), make_float2(nm.z, nm.w), make_float2(pa.z, pa.w),
+                                    make_float2(pb.z, pb.w), make_float2(pi.z, pi.w), a.slope);
+        if constexpr (decltype(edge)::value) {
+          const bool ok = r >= okLo && r < okHi;
+          v01.x = ok ? v01.x : 0.f, v01.y = ok ? v01.y : 0.f, v23.x = ok ? v23.x : 0.f, v23.y = ok ? v23.y : 0.f;
+        }
         if constexpr (!F16) {
           float4 h, l;
           h.x = tf32Round(v01.x), h.y = tf32Round(v01.y), h.z = tf32Round(v23.x), h.w = tf32Round(v23.y);
           const float2 l01 = __fadd2_rn(v01, make_float2(-h.x, -h.y)), l23 = __fadd2_rn(v23, make_float2(-h.z, -h.w));
           l = make_float4(l01.x, l01.y, l23.x, l23.y);
-          if (inr) {
-            *reinterpret_cast<float4*>(hi + r * 4) = h;
-            *reinterpret_cast<float4*>(lo + r * 4) = l;
-          }
+          *reinterpret_cast<float4*>(hi + r * 4) = h;
+          *reinterpret_cast<float4*>(lo + r * 4) = l;
         } else {
           // hi = f16(v), lo = f16((v - hi) * 2^11); 4 channels = 8 bytes of the row's 16-byte K chunk (channel groups
           // 2 j and 2 j + 1 share chunk j). A value beyond the f16 range becomes infinite here and is reported below.
-          big = fmaxf(big, fmaxf(fmaxf(fabsf(v01.x), fabsf(v01.y)), fmaxf(fabsf(v23.x), fabsf(v23.y))));
+          big = max3(max3(big, fabsf(v01.x), fabsf(v01.y)), fabsf(v23.x), fabsf(v23.y));
           const __half2 h01 = __float22half2_rn(v01), h23 = __float22half2_rn(v23);
           const float2 sc = make_float2(kLoScale, kLoScale);
           const float2 f01 = __half22float2(h01), f23 = __half22float2(h23);
@@ -1214,11 +1217,21 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           uint2 hw, lw;
           hw.x = *reinterpret_cast<const uint32_t*>(&h01), hw.y = *reinterpret_cast<const uint32_t*>(&h23);
           lw.x = *reinterpret_cast<const uint32_t*>(&l01), lw.y = *reinterpret_cast<const uint32_t*>(&l23);
-          if (inr) {
-            *reinterpret_cast<uint2*>(hi + r * 4) = hw;
-            *reinterpret_cast<uint2*>(lo + r * 4) = lw;
-          }
+          *reinterpret_cast<uint2*>(hi + r * 4) = hw;
+          *reinterpret_cast<uint2*>(lo + r * 4) = lw;
         }
+      };
+      const int r0 = hf * (NTK / 2) + lane, rx = extRow(rawBuf);
+      const float* const sp0 = raw + cg * 4 * NTK + r0;
+      const float* const spx = raw + KC * NTK + cg * 4 * ext + rx - NTK;
+      if (okLo == 0 && okHi == rows) {  // all but the tiles at the ends of the valid range
+#pragma unroll
+        for (int sl = 0; sl < SLOTS; ++sl) stage(std::false_type{}, r0 + sl * 32, sp0 + sl * 32, NTK);
+        if (rx < rows) stage(std::false_type{}, rx, spx, ext);
+      } else {
+#pragma unroll 2
+        for (int sl = 0; sl < SLOTS; ++sl) stage(std::true_type{}, r0 + sl * 32, sp0 + sl * 32, NTK);
+        if (rx < rows) stage(std::true_type{}, rx, spx, ext);
       }
       if (F16 && big > 65504.f) atomicOr(a.status, kStatusF16Range);
       fenceProxyAsync();  // generic-proxy stores -> visible to the tensor core (async proxy)
@@ -1275,17 +1288,16 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
     } else if (warp == RAW_WARP) {
       // ---------------------------------------------------------------- raw-window loader (aligned route)
-      // Per (tile, chunk): the 16 channels' windows [pos0 & ~3, + 2 half) as two boxes of `half` columns (a box
-      // holds at most 256 elements per dimension). Columns outside [0, L) arrive as zeros and are never used: the
-      // producers write the zero padding themselves, after the activation.
+      // Per (tile, chunk): the 16 channels' windows from the 16-byte boundary at or below their first column, as two boxes
+      // (a box holds at most 256 elements per dimension): the tile's columns and what lies beyond them. Columns outside
+      // [0, L) arrive as zeros and are never used: the producers write the zero padding themselves, after the activation.
       if (a.tmaIn && lane == 0) {
         uint32_t rb = 0, ph = 1, issued = 0;
         long long wR = 0;
         bool dead = false;
         const uint32_t bytes = uint32_t(rawBufFloats) * 4;
         for (int t = tile0; t < numTiles && !dead; t += tileStep) {
-          const int64_t pos0 = int64_t(t / a.numCoBlk) * NTK - a.padding;
-          const int x0 = int(pos0 - (pos0 & 3));
+          const int x0 = (t / a.numCoBlk) * NTK - a.padding - a.delta;
           for (int c = 0; c < nChunks16; ++c, ++issued) {
             if (!waitT(&rawEmpty[rb], ph, wR, SLEEP_W_NS)) {
               giveUp(5, 1);
@@ -1295,7 +1307,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             float* dst = sRaw + rb * rawBufFloats;
             mbarArriveExpectTx(&rawFull[rb], bytes);
             tmaLoad2d(dst, &mapX, x0, (cBegin + c) * KC, &rawFull[rb]);
-            tmaLoad2d(dst + KC * half, &mapX, x0 + half, (cBegin + c) * KC, &rawFull[rb]);
+            if (ext) tmaLoad2d(dst + KC * NTK, &mapExt, x0 + NTK, (cBegin + c) * KC, &rawFull[rb]);
             if (++rb == NRAW) rb = 0, ph ^= 1;
           }
         }
@@ -1319,7 +1331,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // lengthens the cover of the drain to this round's and the next round's lo MMAs, shortened the waits but not the
       // tile: the extra code in this loop cost what the waits gave back.)
       const uint64_t dA0 = makeDesc(smemAddr(sW), MT * 16, 128);
-      const uint64_t dB0 = makeDesc(smemAddr(sAct), rows * 16, 128);
+      const uint64_t dB0 = makeDesc(smemAddr(sAct), rows * 16, 128) + uint32_t(a.delta);
       constexpr uint32_t kStageU = W_STAGE_BYTES >> 4, kLoAU = (W_STAGE_BYTES / 2) >> 4, kKsAU = (2 * MT * 16) >> 4;
       // activation buffer: hi half then lo half; one MMA spans two 16-byte K chunks (K8 of f32 or K16 of f16);
       // one staged time row = 16 bytes = one descriptor address unit
@@ -1532,9 +1544,8 @@ __global__ void convtTcPackKernel(const float* __restrict__ w, void* __restrict_
 
 }  // namespace
 
-// Raw staging: every channel's window of rows + 3 floats (the slack of the 16-byte alignment) is kept as two runs of
-// `half` floats, half a multiple of 4 and at most 256 (one TMA box each).
-static int rawHalf(int rows) { return (((rows + 3 + 1) / 2) + 3) & ~3; }
+// Row floats of the second raw-input box (its 16-byte granularity): what a window of `rows` columns has beyond `cols`.
+static int rawExt(int rows, int cols) { return (rows - cols + 3) & ~3; }
 
 // Dynamic shared memory of one CTA and the weight ring it leaves room for: the largest taps-per-slot (<= TAP_GROUP)
 // that still gives PREF_W_STAGES slots, else the deepest ring. Returns 0 when even single-tap slots do not fit.
@@ -1542,9 +1553,8 @@ static size_t convTcSmemBytes(bool split, int64_t ci, int rows, int k, bool f16,
   const int tap = f16 ? Fmt<true>::W_STAGE_BYTES : Fmt<false>::W_STAGE_BYTES;
   const int actRow = f16 ? Fmt<true>::ACT_BYTES_PER_ROW : Fmt<false>::ACT_BYTES_PER_ROW;
   const int nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
-  const int half = rawHalf(rows);
-  if (half > 256) return 0;
-  const SmemLayout base = smemLayout(split, int(ci), rows, half, nb, 0, 0, actRow, tap);
+  const int ext = rawExt(rows, split ? NTS : NT);
+  const SmemLayout base = smemLayout(split, int(ci), rows, ext, nb, 0, 0, actRow, tap);
   if (base.total > uint32_t(kMaxSmem)) return 0;
   const size_t avail = size_t(kMaxSmem) - base.total;
   // Large groups matter more than a deep ring (measured: two slots of four taps beat four slots of three, and at
@@ -1563,7 +1573,7 @@ static size_t convTcSmemBytes(bool split, int64_t ci, int rows, int k, bool f16,
   if (bestG == 0) return 0;
   if (wStages) *wStages = bestWs;
   if (wG) *wG = bestG;
-  return smemLayout(split, int(ci), rows, half, nb, bestWs, bestG, actRow, tap).total;
+  return smemLayout(split, int(ci), rows, ext, nb, bestWs, bestG, actRow, tap).total;
 }
 
 // The hi chain between two drains holds at most MAX_CHAIN MMAs: whole chunks while they fit, and a chunk that alone
@@ -1576,7 +1586,7 @@ bool convTcEligible(const ConvFusedParams& p, bool f16) {
         chainOk(p.k, f16) && (p.k - 1) * p.dilation <= MAX_HALO && p.lo >= 1 && p.padding <= (1 << 20) && p.ci <= 4096 &&
         p.l < (int64_t(1) << 30)))
     return false;
-  return convTcSmemBytes(false, p.ci, NT + int((p.k - 1) * p.dilation), int(p.k), false, nullptr, nullptr) != 0;  // the larger format
+  return convTcSmemBytes(false, p.ci, NT + int((p.k - 1) * p.dilation) + 3, int(p.k), false, nullptr, nullptr) != 0;  // the larger format
 }
 
 int64_t convTcPackFloats(int64_t co, int64_t ci, int64_t k, bool f16) {
@@ -1692,7 +1702,7 @@ int convTcSetIo(int mode) {
 }
 
 struct TcMaps {
-  CUtensorMap x, res, out;
+  CUtensorMap x, ext, res, out;
 };
 
 template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT>
@@ -1713,13 +1723,13 @@ static int launchTc4(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cu
     attr[0].val.clusterDim.x = unsigned(a.split), attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(unsigned(grid)), cfg.blockDim = dim3(NTHREADS), cfg.dynamicSmemBytes = smem, cfg.stream = s;
     cfg.attrs = attr, cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, m.x, m.res, m.out);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, m.x, m.ext, m.res, m.out);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return failCuda("conv (tensor-core)", e);
     }
   } else {
-    kernel<<<grid, NTHREADS, smem, s>>>(a, m.x, m.res, m.out);
+    kernel<<<grid, NTHREADS, smem, s>>>(a, m.x, m.ext, m.res, m.out);
   }
   return launched("conv (tensor-core)");
 }
@@ -1797,11 +1807,18 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercen
   LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
   const int nt = a.split ? NTS : NT;
   a.numTTiles = int(ceilDiv(a.lo, nt));
-  a.rows = nt + (a.k - 1) * a.dilation;
+  // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
+  // argument: it stays zero-filled and is never dereferenced.
+  std::memset(&m, 0, sizeof m);
+  a.tmaIn = makeMap(&m.x, a.x, a.ci, a.l, a.xPitch, nt, KC, false) ? 1 : 0;
+  a.delta = a.tmaIn ? -a.padding & 3 : 0;  // tiles start on multiples of 4 columns
+  a.rows = nt + (a.k - 1) * a.dilation + a.delta;
+  a.ext = rawExt(a.rows, nt);
+  if (a.tmaIn && a.ext)
+    LKC_REQUIRE(makeMap(&m.ext, a.x, a.ci, a.l, a.xPitch, a.ext, KC, false), "conv (tensor-core): tensor map of the input");
   *smem = convTcSmemBytes(a.split != 0, a.ci, a.rows, a.k, f16, &a.wStages, &a.wG);
   LKC_REQUIRE(*smem != 0, "conv (tensor-core): window too large");
   if (a.split && *smem < SPLIT_SMEM) *smem = SPLIT_SMEM;
-  a.half = rawHalf(a.rows);
   a.nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
   a.status = d->status;
   a.prof = (kProf && gProfileOn) ? d->prof : nullptr;
@@ -1811,10 +1828,6 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercen
   a.drainN = n < 1 ? 1 : n;
   const int tiles = a.numTTiles * a.numCoBlk;
   *grid = a.split ? tiles * a.split : (tiles < d->smCount ? tiles : d->smCount);
-  // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
-  // argument: it stays zero-filled and is never dereferenced.
-  std::memset(&m, 0, sizeof m);
-  a.tmaIn = makeMap(&m.x, a.x, a.ci, a.l, a.xPitch, a.half, KC, false) ? 1 : 0;
   a.tmaOut = 0;
   if (boxesOk && a.co % MT == 0 && makeMap(&m.out, a.out, a.co, a.lo, a.outPitch, BOX, BOX, true) &&
       (!a.residual || makeMap(&m.res, a.residual, a.co, a.lo, a.resPitch, BOX, BOX, true)))
@@ -1860,7 +1873,7 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
 
 bool convtTcEligible(int64_t ci, int64_t co, int64_t k, int64_t stride, int64_t padding) {
   return (stride == 6 || stride == 10) && k == 2 * stride && 2 * padding == stride && ci % KC == 0 && ci >= KC &&
-         ci <= 4096 && co >= 1 && convTcSmemBytes(false, ci, NT + 2, 3, false, nullptr, nullptr) != 0;
+         ci <= 4096 && co >= 1 && convTcSmemBytes(false, ci, NT + 2 + 3, 3, false, nullptr, nullptr) != 0;
 }
 
 int64_t convtTcPackFloats(int64_t ci, int64_t co, int64_t stride, bool f16) {
