@@ -103,9 +103,12 @@ constexpr int STAGE_FLOATS = 32 * STAGE_PITCH;
 constexpr int BOX = 32, BOX_BYTES = BOX * BOX * 4;  // residual / output boxes of the aligned route: 32 co x 32 t
 static_assert(BOX_BYTES <= STAGE_FLOATS * 4, "a swizzled box fits in a warp's tile");
 constexpr int PART_PITCH = NTS + 4;  // floats per row of a split tile's partial: rows 16-byte aligned, 4 banks apart
-constexpr int PART_BYTES = MT * PART_PITCH * 4;
+// A split tile's memory behind its MMAs, over the operand buffers: this CTA's partial tile, then the rows that the CTAs of the
+// cluster send it. Those are at most split * (rows a CTA owns, rounded up; 2 channels of 10 rows and a gap of 2 over 8 CTAs).
+constexpr int PART_ROWS = 176, PART_BYTES = MT * PART_PITCH * 4, RECV_BYTES = PART_ROWS * PART_PITCH * 4;
 constexpr size_t SPLIT_SMEM = 120 * 1024;  // more than half an SM's: one CTA per SM, for whose TMEM two would compete
 constexpr int MAX_SPLIT = 8;     // CTAs of a split tile (the portable cluster size)
+static_assert(MAX_SPLIT <= EPI_WARPS, "an epilogue warp per receiver");
 constexpr int MAX_HALO = 50;     // (K - 1) * dilation of the widest Kokoro conv (K 11, dilation 5)
 constexpr int MAX_W_STAGES = 4, MIN_W_STAGES = 2, PREF_W_STAGES = 2;  // weight ring slots
 constexpr int TAP_GROUP = 6;  // most taps per weight slot: one bulk copy, one wait, MMAs back to back, one release
@@ -133,7 +136,7 @@ __host__ __device__ inline SmemLayout smemLayout(bool split, int ci, int rows, i
   s.raw = (s.act + uint32_t(nb) * actRowBytes * rows + 127u) & ~127u;
   s.w = s.raw + uint32_t(NRAW) * KC * ((split ? NTS : NT) + ext) * 4;  // a multiple of 128
   s.par = s.w + uint32_t(wStages) * wG * wStageBytes;
-  if (split && s.par < uint32_t(PART_BYTES)) s.par = PART_BYTES;  // a split tile's partial lies over the operand buffers
+  if (split && s.par < uint32_t(PART_BYTES + RECV_BYTES)) s.par = PART_BYTES + RECV_BYTES;
   s.bar = s.par + uint32_t(4) * ci * 4;
   s.total = s.bar + 512;
   return s;
@@ -161,6 +164,7 @@ struct TcArgs {
   int tmaOut;      // 1: out (and residual) rows are 16-byte aligned, boxes go by TMA
   int numTTiles, numCoBlk;
   int split;       // 0 = a persistent CTA per SM over 256-column tiles; else the CTAs that share one 128-column tile
+  int early;       // the launch may overlap the end of the one before it (programmatic dependent launch)
   int* status;
   long long* prof;  // null, or 16 cycle counters summed over CTAs (see convTcProfile)
 };
@@ -272,6 +276,11 @@ __device__ __forceinline__ void cpAsyncWait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Programmatic dependent launch. wait: until every kernel this launch depends on has finished and its writes are visible.
+// launch: the kernel that follows may start (it waits in the same way before it touches what this one writes or reads).
+__device__ __forceinline__ void dependenciesWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependentsLaunch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ void tmemAlloc(uint32_t* slot, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(slot)), "r"(cols)
                : "memory");
@@ -282,34 +291,31 @@ __device__ __forceinline__ void tmemRelinquish() {
 __device__ __forceinline__ void tmemDealloc(uint32_t addr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
 }
-// Cluster of the split form: this CTA's rank, the barrier of all threads of all its CTAs (release / acquire: shared-memory
-// writes before it are visible to every CTA after it), and loads from the same offset in another CTA's shared memory.
+// Cluster of the split form: this CTA's rank, the two halves of the barrier of all threads of all its CTAs (release /
+// acquire), and the address of another CTA's copy of this CTA's shared memory.
 __device__ __forceinline__ uint32_t clusterRank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void clusterSync() {
+__device__ __forceinline__ void clusterArrive() {
   __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void clusterWait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t peerAddr(uint32_t addr, uint32_t rank) {
   uint32_t r;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ float4 peerLoad4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr)
+// Bulk copy into another CTA's shared memory, counted by a barrier there (both as peerAddr gives them).
+__device__ __forceinline__ void bulkCopyPeer(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "r"(smemAddr(src)), "r"(bytes), "r"(bar)
                : "memory");
-  return v;
-}
-__device__ __forceinline__ float peerLoad(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-  return v;
 }
 // D[tmem] (+)= A[smem desc] * B[smem desc], kind::tf32, issued by one thread.
 __device__ __forceinline__ void mmaTf32(uint32_t dTmem, uint64_t descA, uint64_t descB, uint32_t idesc, uint32_t accum) {
@@ -433,28 +439,45 @@ __device__ __forceinline__ float warpSum(float v) {
   return v;
 }
 
-// Second half of a split tile, one epilogue warp. `parts` = shared-memory address of the partial tiles, the same in every
-// CTA of the cluster.
+// Second half of a split tile, one epilogue warp. The CTAs of the cluster own a run of its output channels each. Every CTA
+// copies the rows of its partial tile to their owners (send); the owner adds the partials in rank order out of its own shared
+// memory (finish). One bulk copy per pair of CTAs: loads or stores from one SM to another move about 11 bytes per clock
+// (5-7 k clocks for the 56 KB of a CTA).
 // conv: a unit is one output channel of the tile, four columns per lane; the rank's 128 / split channels go round robin
 // over the epilogue warps, UB at a time so that their loads overlap. What does not depend on the contraction (bias,
 // residual) is loaded by prefetch(), for the first UB units before the accumulation.
 // ConvTranspose: a unit is one output channel x 32 input-rate columns, whose 32 * TS output samples are one run.
-// Bound by the SM-to-SM reads (about 11 bytes per clock and SM measured: 5-7 k clocks for the 56 KB of eight CTAs), which
-// is why the split tile is 128 and not 256 columns wide.
 template <int TS>
 struct SplitTail {
   static constexpr int UB = 4;
   float4 res[UB];
   float bias[UB];
   int row0, units, tt, cb;
+  int slot;  // rows that a CTA keeps per sender, enough for the largest share
+
+  // Rows [first, last) of the tile that CTA r owns. ConvTranspose: from its first channel's to its last one's, with the zero
+  // rows between two groups of 32.
+  static __device__ __forceinline__ void share(int split, int r, int& first, int& last) {
+    if constexpr (TS == 0) {
+      first = MT * r / split, last = MT * (r + 1) / split;
+    } else {
+      constexpr int CQ = 32 / TS, CH = 4 * CQ;
+      const int c0 = CH * r / split, c1 = CH * (r + 1) / split - 1;
+      first = (c0 / CQ) * 32 + (c0 % CQ) * TS, last = (c1 / CQ) * 32 + (c1 % CQ) * TS + TS;
+    }
+  }
 
   __device__ __forceinline__ SplitTail(const TcArgs& a, int tile, int rank) {
     tt = tile / a.numCoBlk, cb = tile - tt * a.numCoBlk;
     if constexpr (TS == 0) {
       row0 = MT * rank / a.split, units = MT * (rank + 1) / a.split - row0;
+      slot = (MT + a.split - 1) / a.split;
     } else {
       constexpr int CH = 4 * (32 / TS);
       row0 = CH * rank / a.split, units = (NTS / 32) * (CH * (rank + 1) / a.split - row0);  // row0: first channel
+      constexpr int CQ = 32 / TS;
+      const int n = (CH + a.split - 1) / a.split;  // channels: n * TS rows and the gaps between at most this many groups
+      slot = n * TS + (n + CQ - 2) / CQ * (32 - CQ * TS);
     }
   }
 
@@ -484,7 +507,21 @@ struct SplitTail {
     }
   }
 
-  __device__ __forceinline__ void finish(const TcArgs& a, uint32_t parts, int warp, int lane) {
+  // What CTA `to` owns of this CTA's partial tile. `recv` = where every CTA of the cluster receives, counted by `bar`.
+  __device__ __forceinline__ void send(const TcArgs& a, const float* tile, const float* recv, uint64_t* bar, int rank, int to) const {
+    int first, last;
+    share(a.split, to, first, last);
+    bulkCopyPeer(peerAddr(smemAddr(recv + rank * slot * PART_PITCH), to), tile + first * PART_PITCH,
+                 uint32_t((last - first) * PART_PITCH * 4), peerAddr(smemAddr(bar), to));
+  }
+  // Bytes that CTA `rank` receives.
+  static __device__ __forceinline__ uint32_t expected(const TcArgs& a, int rank) {
+    int first, last;
+    share(a.split, rank, first, last);
+    return uint32_t(a.split * (last - first) * PART_PITCH * 4);
+  }
+
+  __device__ __forceinline__ void finish(const TcArgs& a, const float* parts, int warp, int lane) {
     if constexpr (TS == 0) {
       const bool vecOut = ((reinterpret_cast<uintptr_t>(a.out) | uintptr_t(a.outPitch * 4)) & 15) == 0;
       const int64_t tChunk = int64_t(tt) * NTS, col = tChunk + lane * 4;
@@ -496,15 +533,14 @@ struct SplitTail {
         float4 acc[UB];
 #pragma unroll
         for (int e = 0; e < UB; ++e) acc[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-        const uint32_t at = parts + uint32_t(((row0 + u0) * PART_PITCH + lane * 4) * 4);
+        const float* at = parts + u0 * PART_PITCH + lane * 4;
         if (mine > 0) {
 #pragma unroll 4
-          for (int r = 0; r < a.split; ++r) {
-            const uint32_t peer = peerAddr(at, r);
+          for (int r = 0; r < a.split; ++r, at += slot * PART_PITCH) {
             float4 v[UB];
 #pragma unroll
             for (int e = 0; e < UB; ++e)
-              if (u0 + e * EPI_WARPS < units) v[e] = peerLoad4(peer + uint32_t(e * EPI_WARPS * PART_PITCH * 4));
+              if (u0 + e * EPI_WARPS < units) v[e] = *reinterpret_cast<const float4*>(at + e * EPI_WARPS * PART_PITCH);
               else v[e] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int e = 0; e < UB; ++e) acc[e].x += v[e].x, acc[e].y += v[e].y, acc[e].z += v[e].z, acc[e].w += v[e].w;
@@ -548,6 +584,7 @@ struct SplitTail {
     } else {
       constexpr int CQ = 32 / TS, CH = 4 * CQ, SEGS = NTS / 32;
       const int64_t uEnd = a.lo * TS;
+      const int firstRow = (row0 / CQ) * 32 + (row0 % CQ) * TS;
 #pragma unroll 1
       for (int u = warp; u < units; u += EPI_WARPS) {
         const int ch = row0 + u / SEGS, seg = u % SEGS, co = cb * CH + ch;
@@ -557,18 +594,18 @@ struct SplitTail {
         const float* const rrow = a.residual ? a.residual + int64_t(co) * a.resPitch : nullptr;
         const float b = a.bias ? a.bias[co] : 0.f;
         float acc[TS], rs[TS];
-        uint32_t off[TS];
+        const float* off[TS];
 #pragma unroll
         for (int f = 0; f < TS; ++f) {
           const int idx = f * 32 + lane;
-          off[f] = parts + uint32_t((((ch / CQ) * 32 + (ch % CQ) * TS + idx % TS) * PART_PITCH + seg * 32 + idx / TS) * 4);
+          off[f] = parts + ((ch / CQ) * 32 + (ch % CQ) * TS - firstRow + idx % TS) * PART_PITCH + seg * 32 + idx / TS;
           acc[f] = b;
           rs[f] = rrow && o0 + f * 32 < uEnd ? rrow[a.padLeft + o0 + f * 32] : 0.f;
         }
 #pragma unroll 2
         for (int r = 0; r < a.split; ++r)
 #pragma unroll
-          for (int f = 0; f < TS; ++f) acc[f] += peerLoad(peerAddr(off[f], r));
+          for (int f = 0; f < TS; ++f) acc[f] += off[f][r * slot * PART_PITCH];
 #pragma unroll
         for (int f = 0; f < TS; ++f) {
           const int64_t o = o0 + f * 32;
@@ -584,11 +621,11 @@ struct SplitTail {
 // PARTIAL: Co is not a multiple of 128 (the last output-channel block has rows that do not exist).
 // TS: 0 = conv1d; 6 / 10 = polyphase ConvTranspose1d of that stride (see the comment above convtTcPackKernel).
 // TMAO: residual and output boxes travel by TMA (rows 16-byte aligned; conv1d with Co % 128 == 0 only).
-// SPLIT: a cluster of a.split CTAs shares one 128-column tile. Each CTA contracts its own run of input-channel chunks and
-// leaves its partial tile in its shared memory (over the operand buffers, which nothing reads any more); after the
-// cluster barrier it finishes a slice of the output channels: the partials are added in rank order over distributed
-// shared memory, then bias, residual, scale, statistics and coalesced stores. For launches with fewer tiles than SMs,
-// where one tile's serial chain of chunks is the launch's time (see splitFor).
+// SPLIT: a cluster of a.split CTAs shares one 128-column tile. Each CTA contracts its own run of input-channel chunks. When
+// the MMAs of all of them are done (a cluster barrier under the last drain) it sends the rows of its partial tile to the CTAs
+// that own them, over the operand buffers there, which nothing reads any more; when it has all of its own it finishes them:
+// the partials are added in rank order, then bias, residual, scale, statistics and coalesced stores. For launches with fewer
+// tiles than SMs, where one tile's serial chain of chunks is the launch's time (see splitFor).
 template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT>
 __global__ void __launch_bounds__(NTHREADS, 1)
     convTcKernel(const TcArgs a, const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapExt,
@@ -622,7 +659,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   uint64_t* const rawFull = loEmpty + 1;
   uint64_t* const rawEmpty = rawFull + NRAW;
   uint64_t* const resBar = rawEmpty + NRAW;  // one per epilogue warp
-  uint32_t* const tmemSlot = reinterpret_cast<uint32_t*>(resBar + EPI_WARPS);
+  uint64_t* const recvBar = resBar + EPI_WARPS;  // split form: the rows from the CTAs of the cluster
+  uint64_t* const tileBar = recvBar + 1;     // and this CTA's partial tile, complete
+  uint32_t* const tmemSlot = reinterpret_cast<uint32_t*>(tileBar + 1);
   volatile int* const abortFlag = reinterpret_cast<int*>(tmemSlot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -649,6 +688,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     mbarInit(loFull, 1), mbarInit(loEmpty, EPI_WARPS);
     for (int i = 0; i < NRAW; ++i) mbarInit(&rawFull[i], 1), mbarInit(&rawEmpty[i], PRO_WARPS);
     for (int i = 0; i < EPI_WARPS; ++i) mbarInit(&resBar[i], 1);
+    mbarInit(recvBar, 1), mbarInit(tileBar, EPI_WARPS);
     *abortFlag = 0;
     fenceBarrierInit();
   }
@@ -694,6 +734,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (warp < EPI_WARPS) {
     // ------------------------------------------------------------------ accumulate + epilogue
     regInc<EPI_REGS>();
+    dependenciesWait();
     const int q = warp & 3, g = warp >> 2;  // TMEM lane quarter, 128-column half of the tile
     float* const tile = sStage + warp * STAGE_FLOATS;                                  // unaligned route: [32][33]
     unsigned char* const box = smemRaw + warp * BOX_BYTES;                             // aligned route: swizzled 32 x 32
@@ -705,8 +746,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const uint32_t laneBase = uint32_t(q * 32) << 16;
     constexpr uint32_t kSleepEpi = SPLIT ? SLEEP_EPI_SPLIT_NS : SLEEP_EPI_NS;
     uint32_t groupIt = 0, tileIt = 0, resIt = 0;
-    bool dead = false, resInFlight = false;
+    bool dead = false, resInFlight = false, arrived = false;
     SplitTail<TS> tail(a, tile0, rank);
+    float* const recv = sStage + PART_BYTES / 4;
+    if (SPLIT && threadIdx.x == 0) mbarArriveExpectTx(recvBar, tail.expected(a, rank));
     if constexpr (SPLIT) tail.prefetch(a, warp, lane);
     long long wHi = 0, wLo = 0, cPre = 0, cFin = 0;
     const long long tStart = kProf ? clock64() : 0;
@@ -825,6 +868,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           return false;
         }
         tcFenceAfter();
+        // Everything this CTA's MMAs read is read: peers may write over the operand buffers.
+        if (SPLIT && groupIt + 1 == uint32_t(nGroups)) clusterArrive(), arrived = true;
 #pragma unroll
         for (int b = 0; b < EC / 16; ++b) {
           uint32_t v[16];
@@ -898,10 +943,21 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (dead) break;
       const long long tFin = kProf ? clock64() : 0;
       if constexpr (SPLIT) {
-        // the last drain followed every MMA of this CTA, so the operand buffers are free
-        float* const row = reinterpret_cast<float*>(smemRaw) + (q * 32 + lane) * PART_PITCH + g * EC;
+        float* const row = sStage + (q * 32 + lane) * PART_PITCH + g * EC;
 #pragma unroll
         for (int j = 0; j < EC; j += 4) *reinterpret_cast<float4*>(row + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
+        fenceProxyAsync();  // generic-proxy stores -> visible to the bulk copies
+        __syncwarp();
+        if (lane == 0) mbarArrive(tileBar);
+        clusterWait();
+        if (warp < a.split) {
+          if (!mbarWait(tileBar, 0, abortFlag, 0)) {
+            giveUp(1, 5);
+            dead = true;
+          } else if (lane == 0) {
+            tail.send(a, sStage, recv, recvBar, rank, warp);
+          }
+        }
         if (kProf) cFin += clock64() - tFin;
         continue;
       }
@@ -1051,8 +1107,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (kProf) cFin += clock64() - tFin;
     }
     if constexpr (SPLIT) {
-      clusterSync();
-      tail.finish(a, smemAddr(smemRaw), warp, lane);
+      if (dead) {  // the arrival that the peers wait for
+        if (!arrived) clusterArrive(), clusterWait();
+      } else if (!mbarWait(recvBar, 0, abortFlag, 0)) {
+        giveUp(1, 4);
+      } else {
+        tail.finish(a, recv, warp, lane);
+      }
     }
     // Copies of this warp still in flight must end before the CTA may exit: a residual box after an abort, and the
     // output boxes on every path.
@@ -1063,6 +1124,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   } else if (warp < EPI_WARPS + PRO_WARPS) {
     // ------------------------------------------------------------------ activation producers
     regDec<PRO_REGS>();
+    dependenciesWait();
     const int pw = warp - EPI_WARPS;
     const int cg = pw & 3, hf = pw >> 2;  // channel group of 4 inside the 16-channel chunk; half of the tile's columns
     // A warp stages the rows of its half, SLOTS per lane, with addresses that are immediates. The rows beyond the tile's
@@ -1251,6 +1313,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     regDec<CTL_REGS>();
     if (warp == W_WARP) {
       // ---------------------------------------------------------------- weight producer
+      dependenciesWait();  // the pack may have been queued just before; the input window is waited for longer anyway
       uint32_t wIt = 0, ws = 0, wPh = 1;  // stages issued, ring slot, parity of the slot's previous release
       bool dead = false;
       long long wW = 0;
@@ -1292,6 +1355,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // (a box holds at most 256 elements per dimension): the tile's columns and what lies beyond them. Columns outside
       // [0, L) arrive as zeros and are never used: the producers write the zero padding themselves, after the activation.
       if (a.tmaIn && lane == 0) {
+        dependenciesWait();
         uint32_t rb = 0, ph = 1, issued = 0;
         long long wR = 0;
         bool dead = false;
@@ -1447,6 +1511,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
         tilePar ^= 1;
       }
+      dependentsLaunch();  // this CTA's tensor work is queued; what follows it may set itself up under the tail
       __syncwarp();
       if (kProf) profAdd(0, wBf), profAdd(1, wHe), profAdd(2, wWf), profAdd(3, wLe), profAdd(4, clock64() - tStart);
     }
@@ -1454,8 +1519,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 
   tcFenceBefore();
   if constexpr (SPLIT) {
-    if (warp >= EPI_WARPS) clusterSync();  // the epilogue warps' part of the first barrier is in their branch
-    clusterSync();                         // no CTA leaves while another reads its partial tile
+    if (warp >= EPI_WARPS) clusterArrive(), clusterWait();  // the epilogue warps' part of the first barrier is in their branch
+    clusterArrive(), clusterWait();                         // no CTA leaves before what it sent has arrived
   }
   __syncthreads();
   if (warp == MMA_WARP) {
@@ -1554,7 +1619,8 @@ static size_t convTcSmemBytes(bool split, int64_t ci, int rows, int k, bool f16,
   const int actRow = f16 ? Fmt<true>::ACT_BYTES_PER_ROW : Fmt<false>::ACT_BYTES_PER_ROW;
   const int nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
   const int ext = rawExt(rows, split ? NTS : NT);
-  const SmemLayout base = smemLayout(split, int(ci), rows, ext, nb, 0, 0, actRow, tap);
+  SmemLayout base = smemLayout(split, int(ci), rows, ext, nb, 0, 0, actRow, tap);
+  base.total -= base.par - base.w;  // without the split form's memory behind the MMAs, which the ring may lie in
   if (base.total > uint32_t(kMaxSmem)) return 0;
   const size_t avail = size_t(kMaxSmem) - base.total;
   // Large groups matter more than a deep ring (measured: two slots of four taps beat four slots of three, and at
@@ -1573,7 +1639,8 @@ static size_t convTcSmemBytes(bool split, int64_t ci, int rows, int k, bool f16,
   if (bestG == 0) return 0;
   if (wStages) *wStages = bestWs;
   if (wG) *wG = bestG;
-  return smemLayout(split, int(ci), rows, ext, nb, bestWs, bestG, actRow, tap).total;
+  const size_t total = smemLayout(split, int(ci), rows, ext, nb, bestWs, bestG, actRow, tap).total;
+  return total <= size_t(kMaxSmem) ? total : 0;
 }
 
 // The hi chain between two drains holds at most MAX_CHAIN MMAs: whole chunks while they fit, and a chunk that alone
@@ -1716,20 +1783,22 @@ static int launchTc4(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cu
     if (e != cudaSuccess) return failCuda("conv (tensor-core): cudaFuncSetAttribute", e);
     configured[dev] = true;
   }
-  if constexpr (SPLIT) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = unsigned(a.split), attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(unsigned(grid)), cfg.blockDim = dim3(NTHREADS), cfg.dynamicSmemBytes = smem, cfg.stream = s;
-    cfg.attrs = attr, cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, m.x, m.ext, m.res, m.out);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return failCuda("conv (tensor-core)", e);
-    }
-  } else {
-    kernel<<<grid, NTHREADS, smem, s>>>(a, m.x, m.ext, m.res, m.out);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.gridDim = dim3(unsigned(grid)), cfg.blockDim = dim3(NTHREADS), cfg.dynamicSmemBytes = smem, cfg.stream = s, cfg.attrs = attr;
+  if (a.early) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (SPLIT) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = unsigned(a.split), attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a, m.x, m.ext, m.res, m.out);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return failCuda("conv (tensor-core)", e);
   }
   return launched("conv (tensor-core)");
 }
@@ -1828,6 +1897,11 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercen
   a.drainN = n < 1 ? 1 : n;
   const int tiles = a.numTTiles * a.numCoBlk;
   *grid = a.split ? tiles * a.split : (tiles < d->smCount ? tiles : d->smCount);
+  // A launch of one round starts as the SMs come free and sets itself up under the end of the one before it: 3 us of a split
+  // launch's 14. CTAs that wait hold SMs that a ready launch of another stream could use, so beside other launches this is for
+  // those of so few tiles that the launches beside them are split as well. us per forward, no launch early / every split one:
+  // T = 24 366 / 337, T = 80 528 / 513, T = 121 598 / 633, T = 320 934 / 992.
+  a.early = smPercent == 100 ? tiles <= d->smCount : a.split && tiles * 8 <= d->smCount;
   a.tmaOut = 0;
   if (boxesOk && a.co % MT == 0 && makeMap(&m.out, a.out, a.co, a.lo, a.outPitch, BOX, BOX, true) &&
       (!a.residual || makeMap(&m.res, a.residual, a.co, a.lo, a.resPitch, BOX, BOX, true)))

@@ -119,9 +119,12 @@ def test_conv1d_fused(cuda, ci, co, l, k, d, variant):
 # Ci far above Co, and on a 148-SM device the last length with two CTAs per tile and the first without.
 SPLIT_CASES = [(48, 129, 129, 3, 1), (80, 128, 257, 5, 2), (112, 256, 1, 7, 1), (16, 22, 127, 1, 1), (1104, 64, 97, 3, 1),
                (128, 128, 9472, 3, 1), (128, 128, 9473, 3, 1)]
+# Windows that reach 28, 30, 48 and 50 columns beyond a tile, with and without the up to three columns in front of a 16-byte
+# boundary (31 to 53 staged rows beyond the tile: one or two slots of 32), both tile widths, first and last columns of a row.
+WINDOW_CASES = [(32, 128, 515, 8, 4), (32, 128, 512, 7, 5), (32, 128, 19001, 7, 5), (48, 128, 700, 9, 6), (48, 128, 19003, 11, 5)]
 
 
-@pytest.mark.parametrize("ci,co,l,k,d", SPLIT_CASES)
+@pytest.mark.parametrize("ci,co,l,k,d", SPLIT_CASES + WINDOW_CASES)
 @pytest.mark.parametrize("padded", [False, True])
 def test_conv1d_few_tiles(cuda, ci, co, l, k, d, padded):
     """Channels of a tile contracted by several CTAs, on both row layouts, with residual and scale: against the float64
