@@ -321,6 +321,33 @@ typedef struct LkcResblockIo {
   int64_t workspace_bytes;
   int64_t launches; /* out */
 } LkcResblockIo;
+/* One AdainResBlk1d of the decoder (models/kokoro/model.py:158-221). cin: channels of its input including the zero rows that
+ * pad it to a multiple of 16; gb: offset of (gamma | beta) of norm1 (of cin channels each, padded likewise) and norm2. The
+ * pool (up) is the depthwise ConvTranspose1d of stride 2, K 3, padding 1, output padding 1. */
+typedef struct LkcDecoderBlock {
+  int64_t cin, cout, up;
+  const void *w1, *b1, *w2, *b2, *w1x1, *b1x1, *pool_w, *pool_b; /* w1x1 f32[cout, cin, 1]; pool_w f32[cin, 1, 3] */
+  const LkcConvState *state1, *state2, *state1x1;
+  int64_t gb1, gb2;
+} LkcDecoderBlock;
+/* The decoder (models/kokoro/model.py:704-717): encode, then four blocks over [block output, asr_res, F0, N, zero rows]. */
+typedef struct LkcDecoder {
+  const void *bank_wt, *bank_b;
+  int64_t bank_n;
+  const void *f0_w, *f0_b, *n_w, *n_b; /* f32[1, 1, 3], f32[1]: stride 2, padding 1 */
+  const void *asr_w, *asr_b;           /* f32[64, 512, 1], f32[64] */
+  const LkcConvState* asr_state;
+  LkcDecoderBlock block[5];
+} LkcDecoder;
+typedef struct LkcDecoderIo {
+  const void *asr, *f0, *n, *s; /* f32[512, frames] (rows asr_pitch floats apart), f32[2 frames] twice, f32[128] */
+  void* out;                    /* f32[512, 2 frames], rows out_pitch floats apart */
+  int64_t frames, asr_pitch, out_pitch;
+  void* workspace;
+  int64_t workspace_bytes;
+  void* side;       /* a stream for the shortcuts; joined back before the call's last kernel */
+  int64_t launches; /* out: kernels queued */
+} LkcDecoderIo;
 typedef struct LkcModel LkcModel;
 /* The handle copies the struct and keeps the events of the stream joins and the memory plans of the last lengths. Calls on
  * one handle may come from several threads. */
@@ -328,6 +355,10 @@ LKC_API LkcModel* lkc_generator_create(const LkcGenerator* w);
 LKC_API void lkc_model_destroy(LkcModel* m);
 LKC_API int lkc_generator_workspace(LkcModel* m, int64_t t, int concurrent, int64_t* bytes, int64_t* unplanned);
 LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, void* stream);
+/* The decoder's forward as one call, under the same rules; the handle of one model is refused by the calls of the other. */
+LKC_API LkcModel* lkc_decoder_create(const LkcDecoder* w);
+LKC_API int lkc_decoder_workspace(LkcModel* m, int64_t frames, int64_t* bytes);
+LKC_API int lkc_decoder_forward(LkcModel* m, LkcDecoderIo* io, void* stream);
 LKC_API int lkc_resblock(const LkcResblock* w, LkcResblockIo* io, void* stream);
 
 /* ---- device-side test harness (the data path of the reference's RUN2 message, include/lokinfer/remote/server.h:30-47)

@@ -52,6 +52,28 @@ class LkcGeneratorIo(ctypes.Structure):
                 ("launches", ctypes.c_int64)]
 
 
+class LkcDecoderBlock(ctypes.Structure):
+    _fields_ = [("cin", ctypes.c_int64), ("cout", ctypes.c_int64), ("up", ctypes.c_int64), ("w1", ctypes.c_void_p),
+                ("b1", ctypes.c_void_p), ("w2", ctypes.c_void_p), ("b2", ctypes.c_void_p), ("w1x1", ctypes.c_void_p),
+                ("b1x1", ctypes.c_void_p), ("pool_w", ctypes.c_void_p), ("pool_b", ctypes.c_void_p), ("state1", ctypes.c_void_p),
+                ("state2", ctypes.c_void_p), ("state1x1", ctypes.c_void_p), ("gb1", ctypes.c_int64),
+                ("gb2", ctypes.c_int64)]
+
+
+class LkcDecoder(ctypes.Structure):
+    _fields_ = [("bank_wt", ctypes.c_void_p), ("bank_b", ctypes.c_void_p), ("bank_n", ctypes.c_int64),
+                ("f0_w", ctypes.c_void_p), ("f0_b", ctypes.c_void_p), ("n_w", ctypes.c_void_p), ("n_b", ctypes.c_void_p),
+                ("asr_w", ctypes.c_void_p), ("asr_b", ctypes.c_void_p), ("asr_state", ctypes.c_void_p),
+                ("block", LkcDecoderBlock * 5)]
+
+
+class LkcDecoderIo(ctypes.Structure):
+    _fields_ = [("asr", ctypes.c_void_p), ("f0", ctypes.c_void_p), ("n", ctypes.c_void_p), ("s", ctypes.c_void_p),
+                ("out", ctypes.c_void_p), ("frames", ctypes.c_int64), ("asr_pitch", ctypes.c_int64),
+                ("out_pitch", ctypes.c_int64), ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_int64),
+                ("side", ctypes.c_void_p), ("launches", ctypes.c_int64)]
+
+
 class LkcResblockIo(ctypes.Structure):
     _fields_ = [("x", ctypes.c_void_p), ("stats", ctypes.c_void_p), ("bank", ctypes.c_void_p), ("out", ctypes.c_void_p),
                 ("out_stats", ctypes.c_void_p), ("l", ctypes.c_int64), ("x_pitch", ctypes.c_int64),
@@ -124,6 +146,12 @@ def lib():
                                               ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]
         l.lkc_generator_forward.restype = ctypes.c_int
         l.lkc_generator_forward.argtypes = [ctypes.c_void_p, ctypes.POINTER(LkcGeneratorIo), ctypes.c_void_p]
+        l.lkc_decoder_create.restype = ctypes.c_void_p
+        l.lkc_decoder_create.argtypes = [ctypes.POINTER(LkcDecoder)]
+        l.lkc_decoder_workspace.restype = ctypes.c_int
+        l.lkc_decoder_workspace.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.POINTER(ctypes.c_int64)]
+        l.lkc_decoder_forward.restype = ctypes.c_int
+        l.lkc_decoder_forward.argtypes = [ctypes.c_void_p, ctypes.POINTER(LkcDecoderIo), ctypes.c_void_p]
         l.lkc_resblock.restype = ctypes.c_int
         l.lkc_resblock.argtypes = [ctypes.POINTER(LkcResblock), ctypes.POINTER(LkcResblockIo), ctypes.c_void_p]
         _lib = l

@@ -1805,7 +1805,7 @@ static int launchTc4(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cu
 
 template <int ACT, bool PARTIAL, int TS, bool F16>
 static int launchTc3(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cudaStream_t s) {
-  if constexpr (F16) {  // the second half of a split tile handles every Co and alignment
+  if constexpr (F16 || (ACT == 0 && TS == 0)) {  // the second half of a split tile handles every Co and alignment
     if (a.split) return launchTc4<ACT, false, TS, F16, false, true>(a, m, grid, smem, s);
   }
   if constexpr (TS == 0 && !PARTIAL) {
@@ -1853,8 +1853,10 @@ int convTcProfile(int enable, long long* out16) {
 // 48 clusters of three where 45 fit, 36 us against 30 us unsplit and 21 us with two CTAs per tile.
 // Measured (us, persistent -> split): [256, 240] K = 11: 52 -> 15; [256, 1210] K = 7: 49 -> 17; [128, 1441] K = 3: 29 -> 12;
 // [1104 -> 1024, 61] K = 3: 130 -> 19; [256, 3200] K = 11, two CTAs per tile: 52 -> 30.
-static int splitFor(bool f16, int ci, int64_t lo, int64_t coBlocks, int sms, const int32_t* clusters) {
-  if (!f16) return 0;
+// Of the convs with tf32 halves the pointwise ones without an activation split (the decoder's shortcuts).
+static bool splits(bool f16, int64_t k, Act act) { return f16 || (k == 1 && act == Act::None); }
+static int splitFor(bool can, int ci, int64_t lo, int64_t coBlocks, int sms, const int32_t* clusters) {
+  if (!can) return 0;
   const int n = ci / KC;
   const int64_t tiles = ceilDiv(lo, NTS) * coBlocks;
   for (int sp = int(std::min<int64_t>(std::min(MAX_SPLIT, n), sms / tiles)); sp >= 2; --sp) {
@@ -1869,10 +1871,10 @@ int convTcSplitRule(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* 
 }
 
 // Launch geometry and tensor maps shared by the conv and ConvTranspose entry points.
-static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercent, int* grid, size_t* smem) {
+static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool canSplit, bool boxesOk, int smPercent, int* grid, size_t* smem) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
-  a.split = splitFor(f16, a.ci, a.lo, a.numCoBlk, d->smCount * smPercent / 100, d->clusters);
+  a.split = splitFor(canSplit, a.ci, a.lo, a.numCoBlk, d->smCount * smPercent / 100, d->clusters);
   LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
   const int nt = a.split ? NTS : NT;
   a.numTTiles = int(ceilDiv(a.lo, nt));
@@ -1912,7 +1914,7 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool boxesOk, int smPercen
 bool convTcSplits(const ConvFusedParams& p, bool f16) {
   const DeviceInfo* d = nullptr;
   return deviceInfo(&d) == 0 &&
-         splitFor(f16, int(p.ci), p.lo, ceilDiv(p.co, MT), d->smCount * p.smPercent / 100, d->clusters) != 0;
+         splitFor(splits(f16, p.k, p.act), int(p.ci), p.lo, ceilDiv(p.co, MT), d->smCount * p.smPercent / 100, d->clusters) != 0;
 }
 
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {
@@ -1934,7 +1936,7 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
   a.numCoBlk = int(coBlk);
   int grid = 0;
   size_t smem = 0;
-  if (int rc = finishArgs(a, m, f16, true, p.smPercent, &grid, &smem)) return rc;
+  if (int rc = finishArgs(a, m, f16, splits(f16, p.k, p.act), true, p.smPercent, &grid, &smem)) return rc;
   switch (p.act) {
     case Act::None: return launchTc<0>(a, m, f16, grid, smem, s);
     case Act::Snake: return launchTc<1>(a, m, f16, grid, smem, s);
@@ -1989,7 +1991,7 @@ int convtTc(const ConvtParams& p, const float* wp, bool f16, cudaStream_t s) {
   a.numCoBlk = int(coBlk);
   int grid = 0;
   size_t smem = 0;
-  if (int rc = finishArgs(a, m, f16, false, p.smPercent, &grid, &smem)) return rc;
+  if (int rc = finishArgs(a, m, f16, f16, false, p.smPercent, &grid, &smem)) return rc;
   if (p.stride == 6) return launchTc2<2, false, 6>(a, m, f16, grid, smem, s);
   return launchTc2<2, false, 10>(a, m, f16, grid, smem, s);
 }

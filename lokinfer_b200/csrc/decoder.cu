@@ -57,7 +57,86 @@ __global__ void concatRowsKernel(const ConcatArgs a, float* __restrict__ out) {
   }
 }
 
+// The rows around the convs' results in the decoder's two kinds of block input, in one pass: enc = [asr (512 rows), F0, N,
+// zeros], and of cat the rows from catRow on = [F0, N, zeros], where F0 / N are the pitch and energy curves f32[2 l] through
+// their 3-tap convs of stride 2 and padding 1. One block row per channel row of enc, lanes along time.
+__global__ void decoderInputsKernel(const float* __restrict__ asr, int64_t asrPitch, const float* __restrict__ f0,
+                                    const float* __restrict__ n, const float* __restrict__ f0w, const float* __restrict__ f0b,
+                                    const float* __restrict__ nw, const float* __restrict__ nb, float* __restrict__ enc,
+                                    float* __restrict__ cat, int64_t catRow, int64_t catRows, int64_t l, int64_t pitch) {
+  const int64_t row = blockIdx.y;
+  for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < l; j += int64_t(gridDim.x) * blockDim.x) {
+    float v = 0.f;
+    if (row < 512) {
+      v = asr[row * asrPitch + j];
+    } else if (row < 514) {
+      const float *x = row == 512 ? f0 : n, *w = row == 512 ? f0w : nw;
+      if (j > 0) v = fmaf(x[2 * j - 1], w[0], v);
+      v = fmaf(x[2 * j], w[1], v);
+      v = fmaf(x[2 * j + 1], w[2], v);
+      v += *(row == 512 ? f0b : nb);
+    }
+    enc[row * pitch + j] = v;
+    if (row >= 512 && row - 512 + catRow < catRows) cat[(row - 512 + catRow) * pitch + j] = v;
+  }
+}
+
+// leaky((x - mean) * scale + beta) through the depthwise ConvTranspose1d of stride 2, K 3, padding 1, output padding 1:
+// out[2 j] = b + a_j w1, out[2 j + 1] = b + a_j w2 + a_(j + 1) w0. Bound by memory: 4 bytes read (the neighbour's column from
+// cache) and 8 written per element, where AdaIN, leaky and the transposed conv as kernels of their own moved 36.
+__global__ void adainLeakyPoolKernel(const float* __restrict__ x, const float* __restrict__ affine,
+                                     const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ out,
+                                     int64_t c, int64_t l, int64_t xPitch, int64_t outPitch, float slope) {
+  const int64_t ch = blockIdx.y;
+  const float mean = affine[ch], scale = affine[c + ch], beta = affine[2 * c + ch], b = bias[ch];
+  const float w0 = w[3 * ch], w1 = w[3 * ch + 1], w2 = w[3 * ch + 2];
+  const float* const xr = x + ch * xPitch;
+  float* const o = out + ch * outPitch;
+  auto act = [&](float v) {
+    v = fmaf(v - mean, scale, beta);
+    return v >= 0.f ? v : v * slope;
+  };
+  for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < l; j += int64_t(gridDim.x) * blockDim.x) {
+    const float a0 = act(xr[j]);
+    float odd = fmaf(a0, w2, b);
+    if (j + 1 < l) odd = fmaf(act(xr[j + 1]), w0, odd);
+    o[2 * j] = fmaf(a0, w1, b), o[2 * j + 1] = odd;
+  }
+}
+
+__global__ void upsampleRows2Kernel(const float* __restrict__ x, float* __restrict__ out, int64_t l, int64_t xPitch,
+                                    int64_t outPitch) {
+  for (int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; j < l; j += int64_t(gridDim.x) * blockDim.x) {
+    const float v = x[blockIdx.y * xPitch + j];
+    out[blockIdx.y * outPitch + 2 * j] = v, out[blockIdx.y * outPitch + 2 * j + 1] = v;
+  }
+}
+
+inline dim3 rowGrid(int64_t l, int64_t rows) {
+  const int64_t b = ceilDiv(l, kThreads);
+  return dim3(unsigned(b < 64 ? b : 64), unsigned(rows));
+}
+
 }  // namespace
+
+int decoderInputs(const float* asr, int64_t asrPitch, const float* f0, const float* n, const float* f0w, const float* f0b,
+                  const float* nw, const float* nb, float* enc, int64_t encRows, float* cat, int64_t catRow, int64_t catRows,
+                  int64_t l, int64_t pitch, cudaStream_t s) {
+  // the rows of cat ride on those of enc: both have F0, N and zeros up to a multiple of 16 (514 -> 528, 1090 -> 1104)
+  LKC_REQUIRE(encRows - 512 >= catRows - catRow, "decoder: block inputs");
+  decoderInputsKernel<<<rowGrid(l, encRows), kThreads, 0, s>>>(asr, asrPitch, f0, n, f0w, f0b, nw, nb, enc, cat, catRow,
+                                                               catRows, l, pitch);
+  return launched("decoder inputs");
+}
+int adainLeakyPool(const float* x, const float* affine, const float* w, const float* bias, float* out, int64_t c, int64_t l,
+                   int64_t xPitch, int64_t outPitch, float slope, cudaStream_t s) {
+  adainLeakyPoolKernel<<<rowGrid(l, c), kThreads, 0, s>>>(x, affine, w, bias, out, c, l, xPitch, outPitch, slope);
+  return launched("decoder pool");
+}
+int upsampleRows2(const float* x, float* out, int64_t c, int64_t l, int64_t xPitch, int64_t outPitch, cudaStream_t s) {
+  upsampleRows2Kernel<<<rowGrid(l, c), kThreads, 0, s>>>(x, out, l, xPitch, outPitch);
+  return launched("decoder upsample");
+}
 }  // namespace lkc
 
 using namespace lkc;

@@ -136,6 +136,13 @@ int addRows(const float* a, const float* b, float* out, int64_t n, cudaStream_t 
 int add3Scale(const float* a, const float* b, const float* c, float* out, int64_t n, float scale, cudaStream_t s);
 int spaceToDepth(const float* x, float* y, int64_t ci, int64_t l, int64_t rows, int64_t ly, int64_t xPitch, int64_t yPitch,
                  int64_t stride, int64_t pad, cudaStream_t s);
+// Decoder (decoder.cu): rows 512, 513 and up of a block input [512 + tail, l], see there.
+int decoderInputs(const float* asr, int64_t asrPitch, const float* f0, const float* n, const float* f0w, const float* f0b,
+                  const float* nw, const float* nb, float* enc, int64_t encRows, float* cat, int64_t catRow, int64_t catRows,
+                  int64_t l, int64_t pitch, cudaStream_t s);
+int adainLeakyPool(const float* x, const float* affine, const float* w, const float* bias, float* out, int64_t c, int64_t l,
+                   int64_t xPitch, int64_t outPitch, float slope, cudaStream_t s);
+int upsampleRows2(const float* x, float* out, int64_t c, int64_t l, int64_t xPitch, int64_t outPitch, cudaStream_t s);
 int istftLogits(const float* x, float* out, int64_t l, int64_t pitch, int nfft, int hop, cudaStream_t s);
 
 }  // namespace lkc

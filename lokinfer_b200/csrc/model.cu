@@ -323,6 +323,82 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
   });
 }
 
+// The decoder (models/kokoro/model.py:704-717), stream 1 for the shortcuts. A block's input is ONE buffer `cat` for the four
+// decode blocks: rows [0, 1024) are what the block before wrote (a block reads them in its first conv and its shortcut, both
+// before its second conv overwrites them), the others asr_res, F0, N and zero rows, written once. So nothing is concatenated
+// between blocks, and the chunk statistics of the block's rows come from the epilogue that wrote them.
+constexpr int64_t kDecIn[2] = {528, 1104}, kDecCh = 1024, kDecOut = 512;
+constexpr float kDecSlope = 0.2f, kSqrtHalf = 0.7071067811865476f;
+
+void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
+  const int64_t f = io.frames;
+  const Buf none;
+  auto from = [](Buf b, int64_t floats) {  // the same buffer from an offset on
+    if (b.p) b.p += floats;
+    return b;
+  };
+  Buf bank = e.alloc(0, m.bank_n), enc = e.rows(0, kDecIn[0], f), cat = e.rows(0, kDecIn[1], f);
+  Buf encStats = statsBuf(e, 0, kDecIn[0], f), catStats = statsBuf(e, 0, kDecIn[1], f);
+  const int64_t pitch = enc.pitch, chunkFloats = 2 * statChunks(f);
+  e.launch(0, {bank}, [&](cudaStream_t st) { return gemmBias(FP(io.s), FP(m.bank_wt), FP(m.bank_b), bank.p, 1, 128, m.bank_n, st); });
+  e.launch(0, {enc, cat}, [&](cudaStream_t st) {
+    return decoderInputs(FP(io.asr), io.asr_pitch, FP(io.f0), FP(io.n), FP(m.f0_w), FP(m.f0_b), FP(m.n_w), FP(m.n_b), enc.p,
+                         kDecIn[0], cat.p, kDecCh + 64, kDecIn[1], f, pitch, st);
+  });
+  e.join(1, 0);
+  conv(e, 1, Act::None, enc, f, 512, 64, 1, 1, 0, m.asr_w, m.asr_b, none, nullptr, 0.f, m.asr_state, none,
+       from(cat, kDecCh * pitch), from(catStats, kDecCh * chunkFloats), 100);
+  e.launch(1, {cat, catStats}, [&](cudaStream_t st) {
+    return channelStats(cat.p + (kDecCh + 64) * pitch, catStats.p + (kDecCh + 64) * chunkFloats, kDecIn[1] - kDecCh - 64, f,
+                        pitch, statChunks(f), st);
+  });
+  e.launch(0, {enc, encStats}, [&](cudaStream_t st) { return channelStats(enc.p, encStats.p, kDecIn[0], f, pitch, statChunks(f), st); });
+
+  // AdaIN -> leaky -> conv k 3 [+ residual, scaled]; see adainConv
+  auto leakyConv = [&](Buf x, Buf stats, int64_t l, int64_t ci, int64_t co, const void* w, const void* b, const LkcConvState* state,
+                       int64_t gbAt, Buf residual, Buf out, Buf outStats) {
+    const Buf af = e.alloc(0, 3 * ci);
+    ConvFusedParams p;
+    p.x = x.p, p.w = FP(w), p.bias = FP(b), p.affine = af.p, p.residual = residual.p, p.out = out.p, p.stats = outStats.p;
+    p.ci = ci, p.l = l, p.co = co, p.k = 3, p.padding = 1, p.lo = l;
+    p.xPitch = x.pitch, p.resPitch = residual.pitch, p.outPitch = out.pitch;
+    p.act = Act::Leaky, p.slope = kDecSlope, p.state = state, p.outScale = residual.pitch ? kSqrtHalf : 1.f;
+    const float* gb = bank.p + gbAt;
+    if (e.running() && convFoldsAffine(p))
+      p.statsIn = stats.p, p.gb = gb, p.eps = kEps;
+    else
+      e.launch(0, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, ci, l, kEps, st); });
+    e.launch(0, {x, stats, bank, af, residual, out, outStats}, [&](cudaStream_t st) { return convFused(p, st); });
+  };
+
+  for (int i = 0; i < 5; ++i) {
+    const LkcDecoderBlock& b = m.block[i];
+    const Buf x = i == 0 ? enc : cat, stats = i == 0 ? encStats : catStats;
+    const int64_t l = b.up ? 2 * f : f;
+    Buf h = e.rows(0, b.cout, l), hStats = statsBuf(e, 0, b.cout, l), sc = e.rows(0, b.cout, f);
+    e.join(1, 0);
+    conv(e, 1, Act::None, x, f, b.cin, b.cout, 1, 1, 0, b.w1x1, b.b1x1, none, nullptr, 0.f, b.state1x1, none, sc, none, 100);
+    if (!b.up) {
+      leakyConv(x, stats, f, b.cin, b.cout, b.w1, b.b1, b.state1, b.gb1, none, h, hStats);
+      e.join(0, 1);
+      leakyConv(h, hStats, f, b.cout, b.cout, b.w2, b.b2, b.state2, b.gb2, sc, cat, catStats);
+    } else {
+      const Buf up = e.rows(1, b.cout, l);
+      e.launch(1, {sc, up}, [&](cudaStream_t st) { return upsampleRows2(sc.p, up.p, b.cout, f, sc.pitch, up.pitch, st); });
+      const Buf af = e.alloc(0, 3 * b.cin), r = e.rows(0, b.cin, l);
+      e.launch(0, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, bank.p + b.gb1, af.p, b.cin, f, kEps, st); });
+      e.launch(0, {x, af, r}, [&](cudaStream_t st) {
+        return adainLeakyPool(x.p, af.p, FP(b.pool_w), FP(b.pool_b), r.p, b.cin, f, x.pitch, r.pitch, kDecSlope, st);
+      });
+      conv(e, 0, Act::None, r, l, b.cin, b.cout, 3, 1, 1, b.w1, b.b1, none, nullptr, 0.f, b.state1, none, h, hStats, 100);
+      e.join(0, 1);
+      Buf out;
+      out.p = static_cast<float*>(io.out), out.pitch = io.out_pitch;
+      leakyConv(h, hStats, l, b.cout, b.cout, b.w2, b.b2, b.state2, b.gb2, up, out, none);
+    }
+  }
+}
+
 }  // namespace
 }  // namespace lkc
 
@@ -333,7 +409,9 @@ bool isConcurrent(int64_t mode) { return mode != 0 && mode != LKC_UNPLANNED; }
 }  // namespace
 
 struct LkcModel {
+  bool isDecoder = false;
   LkcGenerator w;
+  LkcDecoder dec;
   cudaEvent_t events[kEvents] = {};
   std::mutex mutex;
   std::list<std::shared_ptr<const Plan>> plans;  // most recently used first
@@ -350,10 +428,16 @@ struct LkcModel {
       }
     auto p = std::make_shared<Plan>();
     p->key = key;
-    LkcGeneratorIo io{};
-    io.t = t;
     Exec e(concurrent);
-    generator(e, w, io);
+    if (isDecoder) {
+      LkcDecoderIo io{};
+      io.frames = t;
+      decoder(e, dec, io);
+    } else {
+      LkcGeneratorIo io{};
+      io.t = t;
+      generator(e, w, io);
+    }
     if (int rc = e.finishPlan(p.get(), overlay)) return rc;
     plans.push_front(p);
     if (plans.size() > kPlans) plans.pop_back();
@@ -374,6 +458,18 @@ bool resblockFits(const LkcResblock& w, int64_t c, int64_t bankN) {
   for (int i = 0; i < 6; ++i)
     if (w.gb[i] > bankN - 2 * c || (w.state[i] && !stateFits(w.state[i], c, c, w.k, 0))) return false;
   return true;
+}
+// The handle with its events, or null (and the handle gone).
+LkcModel* withEvents(LkcModel* m) {
+  for (cudaEvent_t& ev : m->events) {
+    const cudaError_t err = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (err != cudaSuccess) {
+      failCuda("model: cudaEventCreate", err);
+      lkc_model_destroy(m);
+      return nullptr;
+    }
+  }
+  return m;
 }
 }  // namespace
 
@@ -401,15 +497,31 @@ extern "C" LKC_API LkcModel* lkc_generator_create(const LkcGenerator* w) {
     return nullptr;
   }
   m->w = *w;
-  for (cudaEvent_t& ev : m->events) {
-    const cudaError_t err = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-    if (err != cudaSuccess) {
-      failCuda("generator_create: cudaEventCreate", err);
-      lkc_model_destroy(m);
-      return nullptr;
-    }
+  return withEvents(m);
+}
+
+extern "C" LKC_API LkcModel* lkc_decoder_create(const LkcDecoder* w) {
+  const char* bad = nullptr;
+  if (!w) bad = "decoder_create: null weights";
+  if (!bad && (!w->bank_wt || !w->bank_b || w->bank_n < 1 || w->bank_n > 0x7fffffff || !w->f0_w || !w->f0_b || !w->n_w ||
+               !w->n_b || !w->asr_w || !w->asr_b || !stateFits(w->asr_state, 64, 512, 1, 0)))
+    bad = "decoder_create: null weight or bad asr_res";
+  for (int i = 0; !bad && i < 5; ++i) {
+    const LkcDecoderBlock& b = w->block[i];
+    const int64_t cin = kDecIn[i > 0], cout = i == 4 ? kDecOut : kDecCh;
+    if (b.cin != cin || b.cout != cout || b.up != (i == 4) || !b.w1 || !b.b1 || !b.w2 || !b.b2 || !b.w1x1 || !b.b1x1 ||
+        (b.up && (!b.pool_w || !b.pool_b)) || !stateFits(b.state1, cout, cin, 3, 0) || !stateFits(b.state2, cout, cout, 3, 0) ||
+        !stateFits(b.state1x1, cout, cin, 1, 0) || b.gb1 < 0 || b.gb1 > w->bank_n - 2 * cin || b.gb2 < 0 ||
+        b.gb2 > w->bank_n - 2 * cout)
+      bad = "decoder_create: bad block";
   }
-  return m;
+  LkcModel* m = bad ? nullptr : new (std::nothrow) LkcModel;
+  if (!m) {
+    fail(bad ? bad : "decoder_create: out of host memory");
+    return nullptr;
+  }
+  m->isDecoder = true, m->dec = *w;
+  return withEvents(m);
 }
 
 extern "C" LKC_API void lkc_model_destroy(LkcModel* m) {
@@ -420,7 +532,7 @@ extern "C" LKC_API void lkc_model_destroy(LkcModel* m) {
 }
 
 extern "C" LKC_API int lkc_generator_workspace(LkcModel* m, int64_t t, int concurrent, int64_t* bytes, int64_t* unplanned) {
-  LKC_REQUIRE(m && bytes, "generator_workspace: null argument");
+  LKC_REQUIRE(m && bytes && !m->isDecoder, "generator_workspace: null argument or a decoder's handle");
   LKC_REQUIRE(t >= 1 && t < (int64_t(1) << 24), "generator_workspace: t out of range");
   return noThrow([&] {
     std::lock_guard<std::mutex> lock(m->mutex);
@@ -434,6 +546,7 @@ extern "C" LKC_API int lkc_generator_workspace(LkcModel* m, int64_t t, int concu
 
 extern "C" LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, void* stream) {
   LKC_REQUIRE(m && io && io->x && io->har && io->s && io->audio && io->workspace, "generator_forward: null argument");
+  LKC_REQUIRE(!m->isDecoder, "generator_forward: a decoder's handle");
   LKC_REQUIRE(io->t >= 1 && io->t < (int64_t(1) << 24), "generator_forward: t out of range");
   LKC_REQUIRE(io->x_pitch >= io->t && io->har_pitch >= 60 * io->t + 1 && (!io->post || io->post_pitch >= 60 * io->t + 1),
               "generator_forward: a row pitch is smaller than the row");
@@ -448,6 +561,40 @@ extern "C" LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, vo
     Exec e(isConcurrent(io->concurrent), *p, static_cast<char*>(io->workspace), S(stream),
            reinterpret_cast<const cudaStream_t*>(io->side), m->events);
     generator(e, m->w, *io);
+    if (e.rc != 0) e.joinForked();
+    io->launches = e.launches;
+    return e.rc;
+  });
+}
+
+extern "C" LKC_API int lkc_decoder_workspace(LkcModel* m, int64_t frames, int64_t* bytes) {
+  LKC_REQUIRE(m && bytes && m->isDecoder, "decoder_workspace: null argument or a generator's handle");
+  LKC_REQUIRE(frames >= 1 && frames < (int64_t(1) << 24), "decoder_workspace: frames out of range");
+  return noThrow([&] {
+    std::lock_guard<std::mutex> lock(m->mutex);
+    std::shared_ptr<const Plan> p;
+    if (int rc = m->plan(frames, 1, &p)) return rc;
+    *bytes = p->bytes;
+    return 0;
+  });
+}
+
+extern "C" LKC_API int lkc_decoder_forward(LkcModel* m, LkcDecoderIo* io, void* stream) {
+  LKC_REQUIRE(m && io && io->asr && io->f0 && io->n && io->s && io->out && io->workspace && io->side,
+              "decoder_forward: null argument");
+  LKC_REQUIRE(m->isDecoder, "decoder_forward: a generator's handle");
+  LKC_REQUIRE(io->frames >= 1 && io->frames < (int64_t(1) << 24), "decoder_forward: frames out of range");
+  LKC_REQUIRE(io->asr_pitch >= io->frames && io->out_pitch >= 2 * io->frames, "decoder_forward: a row pitch is smaller than the row");
+  LKC_REQUIRE((reinterpret_cast<uintptr_t>(io->workspace) & 255) == 0, "decoder_forward: the workspace must be 256-byte aligned");
+  return noThrow([&] {  // as lkc_generator_forward
+    std::lock_guard<std::mutex> lock(m->mutex);
+    std::shared_ptr<const Plan> p;
+    if (int rc = m->plan(io->frames, 1, &p)) return rc;
+    LKC_REQUIRE(io->workspace_bytes >= p->bytes, "decoder_forward: the workspace is too small (lkc_decoder_workspace)");
+    cudaStream_t side[kStreams - 1];
+    for (cudaStream_t& s : side) s = S(io->side);
+    Exec e(true, *p, static_cast<char*>(io->workspace), S(stream), side, m->events);
+    decoder(e, m->dec, *io);
     if (e.rc != 0) e.joinForked();
     io->launches = e.launches;
     return e.rc;

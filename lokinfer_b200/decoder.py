@@ -11,10 +11,14 @@ the padding contributes exact zeros and every conv of the stack runs on tcgen05.
 """
 from __future__ import annotations
 
+import ctypes
+import operator
+
 import numpy as np
 import torch
 
-from . import ops
+from . import _lib, ops
+from .generator import _Held, _Model
 from .synth import DECODER_BLOCKS
 
 SQRT1_2 = 0.7071067811865476
@@ -67,6 +71,97 @@ class Decoder:
         self.bank_b = torch.cat(bias).contiguous()
         self._ident = {c: torch.stack([torch.zeros(c), torch.ones(c), torch.zeros(c)]).to(self.device).contiguous()
                        for c in {512} | {_pad16(cin) for _, cin, _, _ in DECODER_BLOCKS}}
+        self._model = None  # (getters of its weights and states, _Model) of the whole-forward call
+        self._side = None
+
+    # The forward as one library call (lkc_decoder_forward). It computes what the composition in forward() computes with a
+    # third of its launches (block inputs are never concatenated, statistics come from the convs that wrote the rows), the
+    # shortcuts beside the convs, and no trip through Python per kernel: 48 op calls took 1.7 ms at any length. The
+    # composition remains for single kernels (ops.Profile with timing, ops.tracing), the CUDA-core path, convs without a
+    # tensor-core state and operands that the whole call would not check.
+
+    _NAMES = tuple(["decoder.asr_res.0.weight", "decoder.asr_res.0.bias"]
+                   + [f"decoder.{c}.{p}" for c in ("F0_conv", "N_conv") for p in ("weight", "bias")]
+                   + [f"{name}.{p}" for name, _, _, up in DECODER_BLOCKS
+                      for p in ["conv1.weight", "conv1.bias", "conv2.weight", "conv2.bias", "conv1x1.weight", "conv1x1.bias"]
+                      + (["pool.weight", "pool.bias"] if up else [])])
+    _STATES = tuple(["decoder.asr_res.0"]
+                    + [f"{name}.{c}" for name, _, _, _ in DECODER_BLOCKS for c in ("conv1", "conv2", "conv1x1")])
+    _GET_W, _GET_S = operator.itemgetter(*_NAMES), operator.itemgetter(*_STATES)
+
+    def _is(self, t, *shape):
+        return tuple(t.shape) == shape and t.dtype == torch.float32 and t.is_contiguous() and t.device == self.bank_b.device
+
+    def _whole_model(self):
+        """_Model of lkc_decoder_forward, or None when some conv has no tensor-core state."""
+        try:
+            ws, states = self._GET_W(self.w), self._GET_S(self.state)
+        except KeyError:
+            return None
+        pieces = (*ws, *states, self.bank_wt, self.bank_b, self.bank_off)
+        if self._model is not None and self._model.held.current(pieces):
+            return self._model
+        w, st, n = dict(zip(self._NAMES, ws)), dict(zip(self._STATES, states)), int(self.bank_b.shape[0])
+
+        def has(conv, co, ci, k):
+            s = st[conv]
+            return s is not None and s.shape == (co, ci, k) and self._is(w[conv + ".weight"], co, ci, k) and self._is(w[conv + ".bias"], co)
+
+        ok = (self._is(self.bank_wt, 128, n) and self._is(self.bank_b, n) and has("decoder.asr_res.0", 64, 512, 1)
+              and all(self._is(w[f"decoder.{c}.weight"], 1, 1, 3) and self._is(w[f"decoder.{c}.bias"], 1)
+                      for c in ("F0_conv", "N_conv")))
+        d = _lib.LkcDecoder()
+        for b, (name, cin, cout, up) in zip(d.block, DECODER_BLOCKS):
+            ci = _pad16(cin)
+            ok = (ok and has(name + ".conv1", cout, ci, 3) and has(name + ".conv2", cout, cout, 3)
+                  and has(name + ".conv1x1", cout, ci, 1)
+                  and (not up or (self._is(w[name + ".pool.weight"], ci, 1, 3) and self._is(w[name + ".pool.bias"], ci)))
+                  and not bool(up and self.gb_pad[name] != ci - cin))
+            (b.gb1, n1), (b.gb2, n2) = self.bank_off[name + ".norm1.fc"], self.bank_off[name + ".norm2.fc"]
+            if not (ok and n1 == 2 * ci and n2 == 2 * cout):
+                return None
+            b.cin, b.cout, b.up = ci, cout, int(up)
+            b.w1, b.b1 = w[name + ".conv1.weight"].data_ptr(), w[name + ".conv1.bias"].data_ptr()
+            b.w2, b.b2 = w[name + ".conv2.weight"].data_ptr(), w[name + ".conv2.bias"].data_ptr()
+            b.w1x1, b.b1x1 = w[name + ".conv1x1.weight"].data_ptr(), w[name + ".conv1x1.bias"].data_ptr()
+            if up:
+                b.pool_w, b.pool_b = w[name + ".pool.weight"].data_ptr(), w[name + ".pool.bias"].data_ptr()
+            b.state1, b.state2, b.state1x1 = (st[name + c].handle for c in (".conv1", ".conv2", ".conv1x1"))
+        d.bank_wt, d.bank_b, d.bank_n = self.bank_wt.data_ptr(), self.bank_b.data_ptr(), n
+        d.f0_w, d.f0_b = w["decoder.F0_conv.weight"].data_ptr(), w["decoder.F0_conv.bias"].data_ptr()
+        d.n_w, d.n_b = w["decoder.N_conv.weight"].data_ptr(), w["decoder.N_conv.bias"].data_ptr()
+        d.asr_w, d.asr_b = w["decoder.asr_res.0.weight"].data_ptr(), w["decoder.asr_res.0.bias"].data_ptr()
+        d.asr_state = st["decoder.asr_res.0"].handle
+        with torch.cuda.device(self.bank_b.device):
+            self._model = _Model(d, _Held(pieces), "lkc_decoder_create")
+            if self._side is None:
+                self._side = torch.cuda.Stream(self.bank_b.device)
+        return self._model
+
+    def _takes(self, asr, f0, n_curve, s):
+        """Whether the whole call may have these operands, whose addresses go to the kernels unchecked."""
+        dev = self.bank_b.device
+        return (all(isinstance(t, torch.Tensor) and t.device == dev and t.dtype == torch.float32 for t in (asr, f0, n_curve, s))
+                and asr.shape[1] >= 1 and asr.stride(1) == 1 and asr.stride(0) >= asr.shape[1]
+                and all(t.is_contiguous() for t in (f0, n_curve, s)) and s.numel() == 128)
+
+    def _forward_whole(self, model, asr, f0, n_curve, s):
+        dev, frames, lib = self.bank_b.device, int(asr.shape[1]), _lib.lib()
+        size = ctypes.c_int64(0)
+        with torch.cuda.device(dev):
+            out = ops.empty_rows(512, 2 * frames, dev)
+            rc = lib.lkc_decoder_workspace(model.handle, frames, ctypes.byref(size))
+            if rc == 0:
+                ws = torch.empty(size.value, dtype=torch.uint8, device=dev)
+                io = _lib.LkcDecoderIo()
+                io.asr, io.f0, io.n, io.s = asr.data_ptr(), f0.data_ptr(), n_curve.data_ptr(), s.data_ptr()
+                io.out, io.frames, io.asr_pitch, io.out_pitch = out.data_ptr(), frames, asr.stride(0), out.stride(0)
+                io.workspace, io.workspace_bytes, io.side = ws.data_ptr(), size.value, self._side.cuda_stream
+                rc = lib.lkc_decoder_forward(model.handle, ctypes.byref(io), ops._stream())
+        if rc != 0:
+            raise _lib.LkcError("decoder forward: " + _lib.last_error())
+        ops.count_launches(io.launches)
+        return out
 
     def _style(self, s):
         bank = ops.gemm_bias_f32_cuda(s.reshape(1, -1), self.bank_wt, self.bank_b).reshape(-1)
@@ -139,6 +234,10 @@ class Decoder:
         frames = int(asr.shape[1])
         ops.check(tuple(f0.shape) == (2 * frames,) and tuple(n_curve.shape) == (2 * frames,),
                   "f0 and n_curve must be f32[2F]")
+        if fused and not ops.op_by_op() and self._takes(asr, f0, n_curve, s):
+            model = self._whole_model()
+            if model is not None:
+                return self._forward_whole(model, asr, f0, n_curve, s)
         gb = self._style(s)
         f0d = ops.conv1d_f32_cuda(f0.reshape(1, -1), w["decoder.F0_conv.weight"], w["decoder.F0_conv.bias"], stride=2,
                                   padding=1)

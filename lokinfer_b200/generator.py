@@ -57,11 +57,11 @@ class _Held:
 
 
 class _Model:
-    """Handle of lkc_generator_create; a call in flight in another thread keeps the one it was given."""
+    """Handle of lkc_generator_create (or lkc_decoder_create); a call in flight in another thread keeps the one it was given."""
 
-    def __init__(self, struct, held):
+    def __init__(self, struct, held, create="lkc_generator_create"):
         self.held = held
-        self.handle = _lib.lib().lkc_generator_create(ctypes.byref(struct))
+        self.handle = getattr(_lib.lib(), create)(ctypes.byref(struct))
         if not self.handle:
             raise _lib.LkcError(_lib.last_error())
 

@@ -78,3 +78,95 @@ def test_decoder_feeds_generator(cuda):
     ref = O.generator(gsd, rx, O.T(gin["har"]), O.T(inp["s"])).numpy()
     assert audio.shape == ref.shape == (600 * frames,)
     assert np.abs(audio - ref).max() <= 1e-4
+
+
+@pytest.fixture(scope="module")
+def dec(cuda):
+    from lokinfer_b200 import Decoder
+    return Decoder(synth.decoder_weights(0), cuda)
+
+
+def _composed(dec, *a):
+    """The op-by-op form: a result allocator of one's own makes the whole call stand back."""
+    from lokinfer_b200 import ops
+    with ops.use_allocator(lambda shape, device: torch.empty(shape, dtype=torch.float32, device=device)):
+        return dec.forward(*a)
+
+
+def _args(cuda, frames, seed):
+    inp = synth.decoder_inputs(frames, seed)
+    return dev(cuda, inp["asr"], inp["f0"], inp["n"], inp["s"])
+
+
+@pytest.mark.parametrize("frames", [1, 2, 61, 64, 127, 129, 300, 1040])
+def test_whole_decoder_agrees_with_the_composition(cuda, dec, frames):
+    """The whole call differs from the op-by-op form in who computes the statistics and in how partial sums are split, not
+    beyond rounding. One column: the variance is zero, what is left of it is rounding times 1 / sqrt(eps) (316), twice per
+    block."""
+    from lokinfer_b200 import ops
+    a = _args(cuda, frames, 30 + frames)
+    got, want = dec.forward(*a), _composed(dec, *a)
+    assert got.shape == want.shape == (512, 2 * frames) and got.is_contiguous()
+    assert rel_l2(got.cpu().numpy(), want.cpu().numpy()) <= (10 if frames > 2 else 3160) * REL_L2
+    assert torch.equal(got, dec.forward(*a)) and ops.conv_tc_status() == 0
+
+
+def test_whole_decoder_takes_row_pitches_and_leaves_the_rest(cuda, dec):
+    """A view of wider rows, a stream of the caller's, replaced weights; operands that the call cannot take by their
+    addresses go op by op or are refused as before."""
+    from lokinfer_b200 import Decoder, ops
+    a = _args(cuda, 50, 7)
+    want = dec.forward(*a)
+    wide = torch.full((512, 56), float("nan"), device=cuda)
+    wide[:, :50] = a[0]
+    with ops.padded_rows():
+        got = dec.forward(wide[:, :50], *a[1:])
+    assert torch.equal(got, want)
+    with torch.cuda.stream(torch.cuda.Stream(device=cuda)):
+        torch.cuda.current_stream().wait_stream(torch.cuda.default_stream(cuda))
+        got = dec.forward(*a)
+        torch.cuda.current_stream().synchronize()
+    assert torch.equal(got, want)
+    for bad in ([a[0][:, :49], *a[1:]], [a[0].cpu(), *a[1:]], [a[0].double(), *a[1:]], [a[0], a[1][:-1], a[2], a[3]]):
+        with pytest.raises((ops.OpError, RuntimeError)):
+            dec.forward(*bad)
+    other = Decoder(synth.decoder_weights(0), cuda)
+    other.forward(*a)
+    other.w["decoder.encode.conv2.bias"] = other.w["decoder.encode.conv2.bias"] + 1.0
+    got, want2 = other.forward(*a), _composed(other, *a)
+    assert rel_l2(got.cpu().numpy(), want2.cpu().numpy()) <= 10 * REL_L2 and rel_l2(got.cpu().numpy(), want.cpu().numpy()) > 1e-3
+
+
+def test_one_decoder_in_several_threads(cuda, dec):
+    import threading
+    jobs = [_args(cuda, f, f) for f in (5, 61, 200)]
+    want = [dec.forward(*j).clone() for j in jobs]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream(device=cuda)):
+            for _ in range(10):
+                if not torch.equal(dec.forward(*jobs[i]), want[i]):
+                    wrong.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
+def test_whole_decoder_in_a_graph(cuda, dec):
+    a = _args(cuda, 61, 3)
+    want = dec.forward(*a).clone()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        out = dec.forward(*a)
+    out.zero_()
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)

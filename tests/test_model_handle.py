@@ -94,3 +94,44 @@ def test_weights_that_do_not_fit_are_refused(change, message):
     w = Weights()
     change(w)
     assert message in (w.create() or "")
+
+
+def test_decoder_weights_are_checked():
+    """lkc_decoder_create: states of the five blocks' shapes, AdaIN parameters inside the bank."""
+    lib, states = _lib.lib(), []
+
+    def conv(co, ci, k):
+        states.append(lib.lkc_conv1d_state_create_as(ADDR, co, ci, k, 0))
+        return states[-1]
+
+    def create(change=lambda d: None):
+        d = _lib.LkcDecoder()
+        d.bank_wt = d.bank_b = d.f0_w = d.f0_b = d.n_w = d.n_b = d.asr_w = d.asr_b = ADDR
+        d.bank_n, d.asr_state = BANK_N, conv(64, 512, 1)
+        for i, b in enumerate(d.block):
+            b.cin, b.cout, b.up = (528, 1104)[i > 0], 512 if i == 4 else 1024, int(i == 4)
+            b.w1 = b.b1 = b.w2 = b.b2 = b.w1x1 = b.b1x1 = b.pool_w = b.pool_b = ADDR
+            b.state1, b.state2, b.state1x1 = conv(b.cout, b.cin, 3), conv(b.cout, b.cout, 3), conv(b.cout, b.cin, 1)
+            b.gb1, b.gb2 = BANK_N - 2 * b.cin, BANK_N - 2 * b.cout
+        change(d)
+        handle = lib.lkc_decoder_create(ctypes.byref(d))
+        if handle:
+            lib.lkc_model_destroy(handle)
+            return None
+        return None if "cudaEventCreate" in _lib.last_error() else _lib.last_error()
+
+    def setter(path, value):
+        def change(d):
+            *head, last = path
+            for p in head:
+                d = d[p] if isinstance(p, int) else getattr(d, p)
+            setattr(d, last, value)
+        return change
+
+    assert create() is None
+    for path, value in ((("asr_state",), None), (("bank_n",), 100), (("block", 0, "cin"), 1104), (("block", 4, "up"), 0),
+                        (("block", 2, "w1x1"), None), (("block", 4, "pool_w"), None), (("block", 1, "gb1"), BANK_N - 2207),
+                        (("block", 3, "gb2"), -1), (("block", 1, "state2"), states[0])):
+        assert "decoder_create" in (create(setter(path, value)) or ""), path
+    for st in states:
+        lib.lkc_conv1d_state_destroy(st)
