@@ -244,8 +244,9 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
   har.p = const_cast<float*>(FP(io.har)), har.pitch = io.har_pitch;
 
   Buf bank = e.alloc(0, m.bank_n);
-  e.launch(0, {bank}, [&](cudaStream_t st) { return gemmBias(FP(io.s), FP(m.bank_wt), FP(m.bank_b), bank.p, 1, 128, m.bank_n, st); });
-  e.join(1, 0), e.join(2, 0);
+  e.join(1, 0), e.join(2, 0), e.join(3, 0);
+  // the style bank beside the first convs: the noise branches need it for their first AdaIN
+  e.launch(3, {bank}, [&](cudaStream_t st) { return gemmBias(FP(io.s), FP(m.bank_wt), FP(m.bank_b), bank.p, 1, 128, m.bank_n, st); });
 
   auto upsample = [&](int i, Buf in, int64_t lin, Buf res) {
     Buf u = e.rows(0, kCh[i], len[i]);
@@ -288,6 +289,7 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
     Buf xs = e.rows(s, kCh[i], len[i]), xst = statsBuf(e, s, kCh[i], len[i]);
     conv(e, s, Act::None, y, ly, n.rows, kCh[i], n.taps, 1, 0, n.w, n.b, none, nullptr, 0.f, n.state, none, xs, xst,
          kNoiseSms[i]);
+    e.join(s, 3);
     if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], AddUpsampled{e, u0, kCh[0], len[0]}, kNoiseSms[i]);
     else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], PlainResidual{}, kNoiseSms[i]);
   }
