@@ -157,6 +157,12 @@ int convFused(const ConvFusedParams& p, cudaStream_t s) {
   return convSimt(p, 1, s);
 }
 
+int convStatCols(const ConvFusedParams& p) {
+  if (gConvPath == 1 || p.state == nullptr) return 128;
+  const bool f16 = static_cast<const ConvState*>(p.state)->f16;
+  return convTcEligible(p, f16) ? convTcStatCols(p, f16) : 128;
+}
+
 bool convFoldsAffine(const ConvFusedParams& p) {
   if (gConvPath == 1 || p.state == nullptr) return false;
   const bool f16 = static_cast<const ConvState*>(p.state)->f16;

@@ -154,8 +154,10 @@ struct TcArgs {
   int padLeft;       // ConvTranspose: 1 = one-sample left reflect pad
   float slope, outScale;
   int delta;       // columns between the 16-byte boundary a tile's window is loaded from and its first column (0: 4-byte route)
-  int rows;        // staged time rows per buffer = tile columns + (k-1)*dilation + delta
-  int ext;         // raw staging: [16][tile columns], then [16][ext] with the rows - tile columns beyond them (two TMA boxes)
+  int tileCols;    // time columns per tile: NTS split, else 32 .. NT in steps of 32 (see tileColsFor)
+  int mainRows;    // staged rows that every lane has a slot for: the window up to NT (split: NTS) rows, a multiple of 64
+  int rows;        // staged time rows per buffer: at least tileCols + (k-1)*dilation + delta and mainRows
+  int ext;         // raw staging: [16][NT or NTS], then [16][ext] with the rows beyond them (two TMA boxes)
   int wStages;     // weight ring depth (slots)
   int nb;          // activation buffers
   int wG;          // taps per weight slot: the k taps of a chunk go in ceil(k / wG) groups of near-equal size
@@ -164,6 +166,7 @@ struct TcArgs {
   int tmaOut;      // 1: out (and residual) rows are 16-byte aligned, boxes go by TMA
   int numTTiles, numCoBlk;
   int split;       // 0 = a persistent CTA per SM over 256-column tiles; else the CTAs that share one 128-column tile
+  int fine;        // stats: a (mean, M2) pair per 32 columns, not per 128
   int early;       // the launch may overlap the end of the one before it (programmatic dependent launch)
   int* status;
   long long* prof;  // null, or 16 cycle counters summed over CTAs (see convTcProfile)
@@ -275,11 +278,6 @@ template <int N>
 __device__ __forceinline__ void cpAsyncWait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-
-// Programmatic dependent launch. wait: until every kernel this launch depends on has finished and its writes are visible.
-// launch: the kernel that follows may start (it waits in the same way before it touches what this one writes or reads).
-__device__ __forceinline__ void dependenciesWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void dependentsLaunch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __device__ __forceinline__ void tmemAlloc(uint32_t* slot, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(slot)), "r"(cols)
@@ -636,7 +634,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // Dhi buffers: a 128-column tile leaves room for two, so that the hi MMAs of a drain group need not wait for the drain
   // of the one before (the lo MMAs that cover it are shorter here)
   constexpr int HB = SPLIT ? 2 : 1;
-  constexpr uint32_t kIdesc = idescOf(F16, NTK);
+  const uint32_t kIdesc = SPLIT ? idescOf(F16, NTS) : idescOf(F16, 0) | (uint32_t(a.tileCols >> 3) << 17);
   const int NB = a.nb;
   extern __shared__ __align__(1024) unsigned char smemRaw[];
   const int rows = a.rows, ext = a.ext;
@@ -670,6 +668,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     if (threadIdx.x == 0) atomicOr(a.status, (6 << 8) | 1);
     return;
   }
+  const int W = SPLIT ? NTS : a.tileCols;
   const int numTiles = a.numTTiles * a.numCoBlk;
   // tiles of this CTA: tile0, tile0 + tileStep, ...; its chunks of a tile: cBegin .. cBegin + nChunks16
   const int rank = SPLIT ? int(clusterRank()) : 0;
@@ -735,7 +734,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // ------------------------------------------------------------------ accumulate + epilogue
     regInc<EPI_REGS>();
     dependenciesWait();
-    const int q = warp & 3, g = warp >> 2;  // TMEM lane quarter, 128-column half of the tile
+    const int q = warp & 3, g = warp >> 2;  // TMEM lane quarter, half of the tile
+    // 32-column batches of this warp (of 256 columns: 4) and its first column
+    const int nb0 = SPLIT ? EC / 32 : ((W >> 5) + 1) >> 1, nbat = SPLIT ? EC / 32 : (g ? (W >> 5) - nb0 : nb0), gcol = g * nb0 * 32;
     float* const tile = sStage + warp * STAGE_FLOATS;                                  // unaligned route: [32][33]
     unsigned char* const box = smemRaw + warp * BOX_BYTES;                             // aligned route: swizzled 32 x 32
     unsigned char* const boxRow = box + lane * 128;                                    // this lane's row of the box
@@ -756,9 +757,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     for (int t = tile0; t < numTiles && !dead; t += tileStep, ++tileIt) {
       const int tt = t / a.numCoBlk, cb = t - tt * a.numCoBlk;
       const long long tPre = kProf ? clock64() : 0;
-      const int64_t tChunk = int64_t(tt) * NTK + g * EC;  // first output column of this warp's 128-column chunk
+      const int64_t tChunk = int64_t(tt) * W + gcol;  // first output column of this warp
       const int64_t nValid64 = a.lo - tChunk;
-      const int nValid = nValid64 <= 0 ? 0 : (nValid64 < 128 ? int(nValid64) : 128);
+      const int nValid = nValid64 <= 0 ? 0 : (nValid64 < nbat * 32 ? int(nValid64) : nbat * 32);
       // conv: the warp's rows are 32 consecutive output channels. ConvTranspose: rows are (channel, phase) pairs,
       // CQ channels x TS phases per warp (lane = cl * TS + r), the last 32 - CQ * TS rows are zero padding.
       constexpr int CQ = TS ? 32 / TS : 32, ROWS = TS ? CQ * TS : 32;
@@ -872,8 +873,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (SPLIT && groupIt + 1 == uint32_t(nGroups)) clusterArrive(), arrived = true;
 #pragma unroll
         for (int b = 0; b < EC / 16; ++b) {
+          if (!SPLIT && b >= 2 * nbat) break;
           uint32_t v[16];
-          tmemLoad16Async(tmemHi + hb * NTK + laneBase + g * EC + b * 16, v);
+          tmemLoad16Async(tmemHi + hb * NTK + laneBase + gcol + b * 16, v);
           tmemWaitLoads();
 #pragma unroll
           for (int j = 0; j < 16; j += 2) {  // packed f32x2 adds: half the instructions of the accumulate loop
@@ -896,12 +898,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       // One copy of the fetch and of the drain in the code (this kernel is far larger than the instruction cache,
       // and straight-line code that runs once per tile is fetched at a fraction of the issue rate); only the add
       // needs static register indices.
-      const int nPre = hasRes && nGroups < 4 ? 4 - nGroups : 0;
+      const int nPre = hasRes && nGroups < nbat ? nbat - nGroups : 0;
       const int nSteps = nPre + nGroups, preAt = nGroups == 1 ? 0 : 1;  // first step without a drain
       int rb = 0;  // next residual batch
 #pragma unroll 1
       for (int c = 0; c < nSteps && !dead; ++c) {
-        const bool doRes = hasRes && rb < 4;
+        const bool doRes = hasRes && rb < nbat;
         if (doRes) fetchResidual(rb);
         if (c == nSteps - 1) {
           // Last step of the tile (always a drain): Dlo is complete before the last hi MMAs are, so it is folded in
@@ -914,9 +916,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           tcFenceAfter();
 #pragma unroll
           for (int b = 0; b < EC / 32; ++b) {  // two 16-column loads in flight per wait
+            if (!SPLIT && b >= nbat) break;
             uint32_t va[16], vb[16];
-            tmemLoad16Async(tmemLo + laneBase + g * EC + b * 32, va);
-            tmemLoad16Async(tmemLo + laneBase + g * EC + b * 32 + 16, vb);
+            tmemLoad16Async(tmemLo + laneBase + gcol + b * 32, va);
+            tmemLoad16Async(tmemLo + laneBase + gcol + b * 32 + 16, vb);
             tmemWaitLoads();
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
@@ -943,7 +946,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       if (dead) break;
       const long long tFin = kProf ? clock64() : 0;
       if constexpr (SPLIT) {
-        float* const row = sStage + (q * 32 + lane) * PART_PITCH + g * EC;
+        float* const row = sStage + (q * 32 + lane) * PART_PITCH + gcol;
 #pragma unroll
         for (int j = 0; j < EC; j += 4) *reinterpret_cast<float4*>(row + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
         fenceProxyAsync();  // generic-proxy stores -> visible to the bulk copies
@@ -1048,7 +1051,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             __syncwarp();
           }
         }
-        if (a.stats && nValid > 0 && (!PARTIAL || co < a.co)) {
+        if (a.stats && a.fine && (!PARTIAL || co < a.co)) {  // a pair per 32 columns
+          float2* const st = reinterpret_cast<float2*>(a.stats) + int64_t(co) * a.nchunks + tChunk / 32;
+#pragma unroll
+          for (int b = 0; b < 4; ++b)
+            if (b * 32 < nValid) st[b] = make_float2(pMean[b], pM2[b]);
+        } else if (a.stats && nValid > 0 && (!PARTIAL || co < a.co)) {
           // exact combine of the four 32-column partials: mean = sum n_b m_b / n, M2 = sum M2_b + sum n_b (m_b - mean)^2
           float sum = 0.f;
 #pragma unroll
@@ -1078,6 +1086,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
+          if (b >= nbat) break;
           const int64_t u0 = (tChunk + b * 32) * TS;
           if (lane < ROWS) {
 #pragma unroll
@@ -1130,7 +1139,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // A warp stages the rows of its half, SLOTS per lane, with addresses that are immediates. The rows beyond the tile's
     // columns (at most 53) take one more slot for up to 32 of them: the first 32 go to the warps of half `raw buffer`, so
     // that the halves take turns, the rest to the other half.
-    constexpr int SLOTS = NTK / 64;
+    const int halfRows = a.mainRows / 2, slots = a.mainRows / 64;
     const bool tmaIn = a.tmaIn != 0;
     // per-channel parameters, once: sPar = [-mean | a | b | inv] with a = scale, b = beta (x alpha for Snake), inv = 1/alpha
     // Split form with statsIn: each CTA folds the chunk statistics of its own channels into mean / scale / beta, with the
@@ -1195,9 +1204,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           for (int j = 0; j < 4; ++j) cpAsync4(dst + j * pitch, src + j * a.xPitch);
         }
       };
-      const int r0 = hf * (NTK / 2) + lane;
-#pragma unroll
-      for (int sl = 0; sl < SLOTS; ++sl) copy(r0 + sl * 32, base + cg * 4 * NTK + r0 + sl * 32, NTK);
+      const int r0 = hf * halfRows + lane;
+#pragma unroll 1
+      for (int sl = 0; sl < slots; ++sl) copy(r0 + sl * 32, base + cg * 4 * NTK + r0 + sl * 32, NTK);
       const int r = extRow(rb);
       if (r < rows) copy(r, base + KC * NTK + cg * 4 * ext + r - NTK, ext);
     };
@@ -1206,7 +1215,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     uint32_t buf = 0, bufPar = 1, rawBuf = 0, rawPar = 0;  // activation buffer + parity of its last release; raw buffer + parity of its fill
     long long wB = 0, wCp = 0, cTr = 0;
     const long long tStart = kProf ? clock64() : 0;
-    int64_t pos0 = int64_t(t / a.numCoBlk) * NTK - a.padding;  // input position of row 0 of the current tile's window
+    int64_t pos0 = int64_t(t / a.numCoBlk) * W - a.padding;  // input position of row 0 of the current tile's window
     if (!tmaIn) {
       if (t < numTiles) issueCopies(pos0, c, 0);
       cpAsyncCommit();
@@ -1216,7 +1225,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       int64_t posN = pos0;
       if (cn == nChunks16) {
         cn = 0, tn = t + tileStep;
-        posN = int64_t(tn / a.numCoBlk) * NTK - a.padding;
+        posN = int64_t(tn / a.numCoBlk) * W - a.padding;
       }
       if (tmaIn) {
         if (!waitT(&rawFull[rawBuf], rawPar, wCp, SLEEP_PRO_NS)) {
@@ -1283,16 +1292,21 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           *reinterpret_cast<uint2*>(lo + r * 4) = lw;
         }
       };
-      const int r0 = hf * (NTK / 2) + lane, rx = extRow(rawBuf);
+      const int r0 = hf * halfRows + lane, rx = extRow(rawBuf);
       const float* const sp0 = raw + cg * 4 * NTK + r0;
       const float* const spx = raw + KC * NTK + cg * 4 * ext + rx - NTK;
       if (okLo == 0 && okHi == rows) {  // all but the tiles at the ends of the valid range
+        auto all = [&](auto n) {
 #pragma unroll
-        for (int sl = 0; sl < SLOTS; ++sl) stage(std::false_type{}, r0 + sl * 32, sp0 + sl * 32, NTK);
+          for (int sl = 0; sl < decltype(n)::value; ++sl) stage(std::false_type{}, r0 + sl * 32, sp0 + sl * 32, NTK);
+        };
+        if (SPLIT || slots == 2) all(std::integral_constant<int, 2>{});
+        else if (slots == 4) all(std::integral_constant<int, 4>{});
+        else all(std::integral_constant<int, 3>{});
         if (rx < rows) stage(std::false_type{}, rx, spx, ext);
       } else {
 #pragma unroll 2
-        for (int sl = 0; sl < SLOTS; ++sl) stage(std::true_type{}, r0 + sl * 32, sp0 + sl * 32, NTK);
+        for (int sl = 0; sl < slots; ++sl) stage(std::true_type{}, r0 + sl * 32, sp0 + sl * 32, NTK);
         if (rx < rows) stage(std::true_type{}, rx, spx, ext);
       }
       if (F16 && big > 65504.f) atomicOr(a.status, kStatusF16Range);
@@ -1361,7 +1375,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         bool dead = false;
         const uint32_t bytes = uint32_t(rawBufFloats) * 4;
         for (int t = tile0; t < numTiles && !dead; t += tileStep) {
-          const int x0 = (t / a.numCoBlk) * NTK - a.padding - a.delta;
+          const int x0 = (t / a.numCoBlk) * W - a.padding - a.delta;
           for (int c = 0; c < nChunks16; ++c, ++issued) {
             if (!waitT(&rawEmpty[rb], ph, wR, SLEEP_W_NS)) {
               giveUp(5, 1);
@@ -1610,7 +1624,7 @@ __global__ void convtTcPackKernel(const float* __restrict__ w, void* __restrict_
 }  // namespace
 
 // Row floats of the second raw-input box (its 16-byte granularity): what a window of `rows` columns has beyond `cols`.
-static int rawExt(int rows, int cols) { return (rows - cols + 3) & ~3; }
+static int rawExt(int rows, int cols) { return rows <= cols ? 0 : (rows - cols + 3) & ~3; }
 
 // Dynamic shared memory of one CTA and the weight ring it leaves room for: the largest taps-per-slot (<= TAP_GROUP)
 // that still gives PREF_W_STAGES slots, else the deepest ring. Returns 0 when even single-tap slots do not fit.
@@ -1871,19 +1885,41 @@ int convTcSplitRule(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* 
 }
 
 // Launch geometry and tensor maps shared by the conv and ConvTranspose entry points.
-static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool canSplit, bool boxesOk, int smPercent, int* grid, size_t* smem) {
+// Columns per tile of the persistent form, for a launch that may spread over smPercent of the device's SMs.
+// Alone, the launch's time is the rounds of tiles that its busiest SM runs times a tile's time, which is about that of its
+// columns plus 48 more: a narrower tile pays where it takes fewer SM-columns in whole rounds.
+// Beside other launches the columns all together count, of which wide tiles cost fewer, unless there are few: then the
+// narrowest tiles that find room in one round of the launch's share shorten its chain.
+// Widths other than NT leave chunk statistics per 32 columns, which the caller has to take (fineOk).
+static int tileColsFor(bool fineOk, int64_t lo, int64_t coBlocks, int sms, int smPercent) {
+  int best = NT;
+  if (!fineOk) return best;
+  int64_t cost = ceilDiv(ceilDiv(lo, NT) * coBlocks, sms) * (NT + 48);
+  for (int w = NT - 32; w >= 160; w -= 32) {
+    const int64_t tiles = ceilDiv(lo, w) * coBlocks, c = ceilDiv(tiles, sms) * (w + 48);
+    if (smPercent < 100 ? tiles <= int64_t(sms) * smPercent / 100 : c < cost) best = w, cost = c;
+  }
+  return best;
+}
+
+static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool canSplit, bool boxesOk, bool fineOk, int smPercent, int* grid, size_t* smem) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
   a.split = splitFor(canSplit, a.ci, a.lo, a.numCoBlk, d->smCount * smPercent / 100, d->clusters);
   LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
-  const int nt = a.split ? NTS : NT;
-  a.numTTiles = int(ceilDiv(a.lo, nt));
+  const int nt = a.split ? NTS : NT;  // staged columns of the first box
+  a.tileCols = a.split ? NTS : tileColsFor(fineOk, a.lo, a.numCoBlk, d->smCount, smPercent);
+  a.fine = a.tileCols != NT && !a.split;
+  if (a.stats && a.fine) a.nchunks = ceilDiv(a.lo, 32);
+  a.numTTiles = int(ceilDiv(a.lo, a.tileCols));
   // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
   // argument: it stays zero-filled and is never dereferenced.
   std::memset(&m, 0, sizeof m);
   a.tmaIn = makeMap(&m.x, a.x, a.ci, a.l, a.xPitch, nt, KC, false) ? 1 : 0;
   a.delta = a.tmaIn ? -a.padding & 3 : 0;  // tiles start on multiples of 4 columns
-  a.rows = nt + (a.k - 1) * a.dilation + a.delta;
+  const int need = a.tileCols + (a.k - 1) * a.dilation + a.delta;
+  a.mainRows = std::min(nt, (need + 63) & ~63);
+  a.rows = std::max(need, a.mainRows);
   a.ext = rawExt(a.rows, nt);
   if (a.tmaIn && a.ext)
     LKC_REQUIRE(makeMap(&m.ext, a.x, a.ci, a.l, a.xPitch, a.ext, KC, false), "conv (tensor-core): tensor map of the input");
@@ -1917,6 +1953,12 @@ bool convTcSplits(const ConvFusedParams& p, bool f16) {
          splitFor(splits(f16, p.k, p.act), int(p.ci), p.lo, ceilDiv(p.co, MT), d->smCount * p.smPercent / 100, d->clusters) != 0;
 }
 
+int convTcStatCols(const ConvFusedParams& p, bool f16) {
+  const DeviceInfo* d = nullptr;
+  if (!p.fineStats || deviceInfo(&d) != 0 || convTcSplits(p, f16)) return 128;
+  return tileColsFor(true, p.lo, ceilDiv(p.co, MT), d->smCount, p.smPercent) == NT ? 128 : 32;
+}
+
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {
   TcArgs a;
   TcMaps m;
@@ -1936,7 +1978,7 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
   a.numCoBlk = int(coBlk);
   int grid = 0;
   size_t smem = 0;
-  if (int rc = finishArgs(a, m, f16, splits(f16, p.k, p.act), true, p.smPercent, &grid, &smem)) return rc;
+  if (int rc = finishArgs(a, m, f16, splits(f16, p.k, p.act), true, p.fineStats || !p.stats, p.smPercent, &grid, &smem)) return rc;
   switch (p.act) {
     case Act::None: return launchTc<0>(a, m, f16, grid, smem, s);
     case Act::Snake: return launchTc<1>(a, m, f16, grid, smem, s);
@@ -1991,7 +2033,7 @@ int convtTc(const ConvtParams& p, const float* wp, bool f16, cudaStream_t s) {
   a.numCoBlk = int(coBlk);
   int grid = 0;
   size_t smem = 0;
-  if (int rc = finishArgs(a, m, f16, f16, false, p.smPercent, &grid, &smem)) return rc;
+  if (int rc = finishArgs(a, m, f16, f16, false, true, p.smPercent, &grid, &smem)) return rc;
   if (p.stride == 6) return launchTc2<2, false, 6>(a, m, f16, grid, smem, s);
   return launchTc2<2, false, 10>(a, m, f16, grid, smem, s);
 }

@@ -153,13 +153,15 @@ constexpr int kAffineThreads = 128;
 __global__ void __launch_bounds__(kAffineThreads) adainAffineKernel(const float* __restrict__ stats,
                                                                     const float* __restrict__ gb,
                                                                     float* __restrict__ affine, int64_t c, int64_t l,
-                                                                    int64_t nchunks, float eps) {
+                                                                    int64_t nchunks, int statCols, float eps, int alone) {
+  if (alone) dependentsLaunch();
+  dependenciesWait();
   __shared__ double red[kAffineThreads / 32];
   __shared__ double bc;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t ch = blockIdx.x;
   const float2* sc = reinterpret_cast<const float2*>(stats) + ch * nchunks;  // (mean, M2) pairs, 8-byte aligned
-  const double nT = static_cast<double>(kStatChunk), nLast = static_cast<double>(l - (nchunks - 1) * kStatChunk);
+  const double nT = static_cast<double>(statCols), nLast = static_cast<double>(l - (nchunks - 1) * statCols);
   constexpr int R = 8;
   float2 v[R];
 #pragma unroll
@@ -247,8 +249,22 @@ int channelStats(const float* x, float* stats, int64_t c, int64_t l, int64_t pit
   return launched("channel_stats_f32_cuda");
 }
 
-int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s) {
-  adainAffineKernel<<<static_cast<unsigned>(c), kAffineThreads, 0, s>>>(stats, gb, affine, c, l, statChunks(l), eps);
+int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s,
+                int statCols, bool alone) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(unsigned(c)), cfg.blockDim = dim3(kAffineThreads), cfg.stream = s, cfg.attrs = attr;
+  if (alone) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 1;
+  }
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, adainAffineKernel, stats, gb, affine, c, l, ceilDiv(l, statCols), statCols, eps,
+                                           alone ? 1 : 0);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return failCuda("adain_affine_f32_cuda", e);
+  }
   return launched("adain_affine_f32_cuda");
 }
 

@@ -42,6 +42,13 @@ int noThrow(Fn body) {
   }
 }
 
+#ifdef __CUDACC__
+// Programmatic dependent launch. wait: until every kernel this launch depends on has finished and its writes are visible.
+// launch: the kernel that follows may start (it waits in the same way before it touches what this one writes or reads).
+__device__ __forceinline__ void dependenciesWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependentsLaunch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 #define LKC_REQUIRE(cond, msg) \
   do {                         \
     if (!(cond)) return ::lkc::fail(msg); \
@@ -81,12 +88,15 @@ struct ConvFusedParams {
   // AdaIN; the conv computes the affine itself.
   const float *statsIn = nullptr, *gb = nullptr;
   float eps = 0.f;
+  bool fineStats = false;  // stats may come as one pair per 32 columns (convStatCols says which)
 };
 
 // One fused conv, routed to the tensor-core kernel when the shape qualifies, else to the CUDA-core kernel (api.cu).
 int convFused(const ConvFusedParams& p, cudaStream_t s);
 // Whether that route takes p.statsIn / p.gb instead of p.affine (the tensor-core kernel's split form).
 bool convFoldsAffine(const ConvFusedParams& p);
+// Columns per (mean, M2) pair of p.stats on that route: 128, or 32 where p.fineStats lets the tensor-core kernel choose.
+int convStatCols(const ConvFusedParams& p);
 // CUDA-core implicit-GEMM conv for any shape (conv_simt.cu). stride > 1 only for the plain conv1d.
 int convSimt(const ConvFusedParams& p, int64_t stride, cudaStream_t s);
 
@@ -118,6 +128,7 @@ bool convPathForcedSimt();
 bool convPackF16();  // operand format new packs are made in (lkc_set_conv_path)
 bool convTcEligible(const ConvFusedParams& p, bool f16);
 bool convTcSplits(const ConvFusedParams& p, bool f16);  // of an eligible conv
+int convTcStatCols(const ConvFusedParams& p, bool f16);  // of an eligible conv
 int convTcSplitRule(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* clusters);
 int64_t convTcPackFloats(int64_t co, int64_t ci, int64_t k, bool f16);
 int convTcPack(const float* w, float* wp, int64_t co, int64_t ci, int64_t k, bool f16, cudaStream_t s);
@@ -130,7 +141,8 @@ int convTcProfile(int enable, long long* out16);
 // Launchers behind the C-ABI entry points of the same names (elementwise.cu, istft.cu, conv_tc.cu); arguments checked by
 // the caller. Row pitches in floats.
 int channelStats(const float* x, float* stats, int64_t c, int64_t l, int64_t pitch, int64_t statsStride, cudaStream_t s);
-int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s);
+int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s, int statCols = 128,
+                bool alone = false);  // alone: nothing runs beside it, so it and what follows it may start early
 int gemmBias(const float* x, const float* wt, const float* b, float* out, int64_t m, int64_t k, int64_t n, cudaStream_t s);
 int addRows(const float* a, const float* b, float* out, int64_t n, cudaStream_t s);
 int add3Scale(const float* a, const float* b, const float* c, float* out, int64_t n, float scale, cudaStream_t s);

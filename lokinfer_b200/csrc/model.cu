@@ -169,25 +169,27 @@ void conv(Exec& e, int s, Act act, Buf x, int64_t l, int64_t ci, int64_t co, int
 
 // AdaIN -> Snake -> conv [+ residual] of a resblock, c -> c channels of the same length. gb = this AdaIN's (gamma | beta)
 // inside the style bank. The affine is a launch of its own unless the conv's route folds the statistics itself; the
-// plan reserves it either way, as the route may change between two calls (set_conv_path).
-void adainConv(Exec& e, int s, Buf x, Buf stats, int64_t l, int64_t c, int64_t k, int64_t d, const LkcResblock& w, int i,
-               Buf bank, Buf residual, Buf out, Buf outStats, int smPercent) {
+// plan reserves it either way, as the route may change between two calls (set_conv_path). statCols: columns per pair of
+// `stats`; the return value is that of outStats, 128 unless `fine` allows others.
+int adainConv(Exec& e, int s, Buf x, Buf stats, int statCols, int64_t l, int64_t c, int64_t k, int64_t d, const LkcResblock& w,
+              int i, Buf bank, Buf residual, Buf out, Buf outStats, bool fine, int smPercent) {
   const Buf af = e.alloc(s, 3 * c);
   ConvFusedParams p;
   p.x = x.p, p.w = FP(w.w[i]), p.bias = FP(w.b[i]), p.affine = af.p, p.alpha = FP(w.alpha[i]), p.residual = residual.p;
   p.out = out.p, p.stats = outStats.p;
   p.ci = c, p.l = l, p.co = c, p.k = k, p.dilation = d, p.padding = d * (k - 1) / 2, p.lo = l;
   p.xPitch = x.pitch, p.resPitch = residual.pitch, p.outPitch = out.pitch;
-  p.act = Act::Snake, p.state = w.state[i], p.smPercent = smPercent;
+  p.act = Act::Snake, p.state = w.state[i], p.smPercent = smPercent, p.fineStats = fine;
   const float* gb = bank.p + w.gb[i];
-  if (e.running() && convFoldsAffine(p))
+  if (e.running() && statCols == 128 && convFoldsAffine(p))
     p.statsIn = stats.p, p.gb = gb, p.eps = kEps;
   else
-    e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, c, l, kEps, st); });
+    e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, c, l, kEps, st, statCols, smPercent == 100); });
   e.launch(s, {x, stats, bank, af, residual, out, outStats}, [&](cudaStream_t st) { return convFused(p, st); });
+  return e.running() ? convStatCols(p) : 128;
 }
 
-Buf statsBuf(Exec& e, int s, int64_t c, int64_t l) { return e.alloc(s, c * statChunks(l) * 2); }
+Buf statsBuf(Exec& e, int s, int64_t c, int64_t l, int64_t cols = 128) { return e.alloc(s, c * ceilDiv(l, cols) * 2); }
 
 Buf channelStatsOf(Exec& e, int s, Buf x, int64_t c, int64_t l) {
   Buf st = statsBuf(e, s, c, l);
@@ -204,27 +206,30 @@ struct PlainResidual {
 
 // AdaINResBlock1 (models/kokoro/model.py:235-247): three times {affine, Snake conv (dilation 1, 3, 5), affine, Snake conv
 // + residual}. `out` / `outStats` receive the result: the caller's memory where they come with a pointer, else tensors
-// allocated here.
+// allocated here. outStats = null: nobody asks for the result's statistics.
 template <class Residual>
 void resblock(Exec& e, int s, const LkcResblock& w, Buf x, Buf stats, int64_t l, Buf bank, Buf* out, Buf* outStats,
               Residual residual, int smPercent) {
   static const int64_t dil[3] = {1, 3, 5};
   const int64_t c = w.c, k = w.k;
   const Buf none;
+  int statCols = 128;
   for (int j = 0; j < 3; ++j) {
     const int64_t d = dil[j];
     const int i1 = 2 * j, i2 = 2 * j + 1;
     const bool last = j == 2;
     const Buf res = last ? residual.make(x) : x;
-    Buf xt = e.rows(s, c, l), st1 = statsBuf(e, s, c, l);
-    adainConv(e, s, x, stats, l, c, k, d, w, i1, bank, none, xt, st1, smPercent);
-    Buf xn = last && out->p ? *out : e.rows(s, c, l);
-    Buf stn = last && outStats->p ? *outStats : statsBuf(e, s, c, l);
+    Buf xt = e.rows(s, c, l), st1 = statsBuf(e, s, c, l, 32);
+    statCols = adainConv(e, s, x, stats, statCols, l, c, k, d, w, i1, bank, none, xt, st1, true, smPercent);
+    Buf xn = last && out->p ? *out : e.rows(s, c, l), stn;
+    if (!last) stn = statsBuf(e, s, c, l, 32);
+    else if (outStats) stn = outStats->p ? *outStats : statsBuf(e, s, c, l);
     if (last) residual.ready();
-    adainConv(e, s, xt, st1, l, c, k, 1, w, i2, bank, res, xn, stn, smPercent);
+    statCols = adainConv(e, s, xt, st1, statCols, l, c, k, 1, w, i2, bank, res, xn, stn, !last, smPercent);
     x = xn, stats = stn;
   }
-  *out = x, *outStats = stats;
+  *out = x;
+  if (outStats) *outStats = stats;
 }
 
 bool resblockOk(const LkcResblock& w) {
@@ -277,7 +282,7 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
     }
     void ready() const { e.join(1, 0); }
   };
-  Buf noise[2], noiseStats[2];
+  Buf noise[2], noiseStats;
   for (int i = 1; i >= 0; --i) {  // polyphase view of `har`, stride-1 conv, resblock
     const int s = 1 + i;
     const LkcNoiseConv& n = m.noise_conv[i];
@@ -290,11 +295,11 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
     conv(e, s, Act::None, y, ly, n.rows, kCh[i], n.taps, 1, 0, n.w, n.b, none, nullptr, 0.f, n.state, none, xs, xst,
          kNoiseSms[i]);
     e.join(s, 3);
-    if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], AddUpsampled{e, u0, kCh[0], len[0]}, kNoiseSms[i]);
-    else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats[i], PlainResidual{}, kNoiseSms[i]);
+    if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats, AddUpsampled{e, u0, kCh[0], len[0]}, kNoiseSms[i]);
+    else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], nullptr, PlainResidual{}, kNoiseSms[i]);
   }
 
-  Buf in = noise[0], inStats = noiseStats[0], mean;
+  Buf in = noise[0], inStats = noiseStats, mean;
   for (int i = 0; i < 2; ++i) {
     const int64_t l = len[i], c = kCh[i];
     e.join(0, 1 + i);
@@ -303,9 +308,9 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
       inStats = channelStatsOf(e, 0, in, c, l);
     }
     e.join(3, 0), e.join(4, 0);
-    Buf rb[3], st[3];
+    Buf rb[3];
     for (int j = 2; j >= 0; --j)
-      resblock(e, j == 2 ? 0 : (j == 1 ? 3 : 4), m.res[3 * i + j], in, inStats, l, bank, &rb[j], &st[j], PlainResidual{},
+      resblock(e, j == 2 ? 0 : (j == 1 ? 3 : 4), m.res[3 * i + j], in, inStats, l, bank, &rb[j], nullptr, PlainResidual{},
                kBranchSms[i][j]);
     e.join(0, 3), e.join(0, 4);
     mean = e.rows(0, c, l);
@@ -314,11 +319,11 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
     });
   }
 
-  Buf post, postStats = statsBuf(e, 0, 22, len[1]), ident;
+  Buf post, ident;
   if (io.post) post.p = static_cast<float*>(io.post), post.pitch = io.post_pitch;
   else post = e.rows(0, 22, len[1]);
   ident.p = const_cast<float*>(FP(m.ident128));
-  conv(e, 0, Act::Leaky, mean, len[1], 128, 22, 7, 1, 3, m.post_w, m.post_b, ident, nullptr, 0.01f, m.post_state, none, post, postStats,
+  conv(e, 0, Act::Leaky, mean, len[1], 128, 22, 7, 1, 3, m.post_w, m.post_b, ident, nullptr, 0.01f, m.post_state, none, post, none,
        100);
   e.launch(0, {post}, [&](cudaStream_t st) {
     return istftLogits(post.p, static_cast<float*>(io.audio), len[1], post.pitch, 20, 5, st);

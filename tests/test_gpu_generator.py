@@ -414,3 +414,22 @@ def test_captured_forward_keeps_its_weights(cuda):
     torch.cuda.synchronize()
     assert torch.equal(b["audio"], want)
     del filler
+
+
+@pytest.mark.parametrize("stage,l", [(1, 19201), (1, 24833), (1, 28417), (1, 20000), (0, 9601), (0, 12001), (0, 15000)])
+@pytest.mark.parametrize("k", [3, 11])
+def test_whole_resblock_at_other_tile_widths(cuda, gen, stage, l, k):
+    """Lengths whose convs take tiles of 160, 192 or 224 columns inside the whole-block call (statistics per 32 columns):
+    against the op-by-op form, whose tiles are 256 wide, within the rounding of six convs in a row; the last columns alone too,
+    where a tile ends inside the row."""
+    from lokinfer_b200 import ops
+    x = torch.randn((256, 128)[stage], l, generator=torch.Generator(device=cuda).manual_seed(l), device=cuda)
+    gb = gen.style(torch.randn(128, generator=torch.Generator(device=cuda).manual_seed(k), device=cuda))
+    prefix = f"resblocks.{3 * stage + (0 if k == 3 else 2)}"
+    out, st = gen.adain_resblock1_fused(x, gb, prefix, k)
+    with ops.use_allocator(lambda shape, device: torch.empty(shape, dtype=torch.float32, device=device)):
+        want, want_st = gen.adain_resblock1_fused(x, gb, prefix, k)
+    assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 6 * REL_L2
+    assert rel_l2(out[:, -256:].cpu().numpy(), want[:, -256:].cpu().numpy()) <= 6 * REL_L2
+    assert rel_l2(st.cpu().numpy(), want_st.cpu().numpy()) <= 6 * REL_L2
+    assert torch.equal(out, gen.adain_resblock1_fused(x, gb, prefix, k)[0]) and ops.conv_tc_status() == 0
