@@ -154,7 +154,7 @@ struct TcArgs {
   int padLeft;       // ConvTranspose: 1 = one-sample left reflect pad
   float slope, outScale;
   int delta;       // columns between the 16-byte boundary a tile's window is loaded from and its first column (0: 4-byte route)
-  int tileCols;    // time columns per tile: NTS split, else 32 .. NT in steps of 32 (see tileColsFor)
+  int tileCols;    // time columns per tile: NTS split, else 160 .. NT in steps of 32 (see tileColsFor)
   int mainRows;    // staged rows that every lane has a slot for: the window up to NT (split: NTS) rows, a multiple of 64
   int rows;        // staged time rows per buffer: at least tileCols + (k-1)*dilation + delta and mainRows
   int ext;         // raw staging: [16][NT or NTS], then [16][ext] with the rows beyond them (two TMA boxes)
@@ -166,7 +166,6 @@ struct TcArgs {
   int tmaOut;      // 1: out (and residual) rows are 16-byte aligned, boxes go by TMA
   int numTTiles, numCoBlk;
   int split;       // 0 = a persistent CTA per SM over 256-column tiles; else the CTAs that share one 128-column tile
-  int fine;        // stats: a (mean, M2) pair per 32 columns, not per 128
   int early;       // the launch may overlap the end of the one before it (programmatic dependent launch)
   int* status;
   long long* prof;  // null, or 16 cycle counters summed over CTAs (see convTcProfile)
@@ -624,7 +623,8 @@ struct SplitTail {
 // that own them, over the operand buffers there, which nothing reads any more; when it has all of its own it finishes them:
 // the partials are added in rank order, then bias, residual, scale, statistics and coalesced stores. For launches with fewer
 // tiles than SMs, where one tile's serial chain of chunks is the launch's time (see splitFor).
-template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT>
+// NARROW: tiles of a.tileCols < NT columns. A form of its own: the width as a run-time value cost 256-column tiles 5 % (K = 7).
+template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT, bool NARROW>
 __global__ void __launch_bounds__(NTHREADS, 1)
     convTcKernel(const TcArgs a, const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapExt,
                  const __grid_constant__ CUtensorMap mapRes, const __grid_constant__ CUtensorMap mapOut) {
@@ -634,7 +634,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // Dhi buffers: a 128-column tile leaves room for two, so that the hi MMAs of a drain group need not wait for the drain
   // of the one before (the lo MMAs that cover it are shorter here)
   constexpr int HB = SPLIT ? 2 : 1;
-  const uint32_t kIdesc = SPLIT ? idescOf(F16, NTS) : idescOf(F16, 0) | (uint32_t(a.tileCols >> 3) << 17);
+  const uint32_t kIdesc = NARROW ? idescOf(F16, 0) | (uint32_t(a.tileCols >> 3) << 17) : idescOf(F16, NTK);
   const int NB = a.nb;
   extern __shared__ __align__(1024) unsigned char smemRaw[];
   const int rows = a.rows, ext = a.ext;
@@ -668,7 +668,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     if (threadIdx.x == 0) atomicOr(a.status, (6 << 8) | 1);
     return;
   }
-  const int W = SPLIT ? NTS : a.tileCols;
+  static_assert(!(SPLIT && NARROW), "a split tile is one statistics chunk");
+  const int W = NARROW ? a.tileCols : NTK;
   const int numTiles = a.numTTiles * a.numCoBlk;
   // tiles of this CTA: tile0, tile0 + tileStep, ...; its chunks of a tile: cBegin .. cBegin + nChunks16
   const int rank = SPLIT ? int(clusterRank()) : 0;
@@ -736,7 +737,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     dependenciesWait();
     const int q = warp & 3, g = warp >> 2;  // TMEM lane quarter, half of the tile
     // 32-column batches of this warp (of 256 columns: 4) and its first column
-    const int nb0 = SPLIT ? EC / 32 : ((W >> 5) + 1) >> 1, nbat = SPLIT ? EC / 32 : (g ? (W >> 5) - nb0 : nb0), gcol = g * nb0 * 32;
+    const int nb0 = NARROW ? ((W >> 5) + 1) >> 1 : EC / 32, nbat = NARROW && g ? (W >> 5) - nb0 : nb0, gcol = g * nb0 * 32;
     float* const tile = sStage + warp * STAGE_FLOATS;                                  // unaligned route: [32][33]
     unsigned char* const box = smemRaw + warp * BOX_BYTES;                             // aligned route: swizzled 32 x 32
     unsigned char* const boxRow = box + lane * 128;                                    // this lane's row of the box
@@ -873,7 +874,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         if (SPLIT && groupIt + 1 == uint32_t(nGroups)) clusterArrive(), arrived = true;
 #pragma unroll
         for (int b = 0; b < EC / 16; ++b) {
-          if (!SPLIT && b >= 2 * nbat) break;
+          if (NARROW && b >= 2 * nbat) break;
           uint32_t v[16];
           tmemLoad16Async(tmemHi + hb * NTK + laneBase + gcol + b * 16, v);
           tmemWaitLoads();
@@ -916,7 +917,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           tcFenceAfter();
 #pragma unroll
           for (int b = 0; b < EC / 32; ++b) {  // two 16-column loads in flight per wait
-            if (!SPLIT && b >= nbat) break;
+            if (NARROW && b >= nbat) break;
             uint32_t va[16], vb[16];
             tmemLoad16Async(tmemLo + laneBase + gcol + b * 32, va);
             tmemLoad16Async(tmemLo + laneBase + gcol + b * 32 + 16, vb);
@@ -1051,7 +1052,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             __syncwarp();
           }
         }
-        if (a.stats && a.fine && (!PARTIAL || co < a.co)) {  // a pair per 32 columns
+        if (NARROW && a.stats && (!PARTIAL || co < a.co)) {  // a pair per 32 columns
           float2* const st = reinterpret_cast<float2*>(a.stats) + int64_t(co) * a.nchunks + tChunk / 32;
 #pragma unroll
           for (int b = 0; b < 4; ++b)
@@ -1086,7 +1087,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-          if (b >= nbat) break;
+          if (NARROW && b >= nbat) break;
           const int64_t u0 = (tChunk + b * 32) * TS;
           if (lane < ROWS) {
 #pragma unroll
@@ -1139,7 +1140,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     // A warp stages the rows of its half, SLOTS per lane, with addresses that are immediates. The rows beyond the tile's
     // columns (at most 53) take one more slot for up to 32 of them: the first 32 go to the warps of half `raw buffer`, so
     // that the halves take turns, the rest to the other half.
-    const int halfRows = a.mainRows / 2, slots = a.mainRows / 64;
+    const int mainRows = NARROW ? a.mainRows : NTK, halfRows = mainRows / 2, slots = mainRows / 64;
     const bool tmaIn = a.tmaIn != 0;
     // per-channel parameters, once: sPar = [-mean | a | b | inv] with a = scale, b = beta (x alpha for Snake), inv = 1/alpha
     // Split form with statsIn: each CTA folds the chunk statistics of its own channels into mean / scale / beta, with the
@@ -1300,7 +1301,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
           for (int sl = 0; sl < decltype(n)::value; ++sl) stage(std::false_type{}, r0 + sl * 32, sp0 + sl * 32, NTK);
         };
-        if (SPLIT || slots == 2) all(std::integral_constant<int, 2>{});
+        if (!NARROW) all(std::integral_constant<int, NTK / 64>{});
         else if (slots == 4) all(std::integral_constant<int, 4>{});
         else all(std::integral_constant<int, 3>{});
         if (rx < rows) stage(std::false_type{}, rx, spx, ext);
@@ -1684,7 +1685,7 @@ struct DeviceInfo {
 // A cluster lives inside one GPC, of whose SMs a remainder is left over: 148 SMs hold 74 clusters of two, but 45 of three,
 // 33 of four, 26 of five, 22 of six, 15 of seven or eight (one B200; which SMs are fused off differs).
 static void countClusters(DeviceInfo& d) {
-  const auto kernel = convTcKernel<1, false, 0, true, false, true>;
+  const auto kernel = convTcKernel<1, false, 0, true, false, true, false>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) {
     cudaGetLastError();
     return;  // no split launches
@@ -1786,12 +1787,12 @@ struct TcMaps {
   CUtensorMap x, ext, res, out;
 };
 
-template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT>
-static int launchTc4(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cudaStream_t s) {
+template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT, bool NARROW>
+static int launchTc5(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cudaStream_t s) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  const auto kernel = convTcKernel<ACT, PARTIAL, TS, F16, TMAO, SPLIT>;
+  const auto kernel = convTcKernel<ACT, PARTIAL, TS, F16, TMAO, SPLIT, NARROW>;
   if (dev >= 0 && dev < 64 && !configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e != cudaSuccess) return failCuda("conv (tensor-core): cudaFuncSetAttribute", e);
@@ -1815,6 +1816,14 @@ static int launchTc4(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cu
     return failCuda("conv (tensor-core)", e);
   }
   return launched("conv (tensor-core)");
+}
+
+template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT>
+static int launchTc4(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cudaStream_t s) {
+  if constexpr (F16 && !SPLIT) {
+    if (a.tileCols < NT) return launchTc5<ACT, PARTIAL, TS, F16, TMAO, SPLIT, true>(a, m, grid, smem, s);
+  }
+  return launchTc5<ACT, PARTIAL, TS, F16, TMAO, SPLIT, false>(a, m, grid, smem, s);
 }
 
 template <int ACT, bool PARTIAL, int TS, bool F16>
@@ -1861,7 +1870,7 @@ int convTcProfile(int enable, long long* out16) {
 
 // CTAs per tile: 0 = the persistent form. The split form is taken where at least two CTAs per 128-column tile fit on the
 // launch's share of the SMs and all its clusters are resident at a time (clusters[n], see countClusters): there the time is
-// one tile's chain of 16-channel chunks plus about 9 us of fixed cost (launch, first loads, cluster reduction), and the
+// one tile's chain of 16-channel chunks plus about 7 us of fixed cost (launch, first loads, exchange), and the
 // chain shrinks with every CTA. With one CTA per tile it gains little over 256-column tiles (an M128 N128 MMA takes about
 // 0.8 of the time of an N256 one here) and doubles the weight traffic; with a second wave it loses: [128, 6144] K = 11,
 // 48 clusters of three where 45 fit, 36 us against 30 us unsplit and 21 us with two CTAs per tile.
@@ -1890,7 +1899,8 @@ int convTcSplitRule(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* 
 // columns plus 48 more: a narrower tile pays where it takes fewer SM-columns in whole rounds.
 // Beside other launches the columns all together count, of which wide tiles cost fewer, unless there are few: then the
 // narrowest tiles that find room in one round of the launch's share shorten its chain.
-// Widths other than NT leave chunk statistics per 32 columns, which the caller has to take (fineOk).
+// Widths other than NT (a form of the kernel with f16 halves) leave chunk statistics per 32 columns, which the caller has to
+// take (fineOk).
 static int tileColsFor(bool fineOk, int64_t lo, int64_t coBlocks, int sms, int smPercent) {
   int best = NT;
   if (!fineOk) return best;
@@ -1908,9 +1918,8 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool canSplit, bool boxesO
   a.split = splitFor(canSplit, a.ci, a.lo, a.numCoBlk, d->smCount * smPercent / 100, d->clusters);
   LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
   const int nt = a.split ? NTS : NT;  // staged columns of the first box
-  a.tileCols = a.split ? NTS : tileColsFor(fineOk, a.lo, a.numCoBlk, d->smCount, smPercent);
-  a.fine = a.tileCols != NT && !a.split;
-  if (a.stats && a.fine) a.nchunks = ceilDiv(a.lo, 32);
+  a.tileCols = a.split ? NTS : tileColsFor(f16 && fineOk, a.lo, a.numCoBlk, d->smCount, smPercent);
+  if (a.stats && !a.split && a.tileCols != NT) a.nchunks = ceilDiv(a.lo, 32);
   a.numTTiles = int(ceilDiv(a.lo, a.tileCols));
   // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
   // argument: it stays zero-filled and is never dereferenced.
@@ -1956,7 +1965,7 @@ bool convTcSplits(const ConvFusedParams& p, bool f16) {
 int convTcStatCols(const ConvFusedParams& p, bool f16) {
   const DeviceInfo* d = nullptr;
   if (!p.fineStats || deviceInfo(&d) != 0 || convTcSplits(p, f16)) return 128;
-  return tileColsFor(true, p.lo, ceilDiv(p.co, MT), d->smCount, p.smPercent) == NT ? 128 : 32;
+  return tileColsFor(f16, p.lo, ceilDiv(p.co, MT), d->smCount, p.smPercent) == NT ? 128 : 32;
 }
 
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {
