@@ -30,12 +30,12 @@ constexpr float kEps = 1e-5f;  // AdaIN
 // Percent of the SMs that one launch may spread over, as other branches run beside it (on one stream too, so that both
 // ways add the same partial sums): [stage] the k = 3, 7, 11 resblocks, and the two noise branches. What runs beside each
 // other may add up to more than 100: launches of branches rarely coincide for long, and clusters that find no room start
-// when others end. The longer a branch's chain, the more it gets; the first noise branch is waited for one stage earlier than the second. Measured, microseconds
-// per forward of T = 24 / 121 / 240 / 320 / 400 frames: no splitting 877 / 934 / 980 / 1054 / 1086; noise branches and
-// k = 7, 11 even 400 / 734 / 979 / 1052 / 1088; k = 11 at 50 in both stages 400 / 697 / 915 / 1055 / 1086, at 70 in both
-// 432 / 713 / 853 / 1011 / 1076 (stage 0 of T = 240 and 320 gains, stage 1 of T = 24 loses); as below, and with only as
-// many CTAs per tile as the device holds clusters for: 400 / 711 / 853 / 1013 / 1091.
-constexpr int kBranchSms[2][3] = {{26, 36, 70}, {26, 36, 50}}, kNoiseSms[2] = {70, 40};
+// when others end. The longer a branch's chain, the more it gets; the first noise branch is waited for one stage earlier than
+// the second. us per forward of T = 24 / 80 / 121 / 200 / 320 frames, [stage 0 | stage 1 | noise]: 26, 36, 70 | 26, 36, 50 | 70,
+// 40: 337 / 513 / 598 / 757 / 934; 33 each, noise 50: 352 / 517 / 581 / 751 / 877; k = 11 at 90 in stage 0: 336 / 624 / 717 /
+// 759 / 935; as below 333 / 511 / 597 / 705 / 878 (T = 320 gains where stage 0 of k = 11 takes whole tiles instead of halves,
+// T = 200 from the second noise branch). No splitting at all, with an earlier build: 877 at T = 24, 934 at 121.
+constexpr int kBranchSms[2][3] = {{26, 36, 60}, {26, 36, 50}}, kNoiseSms[2] = {60, 50};
 
 // Channels of the two stages, of what goes into their upsamplers, and the upsampling factors.
 constexpr int64_t kCh[2] = {256, 128}, kChIn[2] = {512, 256}, kUp[2] = {10, 6};
