@@ -1668,7 +1668,7 @@ bool convTcEligible(const ConvFusedParams& p, bool f16) {
         chainOk(p.k, f16) && (p.k - 1) * p.dilation <= MAX_HALO && p.lo >= 1 && p.padding <= (1 << 20) && p.ci <= 4096 &&
         p.l < (int64_t(1) << 30)))
     return false;
-  return convTcSmemBytes(false, p.ci, NT + int((p.k - 1) * p.dilation) + 3, int(p.k), false, nullptr, nullptr) != 0;  // the larger format
+  return convTcSmemBytes(false, p.ci, NT + int((p.k - 1) * p.dilation), int(p.k), false, nullptr, nullptr) != 0;  // the larger format
 }
 
 int64_t convTcPackFloats(int64_t co, int64_t ci, int64_t k, bool f16) {
@@ -1925,14 +1925,18 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool canSplit, bool boxesO
   // argument: it stays zero-filled and is never dereferenced.
   std::memset(&m, 0, sizeof m);
   a.tmaIn = makeMap(&m.x, a.x, a.ci, a.l, a.xPitch, nt, KC, false) ? 1 : 0;
-  a.delta = a.tmaIn ? -a.padding & 3 : 0;  // tiles start on multiples of 4 columns
-  const int need = a.tileCols + (a.k - 1) * a.dilation + a.delta;
-  a.mainRows = std::min(nt, (need + 63) & ~63);
-  a.rows = std::max(need, a.mainRows);
-  a.ext = rawExt(a.rows, nt);
+  auto layOut = [&] {
+    a.delta = a.tmaIn ? -a.padding & 3 : 0;  // tiles start on multiples of 4 columns
+    const int need = a.tileCols + (a.k - 1) * a.dilation + a.delta;
+    a.mainRows = std::min(nt, (need + 63) & ~63);
+    a.rows = std::max(need, a.mainRows);
+    a.ext = rawExt(a.rows, nt);
+    *smem = convTcSmemBytes(a.split != 0, a.ci, a.rows, a.k, f16, &a.wStages, &a.wG);
+  };
+  layOut();
+  if (*smem == 0 && a.tmaIn) a.tmaIn = 0, layOut();  // no room for the rows in front of the window: the 4-byte route has none
   if (a.tmaIn && a.ext)
     LKC_REQUIRE(makeMap(&m.ext, a.x, a.ci, a.l, a.xPitch, a.ext, KC, false), "conv (tensor-core): tensor map of the input");
-  *smem = convTcSmemBytes(a.split != 0, a.ci, a.rows, a.k, f16, &a.wStages, &a.wG);
   LKC_REQUIRE(*smem != 0, "conv (tensor-core): window too large");
   if (a.split && *smem < SPLIT_SMEM) *smem = SPLIT_SMEM;
   a.nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
@@ -2000,7 +2004,7 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
 
 bool convtTcEligible(int64_t ci, int64_t co, int64_t k, int64_t stride, int64_t padding) {
   return (stride == 6 || stride == 10) && k == 2 * stride && 2 * padding == stride && ci % KC == 0 && ci >= KC &&
-         ci <= 4096 && co >= 1 && convTcSmemBytes(false, ci, NT + 2 + 3, 3, false, nullptr, nullptr) != 0;
+         ci <= 4096 && co >= 1 && convTcSmemBytes(false, ci, NT + 2, 3, false, nullptr, nullptr) != 0;
 }
 
 int64_t convtTcPackFloats(int64_t ci, int64_t co, int64_t stride, bool f16) {

@@ -347,19 +347,21 @@ void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
   Buf bank = e.alloc(0, m.bank_n), enc = e.rows(0, kDecIn[0], f), cat = e.rows(0, kDecIn[1], f);
   Buf encStats = statsBuf(e, 0, kDecIn[0], f), catStats = statsBuf(e, 0, kDecIn[1], f);
   const int64_t pitch = enc.pitch, chunkFloats = 2 * statChunks(f);
-  e.launch(0, {bank}, [&](cudaStream_t st) { return gemmBias(FP(io.s), FP(m.bank_wt), FP(m.bank_b), bank.p, 1, 128, m.bank_n, st); });
+  e.join(1, 0);
+  e.launch(1, {bank}, [&](cudaStream_t st) { return gemmBias(FP(io.s), FP(m.bank_wt), FP(m.bank_b), bank.p, 1, 128, m.bank_n, st); });
   e.launch(0, {enc, cat}, [&](cudaStream_t st) {
     return decoderInputs(FP(io.asr), io.asr_pitch, FP(io.f0), FP(io.n), FP(m.f0_w), FP(m.f0_b), FP(m.n_w), FP(m.n_b), enc.p,
                          kDecIn[0], cat.p, kDecCh + 64, kDecIn[1], f, pitch, st);
   });
-  e.join(1, 0);
+  e.launch(0, {enc, encStats}, [&](cudaStream_t st) { return channelStats(enc.p, encStats.p, kDecIn[0], f, pitch, statChunks(f), st); });
+  e.join(0, 1);  // the style bank
+  e.join(1, 0);  // the block inputs
   conv(e, 1, Act::None, enc, f, 512, 64, 1, 1, 0, m.asr_w, m.asr_b, none, nullptr, 0.f, m.asr_state, none,
        from(cat, kDecCh * pitch), from(catStats, kDecCh * chunkFloats), 100);
   e.launch(1, {cat, catStats}, [&](cudaStream_t st) {
     return channelStats(cat.p + (kDecCh + 64) * pitch, catStats.p + (kDecCh + 64) * chunkFloats, kDecIn[1] - kDecCh - 64, f,
                         pitch, statChunks(f), st);
   });
-  e.launch(0, {enc, encStats}, [&](cudaStream_t st) { return channelStats(enc.p, encStats.p, kDecIn[0], f, pitch, statChunks(f), st); });
 
   // AdaIN -> leaky -> conv k 3 [+ residual, scaled]; see adainConv
   auto leakyConv = [&](Buf x, Buf stats, int64_t l, int64_t ci, int64_t co, const void* w, const void* b, const LkcConvState* state,

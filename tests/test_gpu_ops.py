@@ -374,7 +374,9 @@ def test_conv1d_weights_beyond_f16_range_fall_back_to_tf32_pack(cuda):
 
 
 TF32_CASES = [(128, 128, 1201, 3, 1), (128, 128, 1201, 7, 3), (256, 256, 640, 11, 5), (128, 128, 257, 7, 1),
-              (16, 128, 700, 7, 3), (128, 22, 5000, 7, 1), (128, 128, 19201, 11, 3)]
+              (16, 128, 700, 7, 3), (128, 22, 5000, 7, 1), (128, 128, 19201, 11, 3),
+              # aligned rows, but shared memory only for a window without the rows in front of it: the 4-byte route
+              (2928, 16, 300, 11, 5)]
 
 
 @pytest.mark.parametrize("ci,co,l,k,d", TF32_CASES)
