@@ -71,8 +71,11 @@ class Decoder:
         self.bank_b = torch.cat(bias).contiguous()
         self._ident = {c: torch.stack([torch.zeros(c), torch.ones(c), torch.zeros(c)]).to(self.device).contiguous()
                        for c in {512} | {_pad16(cin) for _, cin, _, _ in DECODER_BLOCKS}}
-        self._model = None  # (getters of its weights and states, _Model) of the whole-forward call
-        self._side = None
+        self._init_calls()
+
+    def _init_calls(self):
+        self._model = None  # _Model of the whole-forward call
+        self._side = None  # its second stream
 
     # The forward as one library call (lkc_decoder_forward). It computes what the composition in forward() computes with a
     # third of its launches (block inputs are never concatenated, statistics come from the convs that wrote the rows), the
@@ -99,8 +102,9 @@ class Decoder:
         except KeyError:
             return None
         pieces = (*ws, *states, self.bank_wt, self.bank_b, self.bank_off)
-        if self._model is not None and self._model.held.current(pieces):
-            return self._model
+        model = self._model
+        if model is not None and model.held.current(pieces):
+            return model
         w, st, n = dict(zip(self._NAMES, ws)), dict(zip(self._STATES, states)), int(self.bank_b.shape[0])
 
         def has(conv, co, ci, k):
@@ -133,10 +137,14 @@ class Decoder:
         d.asr_w, d.asr_b = w["decoder.asr_res.0.weight"].data_ptr(), w["decoder.asr_res.0.bias"].data_ptr()
         d.asr_state = st["decoder.asr_res.0"].handle
         with torch.cuda.device(self.bank_b.device):
-            self._model = _Model(d, _Held(pieces), "lkc_decoder_create")
-            if self._side is None:
-                self._side = torch.cuda.Stream(self.bank_b.device)
-        return self._model
+            model = _Model(d, _Held(pieces), "lkc_decoder_create")
+        self._model = model  # complete: another thread may take it from here on
+        return model
+
+    def _side_stream(self):
+        if self._side is None:
+            self._side = torch.cuda.Stream(self.bank_b.device)
+        return self._side
 
     def _takes(self, asr, f0, n_curve, s):
         """Whether the whole call may have these operands, whose addresses go to the kernels unchecked."""
@@ -156,7 +164,7 @@ class Decoder:
                 io = _lib.LkcDecoderIo()
                 io.asr, io.f0, io.n, io.s = asr.data_ptr(), f0.data_ptr(), n_curve.data_ptr(), s.data_ptr()
                 io.out, io.frames, io.asr_pitch, io.out_pitch = out.data_ptr(), frames, asr.stride(0), out.stride(0)
-                io.workspace, io.workspace_bytes, io.side = ws.data_ptr(), size.value, self._side.cuda_stream
+                io.workspace, io.workspace_bytes, io.side = ws.data_ptr(), size.value, self._side_stream().cuda_stream
                 rc = lib.lkc_decoder_forward(model.handle, ctypes.byref(io), ops._stream())
         if rc != 0:
             raise _lib.LkcError("decoder forward: " + _lib.last_error())
