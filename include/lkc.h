@@ -345,7 +345,8 @@ typedef struct LkcDecoderIo {
   int64_t frames, asr_pitch, out_pitch;
   void* workspace;
   int64_t workspace_bytes;
-  void* side;       /* a stream for the shortcuts; joined back before the call's last kernel */
+  void* side;       /* a stream for the shortcuts, joined back before the call's last kernel; left out (they go on the caller's
+                       stream) while it is in a capture that the caller's stream is not in */
   int64_t launches; /* out: kernels queued */
 } LkcDecoderIo;
 typedef struct LkcModel LkcModel;

@@ -576,6 +576,26 @@ extern "C" LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, vo
   });
 }
 
+namespace {
+// Whether `side` can be forked from `stream` and joined back: not while it is in a capture that `stream` is not in. A side
+// stream stays in its caller's capture when that call returns, until the capture ends; a fork from outside would fail and
+// invalidate the capture.
+bool joinable(cudaStream_t stream, cudaStream_t side) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone, sd = cudaStreamCaptureStatusNone;
+  unsigned long long idStream = 0, idSide = 0;
+  if (cudaStreamGetCaptureInfo(side, &sd, &idSide) != cudaSuccess || sd == cudaStreamCaptureStatusInvalidated) {
+    cudaGetLastError();
+    return false;
+  }
+  if (sd == cudaStreamCaptureStatusNone) return true;
+  if (cudaStreamGetCaptureInfo(stream, &st, &idStream) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return st == cudaStreamCaptureStatusActive && idStream == idSide;
+}
+}  // namespace
+
 extern "C" LKC_API int lkc_decoder_workspace(LkcModel* m, int64_t frames, int64_t* bytes) {
   LKC_REQUIRE(m && bytes && m->isDecoder, "decoder_workspace: null argument or a generator's handle");
   LKC_REQUIRE(frames >= 1 && frames < (int64_t(1) << 24), "decoder_workspace: frames out of range");
@@ -601,7 +621,7 @@ extern "C" LKC_API int lkc_decoder_forward(LkcModel* m, LkcDecoderIo* io, void* 
     if (int rc = m->plan(io->frames, 1, &p)) return rc;
     LKC_REQUIRE(io->workspace_bytes >= p->bytes, "decoder_forward: the workspace is too small (lkc_decoder_workspace)");
     cudaStream_t side[kStreams - 1];
-    for (cudaStream_t& s : side) s = S(io->side);
+    for (cudaStream_t& s : side) s = joinable(S(stream), S(io->side)) ? S(io->side) : S(stream);
     Exec e(true, *p, static_cast<char*>(io->workspace), S(stream), side, m->events);
     decoder(e, m->dec, *io);
     if (e.rc != 0) e.joinForked();

@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import ctypes
 import operator
+import threading
 
 import numpy as np
 import torch
@@ -75,7 +76,7 @@ class Decoder:
 
     def _init_calls(self):
         self._model = None  # _Model of the whole-forward call
-        self._side = None  # its second stream
+        self._sides = {}  # calling stream -> the stream of its shortcuts (_side_stream)
 
     # The forward as one library call (lkc_decoder_forward). It computes what the composition in forward() computes with a
     # third of its launches (block inputs are never concatenated, statistics come from the convs that wrote the rows), the
@@ -141,10 +142,26 @@ class Decoder:
         self._model = model  # complete: another thread may take it from here on
         return model
 
-    def _side_stream(self):
-        if self._side is None:
-            self._side = torch.cuda.Stream(self.bank_b.device)
-        return self._side
+    _MAX_SIDES = 16
+    _SIDES_LOCK = threading.Lock()
+
+    def _side_stream(self, caller):
+        """The handle of the stream for the shortcuts of a call on stream `caller`: one per calling stream, so that callers on
+        different streams do not wait for each other, nor one for a capture of another. Its own, as far as torch's pool of 32
+        goes: none of another caller and no calling stream seen so far. The last callers' are kept; a stream that was handed out
+        twice in the end costs overlap, not results (lkc_decoder_forward leaves out one that is in another capture)."""
+        with self._SIDES_LOCK:
+            side = self._sides.pop(caller, None)
+            if side is None:
+                taken = {caller, *self._sides, *(s.cuda_stream for s in self._sides.values())}
+                for _ in range(64):
+                    side = torch.cuda.Stream(self.bank_b.device)
+                    if side.cuda_stream not in taken:
+                        break
+                while len(self._sides) >= self._MAX_SIDES:
+                    del self._sides[next(iter(self._sides))]
+            self._sides[caller] = side  # the last one used at the end
+            return side.cuda_stream
 
     def _takes(self, asr, f0, n_curve, s):
         """Whether the whole call may have these operands, whose addresses go to the kernels unchecked."""
@@ -164,8 +181,9 @@ class Decoder:
                 io = _lib.LkcDecoderIo()
                 io.asr, io.f0, io.n, io.s = asr.data_ptr(), f0.data_ptr(), n_curve.data_ptr(), s.data_ptr()
                 io.out, io.frames, io.asr_pitch, io.out_pitch = out.data_ptr(), frames, asr.stride(0), out.stride(0)
-                io.workspace, io.workspace_bytes, io.side = ws.data_ptr(), size.value, self._side_stream().cuda_stream
-                rc = lib.lkc_decoder_forward(model.handle, ctypes.byref(io), ops._stream())
+                stream = ops._stream()
+                io.workspace, io.workspace_bytes, io.side = ws.data_ptr(), size.value, self._side_stream(stream)
+                rc = lib.lkc_decoder_forward(model.handle, ctypes.byref(io), stream)
         if rc != 0:
             raise _lib.LkcError("decoder forward: " + _lib.last_error())
         ops.count_launches(io.launches)

@@ -63,7 +63,7 @@ def dec(monkeypatch):
 
     def stream(*a, **k):
         n = next(made)
-        time.sleep(0.1)
+        time.sleep(0.02)
         return types.SimpleNamespace(cuda_stream=n)
 
     monkeypatch.setattr(D, "_Model", lambda struct, held, create: types.SimpleNamespace(held=held, handle=1))
@@ -106,3 +106,22 @@ def test_first_use_from_several_threads(dec):
 
     in_threads(lambda: call(dec), late, late)
     assert len(dec.library.calls) == 3 and all(side for _, side in dec.library.calls)
+
+
+def test_every_calling_stream_has_a_side_stream_of_its_own(dec):
+    """Also when the new stream that torch hands out is one that a caller uses already."""
+
+    def on(stream):
+        def job():
+            dec.library.at.stream = stream
+            for _ in range(3):
+                call(dec)
+        return job
+
+    in_threads(*(on(s) for s in (0, 7, 1000, 1002)))
+    sides = {}
+    for stream, side in dec.library.calls:
+        assert sides.setdefault(stream, side) == side != stream
+    assert len(sides) == len(set(sides.values())) == 4
+    in_threads(*(on(s) for s in range(10, 50)))  # many short-lived callers: the store stays bounded
+    assert len(dec._sides) == dec._MAX_SIDES

@@ -170,3 +170,44 @@ def test_whole_decoder_in_a_graph(cuda, dec):
         g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("one_side", [False, True])
+def test_a_capture_beside_a_call_of_another_thread(cuda, dec, monkeypatch, one_side):
+    """While one thread captures a forward, another runs one: the call works and the capture stays valid. one_side: both are
+    handed the same side stream, which is then in the first one's capture."""
+    import threading
+    a, b = _args(cuda, 61, 3), _args(cuda, 200, 4)
+    want = [dec.forward(*x).clone() for x in (a, b)]
+    streams = [torch.cuda.Stream(device=cuda) for _ in range(2)]
+    if one_side:
+        side = torch.cuda.Stream(device=cuda)
+        monkeypatch.setattr(dec, "_side_stream", lambda caller: side.cuda_stream)
+    torch.cuda.synchronize()
+    captured, done = threading.Event(), threading.Event()
+    got, errors = [], []
+
+    def other():
+        try:
+            assert captured.wait(60)
+            with torch.cuda.stream(streams[1]):
+                got.append(dec.forward(*b))
+        except Exception as e:  # a thread's exception would be lost
+            errors.append(repr(e))
+        finally:
+            done.set()
+
+    t, g = threading.Thread(target=other), torch.cuda.CUDAGraph()
+    t.start()
+    with torch.cuda.graph(g, stream=streams[0], capture_error_mode="thread_local"):
+        out = dec.forward(*a)
+        captured.set()
+        assert done.wait(60)
+        again = dec.forward(*a)  # the same capture a second time
+    t.join()
+    torch.cuda.synchronize()
+    assert not errors and torch.equal(got[0], want[1])
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want[0]) and torch.equal(again, want[0])
