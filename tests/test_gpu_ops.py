@@ -488,6 +488,20 @@ def test_channel_stats_and_adain_affine(cuda, c, l):
     np.testing.assert_allclose(got, ref, atol=2e-5 * max(1, np.abs(ref).max()), rtol=1e-4)
 
 
+@pytest.mark.parametrize("l", [1, 3, 127, 128, 129, 131, 700])
+def test_channel_stats_are_the_same_on_every_row_layout(cuda, l):
+    """Rows on 16-byte boundaries, contiguous ones and ones that start 4 to 12 bytes behind a boundary: the same bits."""
+    from lokinfer_b200 import ops
+    pitch = (l + 3) // 4 * 4
+    buf = torch.full((9, pitch + 4), float("nan"), device=cuda)
+    x = torch.randn(9, l, generator=torch.Generator(device=cuda).manual_seed(l), device=cuda) * 3 + 5
+    want = ops.channel_stats_f32_cuda(x)
+    check_stats(want.cpu().numpy(), x.cpu().numpy())
+    for off in range(4):
+        buf[:, off:off + l] = x
+        assert torch.equal(ops.channel_stats_f32_cuda(buf[:, off:off + l]), want)
+
+
 CONVT_CASES = [(8, 32, 5, 4, 2, 0), (16, 40, 37, 8, 4, 1), (512, 256, 26, 20, 10, 0), (512, 256, 294, 20, 10, 0),
                (256, 128, 2940, 12, 6, 1), (256, 128, 1, 12, 6, 1), (64, 64, 700, 12, 6, 1), (16, 8, 33, 6, 3, 1),
                (8, 4, 9, 5, 5, 0), (256, 128, 20800, 12, 6, 1), (512, 256, 2080, 20, 10, 0), (32, 7, 257, 20, 10, 1),
