@@ -215,11 +215,24 @@ __global__ void __launch_bounds__(kAffineThreads) adainAffineKernel(const float*
   }
 }
 
-// out[m, n] = sum_k x[m, k] wt[k, n] + b[n], coalesced over n. Meant for the style bank (M = 1, K = 128), where it is bound by
-// the latency of its loads: GEMV_K threads share a column's sum, so that 16 rows of wt are in flight per thread and 300 to 700
-// blocks run instead of 75 to 180 (T = 24: 12.5 us with one thread per column).
-constexpr int GEMV_N = 64, GEMV_K = 4;
+// out[m, n] = sum_k x[m, k] wt[k, n] + b[n]; one thread per output column, coalesced over n.
 __global__ void gemmBiasKernel(const float* __restrict__ x, const float* __restrict__ wt, const float* __restrict__ b,
+                               float* __restrict__ out, int64_t m, int64_t k, int64_t n) {
+  extern __shared__ float xs[];
+  const int64_t row = blockIdx.y;
+  for (int64_t i = threadIdx.x; i < k; i += blockDim.x) xs[i] = x[row * k + i];
+  __syncthreads();
+  const int64_t col = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  if (col >= n) return;
+  float acc = 0.f;
+  for (int64_t i = 0; i < k; ++i) acc = fmaf(xs[i], wt[i * n + col], acc);
+  out[row * n + col] = acc + b[col];
+}
+
+// The same for few outputs (the style bank: M = 1, K = 128), where the latency of the loads is the time: GEMV_K threads share a
+// column's sum, so that 16 rows of wt are in flight per thread and four times the blocks run.
+constexpr int GEMV_N = 64, GEMV_K = 4;
+__global__ void gemvBiasKernel(const float* __restrict__ x, const float* __restrict__ wt, const float* __restrict__ b,
                                float* __restrict__ out, int64_t m, int64_t k, int64_t n) {
   extern __shared__ float xs[];  // x's row, then the partial sums
   const int64_t row = blockIdx.y;
@@ -269,10 +282,19 @@ int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, i
   return launched("adain_affine_f32_cuda");
 }
 
+// us with one thread per column / with four: [1, 128] x [128, 19104] 5.4 / 3.6, [1, 512] x [512, 19104] 15.5 / 8.1. One is better
+// for sums of fewer than 64 terms (K = 33, N = 100: 2.6 / 3.1) and where the outputs fill the device already, from about 400
+// blocks of 256 on: [300, 512] x [512, 512] (600) 19 / 26, [64, 128] x [128, 19104] 37 / 51, [32, 512] x [512, 4096] (512) 19 / 22;
+// below, [16, 128] x [128, 4096] (256) 5.7 / 5.2, [4, 512] x [512, 19104] (298) 16.7 / 15.6, [4, 128] x [128, 19104] 5.9 / 6.1. Sums
+// of thousands of terms over a wide matrix can go the other way ([32, 4096] x [4096, 4096] 192 / 171).
 int gemmBias(const float* x, const float* wt, const float* b, float* out, int64_t m, int64_t k, int64_t n, cudaStream_t s) {
   static_assert(GEMV_K == 4, "the sum of the parts");
-  dim3 grid(static_cast<unsigned>(ceilDiv(n, GEMV_N)), static_cast<unsigned>(m));
-  gemmBiasKernel<<<grid, GEMV_N * GEMV_K, static_cast<size_t>(k > GEMV_N * GEMV_K ? k : GEMV_N * GEMV_K) * 4, s>>>(x, wt, b, out, m, k, n);
+  constexpr int kGemvThreads = GEMV_N * GEMV_K;
+  const auto grid = [&](int64_t cols) { return dim3(static_cast<unsigned>(ceilDiv(n, cols)), static_cast<unsigned>(m)); };
+  if (k < 64 || m * n > 400 * 256)
+    gemmBiasKernel<<<grid(kThreads), kThreads, static_cast<size_t>(k) * 4, s>>>(x, wt, b, out, m, k, n);
+  else
+    gemvBiasKernel<<<grid(GEMV_N), kGemvThreads, static_cast<size_t>(k > kGemvThreads ? k : kGemvThreads) * 4, s>>>(x, wt, b, out, m, k, n);
   return launched("gemm_bias_f32_cuda");
 }
 

@@ -741,6 +741,19 @@ def test_errors_come_back_as_exceptions(cuda):
     assert ops.istft_logits_f32_cuda(x).shape == (35,)
 
 
+@pytest.mark.parametrize("m,k,n", [(1, 63, 100), (1, 64, 100), (3, 65, 257), (1, 130, 19104), (2, 128, 51200), (2, 128, 51201),
+                                   (300, 65, 700), (1, 1, 1)])
+def test_gemm_bias_sizes(cuda, m, k, n):
+    """Both sides of the rule that shares a column's sum among four threads (64 terms, 102400 outputs), uneven parts, columns
+    beyond the last block. Rounding of a sum of k products of standard normals: k * 2^-24 * k^(1/2), far below the bar."""
+    from lokinfer_b200 import ops
+    r = np.random.default_rng(m * 7 + k)
+    x, wt, b = (r.standard_normal(sh).astype(np.float32) for sh in ((m, k), (k, n), (n,)))
+    got = ops.gemm_bias_f32_cuda(*dev(cuda, x, wt, b)).cpu().numpy()
+    ref = x.astype(np.float64) @ wt.astype(np.float64) + b
+    assert np.abs(got - ref).max() <= 1e-4 and rel_l2(got, ref) <= 1e-6
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("ci,co,l,k,s,p", [(22, 256, 1201, 12, 6, 3), (22, 128, 999, 1, 1, 0), (5, 32, 500, 6, 3, 2),
                                            (22, 256, 124801, 12, 6, 3)])
