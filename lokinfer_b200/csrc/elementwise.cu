@@ -405,13 +405,79 @@ __global__ void spaceToDepthKernel(const float* __restrict__ x, float* __restric
   }
 }
 
+// The same for large strides and small calls: 1 << lc columns at a time, the threads spread over columns and phases, and a gap of
+// one float per 32 in shared memory, since lanes `s` floats apart would meet in one bank where s is a multiple of 32.
+__global__ void spaceToDepthWideKernel(const float* __restrict__ x, float* __restrict__ y, int64_t ci, int64_t l, int64_t rows,
+                                       int64_t ly, int64_t xPitch, int64_t yPitch, int s, int64_t pad, int lc) {
+  extern __shared__ float sx[];
+  const int n = s << lc, last = (1 << lc) - 1;
+  for (int64_t c = blockIdx.y; c < ci + rows - ci * s; c += gridDim.y) {
+    for (int64_t t0 = int64_t(blockIdx.x) << lc; t0 < ly; t0 += int64_t(gridDim.x) << lc) {
+      if (c >= ci) {
+        const int64_t t = t0 + threadIdx.x;
+        if (int(threadIdx.x) <= last && t < ly) y[(ci * s + (c - ci)) * yPitch + t] = 0.f;
+        continue;
+      }
+      const int64_t pos0 = int64_t(s) * t0 - pad;
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int64_t pos = pos0 + i;
+        sx[i + (i >> 5)] = pos >= 0 && pos < l ? x[c * xPitch + pos] : 0.f;
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int r = i >> lc, t = i & last, at = t * s + r;
+        if (t0 + t < ly) y[(c * s + r) * yPitch + t0 + t] = sx[at + (at >> 5)];
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Stride 1: a copy with padding and zero rows, four loads in flight per thread ([22, 124801] 5.4 us, through shared memory 14.6).
+__global__ void spaceToDepthCopyKernel(const float* __restrict__ x, float* __restrict__ y, int64_t ci, int64_t l, int64_t rows,
+                                       int64_t ly, int64_t xPitch, int64_t yPitch, int64_t pad) {
+  for (int64_t c = blockIdx.y; c < rows; c += gridDim.y) {
+    const float* const xr = x + c * xPitch - pad;
+    for (int64_t t = blockIdx.x * int64_t(4 * kThreads) + threadIdx.x; t < ly; t += int64_t(gridDim.x) * 4 * kThreads) {
+      float v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int64_t at = t + j * kThreads;
+        v[j] = c < ci && at >= pad && at - pad < l ? xr[at] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (t + j * kThreads < ly) y[c * yPitch + t + j * kThreads] = v[j];
+    }
+  }
+}
+
 namespace lkc {
+// us for [channels, length], stride: one thread per column and all its phases / the wide form (columns at a time). Few blocks are
+// better spread: [3, 4000], 8 3.6 / 1.9 (16), 15 5.0 / 1.9 (16), 33 8.6 / 2.5 (16); [3, 400000], 17 6.2 / 5.0 (64). So are strides
+// that put a warp's lanes into few banks: [500, 200000], 16 356 / 310 (64), 32 555 / 284, and the largest: [100, 40000], 63 17.6 /
+// 10.2. Otherwise the first reads and writes in longer runs: [500, 200000], 17 241 / 323, 20 250 / 299; [22, 124801], 6 6.8 / 11.9.
 int spaceToDepth(const float* x, float* y, int64_t ci, int64_t l, int64_t rows, int64_t ly, int64_t xPitch, int64_t yPitch,
                  int64_t stride, int64_t pad, cudaStream_t s) {
-  const int threads = stride <= 32 ? kThreads : kThreads / 2;  // at most 32 KB of shared memory
-  const int64_t bx = ceilDiv(ly, threads), by = ci + rows - ci * stride;
-  spaceToDepthKernel<<<dim3(unsigned(bx < 512 ? bx : 512), unsigned(by < 65535 ? by : 65535)), threads,
-                       size_t(stride) * threads * 4, s>>>(x, y, ci, l, rows, ly, xPitch, yPitch, int(stride), pad);
+  const auto grid = [&](int64_t cols, int64_t most, int64_t blockRows) {
+    const int64_t bx = ceilDiv(ly, cols);
+    return dim3(unsigned(bx < most ? bx : most), unsigned(blockRows < 65535 ? blockRows : 65535));
+  };
+  const int64_t blockRows = ci + rows - ci * stride;
+  const bool few = ceilDiv(ly, kThreads) * ci < 296;  // two blocks per SM of a B200
+  if (stride == 1) {
+    spaceToDepthCopyKernel<<<grid(4 * kThreads, 4096, rows), kThreads, 0, s>>>(x, y, ci, l, rows, ly, xPitch, yPitch, pad);
+  } else if (stride < 8 || (stride <= 33 && !few && (stride < 16 || stride % 8 != 0))) {
+    const int threads = stride <= 32 ? kThreads : kThreads / 2;  // at most 32 KB of shared memory
+    spaceToDepthKernel<<<grid(threads, 512, blockRows), threads, size_t(stride) * threads * 4, s>>>(x, y, ci, l, rows, ly, xPitch,
+                                                                                                   yPitch, int(stride), pad);
+  } else {
+    int lc = 6;
+    while (lc > 4 && ceilDiv(ly, int64_t(1) << lc) * ci < 512) --lc;
+    const size_t n = size_t(stride) << lc;  // at most 4096 floats
+    spaceToDepthWideKernel<<<grid(int64_t(1) << lc, 4096, blockRows), kThreads, (n + n / 32) * 4, s>>>(x, y, ci, l, rows, ly, xPitch,
+                                                                                                      yPitch, int(stride), pad, lc);
+  }
   return launched("space_to_depth_f32_cuda");
 }
 }  // namespace lkc

@@ -754,6 +754,29 @@ def test_gemm_bias_sizes(cuda, m, k, n):
     assert np.abs(got - ref).max() <= 1e-4 and rel_l2(got, ref) <= 1e-6
 
 
+@pytest.mark.parametrize("ci,l,s,pad,taps,more", [(3, 700, 1, 0, 1, 13), (2, 701, 1, 5, 3, 0), (3, 3000, 15, 4, 2, 3),
+                                                  (3, 3001, 16, 0, 1, 0), (2, 5003, 32, 7, 2, 5), (1, 4100, 33, 32, 1, 0),
+                                                  (2, 64 * 300 + 9, 64, 63, 1, 70), (70, 64 * 600, 64, 0, 1, 0),
+                                                  (3, 200, 7, 3, 2, 1), (3, 200, 8, 9, 2, 1), (149, 2600, 10, 0, 1, 2),
+                                                  (148, 10239, 20, 1, 1, 0), (148, 10240, 24, 1, 1, 5), (5, 5000, 1, 0, 1, 2)])
+def test_space_to_depth_strides(cuda, ci, l, s, pad, taps, more):
+    """The three kernels and the edges of the rule between them, exactly: stride 1, few and many blocks, multiples of the 32 banks,
+    the largest stride; padding on both sides, zero rows."""
+    from lokinfer_b200 import ops
+    rows, x = ci * s + more, np.random.default_rng(l).standard_normal((ci, l)).astype(np.float32)
+    (dx,) = dev(cuda, x)
+    for padded in (False, True):
+        with ops.padded_rows(padded):
+            y = ops.space_to_depth_f32_cuda(dx, s, pad, taps, rows).cpu().numpy()
+        want = np.zeros((rows, y.shape[1]), np.float32)
+        for c in range(ci):
+            for r in range(s):
+                pos = s * np.arange(y.shape[1]) + r - pad
+                ok = (pos >= 0) & (pos < l)
+                want[c * s + r, ok] = x[c, pos[ok]]
+        np.testing.assert_array_equal(y, want)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("ci,co,l,k,s,p", [(22, 256, 1201, 12, 6, 3), (22, 128, 999, 1, 1, 0), (5, 32, 500, 6, 3, 2),
                                            (22, 256, 124801, 12, 6, 3)])
