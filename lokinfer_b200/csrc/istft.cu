@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(NTHREADS) istftKernel(const IstftArgs a) {
 }
 
 // The generator's own size, n_fft 20 and hop 5: a thread per frame keeps its spectrum in registers and takes the synthesis
-// table from the kernel's parameters (constant memory), so that the transform is 420 multiply-adds with constant operands and
+// table from the kernel's parameters (constant memory), so that the transform is 440 multiply-adds with constant operands and
 // nothing but the overlap-add goes through shared memory. A block computes N2 frames, N2 - 4 of which are its own (every output
 // sample overlaps four). Bound by its expf / sinf / sincosf. The form above builds the table in every block, in double, and
 // spends two shared-memory loads on each multiply-add: 42.5 us at T = 2080 and 14.7 us at T = 24.
@@ -161,7 +161,9 @@ const IstftTable& istft20Table() {
 
 // Checks of the caller done: shared-memory limit, launch.
 int istftLaunch(IstftArgs p, cudaStream_t s) {
-  if (p.nfft == NFFT2 && p.hop == HOP2) {
+  // A frame's 11 bins are one thread's chain there, which few frames do not hide: us general / this one at 2 frames 4.6 / 5.4, at 16
+  // 5.4 / 6.0, 32 6.4 / 6.5, 48 7.3 / 6.6, 128 12.7 / 7.5.
+  if (p.nfft == NFFT2 && p.hop == HOP2 && p.len > 32 * HOP2) {
     const int64_t blocks = ceilDiv(p.len, int64_t(OWN2) * HOP2);
     LKC_REQUIRE(blocks <= 0x7fffffff, "istft_logits_f32_cuda: grid too large");
     istft20Kernel<<<static_cast<unsigned>(blocks), N2, 0, s>>>(p, istft20Table());

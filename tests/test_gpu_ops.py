@@ -581,6 +581,12 @@ def test_istft_logits(cuda, l):
     assert rel_l2(y, ref32) <= REL_L2
 
 
+@pytest.mark.parametrize("l", [32, 33, 34, 126, 129])
+def test_istft_of_few_frames(cuda, l):
+    """Lengths around the one up to which the general kernel serves the generator's size, and one and two blocks of the other."""
+    test_istft_logits(cuda, l)
+
+
 def test_istft_other_sizes(cuda):
     from lokinfer_b200 import ops
     for n_fft, hop, l in ((16, 4, 100), (8, 2, 33), (126, 21, 40)):
