@@ -713,10 +713,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       return ok;
     }
   };
-  auto profAdd = [&](int slot, long long v) {
-    if (kProf && a.prof && lane == 0)
+  auto profAddIf = [&](bool mine, int slot, long long v) {  // one lane of a role adds the counts that it holds
+    if (kProf && a.prof && mine)
       atomicAdd(reinterpret_cast<unsigned long long*>(a.prof + slot), (unsigned long long)v);
   };
+  auto profAdd = [&](int slot, long long v) { profAddIf(lane == 0, slot, v); };
   // First timeout wins the low 16 bits; the flag bits above them are kept. One lane of a role reports; in the MMA issuer the
   // only lane that runs, whichever it is.
   auto giveUp = [&](int role, int code) {
@@ -1528,7 +1529,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       dependentsLaunch();  // this CTA's tensor work is queued; what follows it may set itself up under the tail
       __syncwarp();
-      if (kProf) profAdd(0, wBf), profAdd(1, wHe), profAdd(2, wWf), profAdd(3, wLe), profAdd(4, clock64() - tStart);
+      if (kProf)
+        profAddIf(leader, 0, wBf), profAddIf(leader, 1, wHe), profAddIf(leader, 2, wWf), profAddIf(leader, 3, wLe),
+            profAddIf(leader, 4, clock64() - tStart);
     }
   }
 
