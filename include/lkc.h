@@ -164,6 +164,9 @@ LKC_API void lkc_conv1d_state_destroy(LkcConvState* st);
  * 128-channel tile together, 0 = a CTA per tile. sms = SMs the launch may use; clusters[n], n = 2..8 = clusters of n CTAs
  * resident at a time on the device (9 entries; cudaOccupancyMaxActiveClusters). */
 LKC_API int lkc_conv1d_tc_split(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* clusters);
+/* The rule for the tile width of a conv with f16 halves that is not split and may leave chunk statistics per 32 columns (or none):
+ * 160, 192, 224 or 256 columns, for a launch on sm_percent of sms SMs (100: one that runs alone); 0 for bad arguments. */
+LKC_API int lkc_conv1d_tc_tile_cols(int64_t co, int64_t lo, int sms, int sm_percent);
 LKC_API int lkc_conv1d_tc_status(int* status, int reset);
 /* Stream-ordered form for callers that keep several utterances in flight: queues a 4-byte copy of the status word
  * into status_host (pinned host memory) behind the work already on `stream`; synchronises nothing, clears nothing. */

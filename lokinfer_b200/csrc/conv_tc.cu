@@ -1898,7 +1898,6 @@ int convTcSplitRule(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* 
   return splitFor(true, int(ci), lo, ceilDiv(co, MT), sms, clusters);
 }
 
-// Launch geometry and tensor maps shared by the conv and ConvTranspose entry points.
 // Columns per tile of the persistent form, for a launch that may spread over smPercent of the device's SMs.
 // Alone, the launch's time is the rounds of tiles that its busiest SM runs times a tile's time, which is about that of its
 // columns plus 48 more: a narrower tile pays where it takes fewer SM-columns in whole rounds.
@@ -1917,13 +1916,33 @@ static int tileColsFor(bool fineOk, int64_t lo, int64_t coBlocks, int sms, int s
   return best;
 }
 
-static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool canSplit, bool boxesOk, bool fineOk, int smPercent, int* grid, size_t* smem) {
+int convTcTileRule(int64_t co, int64_t lo, int sms, int smPercent) { return tileColsFor(true, lo, ceilDiv(co, MT), sms, smPercent); }
+
+// The form of a launch. Everybody who has to know it asks here: the launch itself, and the whole-model calls, which give split
+// convs chunk statistics and read the statistics of narrow tiles.
+struct TcForm {
+  int split, tileCols;
+};
+static TcForm formFor(const DeviceInfo& d, bool canSplit, bool fineOk, int64_t ci, int64_t lo, int64_t coBlocks, int smPercent) {
+  TcForm f;
+  f.split = splitFor(canSplit, int(ci), lo, coBlocks, d.smCount * smPercent / 100, d.clusters);
+  f.tileCols = f.split ? NTS : tileColsFor(fineOk, lo, coBlocks, d.smCount, smPercent);
+  return f;
+}
+static int formOf(const ConvFusedParams& p, bool f16, TcForm* f) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
-  a.split = splitFor(canSplit, a.ci, a.lo, a.numCoBlk, d->smCount * smPercent / 100, d->clusters);
+  *f = formFor(*d, splits(f16, p.k, p.act), f16 && (p.fineStats || !p.stats), p.ci, p.lo, ceilDiv(p.co, MT), p.smPercent);
+  return 0;
+}
+
+// Launch geometry and tensor maps shared by the conv and ConvTranspose entry points.
+static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk, int smPercent, int* grid, size_t* smem) {
+  const DeviceInfo* d = nullptr;
+  if (int rc = deviceInfo(&d)) return rc;
+  a.split = form.split, a.tileCols = form.tileCols;
   LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
   const int nt = a.split ? NTS : NT;  // staged columns of the first box
-  a.tileCols = a.split ? NTS : tileColsFor(f16 && fineOk, a.lo, a.numCoBlk, d->smCount, smPercent);
   if (a.stats && !a.split && a.tileCols != NT) a.nchunks = ceilDiv(a.lo, 32);
   a.numTTiles = int(ceilDiv(a.lo, a.tileCols));
   // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
@@ -1966,15 +1985,13 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, bool canSplit, bool boxesO
 }
 
 bool convTcSplits(const ConvFusedParams& p, bool f16) {
-  const DeviceInfo* d = nullptr;
-  return deviceInfo(&d) == 0 &&
-         splitFor(splits(f16, p.k, p.act), int(p.ci), p.lo, ceilDiv(p.co, MT), d->smCount * p.smPercent / 100, d->clusters) != 0;
+  TcForm f;
+  return formOf(p, f16, &f) == 0 && f.split != 0;
 }
 
 int convTcStatCols(const ConvFusedParams& p, bool f16) {
-  const DeviceInfo* d = nullptr;
-  if (!p.fineStats || deviceInfo(&d) != 0 || convTcSplits(p, f16)) return 128;
-  return tileColsFor(f16, p.lo, ceilDiv(p.co, MT), d->smCount, p.smPercent) == NT ? 128 : 32;
+  TcForm f;
+  return formOf(p, f16, &f) == 0 && !f.split && f.tileCols != NT ? 32 : 128;
 }
 
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {
@@ -1996,7 +2013,9 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
   a.numCoBlk = int(coBlk);
   int grid = 0;
   size_t smem = 0;
-  if (int rc = finishArgs(a, m, f16, splits(f16, p.k, p.act), true, p.fineStats || !p.stats, p.smPercent, &grid, &smem)) return rc;
+  TcForm form;
+  if (int rc = formOf(p, f16, &form)) return rc;
+  if (int rc = finishArgs(a, m, f16, form, true, p.smPercent, &grid, &smem)) return rc;
   switch (p.act) {
     case Act::None: return launchTc<0>(a, m, f16, grid, smem, s);
     case Act::Snake: return launchTc<1>(a, m, f16, grid, smem, s);
@@ -2051,7 +2070,10 @@ int convtTc(const ConvtParams& p, const float* wp, bool f16, cudaStream_t s) {
   a.numCoBlk = int(coBlk);
   int grid = 0;
   size_t smem = 0;
-  if (int rc = finishArgs(a, m, f16, f16, false, true, p.smPercent, &grid, &smem)) return rc;
+  const DeviceInfo* d = nullptr;
+  if (int rc = deviceInfo(&d)) return rc;
+  const TcForm form = formFor(*d, f16, f16, p.ci, p.l, coBlk, p.smPercent);
+  if (int rc = finishArgs(a, m, f16, form, false, p.smPercent, &grid, &smem)) return rc;
   if (p.stride == 6) return launchTc2<2, false, 6>(a, m, f16, grid, smem, s);
   return launchTc2<2, false, 10>(a, m, f16, grid, smem, s);
 }

@@ -1,4 +1,5 @@
-"""The rule that splits a conv's tiles over clusters of CTAs (host code): every cluster of a launch is resident at once."""
+"""The rules for the form of a conv launch (host code): how many CTAs share a tile, so that every cluster of the launch is resident
+at once, and how wide the tiles of the others are."""
 import ctypes
 
 import pytest
@@ -37,3 +38,32 @@ def test_lengths_around_the_limits():
     assert split(256, 256, 896) == 8 and split(256, 256, 897) == 6
     assert split(128, 128, 9472) == 2 and split(128, 128, 9473) == 0
     assert split(16, 16, 1) == 0 and split(100, 16, 1) == 0 and split(128, 128, 0) == 0
+
+
+def tile_cols(co, lo, percent=100, sms=SMS):
+    return _lib.lib().lkc_conv1d_tc_tile_cols(co, lo, sms, percent)
+
+
+@pytest.mark.parametrize("co", [22, 128, 256, 512])
+@pytest.mark.parametrize("percent", [26, 50, 99, 100])
+@pytest.mark.parametrize("sms", [SMS, 20])
+def test_tile_widths(co, percent, sms):
+    """Alone: no width takes fewer SM-columns in whole rounds (48 columns of cost beside a tile's own), the widest of equals. Beside
+    other launches: the narrowest that fits one round of the share, else whole tiles. Widths are multiples of the 32 columns that
+    the narrow tiles' statistics cover, so no pair spans two tiles."""
+    blocks, widths = -(-co // 128), (256, 224, 192, 160)
+    for lo in [*range(1, 3000, 97), *range(3001, 130000, 1009), 9472, 9473, 19201, 23680, 23681, 124801]:
+        w = tile_cols(co, lo, percent, sms)
+        tiles = {v: -(-lo // v) * blocks for v in widths}
+        cost = {v: -(-tiles[v] // sms) * (v + 48) for v in widths}
+        if percent == 100:
+            assert w == min(widths, key=lambda v: (cost[v], -v))
+        else:
+            fits = [v for v in widths[1:] if tiles[v] <= sms * percent // 100]
+            assert w == (min(fits) if fits else 256)
+    assert tile_cols(0, 100) == tile_cols(128, 0) == tile_cols(128, 100, 0) == tile_cols(128, 100, 100, 0) == 0
+
+
+def test_tile_widths_of_known_lengths():
+    assert tile_cols(128, 19201) == 160 and tile_cols(256, 12001) == 192  # 121 and 126 tiles on 148 SMs
+    assert tile_cols(128, 124801, 50) == 256 and tile_cols(128, 9601, 50) == 160  # 976 tiles of any width; 61 on 74 SMs
