@@ -3,7 +3,8 @@
 //   out[co, t] = sum_{ci, kk} W[co, ci, kk] * A[ci, t + kk d - pad],  A = act((x - mean) * scale + beta), zero outside
 //   [0, L); epilogue + bias [+ residual] [* oscale] and the per-(channel, 128-column chunk) (mean, M2).
 //
-// GEMM view: D[128 co, 256 t] += Wtap[128 co, 16 ci] * Ashift[16 ci, 256 t] for every 16-channel chunk and tap.
+// GEMM view: D[128 co, 256 t] += Wtap[128 co, 16 ci] * Ashift[16 ci, 256 t] for every 16-channel chunk and tap. Some launches
+// take narrower tiles (tileColsFor: 160, 192 or 224 columns; 128 in the split form).
 // f32 accuracy comes from splitting both operands, v = hi + lo with an 11-bit hi and an 11-bit lo:
 // out = sum Whi Ahi + (sum Wlo Ahi + Whi Alo); the lo*lo term, 2^-22 relative, is dropped. Two operand formats
 // (see Fmt below): f16 halves (default; 3 kind::f16 K16 MMAs per tap and 16 channels) or tf32 halves (6 kind::tf32
@@ -165,7 +166,7 @@ struct TcArgs {
   int tmaIn;       // 1: x rows are 16-byte aligned, the raw windows come by tiled TMA loads
   int tmaOut;      // 1: out (and residual) rows are 16-byte aligned, boxes go by TMA
   int numTTiles, numCoBlk;
-  int split;       // 0 = a persistent CTA per SM over 256-column tiles; else the CTAs that share one 128-column tile
+  int split;       // 0 = a persistent CTA per SM over tiles of tileCols columns; else the CTAs that share one 128-column tile
   int early;       // the launch may overlap the end of the one before it (programmatic dependent launch)
   int* status;
   long long* prof;  // null, or 16 cycle counters summed over CTAs (see convTcProfile)
@@ -1192,8 +1193,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     auto extRow = [&](uint32_t rb) { return NTK + (uint32_t(hf) == rb ? 0 : 32) + lane; };
 
     // Unaligned route: cp.async of this thread's part of the raw window of chunk c of the tile whose window starts at
-    // input position posT (= tile column * NT - padding) into staging buffer rb. Pointer increments only: this runs
-    // once per chunk on every producer thread. A thread copies what it will itself read back.
+    // input position posT (= tile * W - padding) into staging buffer rb. This runs once per chunk on every producer
+    // thread. A thread copies what it will itself read back.
     auto issueCopies = [&](int64_t posT, int c, int rb) {
       const float* xc = a.x + int64_t((cBegin + c) * KC + cg * 4) * a.xPitch + posT;
       float* const base = sRaw + rb * rawBufFloats;
@@ -1874,9 +1875,9 @@ int convTcProfile(int enable, long long* out16) {
 }
 
 // CTAs per tile: 0 = the persistent form. The split form is taken where at least two CTAs per 128-column tile fit on the
-// launch's share of the SMs and all its clusters are resident at a time (clusters[n], see countClusters): there the time is
-// one tile's chain of 16-channel chunks plus about 7 us of fixed cost (launch, first loads, exchange), and the
-// chain shrinks with every CTA. With one CTA per tile it gains little over 256-column tiles (an M128 N128 MMA takes about
+// launch's share of the SMs and all its clusters, by themselves, are resident at a time (clusters[n], see countClusters):
+// there the time is one tile's chain of 16-channel chunks plus about 7 us of fixed cost (launch, first loads, exchange), and
+// the chain shrinks with every CTA. With one CTA per tile it gains little over 256-column tiles (an M128 N128 MMA takes about
 // 0.8 of the time of an N256 one here) and doubles the weight traffic; with a second wave it loses: [128, 6144] K = 11,
 // 48 clusters of three where 45 fit, 36 us against 30 us unsplit and 21 us with two CTAs per tile.
 // Measured (us, persistent -> split): [256, 240] K = 11: 52 -> 15; [256, 1210] K = 7: 49 -> 17; [128, 1441] K = 3: 29 -> 12;
@@ -1975,7 +1976,8 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk,
   // A launch of one round starts as the SMs come free and sets itself up under the end of the one before it: 3 us of a split
   // launch's 14. CTAs that wait hold SMs that a ready launch of another stream could use, so beside other launches this is for
   // those of so few tiles that the launches beside them are split as well. us per forward, no launch early / every split one:
-  // T = 24 366 / 337, T = 80 528 / 513, T = 121 598 / 633, T = 320 934 / 992.
+  // T = 24 366 / 337, T = 80 528 / 513, T = 121 598 / 633, T = 320 934 / 992. A share of 100 % counts as alone, which the
+  // decoder's launches say as well, though its shortcuts run beside its main convs (see there).
   a.early = smPercent == 100 ? tiles <= d->smCount : a.split && tiles * 8 <= d->smCount;
   a.tmaOut = 0;
   if (boxesOk && a.co % MT == 0 && makeMap(&m.out, a.out, a.co, a.lo, a.outPitch, BOX, BOX, true) &&

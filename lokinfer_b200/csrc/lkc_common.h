@@ -83,7 +83,7 @@ struct ConvFusedParams {
   Act act = Act::None;
   float slope = 0.f, outScale = 1.f, inScale = 1.f;
   const void* state = nullptr;
-  int smPercent = 100;  // part of the device's SMs this launch may spread over (others run beside it)
+  int smPercent = 100;  // part of the device's SMs this launch may spread over (others run beside it); 100 is planned as alone
   // Instead of `affine`, where convFoldsAffine: chunk statistics [ci, ceil(l / 128), 2] of x and the (gamma | beta) of its
   // AdaIN; the conv computes the affine itself.
   const float *statsIn = nullptr, *gb = nullptr;
@@ -149,7 +149,8 @@ int addRows(const float* a, const float* b, float* out, int64_t n, cudaStream_t 
 int add3Scale(const float* a, const float* b, const float* c, float* out, int64_t n, float scale, cudaStream_t s);
 int spaceToDepth(const float* x, float* y, int64_t ci, int64_t l, int64_t rows, int64_t ly, int64_t xPitch, int64_t yPitch,
                  int64_t stride, int64_t pad, cudaStream_t s);
-// Decoder (decoder.cu): rows 512, 513 and up of a block input [512 + tail, l], see there.
+// Decoder (decoder.cu): the rows around the convs' results in both kinds of block input; AdaIN, leaky ReLU and the depthwise
+// pool of the upsampling block in one pass; nearest-neighbour upsampling by 2.
 int decoderInputs(const float* asr, int64_t asrPitch, const float* f0, const float* n, const float* f0w, const float* f0b,
                   const float* nw, const float* nb, float* enc, int64_t encRows, float* cat, int64_t catRow, int64_t catRows,
                   int64_t l, int64_t pitch, cudaStream_t s);

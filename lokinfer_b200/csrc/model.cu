@@ -1,7 +1,8 @@
-// Whole-model calls: the generator's forward and one AdaINResBlock1 as ONE call each (host code; every kernel it queues
-// is an entry point of this library). What they replace is the op-by-op composition in generator.py, whose 110 calls
-// through Python (argument checks, argument packing, one allocation per result, stream switches) took 5 ms of host time
-// per forward whatever its length, two to ten times what the GPU needs below 10 s of audio.
+// Whole-model calls: the generator's forward, the decoder's forward and one AdaINResBlock1 as ONE call each (host code; the
+// kernels it queues are those of this library's entry points, and three of the decoder's own). What they replace is the
+// op-by-op compositions in generator.py and decoder.py, whose 110 and 48 calls through Python (argument checks, argument
+// packing, one allocation per result, stream switches) took 5 and 1.7 ms of host time per forward whatever its length, two to
+// ten times what the GPU needs below 10 s of audio.
 //
 // A forward is written once as a sequence of alloc / use / join / launch steps over an Exec and runs in two modes. In
 // plan mode nothing is launched: every tensor's allocation and uses are recorded with the vector clock of the stream
@@ -22,7 +23,7 @@ namespace lkc {
 namespace {
 
 constexpr int kStreams = 5;  // the caller's stream and four side streams
-// Events of the joins, used in turn. A forward makes 14 joins: an event may be recorded again as soon as the wait on it has
+// Events of the joins, used in turn. A generator forward makes 17 joins, a decoder's 13: an event may be recorded again as soon as the wait on it has
 // been queued, which is the case when join() returns.
 constexpr int kEvents = 12;
 constexpr size_t kPlans = 16;
@@ -336,6 +337,12 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
 // between blocks, and the chunk statistics of the block's rows come from the epilogue that wrote them.
 constexpr int64_t kDecIn[2] = {528, 1104}, kDecCh = 1024, kDecOut = 512;
 constexpr float kDecSlope = 0.2f, kSqrtHalf = 0.7071067811865476f;
+// Percent of the SMs (see kBranchSms) of the main convs and of the shortcuts beside them. At 100 each launch is planned, and
+// started early, as if it ran alone; where two coincide, clusters wait for room, which costs less than fewer CTAs per tile.
+// us per forward at F = 61 / 160 / 400 / 600 / 1040: 100 and 100 238 / 286 / 378 / 463 / 618, without early starts 239 / 286 / 390 /
+// 474 / 630; 75 and 25 216 / 287 / 482 / 571 / 743; 100 and 30 210 / 285 / 460 / 509 / 746; 100 and 50 239 / 299 / 410 / 502 / 725.
+// (Up to F = 100 fewer SMs for the shortcuts would be the better choice.)
+constexpr int kDecSms = 100, kDecShortcutSms = 100;
 
 void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
   const int64_t f = io.frames;
@@ -357,7 +364,7 @@ void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
   e.join(0, 1);  // the style bank
   e.join(1, 0);  // the block inputs
   conv(e, 1, Act::None, enc, f, 512, 64, 1, 1, 0, m.asr_w, m.asr_b, none, nullptr, 0.f, m.asr_state, none,
-       from(cat, kDecCh * pitch), from(catStats, kDecCh * chunkFloats), 100);
+       from(cat, kDecCh * pitch), from(catStats, kDecCh * chunkFloats), kDecShortcutSms);
   e.launch(1, {cat, catStats}, [&](cudaStream_t st) {
     return channelStats(cat.p + (kDecCh + 64) * pitch, catStats.p + (kDecCh + 64) * chunkFloats, kDecIn[1] - kDecCh - 64, f,
                         pitch, statChunks(f), st);
@@ -372,6 +379,7 @@ void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
     p.ci = ci, p.l = l, p.co = co, p.k = 3, p.padding = 1, p.lo = l;
     p.xPitch = x.pitch, p.resPitch = residual.pitch, p.outPitch = out.pitch;
     p.act = Act::Leaky, p.slope = kDecSlope, p.state = state, p.outScale = residual.pitch ? kSqrtHalf : 1.f;
+    p.smPercent = kDecSms;
     const float* gb = bank.p + gbAt;
     if (e.running() && convFoldsAffine(p))
       p.statsIn = stats.p, p.gb = gb, p.eps = kEps;
@@ -386,7 +394,8 @@ void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
     const int64_t l = b.up ? 2 * f : f;
     Buf h = e.rows(0, b.cout, l), hStats = statsBuf(e, 0, b.cout, l), sc = e.rows(0, b.cout, f);
     e.join(1, 0);
-    conv(e, 1, Act::None, x, f, b.cin, b.cout, 1, 1, 0, b.w1x1, b.b1x1, none, nullptr, 0.f, b.state1x1, none, sc, none, 100);
+    conv(e, 1, Act::None, x, f, b.cin, b.cout, 1, 1, 0, b.w1x1, b.b1x1, none, nullptr, 0.f, b.state1x1, none, sc, none,
+         kDecShortcutSms);
     if (!b.up) {
       leakyConv(x, stats, f, b.cin, b.cout, b.w1, b.b1, b.state1, b.gb1, none, h, hStats);
       e.join(0, 1);
@@ -399,7 +408,7 @@ void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
       e.launch(0, {x, af, r}, [&](cudaStream_t st) {
         return adainLeakyPool(x.p, af.p, FP(b.pool_w), FP(b.pool_b), r.p, b.cin, f, x.pitch, r.pitch, kDecSlope, st);
       });
-      conv(e, 0, Act::None, r, l, b.cin, b.cout, 3, 1, 1, b.w1, b.b1, none, nullptr, 0.f, b.state1, none, h, hStats, 100);
+      conv(e, 0, Act::None, r, l, b.cin, b.cout, 3, 1, 1, b.w1, b.b1, none, nullptr, 0.f, b.state1, none, h, hStats, kDecSms);
       e.join(0, 1);
       Buf out;
       out.p = static_cast<float*>(io.out), out.pitch = io.out_pitch;

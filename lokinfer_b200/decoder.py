@@ -1,12 +1,12 @@
 """The decoder in front of the Kokoro generator, wired from `ops.*_cuda`: five AdainResBlk1d blocks that turn the
 aligned text features, the pitch curve and the energy curve into the generator's input x [512, 2F]
 (models/kokoro/model.py:158-221 the blocks, :704-717 the stack). Same op sequence as the reference's CPU graph, fused
-(stats -> adain_affine -> conv1d_leaky, :205-221) or basic (:158-174).
+(stats -> adain_affine -> conv1d_leaky, :205-221) or basic (:158-174). forward() is one library call that works on block
+inputs in place (lkc_decoder_forward); the composition from single ops, which concatenates them, stands behind it.
 
 Its convs have 514 / 1090 / 1024 input channels and kernel size 3. The tensor-core kernel stages 16 input channels at
-a time, so the two odd counts are padded here, once, when the weights are uploaded: the row concatenations that build
-the block inputs append zero rows up to the next multiple of 16 and the weights / AdaIN parameters get zero columns
-to match. A zero row has mean 0 and variance 0, its activation is the finite AdaIN bias, and it meets a zero weight:
+a time, so the two odd counts are padded: the block inputs get zero rows up to the next multiple of 16 and the weights /
+AdaIN parameters, once, when they are uploaded, zero columns to match. A zero row has mean 0 and variance 0, its activation is the finite AdaIN bias, and it meets a zero weight:
 the padding contributes exact zeros and every conv of the stack runs on tcgen05.
 """
 from __future__ import annotations
