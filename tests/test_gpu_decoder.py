@@ -98,17 +98,21 @@ def _args(cuda, frames, seed):
     return dev(cuda, inp["asr"], inp["f0"], inp["n"], inp["s"])
 
 
-@pytest.mark.parametrize("frames", [1, 2, 61, 64, 127, 129, 300, 1040])
+@pytest.mark.parametrize("frames", [1, 2, 3, 61, 64, 127, 129, 300, 1040])
 def test_whole_decoder_agrees_with_the_composition(cuda, dec, frames):
     """The whole call differs from the op-by-op form in who computes the statistics and in how partial sums are split, not
-    beyond rounding. One column: the variance is zero, what is left of it is rounding times 1 / sqrt(eps) (316), twice per
-    block."""
+    beyond rounding: within the 1e-5 of one op. Against float64 it is no further off than the composition is, within 1e-5 but at
+    two columns, where the variance of two samples in front of 1 / sqrt(var + eps) magnifies the rounding of both alike."""
     from lokinfer_b200 import ops
-    a = _args(cuda, frames, 30 + frames)
+    inp = synth.decoder_inputs(frames, 30 + frames)
+    a = dev(cuda, inp["asr"], inp["f0"], inp["n"], inp["s"])
     got, want = dec.forward(*a), _composed(dec, *a)
     assert got.shape == want.shape == (512, 2 * frames) and got.is_contiguous()
-    assert rel_l2(got.cpu().numpy(), want.cpu().numpy()) <= (10 if frames > 2 else 3160) * REL_L2
+    assert rel_l2(got.cpu().numpy(), want.cpu().numpy()) <= REL_L2
     assert torch.equal(got, dec.forward(*a)) and ops.conv_tc_status() == 0
+    r64 = O.decoder(synth.decoder_weights(0), *[O.T(inp[k], torch.float64) for k in ("asr", "f0", "n", "s")]).numpy()
+    err, err_ops = rel_l2(got.cpu().numpy(), r64), rel_l2(want.cpu().numpy(), r64)
+    assert err <= 1.2 * err_ops + 1e-7 and (err <= REL_L2 or frames == 2)
 
 
 def test_whole_decoder_takes_row_pitches_and_leaves_the_rest(cuda, dec):
@@ -134,28 +138,36 @@ def test_whole_decoder_takes_row_pitches_and_leaves_the_rest(cuda, dec):
     other.forward(*a)
     other.w["decoder.encode.conv2.bias"] = other.w["decoder.encode.conv2.bias"] + 1.0
     got, want2 = other.forward(*a), _composed(other, *a)
-    assert rel_l2(got.cpu().numpy(), want2.cpu().numpy()) <= 10 * REL_L2 and rel_l2(got.cpu().numpy(), want.cpu().numpy()) > 1e-3
+    assert rel_l2(got.cpu().numpy(), want2.cpu().numpy()) <= REL_L2 and rel_l2(got.cpu().numpy(), want.cpu().numpy()) > 1e-3
 
 
-def test_one_decoder_in_several_threads(cuda, dec):
+@pytest.mark.parametrize("cold", [False, True])
+def test_one_decoder_in_several_threads(cuda, dec, cold):
+    """cold: the threads are the decoder's first users."""
     import threading
+
+    from lokinfer_b200 import Decoder
     jobs = [_args(cuda, f, f) for f in (5, 61, 200)]
     want = [dec.forward(*j).clone() for j in jobs]
     torch.cuda.synchronize()
-    wrong = []
+    user = Decoder(synth.decoder_weights(0), cuda) if cold else dec
+    start, right, errors = threading.Barrier(3), [0, 0, 0], []
 
     def work(i):
-        with torch.cuda.stream(torch.cuda.Stream(device=cuda)):
-            for _ in range(10):
-                if not torch.equal(dec.forward(*jobs[i]), want[i]):
-                    wrong.append(i)
+        try:
+            with torch.cuda.stream(torch.cuda.Stream(device=cuda)):
+                start.wait(60)
+                for _ in range(10):
+                    right[i] += torch.equal(user.forward(*jobs[i]), want[i])
+        except Exception as e:  # a thread's exception would be lost
+            errors.append(repr(e))
 
     threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
     for t in threads:
         t.start()
     for t in threads:
         t.join()
-    assert not wrong
+    assert not errors and right == [10, 10, 10]
 
 
 def test_whole_decoder_in_a_graph(cuda, dec):
