@@ -45,9 +45,9 @@ from lokinfer_b200 import synth  # noqa: E402
 
 # DRAM traffic of one launch of the dominant conv shape (ncu capture, summary under profiles/); algorithmic bytes =
 # x + residual read, out written = 3 * 4 * C * L.
-TRAFFIC = {"bytes": 129688576 + 29296384, "algorithmic": 3 * 4 * 128 * 124801,
+TRAFFIC = {"bytes": 129583360 + 24412928, "algorithmic": 3 * 4 * 128 * 124801,
            "kernel": "convTcKernel, conv1d_snake_res, Ci = Co = 128, L = 124801, K = 11, dilation 5 (one launch)",
-           "source": "profiles/conv_tc_c128_k11_L124801.md"}
+           "source": "profiles/conv_tc_counters.md"}
 
 BATCH_STREAMS = 3  # utterance graphs of one GPU are replayed round-robin on this many streams (config 3)
 METRIC = "kokoro_generator_audio_seconds_per_second"
@@ -676,7 +676,8 @@ def run_batch(args, rank: int, local_rank: int, world: int):
 def run_sweep(args):
     """Conv kernel sweep (f32, batch 1): one fused conv1d_snake_res launch per step at each point, timed with CUDA
     events; prints one JSON line per point with achieved TFLOP/s (2 Co Ci K L / time) and the fraction of the
-    split-operand tensor roofline (measured bf16 peak / 3). --point Ci,Co,L,K,d runs a single point (used for ncu captures)."""
+    split-operand tensor roofline (measured bf16 peak / 3). --point Ci,Co,L,K,d[:Ci,Co,L,K,d...] runs these points alone (used
+    for ncu captures)."""
     from lokinfer_b200 import ops
 
     assert torch.cuda.is_available(), "bench.py needs a CUDA device (there is no CPU path)"
@@ -684,7 +685,7 @@ def run_sweep(args):
     pk = peaks()
     peak = pk["bf16_tflops"] / 3.0
     if args.point:
-        points = [tuple(int(v) for v in args.point.split(","))]
+        points = [tuple(int(v) for v in p.split(",")) for p in args.point.split(":")]
     else:
         points = [(c, c, l, k, d) for c in (128, 256, 512) for k in (3, 7, 11) for d in (1, 3, 5)
                   for l in (320, 3200, 19200, 124800)]
@@ -836,7 +837,7 @@ def main():
     ap.add_argument("--workload", default="single", choices=["single", "batch64"],
                     help="single: one utterance of --t frames per GPU (default, weak scaling); batch64: 64 utterances of "
                          "120..800 frames sharded across the GPUs (strong scaling)")
-    ap.add_argument("--point", default=None, help="single sweep point Ci,Co,L,K,dilation")
+    ap.add_argument("--point", default=None, help="sweep point Ci,Co,L,K,dilation (conv: several, joined by colons)")
     ap.add_argument("--plain-rows", action="store_true",
                     help="conv sweep: contiguous rows instead of rows padded to 16 bytes")
     args = ap.parse_args()
