@@ -430,12 +430,6 @@ __device__ __forceinline__ void regDec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-__device__ __forceinline__ float warpSum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // Second half of a split tile, one epilogue warp. The CTAs of the cluster own a run of its output channels each. Every CTA
 // copies the rows of its partial tile to their owners (send); the owner adds the partials in rank order out of its own shared
 // memory (finish). One bulk copy per pair of CTAs: loads or stores from one SM to another move about 11 bytes per clock
@@ -524,58 +518,73 @@ struct SplitTail {
       const int64_t tChunk = int64_t(tt) * NTS, col = tChunk + lane * 4;
       // valid columns of the tile, and from this lane's first on
       const int nValid = a.lo - tChunk < NTS ? int(a.lo - tChunk) : NTS, mine = nValid - lane * 4;
+      // The UB channels of a warp go side by side through the reductions, whose latency is what this phase lasts (one after the
+      // other: 2.1 us of a launch's 12 at four channels per warp).
 #pragma unroll 1
       for (int u0 = warp; u0 < units; u0 += UB * EPI_WARPS) {
         if (u0 != warp) prefetch(a, u0, lane);
-        float4 acc[UB];
-#pragma unroll
-        for (int e = 0; e < UB; ++e) acc[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float* at = parts + u0 * PART_PITCH + lane * 4;
-        if (mine > 0) {
-#pragma unroll 4
-          for (int r = 0; r < a.split; ++r, at += slot * PART_PITCH) {
-            float4 v[UB];
-#pragma unroll
-            for (int e = 0; e < UB; ++e)
-              if (u0 + e * EPI_WARPS < units) v[e] = *reinterpret_cast<const float4*>(at + e * EPI_WARPS * PART_PITCH);
-              else v[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int e = 0; e < UB; ++e) acc[e].x += v[e].x, acc[e].y += v[e].y, acc[e].z += v[e].z, acc[e].w += v[e].w;
-          }
-        }
-        __syncwarp();
+        float acc[UB][4];
+        bool ok[UB];  // this lane has columns of channel e
 #pragma unroll
         for (int e = 0; e < UB; ++e) {
-          const int u = u0 + e * EPI_WARPS, co = cb * MT + row0 + u;
-          if (u >= units || co >= a.co) continue;  // warp-uniform
-          float v[4] = {acc[e].x, acc[e].y, acc[e].z, acc[e].w};
+          ok[e] = u0 + e * EPI_WARPS < units && cb * MT + row0 + u0 + e * EPI_WARPS < a.co && mine > 0;
+          acc[e][0] = acc[e][1] = acc[e][2] = acc[e][3] = 0.f;
+        }
+        const float* at = parts + u0 * PART_PITCH + lane * 4;
+#pragma unroll 2
+        for (int r = 0; r < a.split; ++r, at += slot * PART_PITCH) {
+#pragma unroll
+          for (int e = 0; e < UB; ++e)
+            if (ok[e]) {
+              const float4 v = *reinterpret_cast<const float4*>(at + e * EPI_WARPS * PART_PITCH);
+              acc[e][0] += v.x, acc[e][1] += v.y, acc[e][2] += v.z, acc[e][3] += v.w;
+            }
+        }
+        __syncwarp();
+        float mean[UB], m2[UB];
+#pragma unroll
+        for (int e = 0; e < UB; ++e) {
           const float rs[4] = {res[e].x, res[e].y, res[e].z, res[e].w};
-          float sum = 0.f, m2 = 0.f;
+          mean[e] = 0.f, m2[e] = 0.f;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            v[j] += bias[e];
-            if (a.residual) v[j] = (v[j] + rs[j]) * a.outScale;
-            if (j < mine) sum += v[j];
+            acc[e][j] += bias[e];
+            if (a.residual) acc[e][j] = (acc[e][j] + rs[j]) * a.outScale;
+            if (j < mine) mean[e] += acc[e][j];
           }
-          float* op = a.out + int64_t(co) * a.outPitch + col;
-          if (vecOut && mine >= 4) {
-            *reinterpret_cast<float4*>(op) = make_float4(v[0], v[1], v[2], v[3]);
-          } else {
+          float* op = a.out + int64_t(cb * MT + row0 + u0 + e * EPI_WARPS) * a.outPitch + col;
+          if (ok[e]) {
+            if (vecOut && mine >= 4) {
+              *reinterpret_cast<float4*>(op) = make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
+            } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (j < mine) op[j] = v[j];
-          }
-          if (a.stats) {
-            const float mean = warpSum(sum) / float(nValid);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (j < mine) m2 = fmaf(v[j] - mean, v[j] - mean, m2);
-            m2 = warpSum(m2);
-            if (lane == 0) {
-              float* st = a.stats + (int64_t(co) * a.nchunks + tt) * 2;
-              st[0] = mean, st[1] = m2;
+              for (int j = 0; j < 4; ++j)
+                if (j < mine) op[j] = acc[e][j];
             }
           }
+        }
+        if (a.stats) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int e = 0; e < UB; ++e) mean[e] += __shfl_xor_sync(0xffffffffu, mean[e], o);
+#pragma unroll
+          for (int e = 0; e < UB; ++e) {
+            mean[e] /= float(nValid);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (j < mine) m2[e] = fmaf(acc[e][j] - mean[e], acc[e][j] - mean[e], m2[e]);
+          }
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int e = 0; e < UB; ++e) m2[e] += __shfl_xor_sync(0xffffffffu, m2[e], o);
+#pragma unroll
+          for (int e = 0; e < UB; ++e)
+            if (lane == 0 && ok[e]) {
+              float* st = a.stats + (int64_t(cb * MT + row0 + u0 + e * EPI_WARPS) * a.nchunks + tt) * 2;
+              st[0] = mean[e], st[1] = m2[e];
+            }
         }
       }
     } else {
@@ -732,8 +741,53 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
   };
 
+  // Split form with statsIn: each CTA folds the chunk statistics of the channels it contracts into their AdaIN affine (sPar, see
+  // the producers). A launch of its own costs 3.5 us plus a gap in front of every conv; here it is one round of loads under the
+  // first weight and input copies, eight lanes per channel on the sixteen warps that have nothing to do yet. In double and
+  // relative to the row's first mean, so that one pass over the pairs gives mean and variance as adainAffineKernel's two do.
+  // (Two passes on the eight producer warps, four lanes per channel: 1.6-1.9 us from the predecessor's end to the constants.)
+  const bool fold = SPLIT && ACT != 0 && TS == 0 && a.statsIn != nullptr;
+  if (fold && warp < EPI_WARPS + PRO_WARPS) {
+    dependenciesWait();
+    constexpr int R = 4;  // pairs per lane in flight
+    const int cEnd = (cBegin + nChunks16) * KC, sub = lane & 7, nch = int((a.l + NTS - 1) / NTS);
+    const double nT = double(NTS), nLast = double(a.l - int64_t(nch - 1) * NTS), invL = 1.0 / double(a.l);
+#pragma unroll 1
+    for (int c0 = cBegin * KC + warp * 4; c0 < cEnd; c0 += (EPI_WARPS + PRO_WARPS) * 4) {  // warp-uniform; KC is a multiple of 4
+      const int c = c0 + (lane >> 3);
+      const float2* const st = reinterpret_cast<const float2*>(a.statsIn) + int64_t(c) * nch;  // 8-byte aligned, as adain_affine wants
+      const float gamma = a.gb[c], beta = a.gb[a.ci + c], al = ACT == 1 ? a.alpha[c] : 1.f;
+      const double first = double(st[0].x);
+      double s1 = 0.0, s2 = 0.0;  // sum of (x - first), sum of (x - first)^2
+#pragma unroll 1
+      for (int t0 = sub; t0 < nch; t0 += 8 * R) {
+        float2 v[R];
+#pragma unroll
+        for (int e = 0; e < R; ++e) v[e] = t0 + 8 * e < nch ? st[t0 + 8 * e] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int e = 0; e < R; ++e) {
+          const int t = t0 + 8 * e;
+          const double cols = t + 1 < nch ? nT : t < nch ? nLast : 0.0, d = double(v[e].x) - first;
+          s1 += cols * d, s2 += double(v[e].y) + cols * d * d;
+        }
+      }
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) s1 += __shfl_xor_sync(0xffffffffu, s1, o), s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      if (sub == 0) {
+        const double dm = s1 * invL, v = s2 * invL - dm * dm;
+        const float var = v < 0.0 ? 0.f : float(v);  // (a NaN stays one)
+        sPar[c] = -float(first + dm);
+        sPar[a.ci + c] = (1.f + gamma) * (1.0f / sqrtf(var + a.eps)) * al;
+        sPar[2 * a.ci + c] = beta * al;
+        sPar[3 * a.ci + c] = 1.f / al;
+      }
+      __syncwarp();
+    }
+  }
+
   if (warp < EPI_WARPS) {
     // ------------------------------------------------------------------ accumulate + epilogue
+    if (fold) asm volatile("bar.arrive 1, %0;" ::"n"((EPI_WARPS + PRO_WARPS) * 32) : "memory");  // the producers wait for this part
     regInc<EPI_REGS>();
     dependenciesWait();
     const int q = warp & 3, g = warp >> 2;  // TMEM lane quarter, half of the tile
@@ -1144,42 +1198,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const int mainRows = NARROW ? a.mainRows : NTK, halfRows = mainRows / 2, slots = mainRows / 64;
     const bool tmaIn = a.tmaIn != 0;
     // per-channel parameters, once: sPar = [-mean | a | b | inv] with a = scale, b = beta (x alpha for Snake), inv = 1/alpha
-    // Split form with statsIn: each CTA folds the chunk statistics of its own channels into mean / scale / beta, with the
-    // arithmetic of adainAffineKernel (Chan combine in double), four lanes per channel. A launch of its own costs
-    // 3.5 us plus a gap in front of every conv; here it is one round of loads under the first weight and input copies.
-    const bool fold = SPLIT && a.statsIn != nullptr;
-    if constexpr (SPLIT) {
-      if (fold) {
-        const int64_t nch = (a.l + 127) / 128;
-        const double nT = 128.0, nLast = double(a.l - (nch - 1) * 128);
-        const int cEnd = (cBegin + nChunks16) * KC, sub = lane & 3;
-        for (int c0 = cBegin * KC + pw * 8; c0 < cEnd; c0 += PRO_WARPS * 8) {  // warp-uniform; KC is a multiple of 8
-          const int c = c0 + (lane >> 2);
-          const float2* st = reinterpret_cast<const float2*>(a.statsIn) + int64_t(c) * nch;  // 8-byte aligned, as adain_affine wants
-          double sum = 0.0, m2 = 0.0;
-#pragma unroll 4
-          for (int64_t t = sub; t < nch; t += 4) sum += double(st[t].x) * (t + 1 < nch ? nT : nLast);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-          sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-          const double mean = sum / double(a.l);
-#pragma unroll 4
-          for (int64_t t = sub; t < nch; t += 4) {
-            const float2 v = st[t];
-            const double dm = double(v.x) - mean;
-            m2 += double(v.y) + (t + 1 < nch ? nT : nLast) * dm * dm;
-          }
-          m2 += __shfl_xor_sync(0xffffffffu, m2, 1);
-          m2 += __shfl_xor_sync(0xffffffffu, m2, 2);
-          if (sub == 0) {
-            const float var = float(m2 / double(a.l)), al = ACT == 1 ? a.alpha[c] : 1.f;
-            sPar[c] = -float(mean);
-            sPar[a.ci + c] = (1.f + a.gb[c]) * (1.0f / sqrtf(var + a.eps)) * al;
-            sPar[2 * a.ci + c] = a.gb[a.ci + c] * al;
-            sPar[3 * a.ci + c] = 1.f / al;
-          }
-        }
-      }
-    }
     for (int c = cBegin * KC + pw * 32 + lane; !fold && c < (cBegin + nChunks16) * KC; c += PRO_WARPS * 32) {
       const float al = ACT == 1 ? a.alpha[c] : 1.f;
       sPar[c] = a.affine ? -a.affine[c] : 0.f;
@@ -1187,7 +1205,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       sPar[2 * a.ci + c] = (a.affine ? a.affine[2 * a.ci + c] : 0.f) * al;
       sPar[3 * a.ci + c] = 1.f / al;
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(PRO_WARPS * 32) : "memory");  // producer warps only
+    if (fold) asm volatile("bar.sync 1, %0;" ::"n"((EPI_WARPS + PRO_WARPS) * 32) : "memory");
+    else asm volatile("bar.sync 1, %0;" ::"n"(PRO_WARPS * 32) : "memory");  // producer warps only
 
     // First row beyond the tile's columns that this lane stages from raw buffer rb.
     auto extRow = [&](uint32_t rb) { return NTK + (uint32_t(hf) == rb ? 0 : 32) + lane; };

@@ -433,3 +433,26 @@ def test_whole_resblock_at_other_tile_widths(cuda, gen, stage, l, k):
     assert rel_l2(out[:, -256:].cpu().numpy(), want[:, -256:].cpu().numpy()) <= 6 * REL_L2
     assert rel_l2(st.cpu().numpy(), want_st.cpu().numpy()) <= 6 * REL_L2
     assert torch.equal(out, gen.adain_resblock1_fused(x, gb, prefix, k)[0]) and ops.conv_tc_status() == 0
+
+
+@pytest.mark.parametrize("l", [1, 2, 127, 128, 129, 1024, 1025, 4097, 9000])
+@pytest.mark.parametrize("stage", [0, 1])
+def test_whole_resblock_with_few_tiles(cuda, gen, stage, l):
+    """Lengths whose convs are split among CTAs, which fold the statistics (1 to 71 pairs per channel) themselves: against the
+    op-by-op form with its adain_affine, within the rounding of six convs in a row. Rows far from zero, and constant ones."""
+    from lokinfer_b200 import ops
+    r = torch.Generator(device=cuda).manual_seed(l)
+    c = (256, 128)[stage]
+    x = torch.randn(c, l, generator=r, device=cuda)
+    x[::5] += 300.0
+    x[::7] = -1234.5
+    gb = gen.style(torch.randn(128, generator=r, device=cuda))
+    prefix = f"resblocks.{3 * stage + 1}"
+    out, st = gen.adain_resblock1_fused(x, gb, prefix, 7)
+    with ops.use_allocator(lambda shape, device: torch.empty(shape, dtype=torch.float32, device=device)):
+        want, want_st = gen.adain_resblock1_fused(x, gb, prefix, 7)
+    d, live = out - x, [i for i in range(c) if i % 5 and i % 7]  # what the block adds; on the big rows x's own rounding hides it
+    assert rel_l2(d[live].cpu().numpy(), (want - x)[live].cpu().numpy()) <= 6 * REL_L2
+    assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 6 * REL_L2
+    assert rel_l2(st[..., 0].cpu().numpy(), want_st[..., 0].cpu().numpy()) <= 6 * REL_L2
+    assert torch.equal(out, gen.adain_resblock1_fused(x, gb, prefix, 7)[0]) and ops.conv_tc_status() == 0
