@@ -65,6 +65,7 @@ namespace {
 constexpr bool kProf = LKC_TC_PROF != 0;
 constexpr int NT = 256;         // time columns per tile (= UMMA N)
 constexpr int NTS = 128;        // time columns per tile of the split form: one statistics chunk
+constexpr int NTS2 = 64;        // the same for rows of no more columns
 constexpr int MT = 128;         // output channels per tile (= UMMA M)
 constexpr int KC = 16;          // input channels per staged chunk (one weight stage, two K8 steps)
 constexpr int MAX_NB = 4;       // most activation (hi / lo) buffers
@@ -103,10 +104,13 @@ constexpr int STAGE_PITCH = 33;  // floats per row of an epilogue transpose tile
 constexpr int STAGE_FLOATS = 32 * STAGE_PITCH;
 constexpr int BOX = 32, BOX_BYTES = BOX * BOX * 4;  // residual / output boxes of the aligned route: 32 co x 32 t
 static_assert(BOX_BYTES <= STAGE_FLOATS * 4, "a swizzled box fits in a warp's tile");
-constexpr int PART_PITCH = NTS + 4;  // floats per row of a split tile's partial: rows 16-byte aligned, 4 banks apart
+// Floats per row of a split tile's partial: rows 16-byte aligned, 4 banks apart.
+__host__ __device__ constexpr int partPitch(int cols) { return cols + 4; }
 // A split tile's memory behind its MMAs, over the operand buffers: this CTA's partial tile, then the rows that the CTAs of the
 // cluster send it. Those are at most split * (rows a CTA owns, rounded up; 2 channels of 10 rows and a gap of 2 over 8 CTAs).
-constexpr int PART_ROWS = 176, PART_BYTES = MT * PART_PITCH * 4, RECV_BYTES = PART_ROWS * PART_PITCH * 4;
+constexpr int PART_ROWS = 176;
+__host__ __device__ constexpr int partBytes(int cols) { return MT * partPitch(cols) * 4; }
+__host__ __device__ constexpr int recvBytes(int cols) { return PART_ROWS * partPitch(cols) * 4; }
 constexpr size_t SPLIT_SMEM = 120 * 1024;  // more than half an SM's: one CTA per SM, for whose TMEM two would compete
 constexpr int MAX_SPLIT = 8;     // CTAs of a split tile (the portable cluster size)
 static_assert(MAX_SPLIT <= EPI_WARPS, "an epilogue warp per receiver");
@@ -130,14 +134,15 @@ constexpr int kMaxSmem = 232448;  // 227 KB per CTA on sm_100
 struct SmemLayout {
   uint32_t act, raw, w, par, bar, total;
 };
-__host__ __device__ inline SmemLayout smemLayout(bool split, int ci, int rows, int ext, int nb, int wStages, int wG,
+// split: columns of a split tile, or 0.
+__host__ __device__ inline SmemLayout smemLayout(int split, int ci, int rows, int ext, int nb, int wStages, int wG,
                                                  int actRowBytes, int wStageBytes) {
   SmemLayout s;
   s.act = split ? 0 : EPI_WARPS * STAGE_FLOATS * 4;  // tiles: [0, act)
   s.raw = (s.act + uint32_t(nb) * actRowBytes * rows + 127u) & ~127u;
-  s.w = s.raw + uint32_t(NRAW) * KC * ((split ? NTS : NT) + ext) * 4;  // a multiple of 128
+  s.w = s.raw + uint32_t(NRAW) * KC * ((split ? split : NT) + ext) * 4;  // a multiple of 128
   s.par = s.w + uint32_t(wStages) * wG * wStageBytes;
-  if (split && s.par < uint32_t(PART_BYTES + RECV_BYTES)) s.par = PART_BYTES + RECV_BYTES;
+  if (split && s.par < uint32_t(partBytes(split) + recvBytes(split))) s.par = partBytes(split) + recvBytes(split);
   s.bar = s.par + uint32_t(4) * ci * 4;
   s.total = s.bar + 512;
   return s;
@@ -155,10 +160,10 @@ struct TcArgs {
   int padLeft;       // ConvTranspose: 1 = one-sample left reflect pad
   float slope, outScale;
   int delta;       // columns between the 16-byte boundary a tile's window is loaded from and its first column (0: 4-byte route)
-  int tileCols;    // time columns per tile: NTS split, else 160 .. NT in steps of 32 (see tileColsFor)
-  int mainRows;    // staged rows that every lane has a slot for: the window up to NT (split: NTS) rows, a multiple of 64
+  int tileCols;    // time columns per tile: NTS or NTS2 split, else 160 .. NT in steps of 32 (see tileColsFor)
+  int mainRows;    // staged rows that every lane has a slot for: the window up to NT (split: tileCols) rows, a multiple of 64
   int rows;        // staged time rows per buffer: at least tileCols + (k-1)*dilation + delta and mainRows
-  int ext;         // raw staging: [16][NT or NTS], then [16][ext] with the rows beyond them (two TMA boxes)
+  int ext;         // raw staging: [16][NT, split: tileCols], then [16][ext] with the rows beyond them (two TMA boxes)
   int wStages;     // weight ring depth (slots)
   int nb;          // activation buffers
   int wG;          // taps per weight slot: the k taps of a chunk go in ceil(k / wG) groups of near-equal size
@@ -166,7 +171,7 @@ struct TcArgs {
   int tmaIn;       // 1: x rows are 16-byte aligned, the raw windows come by tiled TMA loads
   int tmaOut;      // 1: out (and residual) rows are 16-byte aligned, boxes go by TMA
   int numTTiles, numCoBlk;
-  int split;       // 0 = a persistent CTA per SM over tiles of tileCols columns; else the CTAs that share one 128-column tile
+  int split;       // 0 = a persistent CTA per SM over tiles of tileCols columns; else the CTAs that share one such tile
   int early;       // the launch may overlap the end of the one before it (programmatic dependent launch)
   int* status;
   long long* prof;  // null, or 16 cycle counters summed over CTAs (see convTcProfile)
@@ -434,12 +439,15 @@ __device__ __forceinline__ void regDec() {
 // copies the rows of its partial tile to their owners (send); the owner adds the partials in rank order out of its own shared
 // memory (finish). One bulk copy per pair of CTAs: loads or stores from one SM to another move about 11 bytes per clock
 // (5-7 k clocks for the 56 KB of a CTA).
-// conv: a unit is one output channel of the tile, four columns per lane; the rank's 128 / split channels go round robin
-// over the epilogue warps, UB at a time so that their loads overlap. What does not depend on the contraction (bias,
+// conv: a unit is one output channel of the tile, four columns per lane (a warp has two at a time where the tile has 64); the
+// rank's 128 / split channels go round robin over the epilogue warps, UB at a time so that their loads overlap. What does not depend on the contraction (bias,
 // residual) is loaded by prefetch(), for the first UB units before the accumulation.
 // ConvTranspose: a unit is one output channel x 32 input-rate columns, whose 32 * TS output samples are one run.
-template <int TS>
+template <int TS, int COLS>
 struct SplitTail {
+  static_assert(TS == 0 || COLS == NTS, "ConvTranspose: 128 columns");
+  static constexpr int PART_PITCH = partPitch(COLS);
+  static constexpr int LPC = COLS / 4, STEP = EPI_WARPS * 32 / LPC;  // lanes per channel, channels that the epilogue warps have at a time
   static constexpr int UB = 4;
   float4 res[UB];
   float bias[UB];
@@ -472,13 +480,14 @@ struct SplitTail {
     }
   }
 
+  // u0: the first channel (of the rank's) of this lane
   __device__ __forceinline__ void prefetch(const TcArgs& a, int u0, int lane) {
     if constexpr (TS == 0) {
       const bool vecRes = a.residual && ((reinterpret_cast<uintptr_t>(a.residual) | uintptr_t(a.resPitch * 4)) & 15) == 0;
-      const int64_t col = int64_t(tt) * NTS + lane * 4;
+      const int64_t col = int64_t(tt) * COLS + lane % LPC * 4;
 #pragma unroll
       for (int e = 0; e < UB; ++e) {
-        const int u = u0 + e * EPI_WARPS, co = cb * MT + row0 + u;
+        const int u = u0 + e * STEP, co = cb * MT + row0 + u;
         res[e] = make_float4(0.f, 0.f, 0.f, 0.f), bias[e] = 0.f;
         if (u < units && co < a.co) {
           if (a.bias) bias[e] = a.bias[co];
@@ -512,31 +521,35 @@ struct SplitTail {
     return uint32_t(a.split * (last - first) * PART_PITCH * 4);
   }
 
+  static __device__ __forceinline__ int firstUnit(int warp, int lane) { return warp * (32 / LPC) + lane / LPC; }
+
   __device__ __forceinline__ void finish(const TcArgs& a, const float* parts, int warp, int lane) {
     if constexpr (TS == 0) {
       const bool vecOut = ((reinterpret_cast<uintptr_t>(a.out) | uintptr_t(a.outPitch * 4)) & 15) == 0;
-      const int64_t tChunk = int64_t(tt) * NTS, col = tChunk + lane * 4;
+      const int sub = lane % LPC;
+      const int64_t tChunk = int64_t(tt) * COLS, col = tChunk + sub * 4;
       // valid columns of the tile, and from this lane's first on
-      const int nValid = a.lo - tChunk < NTS ? int(a.lo - tChunk) : NTS, mine = nValid - lane * 4;
+      const int nValid = a.lo - tChunk < COLS ? int(a.lo - tChunk) : COLS, mine = nValid - sub * 4;
       // The UB channels of a warp go side by side through the reductions, whose latency is what this phase lasts (one after the
       // other: 2.1 us of a launch's 12 at four channels per warp).
 #pragma unroll 1
-      for (int u0 = warp; u0 < units; u0 += UB * EPI_WARPS) {
-        if (u0 != warp) prefetch(a, u0, lane);
+      for (int base = firstUnit(warp, 0); base < units; base += UB * STEP) {  // warp-uniform
+        const int u0 = base + lane / LPC;
+        if (base != firstUnit(warp, 0)) prefetch(a, u0, lane);
         float acc[UB][4];
         bool ok[UB];  // this lane has columns of channel e
 #pragma unroll
         for (int e = 0; e < UB; ++e) {
-          ok[e] = u0 + e * EPI_WARPS < units && cb * MT + row0 + u0 + e * EPI_WARPS < a.co && mine > 0;
+          ok[e] = u0 + e * STEP < units && cb * MT + row0 + u0 + e * STEP < a.co && mine > 0;
           acc[e][0] = acc[e][1] = acc[e][2] = acc[e][3] = 0.f;
         }
-        const float* at = parts + u0 * PART_PITCH + lane * 4;
+        const float* at = parts + u0 * PART_PITCH + sub * 4;
 #pragma unroll 2
         for (int r = 0; r < a.split; ++r, at += slot * PART_PITCH) {
 #pragma unroll
           for (int e = 0; e < UB; ++e)
             if (ok[e]) {
-              const float4 v = *reinterpret_cast<const float4*>(at + e * EPI_WARPS * PART_PITCH);
+              const float4 v = *reinterpret_cast<const float4*>(at + e * STEP * PART_PITCH);
               acc[e][0] += v.x, acc[e][1] += v.y, acc[e][2] += v.z, acc[e][3] += v.w;
             }
         }
@@ -552,7 +565,7 @@ struct SplitTail {
             if (a.residual) acc[e][j] = (acc[e][j] + rs[j]) * a.outScale;
             if (j < mine) mean[e] += acc[e][j];
           }
-          float* op = a.out + int64_t(cb * MT + row0 + u0 + e * EPI_WARPS) * a.outPitch + col;
+          float* op = a.out + int64_t(cb * MT + row0 + u0 + e * STEP) * a.outPitch + col;
           if (ok[e]) {
             if (vecOut && mine >= 4) {
               *reinterpret_cast<float4*>(op) = make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
@@ -565,7 +578,7 @@ struct SplitTail {
         }
         if (a.stats) {
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1)
+          for (int o = LPC / 2; o > 0; o >>= 1)
 #pragma unroll
             for (int e = 0; e < UB; ++e) mean[e] += __shfl_xor_sync(0xffffffffu, mean[e], o);
 #pragma unroll
@@ -576,13 +589,13 @@ struct SplitTail {
               if (j < mine) m2[e] = fmaf(acc[e][j] - mean[e], acc[e][j] - mean[e], m2[e]);
           }
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1)
+          for (int o = LPC / 2; o > 0; o >>= 1)
 #pragma unroll
             for (int e = 0; e < UB; ++e) m2[e] += __shfl_xor_sync(0xffffffffu, m2[e], o);
 #pragma unroll
           for (int e = 0; e < UB; ++e)
-            if (lane == 0 && ok[e]) {
-              float* st = a.stats + (int64_t(cb * MT + row0 + u0 + e * EPI_WARPS) * a.nchunks + tt) * 2;
+            if (sub == 0 && ok[e]) {
+              float* st = a.stats + (int64_t(cb * MT + row0 + u0 + e * STEP) * a.nchunks + tt) * 2;
               st[0] = mean[e], st[1] = m2[e];
             }
         }
@@ -627,18 +640,19 @@ struct SplitTail {
 // PARTIAL: Co is not a multiple of 128 (the last output-channel block has rows that do not exist).
 // TS: 0 = conv1d; 6 / 10 = polyphase ConvTranspose1d of that stride (see the comment above convtTcPackKernel).
 // TMAO: residual and output boxes travel by TMA (rows 16-byte aligned; conv1d with Co % 128 == 0 only).
-// SPLIT: a cluster of a.split CTAs shares one 128-column tile. Each CTA contracts its own run of input-channel chunks. When
+// SPLIT (columns of the tile, or 0): a cluster of a.split CTAs shares one tile of 128 or 64 columns. Each CTA contracts its own run of input-channel chunks. When
 // the MMAs of all of them are done (a cluster barrier under the last drain) it sends the rows of its partial tile to the CTAs
 // that own them, over the operand buffers there, which nothing reads any more; when it has all of its own it finishes them:
 // the partials are added in rank order, then bias, residual, scale, statistics and coalesced stores. For launches with fewer
 // tiles than SMs, where one tile's serial chain of chunks is the launch's time (see splitFor).
 // NARROW: tiles of a.tileCols < NT columns. A form of its own: the width as a run-time value cost 256-column tiles 5 % (K = 7).
-template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT, bool NARROW>
+template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, int SPLIT, bool NARROW>
 __global__ void __launch_bounds__(NTHREADS, 1)
     convTcKernel(const TcArgs a, const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapExt,
                  const __grid_constant__ CUtensorMap mapRes, const __grid_constant__ CUtensorMap mapOut) {
   constexpr int W_STAGE_BYTES = Fmt<F16>::W_STAGE_BYTES, W_STAGE_FLOATS = Fmt<F16>::W_STAGE_FLOATS;
-  constexpr int NTK = SPLIT ? NTS : NT;  // time columns of this kernel's tiles
+  constexpr int NTK = SPLIT ? SPLIT : NT;  // time columns of this kernel's tiles
+  constexpr int PART_PITCH = partPitch(NTK);
   constexpr int EC = NTK / 2;            // columns of one epilogue warp
   // Dhi buffers: a 128-column tile leaves room for two, so that the hi MMAs of a drain group need not wait for the drain
   // of the one before (the lo MMAs that cover it are shorter here)
@@ -746,7 +760,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // first weight and input copies, eight lanes per channel on the sixteen warps that have nothing to do yet. In double and
   // relative to the row's first mean, so that one pass over the pairs gives mean and variance as adainAffineKernel's two do.
   // (Two passes on the eight producer warps, four lanes per channel: 1.6-1.9 us from the predecessor's end to the constants.)
-  const bool fold = SPLIT && ACT != 0 && TS == 0 && a.statsIn != nullptr;
+  const bool fold = SPLIT != 0 && ACT != 0 && TS == 0 && a.statsIn != nullptr;
   if (fold && warp < EPI_WARPS + PRO_WARPS) {
     dependenciesWait();
     constexpr int R = 4;  // pairs per lane in flight
@@ -804,10 +818,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     constexpr uint32_t kSleepEpi = SPLIT ? SLEEP_EPI_SPLIT_NS : SLEEP_EPI_NS;
     uint32_t groupIt = 0, tileIt = 0, resIt = 0;
     bool dead = false, resInFlight = false, arrived = false;
-    SplitTail<TS> tail(a, tile0, rank);
-    float* const recv = sStage + PART_BYTES / 4;
+    SplitTail<TS, SPLIT ? SPLIT : NTS> tail(a, tile0, rank);
+    float* const recv = sStage + partBytes(NTK) / 4;
     if (SPLIT && threadIdx.x == 0) mbarArriveExpectTx(recvBar, tail.expected(a, rank));
-    if constexpr (SPLIT) tail.prefetch(a, warp, lane);
+    if constexpr (SPLIT != 0) tail.prefetch(a, tail.firstUnit(warp, lane), lane);
     long long wHi = 0, wLo = 0, cPre = 0, cFin = 0;
     const long long tStart = kProf ? clock64() : 0;
     for (int t = tile0; t < numTiles && !dead; t += tileStep, ++tileIt) {
@@ -1001,7 +1015,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       if (dead) break;
       const long long tFin = kProf ? clock64() : 0;
-      if constexpr (SPLIT) {
+      if constexpr (SPLIT != 0) {
         float* const row = sStage + (q * 32 + lane) * PART_PITCH + gcol;
 #pragma unroll
         for (int j = 0; j < EC; j += 4) *reinterpret_cast<float4*>(row + j) = make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
@@ -1171,7 +1185,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       if (kProf) cFin += clock64() - tFin;
     }
-    if constexpr (SPLIT) {
+    if constexpr (SPLIT != 0) {
       if (dead) {  // the arrival that the peers wait for
         if (!arrived) clusterArrive(), clusterWait();
       } else if (!mbarWait(recvBar, 0, abortFlag, 0)) {
@@ -1558,7 +1572,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
 
   tcFenceBefore();
-  if constexpr (SPLIT) {
+  if constexpr (SPLIT != 0) {
     if (warp >= EPI_WARPS) clusterArrive(), clusterWait();  // the epilogue warps' part of the first barrier is in their branch
     clusterArrive(), clusterWait();                         // no CTA leaves before what it sent has arrived
   }
@@ -1654,11 +1668,11 @@ static int rawExt(int rows, int cols) { return rows <= cols ? 0 : (rows - cols +
 
 // Dynamic shared memory of one CTA and the weight ring it leaves room for: the largest taps-per-slot (<= TAP_GROUP)
 // that still gives PREF_W_STAGES slots, else the deepest ring. Returns 0 when even single-tap slots do not fit.
-static size_t convTcSmemBytes(bool split, int64_t ci, int rows, int k, bool f16, int* wStages, int* wG) {
+static size_t convTcSmemBytes(int split, int64_t ci, int rows, int k, bool f16, int* wStages, int* wG) {
   const int tap = f16 ? Fmt<true>::W_STAGE_BYTES : Fmt<false>::W_STAGE_BYTES;
   const int actRow = f16 ? Fmt<true>::ACT_BYTES_PER_ROW : Fmt<false>::ACT_BYTES_PER_ROW;
   const int nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
-  const int ext = rawExt(rows, split ? NTS : NT);
+  const int ext = rawExt(rows, split ? split : NT);
   SmemLayout base = smemLayout(split, int(ci), rows, ext, nb, 0, 0, actRow, tap);
   base.total -= base.par - base.w;  // without the split form's memory behind the MMAs, which the ring may lie in
   if (base.total > uint32_t(kMaxSmem)) return 0;
@@ -1693,7 +1707,7 @@ bool convTcEligible(const ConvFusedParams& p, bool f16) {
         chainOk(p.k, f16) && (p.k - 1) * p.dilation <= MAX_HALO && p.lo >= 1 && p.padding <= (1 << 20) && p.ci <= 4096 &&
         p.l < (int64_t(1) << 30)))
     return false;
-  return convTcSmemBytes(false, p.ci, NT + int((p.k - 1) * p.dilation), int(p.k), false, nullptr, nullptr) != 0;  // the larger format
+  return convTcSmemBytes(0, p.ci, NT + int((p.k - 1) * p.dilation), int(p.k), false, nullptr, nullptr) != 0;  // the larger format
 }
 
 int64_t convTcPackFloats(int64_t co, int64_t ci, int64_t k, bool f16) {
@@ -1710,7 +1724,7 @@ struct DeviceInfo {
 // A cluster lives inside one GPC, of whose SMs a remainder is left over: 148 SMs hold 74 clusters of two, but 45 of three,
 // 33 of four, 26 of five, 22 of six, 15 of seven or eight (one B200; which SMs are fused off differs).
 static void countClusters(DeviceInfo& d) {
-  const auto kernel = convTcKernel<1, false, 0, true, false, true, false>;
+  const auto kernel = convTcKernel<1, false, 0, true, false, NTS, false>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) {
     cudaGetLastError();
     return;  // no split launches
@@ -1812,7 +1826,7 @@ struct TcMaps {
   CUtensorMap x, ext, res, out;
 };
 
-template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT, bool NARROW>
+template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, int SPLIT, bool NARROW>
 static int launchTc5(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cudaStream_t s) {
   static bool configured[64] = {};
   int dev = 0;
@@ -1843,9 +1857,9 @@ static int launchTc5(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cu
   return launched("conv (tensor-core)");
 }
 
-template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, bool SPLIT>
+template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, int SPLIT>
 static int launchTc4(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cudaStream_t s) {
-  if constexpr (F16 && !SPLIT) {
+  if constexpr (F16 && SPLIT == 0) {
     if (a.tileCols < NT) return launchTc5<ACT, PARTIAL, TS, F16, TMAO, SPLIT, true>(a, m, grid, smem, s);
   }
   return launchTc5<ACT, PARTIAL, TS, F16, TMAO, SPLIT, false>(a, m, grid, smem, s);
@@ -1854,12 +1868,15 @@ static int launchTc4(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cu
 template <int ACT, bool PARTIAL, int TS, bool F16>
 static int launchTc3(const TcArgs& a, const TcMaps& m, int grid, size_t smem, cudaStream_t s) {
   if constexpr (F16 || (ACT == 0 && TS == 0)) {  // the second half of a split tile handles every Co and alignment
-    if (a.split) return launchTc4<ACT, false, TS, F16, false, true>(a, m, grid, smem, s);
+    if constexpr (TS == 0) {
+      if (a.split && a.tileCols == NTS2) return launchTc4<ACT, false, TS, F16, false, NTS2>(a, m, grid, smem, s);
+    }
+    if (a.split) return launchTc4<ACT, false, TS, F16, false, NTS>(a, m, grid, smem, s);
   }
   if constexpr (TS == 0 && !PARTIAL) {
-    if (a.tmaOut) return launchTc4<ACT, PARTIAL, TS, F16, true, false>(a, m, grid, smem, s);
+    if (a.tmaOut) return launchTc4<ACT, PARTIAL, TS, F16, true, 0>(a, m, grid, smem, s);
   }
-  return launchTc4<ACT, PARTIAL, TS, F16, false, false>(a, m, grid, smem, s);
+  return launchTc4<ACT, PARTIAL, TS, F16, false, 0>(a, m, grid, smem, s);
 }
 
 template <int ACT, bool PARTIAL, int TS = 0>
@@ -1943,16 +1960,19 @@ int convTcTileRule(int64_t co, int64_t lo, int sms, int smPercent) { return tile
 struct TcForm {
   int split, tileCols;
 };
-static TcForm formFor(const DeviceInfo& d, bool canSplit, bool fineOk, int64_t ci, int64_t lo, int64_t coBlocks, int smPercent) {
+// A split tile of a row of up to 64 columns is cut to 64: half of its MMA time, partial tile, exchange and output are padding
+// otherwise. The decoder at F = 61: 244 -> 211 us. Tiles of 64 for longer rows lose more to their number (fewer CTAs per tile, each
+// reading more weights) than their shorter exchange gives: T = 24 320 -> 352, F = 100 244 -> 254.
+static TcForm formFor(const DeviceInfo& d, bool canSplit, bool fineOk, bool conv, int64_t ci, int64_t lo, int64_t coBlocks, int smPercent) {
   TcForm f;
   f.split = splitFor(canSplit, int(ci), lo, coBlocks, d.smCount * smPercent / 100, d.clusters);
-  f.tileCols = f.split ? NTS : tileColsFor(fineOk, lo, coBlocks, d.smCount, smPercent);
+  f.tileCols = f.split ? (conv && lo <= NTS2 ? NTS2 : NTS) : tileColsFor(fineOk, lo, coBlocks, d.smCount, smPercent);
   return f;
 }
 static int formOf(const ConvFusedParams& p, bool f16, TcForm* f) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
-  *f = formFor(*d, splits(f16, p.k, p.act), f16 && (p.fineStats || !p.stats), p.ci, p.lo, ceilDiv(p.co, MT), p.smPercent);
+  *f = formFor(*d, splits(f16, p.k, p.act), f16 && (p.fineStats || !p.stats), true, p.ci, p.lo, ceilDiv(p.co, MT), p.smPercent);
   return 0;
 }
 
@@ -1962,7 +1982,7 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk,
   if (int rc = deviceInfo(&d)) return rc;
   a.split = form.split, a.tileCols = form.tileCols;
   LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
-  const int nt = a.split ? NTS : NT;  // staged columns of the first box
+  const int nt = a.split ? a.tileCols : NT;  // staged columns of the first box
   if (a.stats && !a.split && a.tileCols != NT) a.nchunks = ceilDiv(a.lo, 32);
   a.numTTiles = int(ceilDiv(a.lo, a.tileCols));
   // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
@@ -1975,7 +1995,7 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk,
     a.mainRows = std::min(nt, (need + 63) & ~63);
     a.rows = std::max(need, a.mainRows);
     a.ext = rawExt(a.rows, nt);
-    *smem = convTcSmemBytes(a.split != 0, a.ci, a.rows, a.k, f16, &a.wStages, &a.wG);
+    *smem = convTcSmemBytes(a.split ? nt : 0, a.ci, a.rows, a.k, f16, &a.wStages, &a.wG);
   };
   layOut();
   if (*smem == 0 && a.tmaIn) a.tmaIn = 0, layOut();  // no room for the rows in front of the window: the 4-byte route has none
@@ -2049,7 +2069,7 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
 
 bool convtTcEligible(int64_t ci, int64_t co, int64_t k, int64_t stride, int64_t padding) {
   return (stride == 6 || stride == 10) && k == 2 * stride && 2 * padding == stride && ci % KC == 0 && ci >= KC &&
-         ci <= 4096 && co >= 1 && convTcSmemBytes(false, ci, NT + 2, 3, false, nullptr, nullptr) != 0;
+         ci <= 4096 && co >= 1 && convTcSmemBytes(0, ci, NT + 2, 3, false, nullptr, nullptr) != 0;
 }
 
 int64_t convtTcPackFloats(int64_t ci, int64_t co, int64_t stride, bool f16) {
@@ -2093,7 +2113,7 @@ int convtTc(const ConvtParams& p, const float* wp, bool f16, cudaStream_t s) {
   size_t smem = 0;
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
-  const TcForm form = formFor(*d, f16, f16, p.ci, p.l, coBlk, p.smPercent);
+  const TcForm form = formFor(*d, f16, f16, false, p.ci, p.l, coBlk, p.smPercent);
   if (int rc = finishArgs(a, m, f16, form, false, p.smPercent, &grid, &smem)) return rc;
   if (p.stride == 6) return launchTc2<2, false, 6>(a, m, f16, grid, smem, s);
   return launchTc2<2, false, 10>(a, m, f16, grid, smem, s);

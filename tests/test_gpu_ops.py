@@ -187,6 +187,24 @@ def test_conv1d_few_tiles_other_activations(cuda, ci, co, l, k, d, variant):
     assert ops.conv_tc_status() == 0
 
 
+# Rows of up to 64 columns take tiles of 64: the widths around that and around the 32 columns of an epilogue warp and of a slot of
+# staged rows, windows of 28 to 50 columns more, shares of one channel and of a whole tile's channels, a row of four columns.
+FEW_COLUMNS = [(48, 129, 64, 3, 1), (80, 128, 65, 5, 2), (112, 256, 63, 7, 1), (32, 128, 33, 11, 5), (48, 128, 32, 8, 4),
+               (1104, 64, 61, 3, 1), (128, 128, 4, 7, 5), (64, 22, 31, 9, 6), (528, 256, 64, 1, 1)]
+
+
+@pytest.mark.parametrize("ci,co,l,k,d", FEW_COLUMNS)
+@pytest.mark.parametrize("padded", [False, True])
+def test_conv1d_few_columns(cuda, ci, co, l, k, d, padded):
+    test_conv1d_few_tiles(cuda, ci, co, l, k, d, padded)
+
+
+@pytest.mark.parametrize("ci,co,l,k,d", [(80, 128, 64, 5, 2), (48, 129, 33, 7, 5), (128, 128, 61, 11, 1)])
+@pytest.mark.parametrize("variant", ["snake", "snake_res", "affine"])
+def test_conv1d_few_columns_other_activations(cuda, ci, co, l, k, d, variant):
+    test_conv1d_few_tiles_other_activations(cuda, ci, co, l, k, d, variant)
+
+
 @pytest.mark.parametrize("ci,l,cut,k,d", [(128, 1201, 640, 3, 1), (256, 1000, 384, 11, 5), (48, 700, 128, 7, 3)])
 def test_conv1d_few_tiles_window(cuda, ci, l, cut, k, d):
     """A row in two parts as the time-sharded path holds it: each part a window with real columns of its neighbour beside
