@@ -338,14 +338,23 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
 constexpr int64_t kDecIn[2] = {528, 1104}, kDecCh = 1024, kDecOut = 512;
 constexpr float kDecSlope = 0.2f, kSqrtHalf = 0.7071067811865476f;
 // Percent of the SMs (see kBranchSms) of the main convs and of the shortcuts beside them. At 100 each launch is planned, and
-// started early, as if it ran alone; where two coincide, clusters wait for room, which costs less than fewer CTAs per tile.
-// us per forward at F = 61 / 160 / 400 / 600 / 1040: 100 and 100 238 / 286 / 378 / 463 / 618, without early starts 239 / 286 / 390 /
-// 474 / 630; 75 and 25 216 / 287 / 482 / 571 / 743; 100 and 30 210 / 285 / 460 / 509 / 746; 100 and 50 239 / 299 / 410 / 502 / 725.
-// (Up to F = 100 fewer SMs for the shortcuts would be the better choice.)
-constexpr int kDecSms = 100, kDecShortcutSms = 100;
+// started early, as if it ran alone; where two coincide, clusters wait for room, which for long inputs costs less than fewer CTAs
+// per tile. Short ones have few clusters of many CTAs, of which the device holds few (15 of seven or eight): up to 384 frames the
+// shares are such that the clusters of both fit. us per forward as a graph at F = 61 / 100 / 160 / 300 / 400 / 600, 100 and 100: 215 /
+// 242 / 280 / 332 / 367 / 446; 65 and 35: 194 / 209 / 307 / 316 / 486 / 531; 60 and 40: 219 / 246 / 264 / 344 / 507 / 533; 100 and 30: 194 /
+// 212 / 282 at F = 61 / 100 / 160.
+struct DecSms {
+  int main, shortcut;
+};
+DecSms decSms(int64_t frames) {
+  static const DecSms few[] = {{65, 35}, {60, 40}, {65, 35}};  // by the 128-column tiles of a row
+  const int64_t tiles = ceilDiv(frames, 128);
+  return tiles <= 3 ? few[tiles - 1] : DecSms{100, 100};
+}
 
 void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
   const int64_t f = io.frames;
+  const DecSms sms = decSms(f);
   const Buf none;
   auto from = [](Buf b, int64_t floats) {  // the same buffer from an offset on
     if (b.p) b.p += floats;
@@ -364,7 +373,7 @@ void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
   e.join(0, 1);  // the style bank
   e.join(1, 0);  // the block inputs
   conv(e, 1, Act::None, enc, f, 512, 64, 1, 1, 0, m.asr_w, m.asr_b, none, nullptr, 0.f, m.asr_state, none,
-       from(cat, kDecCh * pitch), from(catStats, kDecCh * chunkFloats), kDecShortcutSms);
+       from(cat, kDecCh * pitch), from(catStats, kDecCh * chunkFloats), sms.shortcut);
   e.launch(1, {cat, catStats}, [&](cudaStream_t st) {
     return channelStats(cat.p + (kDecCh + 64) * pitch, catStats.p + (kDecCh + 64) * chunkFloats, kDecIn[1] - kDecCh - 64, f,
                         pitch, statChunks(f), st);
@@ -379,7 +388,7 @@ void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
     p.ci = ci, p.l = l, p.co = co, p.k = 3, p.padding = 1, p.lo = l;
     p.xPitch = x.pitch, p.resPitch = residual.pitch, p.outPitch = out.pitch;
     p.act = Act::Leaky, p.slope = kDecSlope, p.state = state, p.outScale = residual.pitch ? kSqrtHalf : 1.f;
-    p.smPercent = kDecSms;
+    p.smPercent = sms.main;
     const float* gb = bank.p + gbAt;
     if (e.running() && convFoldsAffine(p))
       p.statsIn = stats.p, p.gb = gb, p.eps = kEps;
@@ -395,7 +404,7 @@ void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
     Buf h = e.rows(0, b.cout, l), hStats = statsBuf(e, 0, b.cout, l), sc = e.rows(0, b.cout, f);
     e.join(1, 0);
     conv(e, 1, Act::None, x, f, b.cin, b.cout, 1, 1, 0, b.w1x1, b.b1x1, none, nullptr, 0.f, b.state1x1, none, sc, none,
-         kDecShortcutSms);
+         sms.shortcut);
     if (!b.up) {
       leakyConv(x, stats, f, b.cin, b.cout, b.w1, b.b1, b.state1, b.gb1, none, h, hStats);
       e.join(0, 1);
@@ -408,7 +417,7 @@ void decoder(Exec& e, const LkcDecoder& m, const LkcDecoderIo& io) {
       e.launch(0, {x, af, r}, [&](cudaStream_t st) {
         return adainLeakyPool(x.p, af.p, FP(b.pool_w), FP(b.pool_b), r.p, b.cin, f, x.pitch, r.pitch, kDecSlope, st);
       });
-      conv(e, 0, Act::None, r, l, b.cin, b.cout, 3, 1, 1, b.w1, b.b1, none, nullptr, 0.f, b.state1, none, h, hStats, kDecSms);
+      conv(e, 0, Act::None, r, l, b.cin, b.cout, 3, 1, 1, b.w1, b.b1, none, nullptr, 0.f, b.state1, none, h, hStats, sms.main);
       e.join(0, 1);
       Buf out;
       out.p = static_cast<float*>(io.out), out.pitch = io.out_pitch;

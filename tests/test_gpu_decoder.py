@@ -115,6 +115,12 @@ def test_whole_decoder_agrees_with_the_composition(cuda, dec, frames):
     assert err <= 1.2 * err_ops + 1e-7 and (err <= REL_L2 or frames == 2)
 
 
+@pytest.mark.parametrize("frames", [32, 33, 65, 128, 256, 257, 384, 385])
+def test_whole_decoder_at_other_tile_counts(cuda, dec, frames):
+    """The lengths where the width of the tiles and the shares of the SMs change."""
+    test_whole_decoder_agrees_with_the_composition(cuda, dec, frames)
+
+
 def test_whole_decoder_takes_row_pitches_and_leaves_the_rest(cuda, dec):
     """A view of wider rows, a stream of the caller's, replaced weights; operands that the call cannot take by their
     addresses go op by op or are refused as before."""
