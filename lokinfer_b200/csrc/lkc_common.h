@@ -143,7 +143,7 @@ int convTcProfile(int enable, long long* out16);
 // the caller. Row pitches in floats.
 int channelStats(const float* x, float* stats, int64_t c, int64_t l, int64_t pitch, int64_t statsStride, cudaStream_t s);
 int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s, int statCols = 128,
-                bool alone = false);  // alone: nothing runs beside it, so it and what follows it may start early
+                bool early = false);  // it may start, and let what follows it start, before what it waits for has ended
 int gemmBias(const float* x, const float* wt, const float* b, float* out, int64_t m, int64_t k, int64_t n, cudaStream_t s);
 int addRows(const float* a, const float* b, float* out, int64_t n, cudaStream_t s);
 int add3Scale(const float* a, const float* b, const float* c, float* out, int64_t n, float scale, cudaStream_t s);

@@ -185,7 +185,7 @@ int adainConv(Exec& e, int s, Buf x, Buf stats, int statCols, int64_t l, int64_t
   if (e.running() && statCols == 128 && convFoldsAffine(p))
     p.statsIn = stats.p, p.gb = gb, p.eps = kEps;
   else
-    e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, c, l, kEps, st, statCols, smPercent == 100); });
+    e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, c, l, kEps, st, statCols, true); });
   e.launch(s, {x, stats, bank, af, residual, out, outStats}, [&](cudaStream_t st) { return convFused(p, st); });
   return e.running() ? convStatCols(p) : 128;
 }
