@@ -456,3 +456,14 @@ def test_whole_resblock_with_few_tiles(cuda, gen, stage, l):
     assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 6 * REL_L2
     assert rel_l2(st[..., 0].cpu().numpy(), want_st[..., 0].cpu().numpy()) <= 6 * REL_L2
     assert torch.equal(out, gen.adain_resblock1_fused(x, gb, prefix, 7)[0]) and ops.conv_tc_status() == 0
+
+
+def test_synthesize_reports_the_status_once(cuda, gen):
+    """An activation beyond the f16 range raises from the call that met it; the next call is clean and right."""
+    from lokinfer_b200 import ops
+    inp, _ = _inputs(cuda, 24)
+    x, har, s = (torch.from_numpy(inp[k]).pin_memory() for k in ("x", "har", "s"))
+    want = gen.synthesize(x, har, s).clone()
+    with pytest.raises(RuntimeError, match="0x10000"):
+        gen.synthesize(x * 1e9, har, s)
+    assert torch.equal(gen.synthesize(x, har, s), want) and ops.conv_tc_status() == 0
