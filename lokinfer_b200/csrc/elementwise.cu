@@ -150,11 +150,11 @@ __global__ void channelStatsKernel(const float* __restrict__ x, float* __restric
 // One 128-thread block per channel: exact combine of the (count, mean, M2) partials in double, two passes. The
 // chunk partials of a channel are read once into registers (up to 8 per thread; longer rows loop), so both passes
 // cost one round of memory latency.
+// Its inputs are not __restrict__: an early launch reads what the one in front of it may still be writing, and loads of read-only
+// data could be moved in front of the wait.
 constexpr int kAffineThreads = 128;
-__global__ void __launch_bounds__(kAffineThreads) adainAffineKernel(const float* __restrict__ stats,
-                                                                    const float* __restrict__ gb,
-                                                                    float* __restrict__ affine, int64_t c, int64_t l,
-                                                                    int64_t nchunks, int statCols, float eps, int early) {
+__global__ void __launch_bounds__(kAffineThreads) adainAffineKernel(const float* stats, const float* gb, float* affine, int64_t c,
+                                                                    int64_t l, int64_t nchunks, int statCols, float eps, int early) {
   if (early) dependentsLaunch();
   dependenciesWait();
   __shared__ double red[kAffineThreads / 32];
