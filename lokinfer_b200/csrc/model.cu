@@ -35,8 +35,10 @@ constexpr float kEps = 1e-5f;  // AdaIN
 // the second. us per forward of T = 24 / 80 / 121 / 200 / 320 frames, [stage 0 | stage 1 | noise]: 26, 36, 70 | 26, 36, 50 | 70,
 // 40: 337 / 513 / 598 / 757 / 934; 33 each, noise 50: 352 / 517 / 581 / 751 / 877; k = 11 at 90 in stage 0: 336 / 624 / 717 /
 // 759 / 935; as below 333 / 511 / 597 / 705 / 878 (T = 320 gains where stage 0 of k = 11 takes whole tiles instead of halves,
-// T = 200 from the second noise branch). No splitting at all, with an earlier build: 877 at T = 24, 934 at 121.
-constexpr int kBranchSms[2][3] = {{26, 36, 60}, {26, 36, 50}}, kNoiseSms[2] = {60, 50};
+// T = 200 from the second noise branch). No splitting at all, with an earlier build: 877 at T = 24, 934 at 121. Stage 0 of k = 3 and 7
+// at 40 (their tiles are split up to T = 160, where at 26 and 36 a whole tile's chain was the branch's time), T = 24 / 80 / 121 / 160 /
+// 200 / 320 / 500 as a graph: 325 / 498 / 587 / 720 / 707 / 869 / 1090 -> 327 / 502 / 554 / 665 / 704 / 868 / 1073.
+constexpr int kBranchSms[2][3] = {{40, 40, 60}, {26, 36, 50}}, kNoiseSms[2] = {60, 50};
 
 // Channels of the two stages, of what goes into their upsamplers, and the upsampling factors.
 constexpr int64_t kCh[2] = {256, 128}, kChIn[2] = {512, 256}, kUp[2] = {10, 6};
