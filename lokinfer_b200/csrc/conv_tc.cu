@@ -4,7 +4,7 @@
 //   [0, L); epilogue + bias [+ residual] [* oscale] and the per-(channel, 128-column chunk) (mean, M2).
 //
 // GEMM view: D[128 co, 256 t] += Wtap[128 co, 16 ci] * Ashift[16 ci, 256 t] for every 16-channel chunk and tap. Some launches
-// take narrower tiles (tileColsFor: 160, 192 or 224 columns; 128 in the split form).
+// take narrower tiles (tileColsFor: 160, 192 or 224 columns; 128 or 64 in the split form).
 // f32 accuracy comes from splitting both operands, v = hi + lo with an 11-bit hi and an 11-bit lo:
 // out = sum Whi Ahi + (sum Wlo Ahi + Whi Alo); the lo*lo term, 2^-22 relative, is dropped. Two operand formats
 // (see Fmt below): f16 halves (default; 3 kind::f16 K16 MMAs per tap and 16 channels) or tf32 halves (6 kind::tf32
@@ -41,7 +41,7 @@
 //   warp 18     raw-window loader of the aligned route (one lane): two tiled TMA loads per chunk, one chunk ahead
 //   warp 19     idle (completes the fifth warpgroup)
 // Launches with few tiles take a second form of the same kernel (template parameter SPLIT): a cluster of CTAs per
-// 128-column tile, each contracting a part of the input channels, reduced over distributed shared memory.
+// 128- or 64-column tile, each contracting a part of the input channels, reduced over distributed shared memory.
 // All hand-offs are mbarriers. Every wait is bounded: on a timeout the kernel records a status word, drains its
 // copies in flight and returns (TMEM is freed on every path).
 #include <cuda.h>
