@@ -357,6 +357,10 @@ typedef struct LkcModel LkcModel;
  * one handle may come from several threads. */
 LKC_API LkcModel* lkc_generator_create(const LkcGenerator* w);
 LKC_API void lkc_model_destroy(LkcModel* m);
+/* The rule for the percent of `sms` SMs that the convs of one resblock of a forward of t frames may spread over, as the other
+ * branches run beside them (host code): stage 0 or 1, branch 0, 1, 2 for k = 3, 7, 11; clusters as in lkc_conv1d_tc_split.
+ * 0 for bad arguments. */
+LKC_API int lkc_generator_branch_sms(int64_t t, int stage, int branch, int sms, const int32_t* clusters);
 LKC_API int lkc_generator_workspace(LkcModel* m, int64_t t, int concurrent, int64_t* bytes, int64_t* unplanned);
 LKC_API int lkc_generator_forward(LkcModel* m, LkcGeneratorIo* io, void* stream);
 /* The decoder's forward as one call, under the same rules; the handle of one model is refused by the calls of the other. */

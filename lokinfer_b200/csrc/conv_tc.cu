@@ -1935,6 +1935,13 @@ int convTcSplitRule(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* 
   return splitFor(true, int(ci), lo, ceilDiv(co, MT), sms, clusters);
 }
 
+int convTcDevice(int* sms, const int32_t** clusters) {
+  const DeviceInfo* d = nullptr;
+  if (int rc = deviceInfo(&d)) return rc;
+  *sms = d->smCount, *clusters = d->clusters;
+  return 0;
+}
+
 // Columns per tile of the persistent form, for a launch that may spread over smPercent of the device's SMs.
 // Alone, the launch's time is the rounds of tiles that its busiest SM runs times a tile's time, which is about that of its
 // columns plus 48 more: a narrower tile pays where it takes fewer SM-columns in whole rounds.

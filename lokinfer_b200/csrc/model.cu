@@ -34,14 +34,28 @@ constexpr float kEps = 1e-5f;  // AdaIN
 // when others end. The longer a branch's chain, the more it gets; the first noise branch is waited for one stage earlier than
 // the second. us per forward of T = 24 / 80 / 121 / 200 / 320 frames, [stage 0 | stage 1 | noise]: 26, 36, 70 | 26, 36, 50 | 70,
 // 40: 337 / 513 / 598 / 757 / 934; 33 each, noise 50: 352 / 517 / 581 / 751 / 877; k = 11 at 90 in stage 0: 336 / 624 / 717 /
-// 759 / 935; as below 333 / 511 / 597 / 705 / 878 (T = 320 gains where stage 0 of k = 11 takes whole tiles instead of halves,
-// T = 200 from the second noise branch). No splitting at all, with an earlier build: 877 at T = 24, 934 at 121. Stage 0 of k = 3 and 7
-// at 40 (their tiles are split up to T = 160, where at 26 and 36 a whole tile's chain was the branch's time), T = 24 / 80 / 121 / 160 /
-// 200 / 320 / 500 as a graph: 325 / 498 / 587 / 720 / 707 / 869 / 1090 -> 327 / 502 / 554 / 665 / 704 / 868 / 1073.
-constexpr int kBranchSms[2][3] = {{40, 40, 60}, {26, 36, 50}}, kNoiseSms[2] = {60, 50};
+// 759 / 935; 26, 36, 60 | 26, 36, 50 | 60, 50: 333 / 511 / 597 / 705 / 878 (T = 320 gains where stage 0 of k = 11 takes whole
+// tiles instead of halves, T = 200 from the second noise branch). No splitting at all, with an earlier build: 877 at T = 24, 934
+// at 121.
+// A resblock whose tiles its share leaves whole gets the other share, with which more lengths are split: a whole tile's chain
+// of 16 channel chunks is then the branch's time. As a graph, T = 72 / 80 / 90 / 100 / 110 / 121 / 140 / 160 / 320 / 640: 26 and 36 for k = 3
+// and 7 of stage 0 at every length 468 / 490 / 502 / 504 / 517 / 584 / 602 / 691 / 866 / 1349; 40 for both, which up to T = 115 only adds
+// CTAs to tiles that have two or three, 462 / 499 / 518 / 520 / 533 / 550 / 573 / 662 / 869 / 1338; as below 469 / 490 / 498 / 505 / 512 / 550 /
+// 564 / 662 / 866 / 1331.
+struct Share {
+  int split, whole;
+};
+constexpr Share kBranchSms[2][3] = {{{26, 40}, {36, 40}, {60, 60}}, {{26, 26}, {36, 36}, {50, 50}}};
+constexpr int kNoiseSms[2] = {60, 50};
 
 // Channels of the two stages, of what goes into their upsamplers, and the upsampling factors.
 constexpr int64_t kCh[2] = {256, 128}, kChIn[2] = {512, 256}, kUp[2] = {10, 6};
+
+// Percent of the SMs of resblock `branch` (k = 3, 7, 11) of a stage whose rows have l columns.
+int branchSms(int stage, int branch, int64_t l, int sms, const int32_t* clusters) {
+  const Share s = kBranchSms[stage][branch];
+  return convTcSplitRule(kCh[stage], kCh[stage], l, sms * s.split / 100, clusters) ? s.split : s.whole;
+}
 
 struct Plan {
   int64_t key = 0, bytes = 0, unplanned = 0;
@@ -250,6 +264,9 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
   Buf x, har;
   x.p = const_cast<float*>(FP(io.x)), x.pitch = io.x_pitch;
   har.p = const_cast<float*>(FP(io.har)), har.pitch = io.har_pitch;
+  int deviceSms = 0;
+  const int32_t* clusters = nullptr;  // the plan does not ask how launches are spread
+  if (e.running() && (e.rc = convTcDevice(&deviceSms, &clusters)) != 0) return;
 
   Buf bank = e.alloc(0, m.bank_n);
   e.join(1, 0), e.join(2, 0), e.join(3, 0);
@@ -314,7 +331,7 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
     Buf rb[3];
     for (int j = 2; j >= 0; --j)
       resblock(e, j == 2 ? 0 : (j == 1 ? 3 : 4), m.res[3 * i + j], in, inStats, l, bank, &rb[j], nullptr, PlainResidual{},
-               kBranchSms[i][j]);
+               e.running() ? branchSms(i, j, l, deviceSms, clusters) : 100);
     e.join(0, 3), e.join(0, 4);
     mean = e.rows(0, c, l);
     e.launch(0, {rb[0], rb[1], rb[2], mean}, [&](cudaStream_t cs) {
@@ -558,6 +575,11 @@ extern "C" LKC_API void lkc_model_destroy(LkcModel* m) {
   for (cudaEvent_t ev : m->events)
     if (ev) cudaEventDestroy(ev);
   delete m;
+}
+
+extern "C" LKC_API int lkc_generator_branch_sms(int64_t t, int stage, int branch, int sms, const int32_t* clusters) {
+  if (t < 1 || t >= (int64_t(1) << 24) || (stage | 1) != 1 || branch < 0 || branch > 2 || sms < 1 || sms > 65535 || !clusters) return 0;
+  return branchSms(stage, branch, stage ? 60 * t + 1 : 10 * t, sms, clusters);
 }
 
 extern "C" LKC_API int lkc_generator_workspace(LkcModel* m, int64_t t, int concurrent, int64_t* bytes, int64_t* unplanned) {

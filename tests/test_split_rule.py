@@ -67,3 +67,24 @@ def test_tile_widths(co, percent, sms):
 def test_tile_widths_of_known_lengths():
     assert tile_cols(128, 19201) == 160 and tile_cols(256, 12001) == 192  # 121 and 126 tiles on 148 SMs
     assert tile_cols(128, 124801, 50) == 256 and tile_cols(128, 9601, 50) == 160  # 976 tiles of any width; 61 on 74 SMs
+
+
+def branch_sms(t, stage, branch, sms=SMS, clusters=CLUSTERS):
+    return _lib.lib().lkc_generator_branch_sms(t, stage, branch, sms, (ctypes.c_int32 * 9)(*clusters))
+
+
+@pytest.mark.parametrize("stage,branch,base,wider", [(0, 0, 26, 40), (0, 1, 36, 40), (0, 2, 60, 60), (1, 0, 26, 26), (1, 1, 36, 36),
+                                                     (1, 2, 50, 50)])
+def test_generator_branches_take_more_sms_only_where_their_tiles_would_be_whole(stage, branch, base, wider):
+    c = (256, 128)[stage]
+    for t in [*range(1, 300), 747, 2080]:
+        whole = split(c, c, (10 * t, 60 * t + 1)[stage], SMS * base // 100) == 0
+        assert branch_sms(t, stage, branch) == (wider if whole else base)
+
+
+def test_generator_branches_of_known_lengths():
+    # k = 3 of stage 0: 18 tiles at T = 115, two CTAs each on 38 SMs; 20 at T = 116, two CTAs each on 59 SMs only
+    assert [branch_sms(t, 0, 0) for t in (24, 80, 100, 115, 116, 160)] == [26, 26, 26, 26, 40, 40]
+    assert [branch_sms(t, 0, 1) for t in (24, 100, 121, 166, 167, 320)] == [36, 36, 36, 36, 40, 40]
+    assert [branch_sms(t, 0, 0, clusters=(0,) * 9) for t in (24, 160)] == [40, 40]  # a device that holds no clusters
+    assert branch_sms(0, 0, 0) == branch_sms(10, 2, 0) == branch_sms(10, -1, 0) == branch_sms(10, 0, 3) == branch_sms(10, 0, 0, 0) == 0
