@@ -6,7 +6,7 @@ import torch
 
 from lokinfer_b200 import synth
 from oracle import kokoro_oracle as O
-from util import REL_L2, WAVE_MAXABS, rel_l2
+from util import REL_L2, WAVE_MAXABS, check_stats, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -435,35 +435,52 @@ def test_whole_resblock_at_other_tile_widths(cuda, gen, stage, l, k):
     assert torch.equal(out, gen.adain_resblock1_fused(x, gb, prefix, k)[0]) and ops.conv_tc_status() == 0
 
 
-@pytest.mark.parametrize("l", [1, 2, 127, 128, 129, 1024, 1025, 4097, 9000])
-@pytest.mark.parametrize("stage", [0, 1])
+# Both stages at their longest split row: 74 tiles, two CTAs each.
+FEW_TILES = [(stage, l) for stage, longest in ((0, 4736), (1, 9472)) for l in (1, 2, 127, 128, 129, 1024, 1025, 4097, longest)]
+
+
+@pytest.mark.parametrize("stage,l", FEW_TILES)
 def test_whole_resblock_with_few_tiles(cuda, gen, stage, l):
-    """Lengths whose convs are split among CTAs, which fold the statistics (1 to 71 pairs per channel) themselves: against the
-    op-by-op form with its adain_affine, within the rounding of six convs in a row. Rows far from zero, and constant ones."""
+    """Lengths whose convs are split among CTAs, which fold the statistics (1 to 37 pairs per channel in stage 0, to 74 in stage 1)
+    themselves: against the op-by-op form with its adain_affine, within the rounding of six convs in a row; the statistics of
+    the result against that result. Rows far from zero, constant ones, and some whose first pair lies far from the others (the
+    fold's variance is taken relative to it)."""
     from lokinfer_b200 import ops
     r = torch.Generator(device=cuda).manual_seed(l)
     c = (256, 128)[stage]
     x = torch.randn(c, l, generator=r, device=cuda)
     x[::5] += 300.0
     x[::7] = -1234.5
+    x[1::11, :128] += 1e4
     gb = gen.style(torch.randn(128, generator=r, device=cuda))
     prefix = f"resblocks.{3 * stage + 1}"
     out, st = gen.adain_resblock1_fused(x, gb, prefix, 7)
     with ops.use_allocator(lambda shape, device: torch.empty(shape, dtype=torch.float32, device=device)):
         want, want_st = gen.adain_resblock1_fused(x, gb, prefix, 7)
-    d, live = out - x, [i for i in range(c) if i % 5 and i % 7]  # what the block adds; on the big rows x's own rounding hides it
+    # what the block adds; on the big rows x's own rounding hides it
+    d, live = out - x, [i for i in range(c) if i % 5 and i % 7 and i % 11 != 1]
     assert rel_l2(d[live].cpu().numpy(), (want - x)[live].cpu().numpy()) <= 6 * REL_L2
+    far = [i for i in range(1, c, 11) if i % 5 and i % 7]
+    assert rel_l2(d[far, 128:].cpu().numpy(), (want - x)[far, 128:].cpu().numpy()) <= 6 * REL_L2
     assert rel_l2(out.cpu().numpy(), want.cpu().numpy()) <= 6 * REL_L2
     assert rel_l2(st[..., 0].cpu().numpy(), want_st[..., 0].cpu().numpy()) <= 6 * REL_L2
+    check_stats(st.cpu().numpy(), out.cpu().numpy())
     assert torch.equal(out, gen.adain_resblock1_fused(x, gb, prefix, 7)[0]) and ops.conv_tc_status() == 0
 
 
-def test_synthesize_reports_the_status_once(cuda, gen):
-    """An activation beyond the f16 range raises from the call that met it; the next call is clean and right."""
+@pytest.mark.parametrize("form", ["har", "f0"])
+def test_synthesize_reports_the_status_once(cuda, gen, form):
+    """An activation beyond the f16 range raises from the call that met it, with that status and no other; the next call is
+    clean and right."""
     from lokinfer_b200 import ops
     inp, _ = _inputs(cuda, 24)
     x, har, s = (torch.from_numpy(inp[k]).pin_memory() for k in ("x", "har", "s"))
-    want = gen.synthesize(x, har, s).clone()
-    with pytest.raises(RuntimeError, match="0x10000"):
-        gen.synthesize(x * 1e9, har, s)
-    assert torch.equal(gen.synthesize(x, har, s), want) and ops.conv_tc_status() == 0
+    f0 = torch.from_numpy(synth.f0_curve(24, 3)).pin_memory()
+
+    def call(x):
+        return gen.synthesize(x, har, s) if form == "har" else gen.synthesize_f0(x, f0, 5, s)
+
+    want = call(x).clone()
+    with pytest.raises(RuntimeError, match=r"reported status 0x10000 "):
+        call(x * 1e9)
+    assert torch.equal(call(x), want) and ops.conv_tc_status() == 0
