@@ -205,7 +205,9 @@ def test_conv1d_few_columns_other_activations(cuda, ci, co, l, k, d, variant):
     test_conv1d_few_tiles_other_activations(cuda, ci, co, l, k, d, variant)
 
 
-@pytest.mark.parametrize("ci,l,cut,k,d", [(128, 1201, 640, 3, 1), (256, 1000, 384, 11, 5), (48, 700, 128, 7, 3)])
+# The last three: a second part of 33, 1 and 64 columns, which takes a tile of 64 (the last one by 16-byte accesses).
+@pytest.mark.parametrize("ci,l,cut,k,d", [(128, 1201, 640, 3, 1), (256, 1000, 384, 11, 5), (48, 700, 128, 7, 3),
+                                          (128, 673, 640, 7, 5), (48, 257, 256, 3, 1), (128, 704, 640, 11, 5)])
 def test_conv1d_few_tiles_window(cuda, ci, l, cut, k, d):
     """A row in two parts as the time-sharded path holds it: each part a window with real columns of its neighbour beside
     it, what lies beyond the utterance not zero, its statistics a slice of the whole row's."""
