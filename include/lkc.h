@@ -160,10 +160,12 @@ LKC_API int64_t lkc_conv1d_tc_pack_floats(int64_t co, int64_t ci, int64_t k);
 LKC_API int lkc_conv1d_tc_pack_f32_cuda(const LkcArgs* a, void* stream);
 LKC_API LkcConvState* lkc_conv1d_state_create(const void* wp, int64_t co, int64_t ci, int64_t k);
 LKC_API void lkc_conv1d_state_destroy(LkcConvState* st);
-/* The rule by which a conv with f16 halves is split (host code, nothing is launched): CTAs that contract one 128-column x
- * 128-channel tile together, 0 = a CTA per tile. sms = SMs the launch may use; clusters[n], n = 2..8 = clusters of n CTAs
- * resident at a time on the device (9 entries; cudaOccupancyMaxActiveClusters). */
+/* The rule by which a conv with f16 halves is split (host code, nothing is launched): CTAs that contract one tile of 128
+ * channels x lkc_conv1d_tc_split_cols columns together, 0 = a CTA per tile. sms = SMs the launch may use; clusters[n], n = 2..8 =
+ * clusters of n CTAs resident at a time on the device (9 entries; cudaOccupancyMaxActiveClusters). */
 LKC_API int lkc_conv1d_tc_split(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* clusters);
+/* Columns per tile of a conv that is split: 64 for rows of no more, else 128; 0 for a bad argument. */
+LKC_API int lkc_conv1d_tc_split_cols(int64_t lo);
 /* The rule for the tile width of a conv with f16 halves that is not split and may leave chunk statistics per 32 columns (or none):
  * 160, 192, 224 or 256 columns, for a launch on sm_percent of sms SMs (100: one that runs alone); 0 for bad arguments. */
 LKC_API int lkc_conv1d_tc_tile_cols(int64_t co, int64_t lo, int sms, int sm_percent);

@@ -115,6 +115,8 @@ def lib():
         l.lkc_conv1d_tc_tile_cols.argtypes = [ctypes.c_int64] * 2 + [ctypes.c_int] * 2
         l.lkc_conv1d_tc_split.restype = ctypes.c_int
         l.lkc_conv1d_tc_split.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int, ctypes.POINTER(ctypes.c_int32)]
+        l.lkc_conv1d_tc_split_cols.restype = ctypes.c_int
+        l.lkc_conv1d_tc_split_cols.argtypes = [ctypes.c_int64]
         l.lkc_generator_branch_sms.restype = ctypes.c_int
         l.lkc_generator_branch_sms.argtypes = [ctypes.c_int64] + [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int32)]
         l.lkc_conv1d_state_create_as.restype = ctypes.c_void_p

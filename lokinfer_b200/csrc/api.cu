@@ -264,6 +264,8 @@ extern "C" LKC_API int lkc_conv1d_tc_split(int64_t ci, int64_t co, int64_t lo, i
   return convTcSplitRule(ci, co, lo, sms, clusters);
 }
 
+extern "C" LKC_API int lkc_conv1d_tc_split_cols(int64_t lo) { return lo < 1 ? 0 : convTcSplitCols(lo); }
+
 extern "C" LKC_API int lkc_conv1d_tc_tile_cols(int64_t co, int64_t lo, int sms, int sm_percent) {
   return co < 1 || co > (1 << 30) || lo < 1 || lo > (1 << 30) || sms < 1 || sm_percent < 1 ? 0 : convTcTileRule(co, lo, sms, sm_percent);
 }

@@ -1962,18 +1962,21 @@ static int tileColsFor(bool fineOk, int64_t lo, int64_t coBlocks, int sms, int s
 
 int convTcTileRule(int64_t co, int64_t lo, int sms, int smPercent) { return tileColsFor(true, lo, ceilDiv(co, MT), sms, smPercent); }
 
+// Columns of a split tile of a conv. Of a row of up to 64, half of a 128-column tile's MMA time, partial tile, exchange and
+// output are padding: the decoder at F = 61 244 -> 215 us. Tiles of 64 for longer rows lose more to their number (fewer CTAs per
+// tile, each reading more weights) than their shorter exchange gives: T = 24 320 -> 352, F = 100 244 -> 254.
+int convTcSplitCols(int64_t lo) { return lo <= NTS2 ? NTS2 : NTS; }
+
 // The form of a launch. Everybody who has to know it asks here: the launch itself, and the whole-model calls, which give split
 // convs chunk statistics and read the statistics of narrow tiles.
 struct TcForm {
   int split, tileCols;
 };
-// A split tile of a row of up to 64 columns is cut to 64: half of its MMA time, partial tile, exchange and output are padding
-// otherwise. The decoder at F = 61: 244 -> 211 us. Tiles of 64 for longer rows lose more to their number (fewer CTAs per tile, each
-// reading more weights) than their shorter exchange gives: T = 24 320 -> 352, F = 100 244 -> 254.
-static TcForm formFor(const DeviceInfo& d, bool canSplit, bool fineOk, bool conv, int64_t ci, int64_t lo, int64_t coBlocks, int smPercent) {
+static TcForm formFor(const DeviceInfo& d, bool canSplit, bool fineOk, bool conv, int64_t ci, int64_t lo, int64_t coBlocks,
+                      int smPercent) {
   TcForm f;
   f.split = splitFor(canSplit, int(ci), lo, coBlocks, d.smCount * smPercent / 100, d.clusters);
-  f.tileCols = f.split ? (conv && lo <= NTS2 ? NTS2 : NTS) : tileColsFor(fineOk, lo, coBlocks, d.smCount, smPercent);
+  f.tileCols = f.split ? (conv ? convTcSplitCols(lo) : NTS) : tileColsFor(fineOk, lo, coBlocks, d.smCount, smPercent);
   return f;
 }
 static int formOf(const ConvFusedParams& p, bool f16, TcForm* f) {

@@ -132,6 +132,7 @@ int convTcStatCols(const ConvFusedParams& p, bool f16);  // of an eligible conv
 int convTcTileRule(int64_t co, int64_t lo, int sms, int smPercent);
 int convTcDevice(int* sms, const int32_t** clusters);  // what the rules are asked with on the current device
 int convTcSplitRule(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* clusters);
+int convTcSplitCols(int64_t lo);
 int64_t convTcPackFloats(int64_t co, int64_t ci, int64_t k, bool f16);
 int convTcPack(const float* w, float* wp, int64_t co, int64_t ci, int64_t k, bool f16, cudaStream_t s);
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s);

@@ -40,6 +40,12 @@ def test_lengths_around_the_limits():
     assert split(16, 16, 1) == 0 and split(100, 16, 1) == 0 and split(128, 128, 0) == 0
 
 
+def test_columns_of_a_split_tile():
+    cols = _lib.lib().lkc_conv1d_tc_split_cols
+    assert [cols(n) for n in (1, 32, 63, 64)] == [64] * 4 and [cols(n) for n in (65, 128, 129, 9472)] == [128] * 4
+    assert cols(0) == cols(-1) == 0
+
+
 def tile_cols(co, lo, percent=100, sms=SMS):
     return _lib.lib().lkc_conv1d_tc_tile_cols(co, lo, sms, percent)
 
