@@ -440,14 +440,15 @@ __device__ __forceinline__ void regDec() {
 // memory (finish). One bulk copy per pair of CTAs: loads or stores from one SM to another move about 11 bytes per clock
 // (5-7 k clocks for the 56 KB of a CTA).
 // conv: a unit is one output channel of the tile, four columns per lane (a warp has two at a time where the tile has 64); the
-// rank's 128 / split channels go round robin over the epilogue warps, UB at a time so that their loads overlap. What does not depend on the contraction (bias,
-// residual) is loaded by prefetch(), for the first UB units before the accumulation.
+// rank's 128 / split channels go round robin over the epilogue warps, UB at a time so that their loads overlap. What does not
+// depend on the contraction (bias, residual) is loaded by prefetch(), for the first UB units before the accumulation.
 // ConvTranspose: a unit is one output channel x 32 input-rate columns, whose 32 * TS output samples are one run.
 template <int TS, int COLS>
 struct SplitTail {
   static_assert(TS == 0 || COLS == NTS, "ConvTranspose: 128 columns");
   static constexpr int PART_PITCH = partPitch(COLS);
-  static constexpr int LPC = COLS / 4, STEP = EPI_WARPS * 32 / LPC;  // lanes per channel, channels that the epilogue warps have at a time
+  static constexpr int LPC = COLS / 4;                // lanes per channel
+  static constexpr int STEP = EPI_WARPS * 32 / LPC;  // channels that the epilogue warps have at a time
   static constexpr int UB = 4;
   float4 res[UB];
   float bias[UB];
@@ -530,8 +531,8 @@ struct SplitTail {
       const int64_t tChunk = int64_t(tt) * COLS, col = tChunk + sub * 4;
       // valid columns of the tile, and from this lane's first on
       const int nValid = a.lo - tChunk < COLS ? int(a.lo - tChunk) : COLS, mine = nValid - sub * 4;
-      // The UB channels of a warp go side by side through the reductions, whose latency is what this phase lasts (one after the
-      // other: 2.1 us of a launch's 12 at four channels per warp).
+      // The UB channels of a warp go side by side through the reductions, whose latency is what this phase lasts (2.1 us of a
+      // launch's 12 one after the other, at four channels per warp).
 #pragma unroll 1
       for (int base = firstUnit(warp, 0); base < units; base += UB * STEP) {  // warp-uniform
         const int u0 = base + lane / LPC;
@@ -640,11 +641,11 @@ struct SplitTail {
 // PARTIAL: Co is not a multiple of 128 (the last output-channel block has rows that do not exist).
 // TS: 0 = conv1d; 6 / 10 = polyphase ConvTranspose1d of that stride (see the comment above convtTcPackKernel).
 // TMAO: residual and output boxes travel by TMA (rows 16-byte aligned; conv1d with Co % 128 == 0 only).
-// SPLIT (columns of the tile, or 0): a cluster of a.split CTAs shares one tile of 128 or 64 columns. Each CTA contracts its own run of input-channel chunks. When
-// the MMAs of all of them are done (a cluster barrier under the last drain) it sends the rows of its partial tile to the CTAs
-// that own them, over the operand buffers there, which nothing reads any more; when it has all of its own it finishes them:
-// the partials are added in rank order, then bias, residual, scale, statistics and coalesced stores. For launches with fewer
-// tiles than SMs, where one tile's serial chain of chunks is the launch's time (see splitFor).
+// SPLIT (columns of the tile, or 0): a cluster of a.split CTAs shares one tile of 128 or 64 columns. Each CTA contracts its own
+// run of input-channel chunks. When the MMAs of all of them are done (a cluster barrier under the last drain) it sends the rows
+// of its partial tile to the CTAs that own them, over the operand buffers there, which nothing reads any more; when it has all
+// of its own it finishes them: the partials are added in rank order, then bias, residual, scale, statistics and coalesced
+// stores. For launches with fewer tiles than SMs, where one tile's serial chain of chunks is the launch's time (see splitFor).
 // NARROW: tiles of a.tileCols < NT columns. A form of its own: the width as a run-time value cost 256-column tiles 5 % (K = 7).
 template <int ACT, bool PARTIAL, int TS, bool F16, bool TMAO, int SPLIT, bool NARROW>
 __global__ void __launch_bounds__(NTHREADS, 1)
@@ -756,10 +757,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   };
 
   // Split form with statsIn: each CTA folds the chunk statistics of the channels it contracts into their AdaIN affine (sPar, see
-  // the producers). A launch of its own costs 3.5 us plus a gap in front of every conv; here it is one round of loads under the
-  // first weight and input copies, eight lanes per channel on the sixteen warps that have nothing to do yet. In double and
-  // relative to the row's first mean, so that one pass over the pairs gives mean and variance as adainAffineKernel's two do.
-  // (Two passes on the eight producer warps, four lanes per channel: 1.6-1.9 us from the predecessor's end to the constants.)
+  // the producers). A launch of its own costs 3.5 us plus a gap in front of every conv; here it is, for rows of up to 32 pairs
+  // (4096 columns), one round of loads under the first weight and input copies, eight lanes per channel on the sixteen warps that
+  // have nothing to do yet. In double and relative to the row's first mean, so that one pass over the pairs gives mean and
+  // variance as adainAffineKernel's two do: a first mean far from the row's costs at most a factor of the number of pairs of 2^-53.
+  // Two passes on eight warps took 1.6-1.9 us; this and the finish phase together 339 -> 320 us at T = 24.
   const bool fold = SPLIT != 0 && ACT != 0 && TS == 0 && a.statsIn != nullptr;
   if (fold && warp < EPI_WARPS + PRO_WARPS) {
     dependenciesWait();
@@ -769,7 +771,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll 1
     for (int c0 = cBegin * KC + warp * 4; c0 < cEnd; c0 += (EPI_WARPS + PRO_WARPS) * 4) {  // warp-uniform; KC is a multiple of 4
       const int c = c0 + (lane >> 3);
-      const float2* const st = reinterpret_cast<const float2*>(a.statsIn) + int64_t(c) * nch;  // 8-byte aligned, as adain_affine wants
+      // 8-byte aligned, as adain_affine wants
+      const float2* const st = reinterpret_cast<const float2*>(a.statsIn) + int64_t(c) * nch;
       const float gamma = a.gb[c], beta = a.gb[a.ci + c], al = ACT == 1 ? a.alpha[c] : 1.f;
       const double first = double(st[0].x);
       double s1 = 0.0, s2 = 0.0;  // sum of (x - first), sum of (x - first)^2
@@ -2026,7 +2029,8 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk,
   // launch's 14. CTAs that wait hold SMs that a ready launch of another stream could use, so beside other launches this is for
   // those of so few tiles that the launches beside them are split as well. us per forward, no launch early / every split one:
   // T = 24 366 / 337, T = 80 528 / 513, T = 121 598 / 633, T = 320 934 / 992. A share of 100 % counts as alone, which the
-  // decoder's launches say as well, though its shortcuts run beside its main convs (see there).
+  // decoder's launches above 384 frames say as well, though its shortcuts run beside its main convs (see there). Of its shorter
+  // ones the main convs of 257 to 384 frames, 24 tiles, are the only ones that do not start early.
   a.early = smPercent == 100 ? tiles <= d->smCount : a.split && tiles * 8 <= d->smCount;
   a.tmaOut = 0;
   if (boxesOk && a.co % MT == 0 && makeMap(&m.out, a.out, a.co, a.lo, a.outPitch, BOX, BOX, true) &&

@@ -263,10 +263,12 @@ int channelStats(const float* x, float* stats, int64_t c, int64_t l, int64_t pit
   return launched("channel_stats_f32_cuda");
 }
 
-// Early between two convs, beside other launches too: its blocks take room that a conv leaves on an SM and wait there, so that the
-// launch itself (1.5 us of a 3.5 us step between two convs) is over when the first conv ends. The conv behind it starts early only
-// where it says so itself. us, before -> now: synthesize T = 320 982 -> 965, forward T = 121 638 -> 617, T = 800 1713 -> 1709, text to
-// waveform F = 160 1288 -> 1257.
+// Early between two convs, beside other launches too: the launch itself (1.5 us of a 3.5 us step between two convs) is over when
+// the first conv ends. Its blocks do not fit beside a conv CTA, which leaves 4096 registers of an SM where a block takes 8192:
+// they wait on SMs that hold no conv, and where there are none start as the first conv's CTAs leave. One that waits keeps a
+// ready conv CTA of another branch off its SM. The conv behind it starts early only where it says so itself. us per forward as
+// a graph, early only where nothing runs beside it -> everywhere: T = 24 324 -> 325, T = 80 507 -> 499, T = 121 559 -> 550, T = 170
+// 679 -> 690, T = 320 881 -> 868, T = 640 1345 -> 1332, T = 800 1511 -> 1505, T = 2080 the same.
 int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s,
                 int statCols, bool early) {
   cudaLaunchConfig_t cfg = {};

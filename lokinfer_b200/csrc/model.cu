@@ -23,8 +23,8 @@ namespace lkc {
 namespace {
 
 constexpr int kStreams = 5;  // the caller's stream and four side streams
-// Events of the joins, used in turn. A generator forward makes 17 joins, a decoder's 13: an event may be recorded again as soon as the wait on it has
-// been queued, which is the case when join() returns.
+// Events of the joins, used in turn. A generator forward makes 17 joins, a decoder's 13: an event may be recorded again as soon
+// as the wait on it has been queued, which is the case when join() returns.
 constexpr int kEvents = 12;
 constexpr size_t kPlans = 16;
 constexpr float kEps = 1e-5f;  // AdaIN
@@ -38,10 +38,10 @@ constexpr float kEps = 1e-5f;  // AdaIN
 // tiles instead of halves, T = 200 from the second noise branch). No splitting at all, with an earlier build: 877 at T = 24, 934
 // at 121.
 // A resblock whose tiles its share leaves whole gets the other share, with which more lengths are split: a whole tile's chain
-// of 16 channel chunks is then the branch's time. As a graph, T = 72 / 80 / 90 / 100 / 110 / 121 / 140 / 160 / 320 / 640: 26 and 36 for k = 3
-// and 7 of stage 0 at every length 468 / 490 / 502 / 504 / 517 / 584 / 602 / 691 / 866 / 1349; 40 for both, which up to T = 115 only adds
-// CTAs to tiles that have two or three, 462 / 499 / 518 / 520 / 533 / 550 / 573 / 662 / 869 / 1338; as below 469 / 490 / 498 / 505 / 512 / 550 /
-// 564 / 662 / 866 / 1331.
+// of 16 channel chunks is then the branch's time. As a graph, T = 72 / 80 / 90 / 100 / 110 / 121 / 140 / 160 / 320 / 640: 26 and 36
+// for k = 3 and 7 of stage 0 at every length 468 / 490 / 502 / 504 / 517 / 584 / 602 / 691 / 866 / 1349; 40 for both, which up to
+// T = 115 only adds CTAs to tiles that have two or three, 462 / 499 / 518 / 520 / 533 / 550 / 573 / 662 / 869 / 1338; as below 469 /
+// 490 / 498 / 505 / 512 / 550 / 564 / 662 / 866 / 1331.
 struct Share {
   int split, whole;
 };
@@ -358,10 +358,16 @@ constexpr int64_t kDecIn[2] = {528, 1104}, kDecCh = 1024, kDecOut = 512;
 constexpr float kDecSlope = 0.2f, kSqrtHalf = 0.7071067811865476f;
 // Percent of the SMs (see kBranchSms) of the main convs and of the shortcuts beside them. At 100 each launch is planned, and
 // started early, as if it ran alone; where two coincide, clusters wait for room, which for long inputs costs less than fewer CTAs
-// per tile. Short ones have few clusters of many CTAs, of which the device holds few (15 of seven or eight): up to 384 frames the
-// shares are such that the clusters of both fit. us per forward as a graph at F = 61 / 100 / 160 / 300 / 400 / 600, 100 and 100: 215 /
-// 242 / 280 / 332 / 367 / 446; 65 and 35: 194 / 209 / 307 / 316 / 486 / 531; 60 and 40: 219 / 246 / 264 / 344 / 507 / 533; 100 and 30: 194 /
-// 212 / 282 at F = 61 / 100 / 160.
+// per tile. Short ones have few clusters of many CTAs, of which the device holds few (15 of seven or eight, see countClusters), and
+// gain when main convs and shortcuts leave each other room: the shares are the best pair measured for their number of tiles, on
+// which the form of the launches depends. us per forward as a graph over five to fourteen lengths of each row:
+//   main, shortcuts | 65, 35  | 60, 40  | 100, 30 | 75, 25  | 100, 100
+//   F = 8 to 64     | 186-193 | 212-220 | 187-193 | 190-197 | 209-217
+//   F = 65 to 128   | 209-210 | 244-247 | 211-212 | 217-219 | 241-242
+//   F = 129 to 256  | 305-309 | 263-268 | 281-285 | 283-288 | 278-283
+//   F = 257 to 384  | 313-322 | 340-353 | 438-450 | 433-441 | 329-334
+//   F = 385 to 512  | 483-499 | 506-525 | 461-470 | 480-489 | 366-370
+//   F = 513 to 1040 | 524-756 | 525-754 | 506-715 | 548-756 | 444-575
 struct DecSms {
   int main, shortcut;
 };
