@@ -524,82 +524,90 @@ struct SplitTail {
 
   static __device__ __forceinline__ int firstUnit(int warp, int lane) { return warp * (32 / LPC) + lane / LPC; }
 
+  // N channels of this lane, u0, u0 + STEP, .., side by side through the reductions, whose latency is what the phase lasts. As many
+  // as there are, in twos: an absent channel takes as long as one. us per launch one after the other / UB always / as it is:
+  // [128, 1441] K = 3, eight CTAs with two channels a warp 11.1 / 11.3 / 10.7; [48, 1210] K = 11, three CTAs, 48 of 128 channels
+  // 11.8 / 12.1 / 11.0; [256, 3200] K = 3, two CTAs with eight a warp 19.6 / 18.6 / 18.5.
+  template <int N>
+  __device__ __forceinline__ void finishChannels(const TcArgs& a, const float* parts, int u0, int lane) {
+    const bool vecOut = ((reinterpret_cast<uintptr_t>(a.out) | uintptr_t(a.outPitch * 4)) & 15) == 0;
+    const int sub = lane % LPC;
+    const int64_t tChunk = int64_t(tt) * COLS, col = tChunk + sub * 4;
+    // valid columns of the tile, and from this lane's first on
+    const int nValid = a.lo - tChunk < COLS ? int(a.lo - tChunk) : COLS, mine = nValid - sub * 4;
+    float acc[N][4];
+    bool ok[N];  // this lane has columns of channel e
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      ok[e] = u0 + e * STEP < units && cb * MT + row0 + u0 + e * STEP < a.co && mine > 0;
+      acc[e][0] = acc[e][1] = acc[e][2] = acc[e][3] = 0.f;
+    }
+    const float* at = parts + u0 * PART_PITCH + sub * 4;
+#pragma unroll 2
+    for (int r = 0; r < a.split; ++r, at += slot * PART_PITCH) {
+#pragma unroll
+      for (int e = 0; e < N; ++e)
+        if (ok[e]) {
+          const float4 v = *reinterpret_cast<const float4*>(at + e * STEP * PART_PITCH);
+          acc[e][0] += v.x, acc[e][1] += v.y, acc[e][2] += v.z, acc[e][3] += v.w;
+        }
+    }
+    __syncwarp();
+    float mean[N], m2[N];
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      const float rs[4] = {res[e].x, res[e].y, res[e].z, res[e].w};
+      mean[e] = 0.f, m2[e] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        acc[e][j] += bias[e];
+        if (a.residual) acc[e][j] = (acc[e][j] + rs[j]) * a.outScale;
+        if (j < mine) mean[e] += acc[e][j];
+      }
+      float* op = a.out + int64_t(cb * MT + row0 + u0 + e * STEP) * a.outPitch + col;
+      if (ok[e]) {
+        if (vecOut && mine >= 4) {
+          *reinterpret_cast<float4*>(op) = make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j < mine) op[j] = acc[e][j];
+        }
+      }
+    }
+    if (!a.stats) return;
+#pragma unroll
+    for (int o = LPC / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int e = 0; e < N; ++e) mean[e] += __shfl_xor_sync(0xffffffffu, mean[e], o);
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      mean[e] /= float(nValid);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j < mine) m2[e] = fmaf(acc[e][j] - mean[e], acc[e][j] - mean[e], m2[e]);
+    }
+#pragma unroll
+    for (int o = LPC / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int e = 0; e < N; ++e) m2[e] += __shfl_xor_sync(0xffffffffu, m2[e], o);
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+      if (sub == 0 && ok[e]) {
+        float* st = a.stats + (int64_t(cb * MT + row0 + u0 + e * STEP) * a.nchunks + tt) * 2;
+        st[0] = mean[e], st[1] = m2[e];
+      }
+  }
+
   __device__ __forceinline__ void finish(const TcArgs& a, const float* parts, int warp, int lane) {
     if constexpr (TS == 0) {
-      const bool vecOut = ((reinterpret_cast<uintptr_t>(a.out) | uintptr_t(a.outPitch * 4)) & 15) == 0;
-      const int sub = lane % LPC;
-      const int64_t tChunk = int64_t(tt) * COLS, col = tChunk + sub * 4;
-      // valid columns of the tile, and from this lane's first on
-      const int nValid = a.lo - tChunk < COLS ? int(a.lo - tChunk) : COLS, mine = nValid - sub * 4;
-      // The UB channels of a warp go side by side through the reductions, whose latency is what this phase lasts (2.1 us of a
-      // launch's 12 one after the other, at four channels per warp).
+      const int have = a.co - cb * MT - row0 < units ? a.co - cb * MT - row0 : units;  // channels that exist
 #pragma unroll 1
-      for (int base = firstUnit(warp, 0); base < units; base += UB * STEP) {  // warp-uniform
+      for (int base = firstUnit(warp, 0); base < have; base += UB * STEP) {  // warp-uniform
         const int u0 = base + lane / LPC;
         if (base != firstUnit(warp, 0)) prefetch(a, u0, lane);
-        float acc[UB][4];
-        bool ok[UB];  // this lane has columns of channel e
-#pragma unroll
-        for (int e = 0; e < UB; ++e) {
-          ok[e] = u0 + e * STEP < units && cb * MT + row0 + u0 + e * STEP < a.co && mine > 0;
-          acc[e][0] = acc[e][1] = acc[e][2] = acc[e][3] = 0.f;
-        }
-        const float* at = parts + u0 * PART_PITCH + sub * 4;
-#pragma unroll 2
-        for (int r = 0; r < a.split; ++r, at += slot * PART_PITCH) {
-#pragma unroll
-          for (int e = 0; e < UB; ++e)
-            if (ok[e]) {
-              const float4 v = *reinterpret_cast<const float4*>(at + e * STEP * PART_PITCH);
-              acc[e][0] += v.x, acc[e][1] += v.y, acc[e][2] += v.z, acc[e][3] += v.w;
-            }
-        }
-        __syncwarp();
-        float mean[UB], m2[UB];
-#pragma unroll
-        for (int e = 0; e < UB; ++e) {
-          const float rs[4] = {res[e].x, res[e].y, res[e].z, res[e].w};
-          mean[e] = 0.f, m2[e] = 0.f;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            acc[e][j] += bias[e];
-            if (a.residual) acc[e][j] = (acc[e][j] + rs[j]) * a.outScale;
-            if (j < mine) mean[e] += acc[e][j];
-          }
-          float* op = a.out + int64_t(cb * MT + row0 + u0 + e * STEP) * a.outPitch + col;
-          if (ok[e]) {
-            if (vecOut && mine >= 4) {
-              *reinterpret_cast<float4*>(op) = make_float4(acc[e][0], acc[e][1], acc[e][2], acc[e][3]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (j < mine) op[j] = acc[e][j];
-            }
-          }
-        }
-        if (a.stats) {
-#pragma unroll
-          for (int o = LPC / 2; o > 0; o >>= 1)
-#pragma unroll
-            for (int e = 0; e < UB; ++e) mean[e] += __shfl_xor_sync(0xffffffffu, mean[e], o);
-#pragma unroll
-          for (int e = 0; e < UB; ++e) {
-            mean[e] /= float(nValid);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (j < mine) m2[e] = fmaf(acc[e][j] - mean[e], acc[e][j] - mean[e], m2[e]);
-          }
-#pragma unroll
-          for (int o = LPC / 2; o > 0; o >>= 1)
-#pragma unroll
-            for (int e = 0; e < UB; ++e) m2[e] += __shfl_xor_sync(0xffffffffu, m2[e], o);
-#pragma unroll
-          for (int e = 0; e < UB; ++e)
-            if (sub == 0 && ok[e]) {
-              float* st = a.stats + (int64_t(cb * MT + row0 + u0 + e * STEP) * a.nchunks + tt) * 2;
-              st[0] = mean[e], st[1] = m2[e];
-            }
-        }
+        if (base + UB / 2 * STEP >= have) finishChannels<UB / 2>(a, parts, u0, lane);
+        else finishChannels<UB>(a, parts, u0, lane);
       }
     } else {
       constexpr int CQ = 32 / TS, CH = 4 * CQ, SEGS = NTS / 32;

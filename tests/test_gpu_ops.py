@@ -193,6 +193,15 @@ FEW_COLUMNS = [(48, 129, 64, 3, 1), (80, 128, 65, 5, 2), (112, 256, 63, 7, 1), (
                (1104, 64, 61, 3, 1), (128, 128, 4, 7, 5), (64, 22, 31, 9, 6), (528, 256, 64, 1, 1)]
 
 
+# Shares of 64, 43, 32, 26, 19, 16 of a tile's 128 channels (chunks over 2 to 8 CTAs) and of the channels of a last tile that exist:
+# an epilogue warp finishes up to four at a time (eight of a 64-column tile), fewer where half of them would be absent.
+@pytest.mark.parametrize("l", [61, 100, 129])
+@pytest.mark.parametrize("ci,co", [(32, 128), (48, 128), (64, 128), (80, 128), (112, 128), (128, 128), (32, 16), (32, 17), (48, 33),
+                                   (64, 161), (128, 130), (256, 1)])
+def test_conv1d_few_tiles_shares(cuda, ci, co, l):
+    test_conv1d_few_tiles(cuda, ci, co, l, 3, 1, True)
+
+
 @pytest.mark.parametrize("ci,co,l,k,d", FEW_COLUMNS)
 @pytest.mark.parametrize("padded", [False, True])
 def test_conv1d_few_columns(cuda, ci, co, l, k, d, padded):
