@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   // (4096 columns), one round of loads under the first weight and input copies, eight lanes per channel on the sixteen warps that
   // have nothing to do yet. In double and relative to the row's first mean, so that one pass over the pairs gives mean and
   // variance as adainAffineKernel's two do: a first mean far from the row's costs at most a factor of the number of pairs of 2^-53.
-  // Two passes on eight warps took 1.6-1.9 us; this and the finish phase together 339 -> 320 us at T = 24.
+  // Two passes on eight warps took 1.6-1.9 us; this and the finish phase's channels side by side together 339 -> 320 us at T = 24.
   const bool fold = SPLIT != 0 && ACT != 0 && TS == 0 && a.statsIn != nullptr;
   if (fold && warp < EPI_WARPS + PRO_WARPS) {
     dependenciesWait();

@@ -267,8 +267,8 @@ int channelStats(const float* x, float* stats, int64_t c, int64_t l, int64_t pit
 // the first conv ends. Its blocks do not fit beside a conv CTA, which leaves 4096 registers of an SM where a block takes 8192:
 // they wait on SMs that hold no conv, and where there are none start as the first conv's CTAs leave. One that waits keeps a
 // ready conv CTA of another branch off its SM. The conv behind it starts early only where it says so itself. us per forward as
-// a graph, early only where nothing runs beside it -> everywhere: T = 24 324 -> 325, T = 80 507 -> 499, T = 121 559 -> 550, T = 170
-// 679 -> 690, T = 320 881 -> 868, T = 640 1345 -> 1332, T = 800 1511 -> 1505, T = 2080 the same.
+// a graph, early only where nothing runs beside it -> everywhere: T = 16 303 -> 306, T = 24 319 -> 319, T = 80 498 -> 488, T = 121
+// 563 -> 552, T = 170 685 -> 688, T = 320 879 -> 867, T = 640 1344 -> 1335, T = 800 1510 -> 1502, T = 2080 the same.
 int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s,
                 int statCols, bool early) {
   cudaLaunchConfig_t cfg = {};

@@ -39,9 +39,9 @@ constexpr float kEps = 1e-5f;  // AdaIN
 // at 121.
 // A resblock whose tiles its share leaves whole gets the other share, with which more lengths are split: a whole tile's chain
 // of 16 channel chunks is then the branch's time. As a graph, T = 72 / 80 / 90 / 100 / 110 / 121 / 140 / 160 / 320 / 640: 26 and 36
-// for k = 3 and 7 of stage 0 at every length 468 / 490 / 502 / 504 / 517 / 584 / 602 / 691 / 866 / 1349; 40 for both, which up to
-// T = 115 only adds CTAs to tiles that have two or three, 462 / 499 / 518 / 520 / 533 / 550 / 573 / 662 / 869 / 1338; as below 469 /
-// 490 / 498 / 505 / 512 / 550 / 564 / 662 / 866 / 1331.
+// for k = 3 and 7 of stage 0 at every length 470 / 489 / 502 / 508 / 516 / 586 / 604 / 691 / 864 / 1346; 40 for both, which up to
+// T = 115 only adds CTAs to tiles that have two or three, 466 / 504 / 514 / 525 / 533 / 554 / 577 / 662 / 866 / 1336; as below 468 /
+// 488 / 503 / 506 / 518 / 552 / 573 / 658 / 867 / 1335.
 struct Share {
   int split, whole;
 };
@@ -362,12 +362,12 @@ constexpr float kDecSlope = 0.2f, kSqrtHalf = 0.7071067811865476f;
 // gain when main convs and shortcuts leave each other room: the shares are the best pair measured for their number of tiles, on
 // which the form of the launches depends. us per forward as a graph over five to fourteen lengths of each row:
 //   main, shortcuts | 65, 35  | 60, 40  | 100, 30 | 75, 25  | 100, 100
-//   F = 8 to 64     | 186-193 | 212-220 | 187-193 | 190-197 | 209-217
-//   F = 65 to 128   | 209-210 | 244-247 | 211-212 | 217-219 | 241-242
-//   F = 129 to 256  | 305-309 | 263-268 | 281-285 | 283-288 | 278-283
-//   F = 257 to 384  | 313-322 | 340-353 | 438-450 | 433-441 | 329-334
-//   F = 385 to 512  | 483-499 | 506-525 | 461-470 | 480-489 | 366-370
-//   F = 513 to 1040 | 524-756 | 525-754 | 506-715 | 548-756 | 444-575
+//   F = 8 to 64     | 178-185 | 205-214 | 179-186 | 184-192 | 202-210
+//   F = 65 to 128   | 204-206 | 239-243 | 207-209 | 212-216 | 237-240
+//   F = 129 to 256  | 304-309 | 262-270 | 282-287 | 283-289 | 278-284
+//   F = 257 to 384  | 315-324 | 339-350 | 440-453 | 435-444 | 330-336
+//   F = 385 to 512  | 482-498 | 501-525 | 465-474 | 478-488 | 366-370
+//   F = 513 to 1040 | 526-756 | 527-754 | 507-718 | 549-757 | 442-578
 struct DecSms {
   int main, shortcut;
 };
