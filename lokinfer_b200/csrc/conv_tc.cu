@@ -1621,33 +1621,95 @@ int convTcSplitCols(int64_t lo) { return lo <= NTS2 ? NTS2 : NTS; }
 // convs chunk statistics and read the statistics of narrow tiles.
 struct TcForm {
   int split, tileCols;
+  bool pair;  // tiles of CTA pairs (conv_pair.cu), 160 columns wide or 128
 };
 static TcForm formFor(const DeviceInfo& d, bool canSplit, bool fineOk, bool conv, int64_t ci, int64_t lo, int64_t coBlocks,
                       int smPercent) {
   TcForm f;
+  f.pair = false;
   f.split = splitFor(canSplit, int(ci), lo, coBlocks, d.smCount * smPercent / 100, d.clusters);
   f.tileCols = f.split ? (conv ? convTcSplitCols(lo) : NTS) : tileColsFor(fineOk, lo, coBlocks, d.smCount, smPercent);
   return f;
 }
+// The pair form (conv_pair.cu) with tiles of w columns, of a conv that is not split. It wants whole pairs of output-channel blocks and
+// rows that the TMA unit can address. Alone it is the faster one wherever it applies: half of the window columns to stage, finer
+// tiles and so fuller last rounds. Beside other launches the SM time of all tiles together counts, which is that of 256-column tiles of
+// one CTA; there it is taken for launches of one round. us per launch alone, 256 columns of one CTA -> pairs: [256, 20800] K = 3 / 7 /
+// 11 54 -> 41, 68 -> 56, 95 -> 73; [256, 8000] 29 -> 18, 35 -> 23, 48 -> 30; [512, 19200] K = 3 / 7 / 11 141 -> 107, 184 -> 164,
+// 275 -> 235. us per generator forward as a graph, without pairs / those of one round of the launch's share / of the device:
+// T = 260 827 / 796 / 796, T = 320 866 / 809 / 809, T = 400 913 / 887 / 887, T = 480 1043 / 1021 / 992, T = 640 1328 / 1333 / 1320,
+// T = 800 1497 / 1497 / 1472; with pairs of two rounds T = 2080 3680 / 3740.
+static bool rowsAligned(const float* p, int64_t pitch) { return ((reinterpret_cast<uintptr_t>(p) | uintptr_t(pitch * 4)) & 15) == 0; }
+static int pairRows(int w, int64_t k, int64_t dilation, int64_t padding) {  // staged window columns of a CTA
+  return w / 2 + int((k - 1) * dilation) + int(-padding & 3);
+}
+static bool pairs(const ConvFusedParams& p, const DeviceInfo& d, int w) {
+  if (p.co % (2 * MT) || d.clusters[2] < 1 || !gTmaEnabled || !encodeTiled() || !rowsAligned(p.x, p.xPitch ? p.xPitch : p.l) ||
+      !rowsAligned(p.out, p.outPitch ? p.outPitch : p.lo) || (p.residual && !rowsAligned(p.residual, p.resPitch ? p.resPitch : p.lo)))
+    return false;
+  int nb, nRaw, ws, wG;
+  const int rows = pairRows(w, p.k, p.dilation, p.padding - p.xOrigin);
+  if (pairSmem(int(p.ci), rows, (rows + 3) & ~3, int(p.k), &nb, &nRaw, &ws, &wG) == 0) return false;
+  return p.smPercent == 100 || ceilDiv(p.lo, w) * (p.co / (2 * MT)) <= d.clusters[2];
+}
 static int formOf(const ConvFusedParams& p, bool f16, TcForm* f) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
-  *f = formFor(*d, splits(f16, p.k, p.act), f16 && (p.fineStats || !p.stats), true, p.ci, p.lo, ceilDiv(p.co, MT), p.smPercent);
+  const bool fineOk = f16 && (p.fineStats || !p.stats);
+  *f = formFor(*d, splits(f16, p.k, p.act), fineOk, true, p.ci, p.lo, ceilDiv(p.co, MT), p.smPercent);
+  if (!f->split && f16 && pairs(p, *d, fineOk ? 160 : 128)) f->pair = true, f->tileCols = fineOk ? 160 : 128;
   return 0;
+}
+
+// Geometry and tensor maps of the pair form. False: a map could not be made, and the launch takes the form of one CTA that leaves
+// the same statistics.
+static bool finishPair(TcArgs& a, TcMaps& m, const DeviceInfo& d, int smPercent, int* grid, size_t* smem) {
+  a.delta = -a.padding & 3;
+  a.rows = pairRows(a.tileCols, a.k, a.dilation, a.padding), a.ext = (a.rows + 3) & ~3;  // ext: columns of a raw buffer
+  int nb = 0;
+  *smem = pairSmem(a.ci, a.rows, a.ext, a.k, &nb, &a.nRaw, &a.wStages, &a.wG);
+  constexpr int tapRows = Fmt<true>::W_STAGE_BYTES / 1024;  // the pack as rows of 1 KB
+  const int64_t wRows = int64_t(a.co / MT) * (a.ci / KC) * a.k * tapRows;
+  if (*smem == 0 || wRows >= (int64_t(1) << 30) || !makeMap(&m.x, a.x, a.ci, a.l, a.xPitch, a.ext, KC, false) ||
+      !makeMap(&m.out, a.out, a.co, a.lo, a.outPitch, BOX, BOX, true) ||
+      (a.residual && !makeMap(&m.res, a.residual, a.co, a.lo, a.resPitch, BOX, BOX, true)) ||
+      !makeMap(&m.w, a.wp, wRows, 256, 256, 256, a.wG * tapRows, false) ||
+      (a.k % a.wG && !makeMap(&m.w1, a.wp, wRows, 256, 256, 256, (a.wG - 1) * tapRows, false)))
+    return false;
+  a.tmaIn = a.tmaOut = 1, a.nb = nb;
+  a.numCoBlk = a.co / (2 * MT);
+  const int tiles = a.numTTiles * a.numCoBlk;
+  *grid = 2 * std::min(tiles, d.clusters[2]);
+  a.early = smPercent == 100 && tiles <= d.clusters[2];
+  return true;
 }
 
 // Launch geometry and tensor maps shared by the conv and ConvTranspose entry points.
 static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk, int smPercent, int* grid, size_t* smem) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
-  a.split = form.split, a.tileCols = form.tileCols;
+  a.split = form.split, a.tileCols = form.tileCols, a.pair = form.pair;
   LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
   const int nt = a.split ? a.tileCols : NT;  // staged columns of the first box
-  if (a.stats && !a.split && a.tileCols != NT) a.nchunks = ceilDiv(a.lo, 32);
+  if (a.stats && !a.split && a.tileCols != NT && a.tileCols != 128) a.nchunks = ceilDiv(a.lo, 32);
   a.numTTiles = int(ceilDiv(a.lo, a.tileCols));
   // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
   // argument: it stays zero-filled and is never dereferenced.
   std::memset(&m, 0, sizeof m);
+  a.nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
+  a.status = d->status;
+  a.prof = (kProf && gProfileOn) ? d->prof : nullptr;
+  // Dhi is drained into the f32 running sums after as many whole chunks as fit in the longest chain of MMAs.
+  const int perChunk = a.k * (f16 ? 1 : 2);
+  const int n = (!f16 && a.k == 1 ? MAX_CHAIN_POINT32 : MAX_CHAIN) / perChunk;
+  a.drainN = n < 1 ? 1 : n;
+  if (a.pair) {
+    const int coBlk = a.numCoBlk;
+    if (finishPair(a, m, *d, smPercent, grid, smem)) return 0;
+    std::memset(&m, 0, sizeof m);
+    a.pair = 0, a.numCoBlk = coBlk, a.nb = Fmt<true>::NB;
+    if (a.tileCols == 128) a.tileCols = NT, a.numTTiles = int(ceilDiv(a.lo, NT));
+  }
   a.tmaIn = makeMap(&m.x, a.x, a.ci, a.l, a.xPitch, nt, KC, false) ? 1 : 0;
   auto layOut = [&] {
     a.delta = a.tmaIn ? -a.padding & 3 : 0;  // tiles start on multiples of 4 columns
@@ -1663,13 +1725,6 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk,
     LKC_REQUIRE(makeMap(&m.ext, a.x, a.ci, a.l, a.xPitch, a.ext, KC, false), "conv (tensor-core): tensor map of the input");
   LKC_REQUIRE(*smem != 0, "conv (tensor-core): window too large");
   if (a.split && *smem < SPLIT_SMEM) *smem = SPLIT_SMEM;
-  a.nb = f16 ? Fmt<true>::NB : Fmt<false>::NB;
-  a.status = d->status;
-  a.prof = (kProf && gProfileOn) ? d->prof : nullptr;
-  // Dhi is drained into the f32 running sums after as many whole chunks as fit in the longest chain of MMAs.
-  const int perChunk = a.k * (f16 ? 1 : 2);
-  const int n = (!f16 && a.k == 1 ? MAX_CHAIN_POINT32 : MAX_CHAIN) / perChunk;
-  a.drainN = n < 1 ? 1 : n;
   const int tiles = a.numTTiles * a.numCoBlk;
   *grid = a.split ? tiles * a.split : (tiles < d->smCount ? tiles : d->smCount);
   // A launch of one round starts as the SMs come free and sets itself up under the end of the one before it: 3 us of a split
@@ -1693,7 +1748,7 @@ bool convTcSplits(const ConvFusedParams& p, bool f16) {
 
 int convTcStatCols(const ConvFusedParams& p, bool f16) {
   TcForm f;
-  return formOf(p, f16, &f) == 0 && !f.split && f.tileCols != NT ? 32 : 128;
+  return formOf(p, f16, &f) == 0 && !f.split && f.tileCols != NT && f.tileCols != 128 ? 32 : 128;
 }
 
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {
@@ -1718,6 +1773,7 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
   TcForm form;
   if (int rc = formOf(p, f16, &form)) return rc;
   if (int rc = finishArgs(a, m, f16, form, true, p.smPercent, &grid, &smem)) return rc;
+  if (a.pair) return convPair(a, m, p.act, grid, smem, s);
   switch (p.act) {
     case Act::None: return launchTc<0>(a, m, f16, grid, smem, s);
     case Act::Snake: return launchTc<1>(a, m, f16, grid, smem, s);

@@ -105,6 +105,8 @@ struct TcArgs {
   int tmaOut;      // 1: out (and residual) rows are 16-byte aligned, boxes go by TMA
   int numTTiles, numCoBlk;
   int split;       // 0 = a persistent CTA per SM over tiles of tileCols columns; else the CTAs that share one such tile
+  int pair;        // 1: tiles of CTA pairs (conv_pair.cu)
+  int nRaw;        // CTA pairs: raw-input staging buffers
   int early;       // the launch may overlap the end of the one before it (programmatic dependent launch)
   int* status;
   long long* prof;  // null, or 16 cycle counters summed over CTAs (see convTcProfile)
@@ -372,7 +374,14 @@ __device__ __forceinline__ void regDec() {
 // Tensor maps of a launch.
 struct TcMaps {
   CUtensorMap x, ext, res, out;
+  CUtensorMap w, w1;  // CTA pairs: the weights of a tap group of wG and of wG - 1 taps
 };
 
 }  // namespace tc
+
+// CTA pairs (conv_pair.cu): the buffers of a launch (activations, raw input, weight slots, taps per slot) with its shared memory, or
+// 0 where they do not fit; the launch.
+size_t pairSmem(int ci, int rows, int rawPitch, int k, int* nb, int* nRaw, int* wStages, int* wG);
+int convPair(const tc::TcArgs& a, const tc::TcMaps& m, Act act, int grid, size_t smem, cudaStream_t s);
+
 }  // namespace lkc

@@ -1,0 +1,74 @@
+"""Convs on CTA pairs (csrc/conv_pair.cu): whole pairs of output-channel blocks, 16-byte aligned rows, too many tiles to be split.
+
+The form is a matter of speed alone: the same products, drains and order of sums as in the form of one CTA, which the contiguous
+call and the 4-byte route take. Results are bit-identical to those, which the other tests hold to the oracle."""
+import pytest
+import torch
+
+from lokinfer_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+# ci, co, l, k, d: one chunk, a chunk for one of the two groups of producer warps, tiles of 128 columns with whole, one-column and
+# empty last halves, rounds of pairs that are full and one over, the widest window, K of one and two tap groups and more than eight
+CASES = [(16, 256, 9600, 3, 1), (48, 256, 4737, 7, 3), (256, 256, 4864, 3, 1), (256, 256, 9472, 11, 5), (256, 256, 9473, 11, 1),
+         (128, 512, 9537, 7, 5), (256, 256, 9600, 1, 1), (32, 256, 20100, 2, 3), (64, 768, 6000, 9, 1), (32, 256, 9500, 16, 1)]
+
+
+def _case(cuda, ci, co, l, k):
+    from lokinfer_b200 import ops
+    x, w, b, affine, alpha, res = (torch.from_numpy(v).to(cuda) for v in synth.conv_case(ci, co, l, k, ci + co + l + k))
+    state = ops.conv1d_prepare_f32_cuda(w)
+    assert state is not None
+    return x, w, b, affine, alpha, res, state
+
+
+@pytest.mark.parametrize("variant", ["snake", "snake_res", "leaky_res_scaled", "affine"])
+@pytest.mark.parametrize("ci,co,l,k,d", CASES)
+def test_pair_form_changes_no_bit(cuda, ci, co, l, k, d, variant):
+    from lokinfer_b200 import ops
+    x, w, b, affine, alpha, res, state = _case(cuda, ci, co, l, k)
+
+    def call(xx, rr):
+        kw = dict(padding=d * (k - 1) // 2, dilation=d, state=state)
+        if variant == "affine":
+            return ops.conv1d_affine_f32_cuda(xx, w, b, affine, **kw)
+        if variant == "leaky_res_scaled":
+            return ops.conv1d_leaky_f32_cuda(xx, w, b, affine, slope=0.2, residual=rr, out_scale=0.7071067811865476, **kw)
+        return ops.conv1d_snake_f32_cuda(xx, w, b, affine, alpha, residual=rr if variant == "snake_res" else None, **kw)
+
+    lo = l + 2 * (d * (k - 1) // 2) - d * (k - 1)
+    res = res[:, :lo].contiguous()
+    ops.set_conv_io("plain")
+    try:
+        ref, ref_stats = call(x, res)
+    finally:
+        ops.set_conv_io("tma")
+    with ops.padded_rows():
+        px, pres = ops.to_cuda(x.cpu().numpy(), cuda, rows=True), ops.to_cuda(res.cpu().numpy(), cuda, rows=True)
+        out, stats = call(px, pres)
+    assert ops.conv_tc_status() == 0
+    assert torch.equal(out, ref)
+    assert torch.equal(stats, ref_stats)
+
+
+@pytest.mark.parametrize("l", [4737, 4800, 9601, 11840, 11841])
+def test_pair_form_in_a_resblock(cuda, l):
+    """Tiles of 160 columns with a pair of statistics per 32, which only whole-block calls take."""
+    import numpy as np
+    from lokinfer_b200 import ops
+    from lokinfer_b200.generator import Generator
+    gen = Generator(synth.generator_weights(3), cuda)
+    r = np.random.default_rng(l)
+    with ops.padded_rows():
+        x = ops.to_cuda(r.standard_normal((256, l), dtype=np.float32), cuda, rows=True)
+        gb = gen.style(torch.from_numpy(r.standard_normal(128, dtype=np.float32)).to(cuda))
+        out, _ = gen.adain_resblock1_fused(x, gb, "resblocks.1", 7)
+        ops.set_conv_io("plain")
+        try:
+            ref, _ = gen.adain_resblock1_fused(x, gb, "resblocks.1", 7)
+        finally:
+            ops.set_conv_io("tma")
+    assert ops.conv_tc_status() == 0
+    # the order in which 6 convs' residuals and statistics are added: a few units of the last place each
+    assert torch.linalg.vector_norm(out - ref) <= 2e-6 * torch.linalg.vector_norm(ref)
