@@ -1661,9 +1661,12 @@ static int formOf(const ConvFusedParams& p, bool f16, TcForm* f) {
   return 0;
 }
 
+enum class Start { BehindAffine, Urgent, Patient };  // see ConvFusedParams
+static Start startOf(const ConvFusedParams& p) { return p.behindAffine ? Start::BehindAffine : p.urgent ? Start::Urgent : Start::Patient; }
+
 // Geometry and tensor maps of the pair form. False: a map could not be made, and the launch takes the form of one CTA that leaves
 // the same statistics.
-static bool finishPair(TcArgs& a, TcMaps& m, const DeviceInfo& d, int smPercent, int* grid, size_t* smem) {
+static bool finishPair(TcArgs& a, TcMaps& m, const DeviceInfo& d, Start start, int smPercent, int* grid, size_t* smem) {
   a.delta = -a.padding & 3;
   a.rows = pairRows(a.tileCols, a.k, a.dilation, a.padding), a.ext = (a.rows + 3) & ~3;  // ext: columns of a raw buffer
   int nb = 0;
@@ -1680,12 +1683,12 @@ static bool finishPair(TcArgs& a, TcMaps& m, const DeviceInfo& d, int smPercent,
   a.numCoBlk = a.co / (2 * MT);
   const int tiles = a.numTTiles * a.numCoBlk;
   *grid = 2 * std::min(tiles, d.clusters[2]);
-  a.early = smPercent == 100 && tiles <= d.clusters[2];
+  a.early = start == Start::BehindAffine || (smPercent == 100 && tiles <= d.clusters[2]);
   return true;
 }
 
 // Launch geometry and tensor maps shared by the conv and ConvTranspose entry points.
-static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk, int smPercent, int* grid, size_t* smem) {
+static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk, Start start, int smPercent, int* grid, size_t* smem) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
   a.split = form.split, a.tileCols = form.tileCols, a.pair = form.pair;
@@ -1705,7 +1708,7 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk,
   a.drainN = n < 1 ? 1 : n;
   if (a.pair) {
     const int coBlk = a.numCoBlk;
-    if (finishPair(a, m, *d, smPercent, grid, smem)) return 0;
+    if (finishPair(a, m, *d, start, smPercent, grid, smem)) return 0;
     std::memset(&m, 0, sizeof m);
     a.pair = 0, a.numCoBlk = coBlk, a.nb = Fmt<true>::NB;
     if (a.tileCols == 128) a.tileCols = NT, a.numTTiles = int(ceilDiv(a.lo, NT));
@@ -1728,12 +1731,17 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk,
   const int tiles = a.numTTiles * a.numCoBlk;
   *grid = a.split ? tiles * a.split : (tiles < d->smCount ? tiles : d->smCount);
   // A launch of one round starts as the SMs come free and sets itself up under the end of the one before it: 3 us of a split
-  // launch's 14. CTAs that wait hold SMs that a ready launch of another stream could use, so beside other launches this is for
-  // those of so few tiles that the launches beside them are split as well. us per forward, no launch early / every split one:
-  // T = 24 366 / 337, T = 80 528 / 513, T = 121 598 / 633, T = 320 934 / 992. A share of 100 % counts as alone, which the
-  // decoder's launches above 384 frames say as well, though its shortcuts run beside its main convs (see there). Of its shorter
-  // ones the main convs of 257 to 384 frames, 24 tiles, are the only ones that do not start early.
-  a.early = smPercent == 100 ? tiles <= d->smCount : a.split && tiles * 8 <= d->smCount;
+  // launch's 14. CTAs that wait hold SMs that a ready launch of another stream could use, so beside other launches this is for the
+  // split ones (in a branch that nobody waits for soon, those of few tiles: T = 64 425 -> 436 with the second noise branch early),
+  // and for any behind its adain_affine, which lets it start only when the conv before has ended. us per generator forward as a
+  // graph, split ones of few tiles / all split ones / behind adain_affine too: T = 121 544 / - / 531 and with all split ones 509,
+  // T = 140 580 -> 560, T = 160 638 -> 627, T = 200 682 / 661 / 647; without split ones T = 320 809 -> 761, T = 480 990 -> 966,
+  // T = 640 1317 -> 1271, T = 800 1470 -> 1450. Decoder F = 320 / 384 308 -> 300, 313 -> 304.
+  // A share of 100 % counts as alone, which the decoder's launches above 384 frames say as well, though its shortcuts run beside
+  // its main convs (see there).
+  a.early = start == Start::BehindAffine ? 1
+            : smPercent == 100           ? tiles <= d->smCount
+                                         : a.split && (start == Start::Urgent || tiles * 8 <= d->smCount);
   a.tmaOut = 0;
   if (boxesOk && a.co % MT == 0 && makeMap(&m.out, a.out, a.co, a.lo, a.outPitch, BOX, BOX, true) &&
       (!a.residual || makeMap(&m.res, a.residual, a.co, a.lo, a.resPitch, BOX, BOX, true)))
@@ -1772,7 +1780,7 @@ int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) 
   size_t smem = 0;
   TcForm form;
   if (int rc = formOf(p, f16, &form)) return rc;
-  if (int rc = finishArgs(a, m, f16, form, true, p.smPercent, &grid, &smem)) return rc;
+  if (int rc = finishArgs(a, m, f16, form, true, startOf(p), p.smPercent, &grid, &smem)) return rc;
   if (a.pair) return convPair(a, m, p.act, grid, smem, s);
   switch (p.act) {
     case Act::None: return launchTc<0>(a, m, f16, grid, smem, s);
@@ -1831,7 +1839,7 @@ int convtTc(const ConvtParams& p, const float* wp, bool f16, cudaStream_t s) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
   const TcForm form = formFor(*d, f16, f16, false, p.ci, p.l, coBlk, p.smPercent);
-  if (int rc = finishArgs(a, m, f16, form, false, p.smPercent, &grid, &smem)) return rc;
+  if (int rc = finishArgs(a, m, f16, form, false, Start::Urgent, p.smPercent, &grid, &smem)) return rc;
   if (p.stride == 6) return launchTc2<2, false, 6>(a, m, f16, grid, smem, s);
   return launchTc2<2, false, 10>(a, m, f16, grid, smem, s);
 }

@@ -155,8 +155,8 @@ __global__ void channelStatsKernel(const float* __restrict__ x, float* __restric
 constexpr int kAffineThreads = 128;
 __global__ void __launch_bounds__(kAffineThreads) adainAffineKernel(const float* stats, const float* gb, float* affine, int64_t c,
                                                                     int64_t l, int64_t nchunks, int statCols, float eps, int early) {
-  if (early) dependentsLaunch();
   dependenciesWait();
+  if (early) dependentsLaunch();  // not before: a conv that waits holds SMs, and what it waits for is then this kernel alone
   __shared__ double red[kAffineThreads / 32];
   __shared__ double bc;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -266,7 +266,7 @@ int channelStats(const float* x, float* stats, int64_t c, int64_t l, int64_t pit
 // Early between two convs, beside other launches too: the launch itself (1.5 us of a 3.5 us step between two convs) is over when
 // the first conv ends. Its blocks do not fit beside a conv CTA, which leaves 4096 registers of an SM where a block takes 8192:
 // they wait on SMs that hold no conv, and where there are none start as the first conv's CTAs leave. One that waits keeps a
-// ready conv CTA of another branch off its SM. The conv behind it starts early only where it says so itself. us per forward as
+// ready conv CTA of another branch off its SM. The conv behind it starts early where it says so itself. us per forward as
 // a graph, early only where nothing runs beside it -> everywhere: T = 16 303 -> 306, T = 24 319 -> 319, T = 80 498 -> 488, T = 121
 // 563 -> 552, T = 170 685 -> 688, T = 320 879 -> 867, T = 640 1344 -> 1335, T = 800 1510 -> 1502, T = 2080 the same.
 int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, int64_t l, float eps, cudaStream_t s,

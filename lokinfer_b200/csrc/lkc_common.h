@@ -88,6 +88,9 @@ struct ConvFusedParams {
   // AdaIN; the conv computes the affine itself.
   const float *statsIn = nullptr, *gb = nullptr;
   float eps = 0.f;
+  // When it may start before what it waits for has ended (convTc's rule): the launch in front of it is its adain_affine, which says so
+  // only when the conv before has ended; false: a branch that nobody waits for soon.
+  bool behindAffine = false, urgent = true;
   bool fineStats = false;  // stats may come as one pair per 32 columns (convStatCols says which)
 };
 

@@ -189,19 +189,19 @@ void conv(Exec& e, int s, Act act, Buf x, int64_t l, int64_t ci, int64_t co, int
 // plan reserves it either way, as the route may change between two calls (set_conv_path). statCols: columns per pair of
 // `stats`; the return value is that of outStats, 128 unless `fine` allows others.
 int adainConv(Exec& e, int s, Buf x, Buf stats, int statCols, int64_t l, int64_t c, int64_t k, int64_t d, const LkcResblock& w,
-              int i, Buf bank, Buf residual, Buf out, Buf outStats, bool fine, int smPercent) {
+              int i, Buf bank, Buf residual, Buf out, Buf outStats, bool fine, int smPercent, bool urgent) {
   const Buf af = e.alloc(s, 3 * c);
   ConvFusedParams p;
   p.x = x.p, p.w = FP(w.w[i]), p.bias = FP(w.b[i]), p.affine = af.p, p.alpha = FP(w.alpha[i]), p.residual = residual.p;
   p.out = out.p, p.stats = outStats.p;
   p.ci = c, p.l = l, p.co = c, p.k = k, p.dilation = d, p.padding = d * (k - 1) / 2, p.lo = l;
   p.xPitch = x.pitch, p.resPitch = residual.pitch, p.outPitch = out.pitch;
-  p.act = Act::Snake, p.state = w.state[i], p.smPercent = smPercent, p.fineStats = fine;
+  p.act = Act::Snake, p.state = w.state[i], p.smPercent = smPercent, p.fineStats = fine, p.urgent = urgent;
   const float* gb = bank.p + w.gb[i];
   if (e.running() && statCols == 128 && convFoldsAffine(p))
     p.statsIn = stats.p, p.gb = gb, p.eps = kEps;
   else
-    e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, c, l, kEps, st, statCols, true); });
+    e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, c, l, kEps, st, statCols, true); }), p.behindAffine = true;
   e.launch(s, {x, stats, bank, af, residual, out, outStats}, [&](cudaStream_t st) { return convFused(p, st); });
   return e.running() ? convStatCols(p) : 128;
 }
@@ -226,7 +226,7 @@ struct PlainResidual {
 // allocated here. outStats = null: nobody asks for the result's statistics.
 template <class Residual>
 void resblock(Exec& e, int s, const LkcResblock& w, Buf x, Buf stats, int64_t l, Buf bank, Buf* out, Buf* outStats,
-              Residual residual, int smPercent) {
+              Residual residual, int smPercent, bool urgent = true) {
   static const int64_t dil[3] = {1, 3, 5};
   const int64_t c = w.c, k = w.k;
   const Buf none;
@@ -237,12 +237,12 @@ void resblock(Exec& e, int s, const LkcResblock& w, Buf x, Buf stats, int64_t l,
     const bool last = j == 2;
     const Buf res = last ? residual.make(x) : x;
     Buf xt = e.rows(s, c, l), st1 = statsBuf(e, s, c, l, 32);
-    statCols = adainConv(e, s, x, stats, statCols, l, c, k, d, w, i1, bank, none, xt, st1, true, smPercent);
+    statCols = adainConv(e, s, x, stats, statCols, l, c, k, d, w, i1, bank, none, xt, st1, true, smPercent, urgent);
     Buf xn = last && out->p ? *out : e.rows(s, c, l), stn;
     if (!last) stn = statsBuf(e, s, c, l, 32);
     else if (outStats) stn = outStats->p ? *outStats : statsBuf(e, s, c, l);
     if (last) residual.ready();
-    statCols = adainConv(e, s, xt, st1, statCols, l, c, k, 1, w, i2, bank, res, xn, stn, !last, smPercent);
+    statCols = adainConv(e, s, xt, st1, statCols, l, c, k, 1, w, i2, bank, res, xn, stn, !last, smPercent, urgent);
     x = xn, stats = stn;
   }
   *out = x;
@@ -316,7 +316,7 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
          kNoiseSms[i]);
     e.join(s, 3);
     if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats, AddUpsampled{e, u0, kCh[0], len[0]}, kNoiseSms[i]);
-    else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], nullptr, PlainResidual{}, kNoiseSms[i]);
+    else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], nullptr, PlainResidual{}, kNoiseSms[i], false);
   }
 
   Buf in = noise[0], inStats = noiseStats, mean;
