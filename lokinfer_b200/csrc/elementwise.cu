@@ -147,18 +147,20 @@ __global__ void channelStatsKernel(const float* __restrict__ x, float* __restric
   }
 }
 
-// One 128-thread block per channel: exact combine of the (count, mean, M2) partials in double, two passes. The
-// chunk partials of a channel are read once into registers (up to 8 per thread; longer rows loop), so both passes
-// cost one round of memory latency.
+// One 128-thread block per channel: exact combine of the (count, mean, M2) partials in double, in one pass relative to the row's
+// first mean (to 0 where that is not finite, so that infinities and NaN come out as from sums). A first mean far from the row's costs
+// at most a factor of the number of pairs of 2^-53, as it is in the variance itself. What bounds it is latency, between two convs:
+// one round of loads (up to 8 pairs per thread in flight; longer rows loop), one of shuffles, one barrier. Two passes with
+// a division each and five barriers cost 0.5 us more per step: us per generator forward as a graph T = 121 514 -> 506, T = 200
+// 642 -> 631, T = 320 761 -> 751, T = 480 967 -> 954.
 // Its inputs are not __restrict__: an early launch reads what the one in front of it may still be writing, and loads of read-only
 // data could be moved in front of the wait.
 constexpr int kAffineThreads = 128;
 __global__ void __launch_bounds__(kAffineThreads) adainAffineKernel(const float* stats, const float* gb, float* affine, int64_t c,
-                                                                    int64_t l, int64_t nchunks, int statCols, float eps, int early) {
+                                                                    int64_t l, int64_t nchunks, int statCols, double invL, float eps, int early) {
   dependenciesWait();
   if (early) dependentsLaunch();  // not before: a conv that waits holds SMs, and what it waits for is then this kernel alone
-  __shared__ double red[kAffineThreads / 32];
-  __shared__ double bc;
+  __shared__ double red[2 * kAffineThreads / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t ch = blockIdx.x;
   const float2* sc = reinterpret_cast<const float2*>(stats) + ch * nchunks;  // (mean, M2) pairs, 8-byte aligned
@@ -170,48 +172,31 @@ __global__ void __launch_bounds__(kAffineThreads) adainAffineKernel(const float*
     const int64_t t = threadIdx.x + int64_t(j) * kAffineThreads;
     v[j] = t < nchunks ? sc[t] : make_float2(0.f, 0.f);
   }
-  double sum = 0.0;
+  const float x0 = sc[0].x, gamma = gb[ch], beta = gb[c + ch];
+  const double pivot = fabsf(x0) <= 3.402823466e38f ? static_cast<double>(x0) : 0.0;
+  double s1 = 0.0, s2 = 0.0;  // sum of (x - pivot), sum of (x - pivot)^2
+  auto add = [&](float2 p, int64_t t) {
+    const double n = t + 1 < nchunks ? nT : nLast, d = static_cast<double>(p.x) - pivot;
+    s1 += n * d, s2 += static_cast<double>(p.y) + n * d * d;
+  };
 #pragma unroll
   for (int j = 0; j < R; ++j) {
     const int64_t t = threadIdx.x + int64_t(j) * kAffineThreads;
-    if (t < nchunks) sum += static_cast<double>(v[j].x) * (t + 1 < nchunks ? nT : nLast);
+    if (t < nchunks) add(v[j], t);
   }
-  for (int64_t t = threadIdx.x + int64_t(R) * kAffineThreads; t < nchunks; t += kAffineThreads)
-    sum += static_cast<double>(sc[t].x) * (t + 1 < nchunks ? nT : nLast);
-  sum = warpSumD(sum);
-  if (lane == 0) red[wid] = sum;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < kAffineThreads / 32; ++w) t += red[w];
-    bc = t / static_cast<double>(l);
-  }
-  __syncthreads();
-  const double mean = bc;
-  double m2 = 0.0;
+  for (int64_t t = threadIdx.x + int64_t(R) * kAffineThreads; t < nchunks; t += kAffineThreads) add(sc[t], t);
 #pragma unroll
-  for (int j = 0; j < R; ++j) {
-    const int64_t t = threadIdx.x + int64_t(j) * kAffineThreads;
-    if (t < nchunks) {
-      const double dm = static_cast<double>(v[j].x) - mean;
-      m2 += static_cast<double>(v[j].y) + (t + 1 < nchunks ? nT : nLast) * dm * dm;
-    }
-  }
-  for (int64_t t = threadIdx.x + int64_t(R) * kAffineThreads; t < nchunks; t += kAffineThreads) {
-    const double dm = static_cast<double>(sc[t].x) - mean;
-    m2 += static_cast<double>(sc[t].y) + (t + 1 < nchunks ? nT : nLast) * dm * dm;
-  }
-  m2 = warpSumD(m2);
-  __syncthreads();
-  if (lane == 0) red[wid] = m2;
+  for (int o = 16; o > 0; o >>= 1) s1 += __shfl_xor_sync(0xffffffffu, s1, o), s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  if (lane == 0) red[wid] = s1, red[kAffineThreads / 32 + wid] = s2;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < kAffineThreads / 32; ++w) t += red[w];
-    const float m = static_cast<float>(mean), var = static_cast<float>(t / static_cast<double>(l));
-    affine[ch] = m;
-    affine[c + ch] = (1.f + gb[ch]) * (1.0f / sqrtf(var + eps));
-    affine[2 * c + ch] = gb[c + ch];
+    s1 = s2 = 0.0;
+    for (int w = 0; w < kAffineThreads / 32; ++w) s1 += red[w], s2 += red[kAffineThreads / 32 + w];
+    const double dm = s1 * invL, q = s2 * invL - dm * dm;
+    const float var = q < 0.0 ? 0.f : static_cast<float>(q);  // (a NaN stays one)
+    affine[ch] = static_cast<float>(pivot + dm);
+    affine[c + ch] = (1.f + gamma) * (1.0f / sqrtf(var + eps));
+    affine[2 * c + ch] = beta;
   }
 }
 
@@ -279,7 +264,7 @@ int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, i
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 1;
   }
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, adainAffineKernel, stats, gb, affine, c, l, ceilDiv(l, statCols), statCols, eps,
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, adainAffineKernel, stats, gb, affine, c, l, ceilDiv(l, statCols), statCols, 1.0 / double(l), eps,
                                            early ? 1 : 0);
   if (e != cudaSuccess) {
     cudaGetLastError();
