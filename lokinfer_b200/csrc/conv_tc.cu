@@ -1759,7 +1759,46 @@ int convTcStatCols(const ConvFusedParams& p, bool f16) {
   return formOf(p, f16, &f) == 0 && !f.split && f.tileCols != NT && f.tileCols != 128 ? 32 : 128;
 }
 
+static int convTcLaunch(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s);
+
+// Columns of the first launch of a conv that goes in two, or 0. Alone, a conv whose tiles fill some rounds of the device and a part
+// of one more lasts as if that were full. Where so few columns are over that they can be split over the CTAs of clusters they are a
+// launch of their own, if that saves more MMA clocks (half a column's width each, three to a tap and chunk) than the split form's
+// fixed cost and a second launch's, at most 24,000 (12 us). The rounds are those of 256-column tiles in both forms of whole tiles, so
+// that rows of every alignment give the same bits; two rounds of pairs have as many columns. Statistics per 32 columns leave no
+// choice: a split tile has one pair.
+// Measured (us, one launch -> two): [512, 9500] K = 7: 96 -> 79; [512, 19200] K = 7: 163 -> 156, K = 11: 233 -> 219;
+// [256, 19201] K = 11: 99 -> 67; [128, 38000] K = 11: 53 -> 41, [128, 40000] 57 -> 46. Unchanged by the rule: [512, 19200] K = 3 (105).
+static int64_t fullRounds(const ConvFusedParams& p, bool f16, const TcForm& form) {
+  const DeviceInfo* d = nullptr;
+  if (deviceInfo(&d) || p.smPercent < 100 || !p.stats || p.fineStats || form.split || !splits(f16, p.k, p.act)) return 0;
+  const int64_t blocks = ceilDiv(p.co, MT), n = p.ci / KC;
+  const int64_t cols = ceilDiv(p.lo, NT) * blocks / d->smCount * d->smCount / blocks * NT;
+  if (cols < 1 || cols >= p.lo || cols > (1 << 24)) return 0;
+  const int split = splitFor(true, int(p.ci), p.lo - cols, blocks, d->smCount, d->clusters);
+  if (!split) return 0;
+  const int64_t saved = 3 * p.k * (n * (blocks % 2 ? NT : NTS) / 2 - ceilDiv(n, split) * NTS / 2);  // pairs: by their tiles
+  return saved > 24000 ? cols : 0;
+}
+
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {
+  TcForm form;
+  if (int rc = formOf(p, f16, &form)) return rc;
+  const int64_t cols = fullRounds(p, f16, form);
+  if (cols == 0) return convTcLaunch(p, wp, f16, s);
+  ConvFusedParams first = p;
+  first.xPitch = p.xPitch ? p.xPitch : p.l, first.resPitch = p.resPitch ? p.resPitch : p.lo;
+  first.outPitch = p.outPitch ? p.outPitch : p.lo, first.statsStride = p.statsStride ? p.statsStride : statChunks(p.lo);
+  ConvFusedParams rest = first;
+  first.lo = cols;
+  rest.lo = p.lo - cols, rest.xOrigin = p.xOrigin + cols, rest.out = p.out + cols;
+  if (p.residual) rest.residual = p.residual + cols;
+  if (p.stats) rest.stats = p.stats + 2 * (cols / NTS);
+  if (int rc = convTcLaunch(first, wp, f16, s)) return rc;
+  return convTcLaunch(rest, wp, f16, s);
+}
+
+static int convTcLaunch(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {
   TcArgs a;
   TcMaps m;
   a.x = p.x, a.wp = wp, a.bias = p.bias, a.affine = p.affine, a.alpha = p.alpha, a.residual = p.residual;
