@@ -41,7 +41,8 @@
 //   warp 18     raw-window loader of the aligned route (one lane): two tiled TMA loads per chunk, one chunk ahead
 //   warp 19     idle (completes the fifth warpgroup)
 // Launches with few tiles take a second form of the same kernel (template parameter SPLIT): a cluster of CTAs per
-// 128- or 64-column tile, each contracting a part of the input channels, reduced over distributed shared memory.
+// 128- or 64-column tile, each contracting a part of the input channels, reduced over distributed shared memory. Whole pairs of
+// output-channel blocks take CTA pairs (conv_pair.cu).
 // All hand-offs are mbarriers. Every wait is bounded: on a timeout the kernel records a status word, drains its
 // copies in flight and returns (TMEM is freed on every path).
 #include <algorithm>

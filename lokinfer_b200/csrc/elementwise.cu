@@ -249,7 +249,7 @@ int channelStats(const float* x, float* stats, int64_t c, int64_t l, int64_t pit
 }
 
 // Early between two convs, beside other launches too: the launch itself (1.5 us of a 3.5 us step between two convs) is over when
-// the first conv ends. Its blocks do not fit beside a conv CTA, which leaves 4096 registers of an SM where a block takes 8192:
+// the first conv ends. Its blocks do not fit beside a conv CTA, which leaves 4096 registers of an SM where a block takes 7168:
 // they wait on SMs that hold no conv, and where there are none start as the first conv's CTAs leave. One that waits keeps a
 // ready conv CTA of another branch off its SM. The conv behind it starts early where it says so itself. us per forward as
 // a graph, early only where nothing runs beside it -> everywhere: T = 16 303 -> 306, T = 24 319 -> 319, T = 80 498 -> 488, T = 121
