@@ -11,8 +11,9 @@
 // of two of a tap's three MMAs in the collector, and stages half as many window columns for an output channel.
 //
 // One thread of the pair's first CTA issues the MMAs of both. Hand-offs that it waits for are barriers of that CTA, at which both
-// CTAs arrive; those that it signals are committed to both. Every wait is bounded, in both CTAs; they set up and leave together (a
-// cluster barrier at either end), so that neither signals into shared memory that is gone.
+// CTAs arrive; those that it signals are committed to both. Every wait is bounded, in both CTAs. They set up and leave together (a
+// cluster barrier at either end), and a CTA arrives at the last one only when every signal that is for it has come: neither signals
+// into shared memory that is gone. Where a wait has run out, and that cannot be waited for, a fence stands in front of the arrival.
 #include <algorithm>
 #include <type_traits>
 
@@ -62,6 +63,7 @@ __device__ __forceinline__ void tmaLoad2dPair(void* dst, const CUtensorMap* map,
 __device__ __forceinline__ void storePeer(uint32_t clusterAddr, int v) {
   asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(clusterAddr), "r"(v) : "memory");
 }
+__device__ __forceinline__ void fenceCluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 // What the A collector does with the operand: nothing, keep it, use what it has for the last time.
 enum class Coll { None, Fill, Last };
 template <Coll C>
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   }
   tcFenceBefore();
   __syncthreads();
-  clusterArrive(), clusterWait();  // the peer's barriers are there
+  clusterArrive(), clusterWait();  // the peer's barriers are there (their fence is above; its flag is older than any wait that gives up)
   tcFenceAfter();
   const uint32_t tmemHi = *tmemSlot, tmemLo = tmemHi + 2 * ACC_COLS;
 
@@ -496,8 +498,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       while (c >= nChunks16) c -= nChunks16, t += pairStep, advance(tt, cb);
     }
-    // The release of the last chunk is a signal to this CTA: it has to be here before the CTA may leave.
-    if (lastBuf >= 0 && !dead && !mbarWait(&bEmpty[lastBuf], lastPar ^ 1, abortFlag, SLEEP_PRO_NS)) dead = 2 << 8 | 3;
+    // The releases of the last NB chunks' buffers are signals to this CTA: they have to be here before it may leave. A group waits for
+    // its last chunk's and for the buffer that it would take next, whose last chunk is NB before that one.
+    if (lastBuf >= 0 && !dead && (!mbarWait(&bEmpty[buf], bufPar, abortFlag, SLEEP_PRO_NS) ||
+                                  !mbarWait(&bEmpty[lastBuf], lastPar ^ 1, abortFlag, SLEEP_PRO_NS)))
+      dead = 2 << 8 | 3;
     if (kProf && pw == 0) profAdd(10, wB), profAdd(11, wCp), profAdd(12, cTr), profAdd(13, clock64() - tStart);
   } else {
     regDec<CTL_REGS>();
@@ -638,6 +643,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       __syncwarp();
       dependentsLaunch();
+      // The epilogues' last releases of the accumulators are signals to this CTA, the second CTA's too: no MMA waits for them.
+      if (leader && !dead && !mbarWait(loEmpty, loPar, abortFlag, SLEEP_EPI_NS)) dead = 4 << 8 | 5;
+      for (int i = 0; i < 2 && leader && !dead; ++i, hiPar ^= hb, hb ^= 1)
+        if (!mbarWait(&hiEmpty[hb], hiPar, abortFlag, SLEEP_EPI_NS)) dead = 4 << 8 | 6;
       if (kProf)
         profAddIf(leader, 0, wBf), profAddIf(leader, 1, wHe), profAddIf(leader, 2, wWf), profAddIf(leader, 3, wLe),
             profAddIf(leader, 4, clock64() - tStart);
@@ -653,6 +662,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     }
     *abortFlag = 1;  // both CTAs of the pair stop
     storePeer(peerAddr(smemAddr(const_cast<int*>(abortFlag)), rank ^ 1), 1);
+    fenceCluster();  // that store and the arrivals that nobody waits for now (releases on every path cost 0.3 to 0.6 us per launch)
   }
   tcFenceBefore();
   clusterArrive(), clusterWait();  // nothing is under way to either CTA's shared memory or TMEM any more

@@ -226,12 +226,12 @@ __device__ __forceinline__ void tmemRelinquish() {
 __device__ __forceinline__ void tmemDealloc(uint32_t addr, uint32_t cols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols) : "memory");
 }
-// Cluster of the split form: this CTA's rank, the two halves of the barrier of all threads of all its CTAs, and the address of
-// another CTA's copy of this CTA's shared memory.
-// The arrivals are relaxed: no data passes by these barriers (the rows that the CTAs send each other are counted by recvBar, whose
-// initialisation has its own fence), they only say that operand buffers are read and that nobody needs this CTA any more. As releases
-// they waited for every store in flight, spills and output rows included: us per forward 313 -> 299 at T = 24, 551 -> 540 at
-// T = 121, the decoder at F = 8 / 61 / 160 / 1040 177 -> 171, 183 -> 177, 260 -> 254, 570 -> 561.
+// Clusters: this CTA's rank, the two halves of the barrier of all threads of all its CTAs, and the address of another CTA's copy of
+// this CTA's shared memory.
+// The arrivals are relaxed: they order nothing in front of them. What the CTAs send each other, rows or signals, is waited for
+// at an mbarrier, whose initialisation has its own fence; the cluster barriers only say that operand buffers are read and that nobody
+// needs this CTA any more. As releases they waited for every store in flight, spills and output rows included: us per forward
+// 313 -> 299 at T = 24, 551 -> 540 at T = 121, the decoder at F = 8 / 61 / 160 / 1040 177 -> 171, 183 -> 177, 260 -> 254, 570 -> 561.
 __device__ __forceinline__ uint32_t clusterRank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));

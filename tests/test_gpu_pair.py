@@ -72,3 +72,21 @@ def test_pair_form_in_a_resblock(cuda, l):
     assert ops.conv_tc_status() == 0
     # the order in which 6 convs' residuals and statistics are added: a few units of the last place each
     assert torch.linalg.vector_norm(out - ref) <= 2e-6 * torch.linalg.vector_norm(ref)
+
+
+@pytest.mark.parametrize("ci,l", [(16, 4737), (48, 9473)])
+def test_pairs_leave_nothing_behind_for_the_next_launch(cuda, ci, l):
+    """A pair's CTAs leave when every signal for their shared memory has come, the second CTA's last ones to the first too. Launches back
+    to back whose last tiles have one column, so that the two CTAs are far apart when they end, in turn with another form that takes
+    over the shared memory; all give the bits of the first."""
+    from lokinfer_b200 import ops
+    x, w, b, affine, _, _, state = _case(cuda, ci, 256, l, 3)
+    few = ops.to_cuda(x[:, :300].cpu().numpy(), cuda)  # split over clusters
+    with ops.padded_rows():
+        px = ops.to_cuda(x.cpu().numpy(), cuda, rows=True)
+        kw = dict(padding=1, state=state)
+        outs = [(ops.conv1d_affine_f32_cuda(px, w, b, affine, **kw), ops.conv1d_affine_f32_cuda(few, w, b, affine, **kw))
+                for _ in range(60)]
+    assert ops.conv_tc_status() == 0
+    for pair, split in outs[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(pair + split, outs[0][0] + outs[0][1]))
