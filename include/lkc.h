@@ -169,6 +169,17 @@ LKC_API int lkc_conv1d_tc_split_cols(int64_t lo);
 /* The rule for the tile width of a conv with f16 halves that is not split and may leave chunk statistics per 32 columns (or none):
  * 160, 192, 224 or 256 columns, for a launch on sm_percent of sms SMs (100: one that runs alone); 0 for bad arguments. */
 LKC_API int lkc_conv1d_tc_tile_cols(int64_t co, int64_t lo, int sms, int sm_percent);
+/* The rule by which a conv with f16 halves goes to CTA pairs if its rows are 16-byte aligned: columns per tile, 160 where it may leave
+ * chunk statistics per 32 columns or none (fine), else 128; 0 = not (a launch that is split, tiles of lkc_conv1d_tc_tile_cols or, where
+ * not fine, 256 columns) or bad arguments. act: 0 none, 1 Snake, 2 leaky; behind_affine: it follows its adain_affine inside a
+ * whole-model call, and starts under it. */
+LKC_API int lkc_conv1d_tc_pair_cols(int64_t ci, int64_t co, int64_t lo, int64_t k, int64_t dilation, int64_t padding, int act, int fine,
+                                    int behind_affine, int sm_percent, int sms, const int32_t* clusters);
+/* The rule by which such a conv, alone and with chunk statistics per 128 columns, goes in two launches: columns of the first, a
+ * multiple of 256; the others are a launch that is split. 0 = one launch, or bad arguments. */
+LKC_API int64_t lkc_conv1d_tc_full_rounds(int64_t ci, int64_t co, int64_t lo, int64_t k, int sms, const int32_t* clusters);
+/* What the rules are asked with on the current device: its SMs, and clusters[0..8] as above. Returns 0 or an error code. */
+LKC_API int lkc_conv1d_tc_device(int* sms, int32_t* clusters);
 LKC_API int lkc_conv1d_tc_status(int* status, int reset);
 /* Stream-ordered form for callers that keep several utterances in flight: queues a 4-byte copy of the status word
  * into status_host (pinned host memory) behind the work already on `stream`; synchronises nothing, clears nothing. */

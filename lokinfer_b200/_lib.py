@@ -115,6 +115,12 @@ def lib():
         l.lkc_conv1d_tc_tile_cols.argtypes = [ctypes.c_int64] * 2 + [ctypes.c_int] * 2
         l.lkc_conv1d_tc_split.restype = ctypes.c_int
         l.lkc_conv1d_tc_split.argtypes = [ctypes.c_int64] * 3 + [ctypes.c_int, ctypes.POINTER(ctypes.c_int32)]
+        l.lkc_conv1d_tc_pair_cols.restype = ctypes.c_int
+        l.lkc_conv1d_tc_pair_cols.argtypes = ([ctypes.c_int64] * 6 + [ctypes.c_int] * 5 + [ctypes.POINTER(ctypes.c_int32)])
+        l.lkc_conv1d_tc_full_rounds.restype = ctypes.c_int64
+        l.lkc_conv1d_tc_full_rounds.argtypes = [ctypes.c_int64] * 4 + [ctypes.c_int, ctypes.POINTER(ctypes.c_int32)]
+        l.lkc_conv1d_tc_device.restype = ctypes.c_int
+        l.lkc_conv1d_tc_device.argtypes = [ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int32)]
         l.lkc_conv1d_tc_split_cols.restype = ctypes.c_int
         l.lkc_conv1d_tc_split_cols.argtypes = [ctypes.c_int64]
         l.lkc_generator_branch_sms.restype = ctypes.c_int

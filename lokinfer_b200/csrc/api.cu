@@ -270,6 +270,36 @@ extern "C" LKC_API int lkc_conv1d_tc_tile_cols(int64_t co, int64_t lo, int sms, 
   return co < 1 || co > (1 << 30) || lo < 1 || lo > (1 << 30) || sms < 1 || sm_percent < 1 ? 0 : convTcTileRule(co, lo, sms, sm_percent);
 }
 
+namespace {
+// What the rules for the form of a conv take: a shape of the tensor-core convs whose lengths and counts multiply in 64 bits.
+bool ruleShape(int64_t ci, int64_t co, int64_t lo, int64_t k, int sms, const int32_t* clusters) {
+  return ci >= 16 && ci % 16 == 0 && ci <= 4096 && co >= 1 && co <= (1 << 30) && lo >= 1 && lo <= (1 << 30) && k >= 1 && k <= 64 &&
+         sms >= 1 && sms <= 65535 && clusters;
+}
+}  // namespace
+
+extern "C" LKC_API int lkc_conv1d_tc_pair_cols(int64_t ci, int64_t co, int64_t lo, int64_t k, int64_t dilation, int64_t padding, int act,
+                                               int fine, int behind_affine, int sm_percent, int sms, const int32_t* clusters) {
+  if (!ruleShape(ci, co, lo, k, sms, clusters) || dilation < 1 || dilation > (1 << 20) || padding < 0 || act < 0 || act > 2 ||
+      sm_percent < 1 || sm_percent > 100)
+    return 0;
+  return convTcPairRule(ci, co, lo, k, dilation, padding, static_cast<Act>(act), fine != 0, behind_affine != 0, sm_percent, sms,
+                        clusters);
+}
+
+extern "C" LKC_API int64_t lkc_conv1d_tc_full_rounds(int64_t ci, int64_t co, int64_t lo, int64_t k, int sms, const int32_t* clusters) {
+  if (!ruleShape(ci, co, lo, k, sms, clusters) || convTcSplitRule(ci, co, lo, sms, clusters)) return 0;
+  return convTcRoundsRule(ci, co, lo, k, sms, clusters);
+}
+
+extern "C" LKC_API int lkc_conv1d_tc_device(int* sms, int32_t* clusters) {
+  LKC_REQUIRE(sms && clusters, "conv1d_tc_device: null out pointer");
+  const int32_t* c = nullptr;
+  if (int rc = convTcDevice(sms, &c)) return rc;
+  std::copy(c, c + 9, clusters);
+  return 0;
+}
+
 extern "C" LKC_API void lkc_conv1d_state_destroy(LkcConvState* st) { delete reinterpret_cast<ConvState*>(st); }
 
 // ints: w(Ci, Co, K) wp(n) padding stride [format]

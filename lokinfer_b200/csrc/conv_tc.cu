@@ -1632,33 +1632,64 @@ static TcForm formFor(const DeviceInfo& d, bool canSplit, bool fineOk, bool conv
   f.tileCols = f.split ? (conv ? convTcSplitCols(lo) : NTS) : tileColsFor(fineOk, lo, coBlocks, d.smCount, smPercent);
   return f;
 }
-// The pair form (conv_pair.cu) with tiles of w columns, of a conv that is not split. It wants whole pairs of output-channel blocks and
-// rows that the TMA unit can address. Alone it is the faster one wherever it applies: half of the window columns to stage, finer
-// tiles and so fuller last rounds. Beside other launches the SM time of all tiles together counts, which is that of 256-column tiles of
-// one CTA; there it is taken for launches of one round. us per launch alone, 256 columns of one CTA -> pairs: [256, 20800] K = 3 / 7 /
-// 11 54 -> 41, 68 -> 56, 95 -> 73; [256, 8000] 29 -> 18, 35 -> 23, 48 -> 30; [512, 19200] K = 3 / 7 / 11 141 -> 107, 184 -> 164,
-// 275 -> 235. us per generator forward as a graph, without pairs / those of one round of the launch's share / of the device:
-// T = 260 827 / 796 / 796, T = 320 866 / 809 / 809, T = 400 913 / 887 / 887, T = 480 1043 / 1021 / 992, T = 640 1328 / 1333 / 1320,
-// T = 800 1497 / 1497 / 1472; with pairs of two rounds T = 2080 3680 / 3740.
+// Columns per (mean, M2) pair that a launch of this form leaves.
+static int statColsOf(int split, int tileCols) { return split || tileCols == NT || tileCols == NTS ? 128 : 32; }
+
 static bool rowsAligned(const float* p, int64_t pitch) { return ((reinterpret_cast<uintptr_t>(p) | uintptr_t(pitch * 4)) & 15) == 0; }
 static int pairRows(int w, int64_t k, int64_t dilation, int64_t padding) {  // staged window columns of a CTA
   return w / 2 + int((k - 1) * dilation) + int(-padding & 3);
 }
-static bool pairs(const ConvFusedParams& p, const DeviceInfo& d, int w) {
-  if (p.co % (2 * MT) || d.clusters[2] < 1 || !gTmaEnabled || !encodeTiled() || !rowsAligned(p.x, p.xPitch ? p.xPitch : p.l) ||
-      !rowsAligned(p.out, p.outPitch ? p.outPitch : p.lo) || (p.residual && !rowsAligned(p.residual, p.resPitch ? p.resPitch : p.lo)))
-    return false;
+// Columns per tile of the pair form (conv_pair.cu), for a conv with f16 halves that is not split and whose rows the TMA unit can
+// address, or 0 where tiles of oneCols columns of one CTA are the faster ones: 160, or 128 where the statistics have to be of 128.
+// Pairs stage half of the window columns and have finer tiles, but theirs come in whole rounds too, and their set-up takes longer.
+// Alone, the clocks of both forms decide: a launch's, a tile's, and per chunk the longest of staging, MMAs and, for pairs, refilling
+// the weight slots (a slot of seven taps takes longer than the MMAs of the other one). The constants are fitted to launches timed in
+// both forms, Ci 16 to 1104, Co 256 to 1024, K 1 to 16, L 1600 to 60000. From 128 channels on (1848 launches): the geometric mean of
+// the times is 0.814 of that without pairs (0.812 if the better form were known; 0.826 with pairs wherever they can run), at worst
+// 1.024 (1.44), up to K = 11 1.008. us, one CTA -> pairs: [256, 20800] K = 3 / 7 / 11 54 -> 40, 68 -> 57, 93 -> 72;
+// [256, 8000] 29 -> 17, 35 -> 23, 48 -> 29; not taken: a resblock of [256, 12000], 126 tiles of 192 columns or 75 of pairs where 74 run
+// at a time, K = 7 / 11 221 -> 267, 285 -> 356; [512, 4800] K = 7 36 -> 37. A launch behind its adain_affine starts under it either way, which
+// makes two rounds of pairs 5000 clocks cheaper (resblock [256, 14000] K = 3 197 -> 186). With few channels memory and set-up are the time,
+// which the clocks do not know ([16, 9600] K = 1 9.3 -> 12.4, [64, 60000] 79 -> 89): pairs have to be 5 % faster by them then, in
+// at most three rounds (1148 launches: 0.957, at worst 1.041, three of [64, 30000]; 1.018 and 1.47 wherever they can run).
+// Beside other launches the SM time of all tiles together counts, which is that of 256-column tiles of one CTA; there pairs are taken for
+// launches of one round. us per generator forward as a graph, without pairs / those of one round of the launch's share / of the device:
+// T = 260 827 / 796 / 796, T = 320 866 / 809 / 809, T = 400 913 / 887 / 887, T = 480 1043 / 1021 / 992, T = 640 1328 / 1333 / 1320,
+// T = 800 1497 / 1497 / 1472; with pairs of two rounds T = 2080 3680 / 3740.
+static int pairColsFor(bool fineOk, int64_t ci, int64_t co, int64_t lo, int64_t k, int64_t dilation, int64_t padding, Act act, int oneCols,
+                       bool behindAffine, int smPercent, int sms, const int32_t* clusters) {
+  if (co % (2 * MT) || clusters[2] < 1) return 0;
+  const int w = fineOk ? 160 : 128, rows = pairRows(w, k, dilation, padding);
   int nb, nRaw, ws, wG;
-  const int rows = pairRows(w, p.k, p.dilation, p.padding - p.xOrigin);
-  if (pairSmem(int(p.ci), rows, (rows + 3) & ~3, int(p.k), &nb, &nRaw, &ws, &wG) == 0) return false;
-  return p.smPercent == 100 || ceilDiv(p.lo, w) * (p.co / (2 * MT)) <= d.clusters[2];
+  if (pairSmem(int(ci), rows, (rows + 3) & ~3, int(k), &nb, &nRaw, &ws, &wG) == 0) return 0;
+  const int64_t rounds = ceilDiv(ceilDiv(lo, w) * (co / (2 * MT)), clusters[2]), n = ci / KC;
+  if (smPercent < 100) return rounds == 1 ? w : 0;
+  const int64_t groups = ceilDiv(k, wG), mma = 3 * k * w / 2 + 172 * groups;
+  const int64_t stage = 840 + (act == Act::Snake ? 14 * rows / 5 : 0), refill = (mma + 1270 * groups + 112 * k) / ws;
+  const int64_t pair = (behindAffine ? 7000 : 12000) + rounds * (5450 + n * std::max(std::max(stage, mma), refill));
+  const int64_t oneStage = 1460 + (act == Act::Snake ? 81 : 20) * (oneCols + (k - 1) * dilation) / 20;
+  const int64_t oneMma = 3 * k * oneCols / 2 + 455 * ceilDiv(k, TAP_GROUP);
+  const int64_t one = 11700 + ceilDiv(ceilDiv(lo, oneCols) * ceilDiv(co, MT), sms) * (1550 + 22 * oneCols + n * std::max(oneStage, oneMma));
+  return (n < 8 ? rounds <= 3 && pair * 21 < one * 20 : pair * 101 < one * 100) ? w : 0;
+}
+int convTcPairRule(int64_t ci, int64_t co, int64_t lo, int64_t k, int64_t dilation, int64_t padding, Act act, bool fineOk,
+                   bool behindAffine, int smPercent, int sms, const int32_t* clusters) {
+  const int64_t blocks = ceilDiv(co, MT);
+  if (splitFor(true, int(ci), lo, blocks, sms * smPercent / 100, clusters)) return 0;
+  return pairColsFor(fineOk, ci, co, lo, k, dilation, padding, act, tileColsFor(fineOk, lo, blocks, sms, smPercent), behindAffine, smPercent,
+                     sms, clusters);
 }
 static int formOf(const ConvFusedParams& p, bool f16, TcForm* f) {
   const DeviceInfo* d = nullptr;
   if (int rc = deviceInfo(&d)) return rc;
   const bool fineOk = f16 && (p.fineStats || !p.stats);
   *f = formFor(*d, splits(f16, p.k, p.act), fineOk, true, p.ci, p.lo, ceilDiv(p.co, MT), p.smPercent);
-  if (!f->split && f16 && pairs(p, *d, fineOk ? 160 : 128)) f->pair = true, f->tileCols = fineOk ? 160 : 128;
+  if (f->split || !f16 || !gTmaEnabled || !encodeTiled() || !rowsAligned(p.x, p.xPitch ? p.xPitch : p.l) ||
+      !rowsAligned(p.out, p.outPitch ? p.outPitch : p.lo) || (p.residual && !rowsAligned(p.residual, p.resPitch ? p.resPitch : p.lo)))
+    return 0;
+  if (const int w = pairColsFor(fineOk, p.ci, p.co, p.lo, p.k, p.dilation, p.padding - p.xOrigin, p.act, f->tileCols, p.behindAffine,
+                                p.smPercent, d->smCount, d->clusters))
+    f->pair = true, f->tileCols = w;
   return 0;
 }
 
@@ -1695,7 +1726,7 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk,
   a.split = form.split, a.tileCols = form.tileCols, a.pair = form.pair;
   LKC_REQUIRE(!a.statsIn || a.split, "conv (tensor-core): only the split form takes chunk statistics");
   const int nt = a.split ? a.tileCols : NT;  // staged columns of the first box
-  if (a.stats && !a.split && a.tileCols != NT && a.tileCols != 128) a.nchunks = ceilDiv(a.lo, 32);
+  if (a.stats && statColsOf(a.split, a.tileCols) == 32) a.nchunks = ceilDiv(a.lo, 32);
   a.numTTiles = int(ceilDiv(a.lo, a.tileCols));
   // TMA routes: tensors whose rows are 16-byte aligned. A map that is not used still has to be a valid kernel
   // argument: it stays zero-filled and is never dereferenced.
@@ -1712,7 +1743,7 @@ static int finishArgs(TcArgs& a, TcMaps& m, bool f16, TcForm form, bool boxesOk,
     if (finishPair(a, m, *d, start, smPercent, grid, smem)) return 0;
     std::memset(&m, 0, sizeof m);
     a.pair = 0, a.numCoBlk = coBlk, a.nb = Fmt<true>::NB;
-    if (a.tileCols == 128) a.tileCols = NT, a.numTTiles = int(ceilDiv(a.lo, NT));
+    if (a.tileCols == NTS) a.tileCols = NT, a.numTTiles = int(ceilDiv(a.lo, NT));
   }
   a.tmaIn = makeMap(&m.x, a.x, a.ci, a.l, a.xPitch, nt, KC, false) ? 1 : 0;
   auto layOut = [&] {
@@ -1757,7 +1788,7 @@ bool convTcSplits(const ConvFusedParams& p, bool f16) {
 
 int convTcStatCols(const ConvFusedParams& p, bool f16) {
   TcForm f;
-  return formOf(p, f16, &f) == 0 && !f.split && f.tileCols != NT && f.tileCols != 128 ? 32 : 128;
+  return formOf(p, f16, &f) == 0 ? statColsOf(f.split, f.tileCols) : 128;
 }
 
 static int convTcLaunch(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s);
@@ -1766,20 +1797,24 @@ static int convTcLaunch(const ConvFusedParams& p, const float* wp, bool f16, cud
 // of one more lasts as if that were full. Where so few columns are over that they can be split over the CTAs of clusters they are a
 // launch of their own, if that saves more MMA clocks (half a column's width each, three to a tap and chunk) than the split form's
 // fixed cost and a second launch's, at most 24,000 (12 us). The rounds are those of 256-column tiles in both forms of whole tiles, so
-// that rows of every alignment give the same bits; two rounds of pairs have as many columns. Statistics per 32 columns leave no
-// choice: a split tile has one pair.
+// that rows of every alignment give the same bits; two rounds of pairs have as many columns where pairs fill the device (where clusters
+// of two leave SMs over, pairColsFor sees the rounds that they take). Statistics per 32 columns leave no choice: a split tile has one
+// pair.
 // Measured (us, one launch -> two): [512, 9500] K = 7: 96 -> 79; [512, 19200] K = 7: 163 -> 156, K = 11: 233 -> 219;
 // [256, 19201] K = 11: 99 -> 67; [128, 38000] K = 11: 53 -> 41, [128, 40000] 57 -> 46. Unchanged by the rule: [512, 19200] K = 3 (105).
+int64_t convTcRoundsRule(int64_t ci, int64_t co, int64_t lo, int64_t k, int sms, const int32_t* clusters) {
+  const int64_t blocks = ceilDiv(co, MT), n = ci / KC;
+  const int64_t cols = ceilDiv(lo, NT) * blocks / sms * sms / blocks * NT;
+  if (cols < 1 || cols >= lo || cols > (1 << 24)) return 0;
+  const int split = splitFor(true, int(ci), lo - cols, blocks, sms, clusters);
+  if (!split) return 0;
+  const int64_t saved = 3 * k * (n * (blocks % 2 ? NT : NTS) / 2 - ceilDiv(n, split) * NTS / 2);  // pairs: by their tiles
+  return saved > 24000 ? cols : 0;
+}
 static int64_t fullRounds(const ConvFusedParams& p, bool f16, const TcForm& form) {
   const DeviceInfo* d = nullptr;
   if (deviceInfo(&d) || p.smPercent < 100 || !p.stats || p.fineStats || form.split || !splits(f16, p.k, p.act)) return 0;
-  const int64_t blocks = ceilDiv(p.co, MT), n = p.ci / KC;
-  const int64_t cols = ceilDiv(p.lo, NT) * blocks / d->smCount * d->smCount / blocks * NT;
-  if (cols < 1 || cols >= p.lo || cols > (1 << 24)) return 0;
-  const int split = splitFor(true, int(p.ci), p.lo - cols, blocks, d->smCount, d->clusters);
-  if (!split) return 0;
-  const int64_t saved = 3 * p.k * (n * (blocks % 2 ? NT : NTS) / 2 - ceilDiv(n, split) * NTS / 2);  // pairs: by their tiles
-  return saved > 24000 ? cols : 0;
+  return convTcRoundsRule(p.ci, p.co, p.lo, p.k, d->smCount, d->clusters);
 }
 
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s) {

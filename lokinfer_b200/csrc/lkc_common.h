@@ -136,6 +136,9 @@ int convTcTileRule(int64_t co, int64_t lo, int sms, int smPercent);
 int convTcDevice(int* sms, const int32_t** clusters);  // what the rules are asked with on the current device
 int convTcSplitRule(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* clusters);
 int convTcSplitCols(int64_t lo);
+int convTcPairRule(int64_t ci, int64_t co, int64_t lo, int64_t k, int64_t dilation, int64_t padding, Act act, bool fineOk,
+                   bool behindAffine, int smPercent, int sms, const int32_t* clusters);
+int64_t convTcRoundsRule(int64_t ci, int64_t co, int64_t lo, int64_t k, int sms, const int32_t* clusters);
 int64_t convTcPackFloats(int64_t co, int64_t ci, int64_t k, bool f16);
 int convTcPack(const float* w, float* wp, int64_t co, int64_t ci, int64_t k, bool f16, cudaStream_t s);
 int convTc(const ConvFusedParams& p, const float* wp, bool f16, cudaStream_t s);
