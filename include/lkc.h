@@ -65,6 +65,8 @@ LKC_API int lkc_kernel_count(void);
 LKC_API const char* lkc_kernel_name(int index); /* sorted */
 LKC_API LkcRunFn lkc_find_kernel(const char* name); /* NULL if unknown */
 LKC_API const char* lkc_last_error(void);
+/* Kernels that the calling thread has queued through this library so far. */
+LKC_API int64_t lkc_launch_count(void);
 /* Library build info: "sm_100a" and the compile-time feature list. */
 LKC_API const char* lkc_build_info(void);
 

@@ -106,6 +106,7 @@ def lib():
         l.lkc_find_kernel.restype = ctypes.c_void_p
         l.lkc_find_kernel.argtypes = [ctypes.c_char_p]
         l.lkc_last_error.restype = ctypes.c_char_p
+        l.lkc_launch_count.restype = ctypes.c_int64
         l.lkc_build_info.restype = ctypes.c_char_p
         l.lkc_conv1d_tc_pack_floats.restype = ctypes.c_int64
         l.lkc_conv1d_tc_pack_floats.argtypes = [ctypes.c_int64] * 3

@@ -11,6 +11,11 @@ namespace {
 thread_local char gError[512] = "";
 }
 
+int64_t& launchCount() {
+  static thread_local int64_t count = 0;
+  return count;
+}
+
 int fail(const char* msg) {
   std::snprintf(gError, sizeof gError, "%s", msg);
   return 1;
@@ -412,5 +417,6 @@ extern "C" LKC_API LkcRunFn lkc_find_kernel(const char* name) {
     if (std::strcmp(kEntries[i].name, name) == 0) return kEntries[i].fn;
   return nullptr;
 }
+extern "C" LKC_API int64_t lkc_launch_count(void) { return launchCount(); }
 extern "C" LKC_API const char* lkc_last_error(void) { return gError; }
 extern "C" LKC_API const char* lkc_build_info(void) { return "lkc sm_100a: tcgen05 split-operand fused conv / convT with TMA tile I/O + cuda-core conv/convT/stats/source/stft/istft"; }

@@ -20,13 +20,16 @@ inline const float* F(const LkcArgs* a, int i) { return static_cast<const float*
 inline float* O(const LkcArgs* a, int i) { return static_cast<float*>(a->ptrs[i]); }
 inline cudaStream_t S(void* stream) { return static_cast<cudaStream_t>(stream); }
 
-// Checks the launch that was just issued (no synchronisation).
+int64_t& launchCount();  // kernels that this thread has queued (api.cu)
+
+// Checks and counts the launch that was just issued (no synchronisation).
 inline int launched(const char* what) {
   cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) {
     cudaGetLastError();
     return failCuda(what, e);
   }
+  ++launchCount();
   return 0;
 }
 

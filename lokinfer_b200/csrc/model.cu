@@ -100,11 +100,15 @@ class Exec {
   // f32[c, l] with rows on 16-byte boundaries
   Buf rows(int s, int64_t c, int64_t l) { return alloc(s, c * ((l + 3) & ~int64_t(3)), (l + 3) & ~int64_t(3)); }
 
-  // One kernel on stream s that reads or writes `bufs`; fn() queues it and returns 0 or an error code.
+  // One op on stream s that reads or writes `bufs`; fn() queues its kernel, or the two that some convs take, and returns 0 or an
+  // error code.
   template <class Fn>
   void launch(int s, std::initializer_list<Buf> bufs, Fn fn) {
     if (running()) {
-      if (rc == 0 && (rc = fn(streams_[s])) == 0) ++launches;
+      if (rc != 0) return;
+      const int64_t before = launchCount();
+      rc = fn(streams_[s]);
+      launches += launchCount() - before;
       return;
     }
     const int l = lane(s);

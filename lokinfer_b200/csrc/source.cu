@@ -203,6 +203,7 @@ float* phaseScratch(int64_t floats) {
 int harmonicSourceLaunch(const float* f0, const float* noise, uint64_t seed, const float* w, const float* b, float* p300,
                          float* out, int64_t n, cudaStream_t s) {
   harmonicPhaseKernel<<<1, 288, 0, s>>>(f0, p300, n);
+  if (int rc = launched("harmonic_source_f32_cuda")) return rc;
   const int64_t samples = n * kUp;
   const int blocks = int(ceilDiv(samples, 256) > 148 * 16 ? 148 * 16 : ceilDiv(samples, 256));
   if (noise) harmonicSourceKernel<false><<<blocks, 256, 0, s>>>(f0, noise, 0, w, b, p300, out, n);

@@ -44,3 +44,23 @@ def test_conv_in_two_launches(cuda, c, l, k, d, plain):
     rms = (o ** 2).sum(2)  # what 128 additions in f32 may lose of it
     assert (stats[..., 0].double() - m).abs().le(2.0 ** -16 * (1 + rms.sqrt())).all()
     assert (stats[..., 1].double() - m2).abs().le(2.0 ** -16 * (1 + rms)).all()
+
+
+def test_both_launches_are_counted(cuda):
+    from lokinfer_b200 import ops
+    from lokinfer_b200.generator import Generator
+    x, w, b, affine, alpha, res = (torch.from_numpy(v).to(cuda) for v in synth.conv_case(256, 256, 19201, 11, 1))
+    state = ops.conv1d_prepare_f32_cuda(w)
+    with ops.Profile(time_kernels=False) as one:
+        ops.conv1d_snake_f32_cuda(x[:, :9472].contiguous(), w, b, affine, alpha, padding=5, state=state)
+    with ops.Profile(time_kernels=False) as two:
+        ops.conv1d_snake_f32_cuda(x, w, b, affine, alpha, residual=res, padding=5, state=state)
+    assert (one.count, two.count) == (1, 2)
+    gen = Generator(synth.generator_weights(3), cuda)
+    gb = gen.style(torch.zeros(128, device=cuda))
+    counts = []
+    for l in (19201, 18944):
+        with ops.Profile(time_kernels=False) as prof:
+            gen.adain_resblock1_fused(x[:, :l].contiguous(), gb, "resblocks.2", 11)
+        counts.append(prof.count)
+    assert counts == [14, 13]  # statistics, six affines and convs; the last one, whose statistics are per 128 columns, in two launches
