@@ -188,7 +188,8 @@ __device__ __forceinline__ void bulkCopyG2S(void* dst, const void* src, uint32_t
                : "memory");
 }
 // Tiled TMA copies of a rank-2 tensor (coordinates: x = innermost = time, y = channel). x * 4 bytes must be a
-// multiple of 16; a load may start outside the tensor (the missing part is filled with zeros), a store is clipped.
+// multiple of 16; a load may start outside the tensor (the missing part is filled with zeros), a store is clipped behind the 16 bytes
+// that the last column is in.
 __device__ __forceinline__ void tmaLoad2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(

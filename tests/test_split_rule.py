@@ -171,4 +171,4 @@ def test_two_launches_of_known_lengths():
     assert [full_rounds(256, 256, lo, 11) for lo in (18944, 18945, 19201, 20800)] == [0, 18944, 18944, 18944]
     assert [full_rounds(128, 128, lo, k) for lo, k in ((37889, 11), (37889, 3), (9473, 11))] == [37888, 0, 0]
     assert full_rounds(512, 512, 19200, 3) == 0 and full_rounds(256, 256, 9473, 11) == 0  # 76 of 148 tiles
-    assert full_rounds(100, 256, 19201, 11) == full_rounds(256, 0, 19201, 11) == full_rounds(256, 256, 0, 11) == full_rounds(256, 256, 19201, 65) == 0
+    assert [full_rounds(*bad) for bad in ((100, 256, 19201, 11), (256, 0, 19201, 11), (256, 256, 0, 11), (256, 256, 19201, 65))] == [0] * 4
