@@ -1,13 +1,15 @@
 // Tensor-core fused conv1d on CTA pairs (tcgen05.mma.cta_group::2): the form of conv_tc.cu's conv for whole pairs of output-channel
-// blocks and 16-byte aligned rows. Same operands (f16 halves), same drains and order of sums, same prologue; see there. What differs:
+// blocks and 16-byte aligned rows. Same operands (f16 halves), same drains, same prologue; see there. What differs:
 //
 //   D[256 co, W t] += Wtap[256 co, 16 ci] * Ashift[16 ci, W t]: each CTA of a pair has 128 of the output channels and stages half
 //   of the tile's columns, of which an MMA reads both halves.
 //
 // W is 160 columns, or 128 where the chunk statistics have to be of 128 columns: Dhi then fits twice beside Dlo into tensor memory,
-// and the hi MMAs of a drain group need not wait for the drain of the one before, nor for the final phase of the tile before.
+// and the hi MMAs of a drain group need not wait for the drain of the one before, nor for the final phase of the tile before. At 128
+// columns the sums are added in the same order too, bit for bit; at 160 a residual is added behind another drain, and statistics are
+// those of narrow tiles.
 // What bounds it: an M128 N256 MMA of the other form reads 96 B/clk of shared memory, an M128 N160 one 115, which leaves the other
-// roles (weights, windows, residual, output: about 50 B/clk at K = 11) too little. A pair reads 83 at W = 160, 68 with the weights
+// roles (weights, windows, residual, output: about 50 B/clk at K = 11) too little. A pair reads 83 at W = 160, 66 with the weights
 // of two of a tap's three MMAs in the collector, and stages half as many window columns for an output channel.
 //
 // One thread of the pair's first CTA issues the MMAs of both. Hand-offs that it waits for are barriers of that CTA, at which both

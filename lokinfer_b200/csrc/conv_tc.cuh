@@ -93,7 +93,7 @@ struct TcArgs {
   int padLeft;       // ConvTranspose: 1 = one-sample left reflect pad
   float slope, outScale;
   int delta;       // columns between the 16-byte boundary a tile's window is loaded from and its first column (0: 4-byte route)
-  int tileCols;    // time columns per tile: NTS or NTS2 split, else 160 .. NT in steps of 32 (see tileColsFor)
+  int tileCols;    // time columns per tile: NTS or NTS2 split, 160 or NTS in pairs, else 160 .. NT in steps of 32 (see tileColsFor)
   int mainRows;    // staged rows that every lane has a slot for: the window up to NT (split: tileCols) rows, a multiple of 64
   int rows;        // staged time rows per buffer: at least tileCols + (k-1)*dilation + delta and mainRows
   int ext;         // raw staging: [16][NT, split: tileCols], then [16][ext] with the rows beyond them (two TMA boxes)

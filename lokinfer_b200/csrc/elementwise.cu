@@ -157,7 +157,8 @@ __global__ void channelStatsKernel(const float* __restrict__ x, float* __restric
 // data could be moved in front of the wait.
 constexpr int kAffineThreads = 128;
 __global__ void __launch_bounds__(kAffineThreads) adainAffineKernel(const float* stats, const float* gb, float* affine, int64_t c,
-                                                                    int64_t l, int64_t nchunks, int statCols, double invL, float eps, int early) {
+                                                                    int64_t l, int64_t nchunks, int statCols, double invL, float eps,
+                                                                    int early) {
   dependenciesWait();
   if (early) dependentsLaunch();  // not before: a conv that waits holds SMs, and what it waits for is then this kernel alone
   __shared__ double red[2 * kAffineThreads / 32];
@@ -264,8 +265,8 @@ int adainAffine(const float* stats, const float* gb, float* affine, int64_t c, i
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 1;
   }
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, adainAffineKernel, stats, gb, affine, c, l, ceilDiv(l, statCols), statCols, 1.0 / double(l), eps,
-                                           early ? 1 : 0);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, adainAffineKernel, stats, gb, affine, c, l, ceilDiv(l, statCols), statCols,
+                                           1.0 / double(l), eps, early ? 1 : 0);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return failCuda("adain_affine_f32_cuda", e);

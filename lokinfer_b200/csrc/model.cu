@@ -32,16 +32,15 @@ constexpr float kEps = 1e-5f;  // AdaIN
 // ways add the same partial sums): [stage] the k = 3, 7, 11 resblocks, and the two noise branches. What runs beside each
 // other may add up to more than 100: launches of branches rarely coincide for long, and clusters that find no room start
 // when others end. The longer a branch's chain, the more it gets; the first noise branch is waited for one stage earlier than
-// the second. us per forward of T = 24 / 80 / 121 / 200 / 320 frames, [stage 0 | stage 1 | noise]: 26, 36, 70 | 26, 36, 50 | 70,
-// 40: 337 / 513 / 598 / 757 / 934; 33 each, noise 50: 352 / 517 / 581 / 751 / 877; k = 11 at 90 in stage 0: 336 / 624 / 717 /
-// 759 / 935; 26, 36, 60 | 26, 36, 50 | 60, 50: 333 / 511 / 597 / 705 / 878 (T = 320 gains where stage 0 of k = 11 takes whole
-// tiles instead of halves, T = 200 from the second noise branch). No splitting at all, with an earlier build: 877 at T = 24, 934
-// at 121.
+// the second. us per forward as a graph, T = 24 / 80 / 121 / 200 / 320 / 640 / 2080 frames: as below 302 / 465 / 506 / 640 / 750 / 1347 /
+// 3936; [stage 0 | stage 1 | noise] 26, 36, 70 | 26, 36, 50 | 70, 40: 302 / 464 / 504 / 703 / 815 / 1342 / 3954; 33 each, noise 50: 304 /
+// 464 / 528 / 657 / 752 / 1340 / 3990; k = 11 at 90 in stage 0: 300 / 475 / 519 / 651 / 772 / 1338 / 3971. No splitting at all, with an
+// earlier build: 877 at T = 24, 934 at 121.
 // A resblock whose tiles its share leaves whole gets the other share, with which more lengths are split: a whole tile's chain
-// of 16 channel chunks is then the branch's time. As a graph, T = 72 / 80 / 90 / 100 / 110 / 121 / 140 / 160 / 320 / 640: 26 and 36
-// for k = 3 and 7 of stage 0 at every length 470 / 489 / 502 / 508 / 516 / 586 / 604 / 691 / 864 / 1346; 40 for both, which up to
-// T = 115 only adds CTAs to tiles that have two or three, 466 / 504 / 514 / 525 / 533 / 554 / 577 / 662 / 866 / 1336; as below 468 /
-// 488 / 503 / 506 / 518 / 552 / 573 / 658 / 867 / 1335.
+// of 16 channel chunks is then the branch's time. T = 72 / 80 / 90 / 100 / 110 / 121 / 140 / 160 / 320 / 640: 26 and 36 for k = 3 and 7 of
+// stage 0 at every length 442 / 467 / 479 / 476 / 489 / 503 / 541 / 615 / 751 / 1340; 40 for both 441 / 471 / 488 / 485 / 501 / 507 / 566 /
+// 619 / 751 / 1342; as below 444 / 465 / 473 / 473 / 488 / 506 / 572 / 620 / 750 / 1347. (It was drawn before the convs started early
+// beside other launches: T = 121 / 140 / 160 586 / 604 / 691 with 26 and 36, 552 / 573 / 658 as below.)
 struct Share {
   int split, whole;
 };
@@ -202,10 +201,12 @@ int adainConv(Exec& e, int s, Buf x, Buf stats, int statCols, int64_t l, int64_t
   p.xPitch = x.pitch, p.resPitch = residual.pitch, p.outPitch = out.pitch;
   p.act = Act::Snake, p.state = w.state[i], p.smPercent = smPercent, p.fineStats = fine, p.urgent = urgent;
   const float* gb = bank.p + w.gb[i];
-  if (e.running() && statCols == 128 && convFoldsAffine(p))
+  if (e.running() && statCols == 128 && convFoldsAffine(p)) {
     p.statsIn = stats.p, p.gb = gb, p.eps = kEps;
-  else
-    e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, c, l, kEps, st, statCols, true); }), p.behindAffine = true;
+  } else {
+    e.launch(s, {stats, bank, af}, [&](cudaStream_t st) { return adainAffine(stats.p, gb, af.p, c, l, kEps, st, statCols, true); });
+    p.behindAffine = true;
+  }
   e.launch(s, {x, stats, bank, af, residual, out, outStats}, [&](cudaStream_t st) { return convFused(p, st); });
   return e.running() ? convStatCols(p) : 128;
 }
@@ -319,8 +320,10 @@ void generator(Exec& e, const LkcGenerator& m, const LkcGeneratorIo& io) {
     conv(e, s, Act::None, y, ly, n.rows, kCh[i], n.taps, 1, 0, n.w, n.b, none, nullptr, 0.f, n.state, none, xs, xst,
          kNoiseSms[i]);
     e.join(s, 3);
-    if (i == 0) resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats, AddUpsampled{e, u0, kCh[0], len[0]}, kNoiseSms[i]);
-    else resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], nullptr, PlainResidual{}, kNoiseSms[i], false);
+    if (i == 0)
+      resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], &noiseStats, AddUpsampled{e, u0, kCh[0], len[0]}, kNoiseSms[i]);
+    else
+      resblock(e, s, m.noise_res[i], xs, xst, len[i], bank, &noise[i], nullptr, PlainResidual{}, kNoiseSms[i], false);
   }
 
   Buf in = noise[0], inStats = noiseStats, mean;
@@ -364,14 +367,14 @@ constexpr float kDecSlope = 0.2f, kSqrtHalf = 0.7071067811865476f;
 // started early, as if it ran alone; where two coincide, clusters wait for room, which for long inputs costs less than fewer CTAs
 // per tile. Short ones have few clusters of many CTAs, of which the device holds few (15 of seven or eight, see countClusters), and
 // gain when main convs and shortcuts leave each other room: the shares are the best pair measured for their number of tiles, on
-// which the form of the launches depends. us per forward as a graph over five to fourteen lengths of each row:
+// which the form of the launches depends. us per forward as a graph over three to six lengths of each row:
 //   main, shortcuts | 65, 35  | 60, 40  | 100, 30 | 75, 25  | 100, 100
-//   F = 8 to 64     | 178-185 | 205-214 | 179-186 | 184-192 | 202-210
-//   F = 65 to 128   | 204-206 | 239-243 | 207-209 | 212-216 | 237-240
-//   F = 129 to 256  | 304-309 | 262-270 | 282-287 | 283-289 | 278-284
-//   F = 257 to 384  | 315-324 | 339-350 | 440-453 | 435-444 | 330-336
-//   F = 385 to 512  | 482-498 | 501-525 | 465-474 | 478-488 | 366-370
-//   F = 513 to 1040 | 526-756 | 527-754 | 507-718 | 549-757 | 442-578
+//   F = 8 to 64     | 171-186 | 197-214 | 173-187 | 179-194 | 194-208
+//   F = 65 to 128   | 194-195 | 226-227 | 196-199 | 203-206 | 223-224
+//   F = 129 to 256  | 293-299 | 254-259 | 276-281 | 275-282 | 265-271
+//   F = 257 to 384  | 297-304 | 320-329 | 436-445 | 419-429 | 322-333
+//   F = 385 to 512  | 469-475 | 492-501 | 456-463 | 466-472 | 349-354
+//   F = 513 to 1040 | 511-569 | 511-571 | 500-706 | 537-576 | 432-568
 struct DecSms {
   int main, shortcut;
 };
