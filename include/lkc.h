@@ -168,13 +168,15 @@ LKC_API void lkc_conv1d_state_destroy(LkcConvState* st);
 LKC_API int lkc_conv1d_tc_split(int64_t ci, int64_t co, int64_t lo, int sms, const int32_t* clusters);
 /* Columns per tile of a conv that is split: 64 for rows of no more, else 128; 0 for a bad argument. */
 LKC_API int lkc_conv1d_tc_split_cols(int64_t lo);
-/* The rule for the tile width of a conv with f16 halves that is not split and may leave chunk statistics per 32 columns (or none):
- * 160, 192, 224 or 256 columns, for a launch on sm_percent of sms SMs (100: one that runs alone); 0 for bad arguments. */
+/* The rule for the tile width of a conv with f16 halves that is not split, does not go to CTA pairs (lkc_conv1d_tc_pair_cols)
+ * and may leave chunk statistics per 32 columns (or none): 160, 192, 224 or 256 columns, for a launch on sm_percent of sms SMs
+ * (100: one that runs alone); 0 for bad arguments. */
 LKC_API int lkc_conv1d_tc_tile_cols(int64_t co, int64_t lo, int sms, int sm_percent);
-/* The rule by which a conv with f16 halves goes to CTA pairs if its rows are 16-byte aligned: columns per tile, 160 where it may leave
- * chunk statistics per 32 columns or none (fine), else 128; 0 = not (a launch that is split, tiles of lkc_conv1d_tc_tile_cols or, where
- * not fine, 256 columns) or bad arguments. act: 0 none, 1 Snake, 2 leaky; behind_affine: it follows its adain_affine inside a
- * whole-model call, and starts under it. */
+/* The rule by which a conv with f16 halves goes to CTA pairs if its rows are 16-byte aligned: columns per tile, 160 where it may
+ * leave chunk statistics per 32 columns or none (fine), else 128. 0 = it does not (it is split, or takes tiles of
+ * lkc_conv1d_tc_tile_cols, 256 columns where not fine), a window that the tensor-core path does not take ((k - 1) * dilation > 50),
+ * or bad arguments. act: 0 none, 1 Snake, 2 leaky; behind_affine: it follows its adain_affine inside a whole-model call and starts
+ * under it. */
 LKC_API int lkc_conv1d_tc_pair_cols(int64_t ci, int64_t co, int64_t lo, int64_t k, int64_t dilation, int64_t padding, int act, int fine,
                                     int behind_affine, int sm_percent, int sms, const int32_t* clusters);
 /* The rule by which such a conv, alone and with chunk statistics per 128 columns, goes in two launches: columns of the first, a

@@ -1675,7 +1675,7 @@ static int pairColsFor(bool fineOk, int64_t ci, int64_t co, int64_t lo, int64_t 
 int convTcPairRule(int64_t ci, int64_t co, int64_t lo, int64_t k, int64_t dilation, int64_t padding, Act act, bool fineOk,
                    bool behindAffine, int smPercent, int sms, const int32_t* clusters) {
   const int64_t blocks = ceilDiv(co, MT);
-  if (splitFor(true, int(ci), lo, blocks, sms * smPercent / 100, clusters)) return 0;
+  if ((k - 1) * dilation > MAX_HALO || splitFor(true, int(ci), lo, blocks, sms * smPercent / 100, clusters)) return 0;
   return pairColsFor(fineOk, ci, co, lo, k, dilation, padding, act, tileColsFor(fineOk, lo, blocks, sms, smPercent), behindAffine, smPercent,
                      sms, clusters);
 }

@@ -141,7 +141,7 @@ def test_pairs_are_left_where_their_rounds_cost_more():
     lib, t = _lib.lib(), (ctypes.c_int32 * 9)(*CLUSTERS)
     good = [256, 256, 9472, 3, 1, 1, 1, 0, 0, 100, SMS]
     assert lib.lkc_conv1d_tc_pair_cols(*good, t) == 128 and lib.lkc_conv1d_tc_pair_cols(*good, None) == 0
-    for i, v in ((0, 100), (1, 0), (2, 0), (3, 0), (4, 0), (5, -1), (6, 3), (9, 0), (9, 101), (10, 0)):
+    for i, v in ((0, 100), (1, 0), (2, 0), (3, 0), (4, 0), (4, 26), (4, 1 << 20), (5, -1), (6, 3), (9, 0), (9, 101), (10, 0)):
         assert lib.lkc_conv1d_tc_pair_cols(*good[:i], v, *good[i + 1:], t) == 0
 
 
